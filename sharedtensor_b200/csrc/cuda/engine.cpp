@@ -523,7 +523,8 @@ void GpuReplica::push_snapshot(int link, float* remote_values) {
 // each, so that kernels of other streams get their turn between two launches.
 int GpuReplica::window_tiles() const {
   if (cfg_.window_tiles > 0) return cfg_.window_tiles < n_tiles_ ? cfg_.window_tiles : n_tiles_;
-  return n_tiles_ > 8192 ? 6144 : n_tiles_;   // 25 M elements, about 0.15 ms of a one-link pass
+  const int windows = (n_tiles_ + 8191) / 8192;   // at most 8192 tiles (34 M elements, about 0.12 ms of a one-link pass) each, all alike
+  return (n_tiles_ + windows - 1) / windows;
 }
 int GpuReplica::n_windows() const {
   const int w = window_tiles();
@@ -532,7 +533,7 @@ int GpuReplica::n_windows() const {
 
 // How a launch covers its window: the grid, and how many consecutive tiles a group owns (0: every n-th tile).
 void GpuReplica::grid_for_launch(int tiles, int* grid, int* chunk, int* tiles_per_group) const {
-  const int groups_per_cta = round_shape_groups(cfg_.shape);
+  const int groups_per_cta = round_groups(cfg_.shape, params_.n_links, params_.n_in);
   if (cfg_.chunk_tiles > 0) {
     // many short-lived CTAs: a group takes a run of `chunk_tiles` consecutive tiles and leaves
     const int t = cfg_.chunk_tiles;
@@ -568,6 +569,7 @@ void GpuReplica::launch(bool do_rx, bool do_tx, int sweeps) {
   params_.round = round_no_++;
   params_.parity = cycle_no_ & 1;
   params_.zero_other = w == 0 ? 1 : 0;
+  params_.follows_window = w != 0 ? 1 : 0;
   params_.do_rx = do_rx ? 1 : 0;
   params_.do_tx = do_tx ? 1 : 0;
   params_.sweeps = sweeps < 1 ? 1 : sweeps;

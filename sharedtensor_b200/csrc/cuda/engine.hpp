@@ -45,7 +45,7 @@ struct GpuConfig {
   bool yield_to_updates = true;  // a running round kernel gives up its SMs when addFromTensor has an update ready
   bool comm_high_priority = false;  // comm stream at the highest stream priority (switches yield_to_updates off)
   int chunk_tiles = 0;       // > 0: short-lived CTAs, a group takes this many consecutive tiles (0: one CTA per SM per launch)
-  int window_tiles = 0;      // tiles a launch covers (0: 6144 for tensors above 8192 tiles, else the whole tensor)
+  int window_tiles = 0;      // tiles a launch covers (0: the tensor in equal parts of at most 8192 tiles)
 };
 
 constexpr size_t kGuardBytes = 256;  // canary before and after every mirror, edge block and the values

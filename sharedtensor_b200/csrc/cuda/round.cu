@@ -1,31 +1,31 @@
 // The sync-round kernel for sm_100a (see round.h for the protocol and ../core/codec.hpp for the arithmetic).
 //
-// A CTA holds up to three independent groups and one publisher warp; a group is four compute warps and one I/O warp
-// and owns every n-th tile of the tensor.  The kinds of warp talk through shared memory and mbarriers only:
+// A CTA holds up to three independent groups; a group is eight compute warps and one service warp and owns every n-th
+// tile of the tensor.  The two kinds of warp talk through a few words of shared memory:
 //
-//   I/O warp      reads its tiles' sequence flags, credits and change marks (32 tiles at a time, one per lane),
-//                 and for every tile with something to do hands the compute warps one *step* per link: it writes
-//                 the step's descriptor (tile, link, which frames arrived, which rings have room), and stages the
-//                 tile's values and the link's mirror into a slot with 1-D TMA bulk copies (cp.async.bulk,
-//                 completion on the slot's `full` mbarrier; every source is this GPU's own memory).  When the
-//                 compute warps have finished a step (`done` mbarrier) it issues the step's bulk stores straight
-//                 from the slot: the decoded frames as a bulk reduce-add into the values (so an update another
-//                 stream adds at the same moment is never overwritten), the stepped mirror, and the packed codes
-//                 and scale bytes into the ring slot of every neighbour on the link (peer stores over NVLink;
-//                 reference src/sharedtensor.c:176-177, two socket writes).  Two steps later, when those stores
-//                 have completed, it hands the step to the publisher warp.
-//   publisher     one warp per CTA: takes the completed steps of all groups, executes the system-scope fence (which
-//                 costs microseconds, and would otherwise stall an I/O warp) and writes sequence flags to the
-//                 receivers and credits to the senders, one ring per lane.
-//   compute warps a thread owns 32 consecutive elements of the tile (read from shared memory through an XOR
-//                 swizzle, so no bank conflicts).  It decodes the frames that arrived (reference 106-111, 124-127)
-//                 into one accumulated step, adds it to its values and to the mirror of the link the frames came
-//                 from, then forms values - mirror, the block's largest magnitude, the exponent code, the codes
-//                 of its 32 elements, and steps the mirror by what the codes say (reference 156-174).
+//   service warp  looks at several of the group's tiles at once, a lane per tile and ring: change mark, sequence flags of the
+//                 in-rings, credits of the out-rings (all loads in flight together).  For every tile with something to
+//                 do it writes a descriptor (tile, which frames arrived, which rings have room, what each link may
+//                 hear) into a bank and arms the bank.  Tiles that all eight compute warps have finished are published
+//                 together behind a system-scope fence: sequence flags to the receivers, credits to the senders.
+//   compute warps walk through the bank, each on its own 512 elements of every tile.  A lane owns four 16-byte pieces
+//                 128 elements apart, so that every access to values, mirrors and frames is a full, coalesced line:
+//                 values and mirror are loaded straight into registers, the frames that arrived are decoded
+//                 (reference 106-111, 124-127), what they say goes into the values as a reduction at the L2 (so an
+//                 update another stream adds at the same moment is never overwritten) and into the mirror of its link,
+//                 then values - mirror is quantised (reference 156-174), the mirror steps by what the codes say, and
+//                 the codes go straight into the ring slots of the link's neighbours (peer stores over NVLink;
+//                 reference src/sharedtensor.c:176-177, two socket writes).
 //
-// Nothing in here waits for another GPU.  The waits are on this CTA's own copies and on its own warps, and every
-// one is bounded: when a wait runs out the group records an error in the status block, stores nothing of the step
-// it was on, marks its tiles for another visit and leaves.
+// What bounds it.  Large tensors: HBM; a visit moves 12 to 18 bytes of values, mirror and frames per element.  Two groups
+// keep 64 KB of loads in flight per SM and the next tile is on its way into the L2 meanwhile.  100 M elements on one link:
+// 0.237 ms to send, 0.328 ms to receive and send, 0.332 ms to receive (0.324, 0.439 and 0.426 ms with tiles staged in
+// shared memory by bulk copies for two groups of four warps, four windows instead of three and no overlap between them).
+// Small tensors: latency.  A launch over one tile takes 10 us in the kernel, of which the look at the tile takes 2, the
+// tile 3 and the fence 2; some hundred tiles take 23 us, of which the fence takes 5 to 8 (see the publication below).
+//
+// Nothing in here waits for another GPU.  The waits are on this group's own warps, and every one is bounded: when a
+// wait runs out the group records an error in the status block, marks its tiles for another visit and leaves.
 //
 // Arithmetic is written with explicit round-to-nearest operations; block statistics are maxima (order does not
 // matter), so codes, scales, mirrors and values are bit-identical to the host codec (../core/codec.cpp).
@@ -46,39 +46,18 @@
 #else
 #define ST_CRUMB(slot, code)
 #endif
-#ifdef ST_ROUND_TIMELINE
-// time stamps (ns, low 32 bits) of the first steps of CTA 0 / group 0 in the debug buffer: [1024 + step * 8 + event]
-#define ST_STAMP(step, ev)                                                                                   \
-  do {                                                                                                       \
-    if (p.dbg != nullptr && blockIdx.x == 0 && g == 0 && lane == 0 && (step) < 24u)                          \
-      *reinterpret_cast<volatile uint32_t*>(p.dbg + 1024 + (step) * 8 + (ev)) = uint32_t(globaltimer_ns()); \
-  } while (0)
-#else
-#define ST_STAMP(step, ev)
-#endif
-#ifdef ST_ROUND_TIMING
-#include <cstdio>
-#define ST_T0() const long long st_t0_ = clock64()
-#define ST_ACC(var) var += clock64() - st_t0_
-#define ST_LAP(var) { const long long st_now_ = clock64(); var += st_now_ - st_lap_; st_lap_ = st_now_; }
-#else
-#define ST_T0()
-#define ST_ACC(var)
-#define ST_LAP(var)
-#endif
 
 namespace st {
 
 namespace {
 
-constexpr int kGroupThreads = 128;  // compute threads of a group: one per 32 consecutive elements of a tile
-constexpr int kTileBytes = kTile * 4;
-constexpr int kPubQueue = 32;
-// Shapes of a CTA (groups x staging slots per group); the launcher picks one, see launch_round.
-//   3 x 2: one CTA per SM, 12 compute warps                (fills the SM's shared memory and registers)
-//   2 x 3: one CTA per SM,  8 compute warps, deeper staging (leaves a third of the registers to other kernels)
-// Either way a group takes every n-th tile of the tensor for the whole launch, or (RoundParams::chunk) a run of
-// consecutive tiles, in which case the grid has many short-lived CTAs and other kernels get SMs in between.
+constexpr int kComputeWarps = 8;                       // of a group
+constexpr int kGroupThreads = (kComputeWarps + 1) * 32;  // and its service warp
+constexpr int kBank = 32;                              // tiles a group has in hand at once
+constexpr int kAhead = 6;                              // tiles in the compute warps' hands below which the service warp looks for more
+constexpr int kPieces = 4;                             // 16-byte pieces of a lane
+constexpr int kWarpElems = kPieces * 128;              // elements of a tile that one warp handles
+static_assert(kComputeWarps * kWarpElems == kTile, "eight warps cover a tile");
 
 // ----------------------------------------------------------------------------------------------
 // small PTX wrappers
@@ -86,6 +65,11 @@ constexpr int kPubQueue = 32;
 __device__ __forceinline__ uint32_t ld_acquire_sys(const uint32_t* p) {
   uint32_t v;
   asm volatile("ld.acquire.sys.global.u32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
+  return v;
+}
+__device__ __forceinline__ uint32_t ld_relaxed_sys(const uint32_t* p) {
+  uint32_t v;
+  asm volatile("ld.relaxed.sys.global.u32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
   return v;
 }
 __device__ __forceinline__ void st_relaxed_sys(uint32_t* p, uint32_t v) {
@@ -98,34 +82,20 @@ __device__ __forceinline__ uint32_t ld_cg_u32(const uint32_t* p) {
   return v;
 }
 __device__ __forceinline__ void st_cg_u32(uint32_t* p, uint32_t v) { asm volatile("st.global.cg.u32 [%0], %1;" ::"l"(p), "r"(v) : "memory"); }
-// frame words and scale bytes were written by a neighbour GPU: read them from the L2, never from this SM's L1
-__device__ __forceinline__ uint4 ld_cg_v4(const void* p) {
-  uint4 v;
-  asm volatile("ld.global.cg.v4.u32 {%0,%1,%2,%3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(p));
-  return v;
-}
-__device__ __forceinline__ uint2 ld_cg_v2(const void* p) {
-  uint2 v;
-  asm volatile("ld.global.cg.v2.u32 {%0,%1}, [%2];" : "=r"(v.x), "=r"(v.y) : "l"(p));
-  return v;
-}
-__device__ __forceinline__ uint32_t ld_cg_word(const void* p) {
-  uint32_t v;
-  asm volatile("ld.global.cg.u32 %0, [%1];" : "=r"(v) : "l"(p));
-  return v;
-}
-__device__ __forceinline__ uint32_t ld_cg_u8(const void* p) {
-  uint32_t v;
-  asm volatile("ld.global.cg.u8 %0, [%1];" : "=r"(v) : "l"(p));
-  return v;
-}
 __device__ __forceinline__ uint32_t smem_u32(const void* p) { return static_cast<uint32_t>(__cvta_generic_to_shared(p)); }
-
+__device__ __forceinline__ uint32_t ld_shared_acquire(const uint32_t* p) {
+  uint32_t v;
+  asm volatile("ld.acquire.cta.shared.u32 %0, [%1];" : "=r"(v) : "r"(smem_u32(p)) : "memory");
+  return v;
+}
+__device__ __forceinline__ void st_shared_release(uint32_t* p, uint32_t v) {
+  asm volatile("st.release.cta.shared.u32 [%0], %1;" ::"r"(smem_u32(p)), "r"(v) : "memory");
+}
+__device__ __forceinline__ void red_shared_release_add(uint32_t* p, uint32_t v) {
+  asm volatile("red.release.cta.shared.add.u32 [%0], %1;" ::"r"(smem_u32(p)), "r"(v) : "memory");
+}
 __device__ __forceinline__ void mbar_init(uint64_t* bar, uint32_t count) {
   asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_u32(bar)), "r"(count) : "memory");
-}
-__device__ __forceinline__ void mbar_expect_tx(uint64_t* bar, uint32_t bytes) {
-  asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(smem_u32(bar)), "r"(bytes) : "memory");
 }
 __device__ __forceinline__ void mbar_arrive(uint64_t* bar) {
   asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(bar)) : "memory");
@@ -141,39 +111,15 @@ __device__ __forceinline__ bool mbar_try_wait(uint64_t* bar, uint32_t parity) {
       : "memory");
   return ok != 0;
 }
-// global -> this CTA's shared memory, completion counted in bytes on `bar`.  Source is always local
-// device memory; size and both addresses are multiples of 16.
-__device__ __forceinline__ void bulk_g2s(void* dst_smem, const void* src_gmem, uint32_t bytes, uint64_t* bar) {
-  asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(
-                   smem_u32(dst_smem)),
-               "l"(src_gmem), "r"(bytes), "r"(smem_u32(bar))
-               : "memory");
-}
-// shared -> global bulk store / reduce (this CTA's memory as source), tracked by bulk async-groups
-__device__ __forceinline__ void bulk_s2g(void* dst_gmem, const void* src_smem, uint32_t bytes) {
-  asm volatile("cp.async.bulk.global.shared::cta.bulk_group [%0], [%1], %2;" ::"l"(dst_gmem), "r"(smem_u32(src_smem)), "r"(bytes)
-               : "memory");
-}
-__device__ __forceinline__ void bulk_reduce_add_f32(float* dst_gmem, const void* src_smem, uint32_t bytes) {
-  asm volatile("cp.reduce.async.bulk.global.shared::cta.bulk_group.add.f32 [%0], [%1], %2;" ::"l"(dst_gmem), "r"(smem_u32(src_smem)),
-               "r"(bytes)
-               : "memory");
-}
+// global -> L2, this GPU's own memory; size and address are multiples of 16
 __device__ __forceinline__ void bulk_prefetch_l2(const void* src_gmem, uint32_t bytes) {
   asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(src_gmem), "r"(bytes) : "memory");
 }
-__device__ __forceinline__ void bulk_commit() { asm volatile("cp.async.bulk.commit_group;" ::: "memory"); }
-__device__ __forceinline__ void bulk_wait_read_all() { asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory"); }
-__device__ __forceinline__ void bulk_wait_all_but_2() { asm volatile("cp.async.bulk.wait_group 2;" ::: "memory"); }
-__device__ __forceinline__ void bulk_wait_all() { asm volatile("cp.async.bulk.wait_group 0;" ::: "memory"); }
-__device__ __forceinline__ void fence_async_smem() { asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); }
 __device__ __forceinline__ uint64_t globaltimer_ns() {
   uint64_t t;
   asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
   return t;
 }
-__device__ __forceinline__ uint32_t ld_shared_volatile(const uint32_t* p) { return *reinterpret_cast<const volatile uint32_t*>(p); }
-__device__ __forceinline__ void st_shared_volatile(uint32_t* p, uint32_t v) { *reinterpret_cast<volatile uint32_t*>(p) = v; }
 
 // Bounded wait on one of this CTA's own barriers; false when `limit_ns` has passed.
 __device__ __forceinline__ bool mbar_wait_bounded(uint64_t* bar, uint32_t parity, uint64_t limit_ns) {
@@ -186,78 +132,106 @@ __device__ __forceinline__ bool mbar_wait_bounded(uint64_t* bar, uint32_t parity
   return false;
 }
 
-// A compute warp's wait for the descriptor of a step.  While the I/O warp looks for work, or there is none, a compute
-// warp may sit here for the whole launch, so the limit is generous; it only covers an I/O warp that never comes back.
-__device__ __forceinline__ bool wait_armed(const uint32_t* armed, uint32_t step, const uint32_t* abort) {
-  if (ld_shared_volatile(armed) > step) return true;
-  const uint64_t t_start = globaltimer_ns();
-  for (uint32_t it = 0; it < (1u << 28); it++) {
-    if (ld_shared_volatile(armed) > step) return true;
-    if (ld_shared_volatile(abort)) return false;
-    if ((it & 63) == 63 && globaltimer_ns() - t_start > 2000ull * 1000 * 1000) return false;
-    __nanosleep(20);
-  }
-  return false;
-}
-
 // ----------------------------------------------------------------------------------------------
-// what the I/O warp tells the compute warps about a step (one per slot, in shared memory)
+// what the service warp tells the compute warps about a tile
 // ----------------------------------------------------------------------------------------------
-struct __align__(16) StepDesc {
+struct __align__(16) TileDesc {
   int32_t tile;
-  int32_t link;
   uint32_t flags;
-  uint32_t sent;                 // publication queue only: the step's frame went out
-  uint32_t in_lo, in_hi;         // per in-ring r one byte: frames available << 6 | first slot
-  uint32_t out_lo, out_hi;       // per out-ring r one byte: has room << 6 | next slot
+  int32_t n_frames;  // entries of the tile's frame list
+  int32_t n_slots;   // entries of the tile's slot list
 };
-constexpr uint32_t kDescFirst = 1;   // the tile's first step: the slot also holds the values
-constexpr uint32_t kDescExit = 2;    // nothing more to do in this launch
-constexpr uint32_t kDescRxAny = 4;   // at least one frame arrived for the tile
-constexpr uint32_t kDescTxOk = 8;    // every out-ring of the link has room
-constexpr uint32_t kDescRxLink = 16; // at least one frame arrived on this step's link
-constexpr uint32_t kDescLast = 32;   // the tile's last step
-constexpr uint32_t kDescNoValues = 128; // the step only receives: the values are not loaded, what arrived goes into them as a reduce-add
-constexpr uint32_t kDescTxWant = 64; // the link may have something to hear: the tile changed here, or frames arrived on another link
-constexpr uint32_t kFlagChanged = 1, kFlagNonsilent = 2, kFlagFailed = 4;  // what the compute warps report about a step
+constexpr uint32_t kDescNoValues = 2;       // the visit only receives: the values are not loaded, what arrived goes into them as a reduction
+constexpr uint32_t kDescTxOk = 1u << 4;     // << link: every out-ring of the link has room
+constexpr uint32_t kDescRxLink = 1u << 8;   // << link: at least one frame arrived on the link
+constexpr int kDescFrameShift = 16;         // + 5 * link: 1 + the place in the frame list of the only frame that arrived on the link (0: none or several)
+constexpr uint32_t kDescTxWant = 1u << 12;  // << link: the link may have something to hear: the tile changed here, or frames arrived on another link
+// what a compute warp adds to a tile's `done` word when it has finished its part
+constexpr uint32_t kDoneWarp = 1, kDoneWarps = 0xff;
+constexpr int kDoneNonsilentShift = 8;      // + 4 * link: warps that found something to say on the link
+constexpr uint32_t kDoneFailed = 1u << 24;  // a wait ran out: nothing of the warp's part was stored
 
-__device__ __forceinline__ uint32_t ctrl_byte(uint32_t lo, uint32_t hi, int r) { return ((r < 4 ? lo : hi) >> ((r & 3) * 8)) & 0xffu; }
+constexpr uint32_t kClaimStop = 0x80000000u;
 
-struct SmemLayout {
-  int slot_stride;  // values tile, mirror tile, payload
-  int off_slots;    // [kGroups][kSlots][slot_stride]
-  int off_desc;     // StepDesc[kGroups][kSlots]
-  int off_pubq;     // StepDesc[kGroups][kPubQueue]
-  int off_bar;      // uint64_t[kGroups][2 * kSlots + 1]: full, done, group sync
-  int off_words;    // uint32_t[kGroups][16]: step flags per slot, armed steps, abort, publication counters
-  int off_red;      // float[kGroups][2][8]: cross-warp partials for blocks of 2048 / 4096 elements
-  int total;
+struct GroupShared {
+  TileDesc desc[kBank];
+  uint64_t frames[kBank][kMaxRings * kRxMax + 1];  // per tile: the frames that arrived (address | link), in ring and sequence order
+  uint64_t slots[kBank][kMaxRings + 1];            // per tile: the ring slots a frame goes into (address | link)
+  uint32_t done[kBank];
+  uint32_t armed;        // tiles armed so far in this launch (bank entry = number % kBank)
+  uint32_t claim;        // tiles the compute warps have started so far | kClaimStop: no new ones
+  uint32_t pad[2];
+  uint64_t gsync;        // the compute warps among themselves (blocks of more than 512 elements)
+  float red[2][2][kComputeWarps];  // two buffers: a warp may be one step ahead of the slowest one
+  alignas(16) uint32_t stage[kComputeWarps][kWarpElems / 4];  // the codes of a warp's part on their way into the ring slots
+  // the service warp's own notes about the tiles in hand: the counters after the visit, what moved per ring (frames
+  // taken | 4: a frame may go out), the change mark found
+  uint32_t rx[kBank][kMaxRings], tx[kBank][kMaxRings];
+  uint8_t moved[kBank][kMaxRings];
+  uint32_t dirty[kBank];
 };
-__host__ __device__ inline SmemLayout smem_layout(int payload_bytes, int kGroups, int kSlots) {
-  SmemLayout m;
-  m.slot_stride = 2 * kTileBytes + ((payload_bytes + 127) & ~127);
-  int off = 0;
-  m.off_slots = off;
-  off += kGroups * kSlots * m.slot_stride;
-  m.off_desc = off;
-  off += kGroups * kSlots * int(sizeof(StepDesc));
-  m.off_pubq = off;
-  off += kGroups * kPubQueue * int(sizeof(StepDesc));
-  m.off_bar = off;
-  off += kGroups * (2 * kSlots + 1) * 8;
-  m.off_words = off;
-  off += kGroups * 16 * 4;
-  m.off_red = off;
-  off += kGroups * 2 * 8 * 4;
-  m.total = (off + 127) & ~127;
-  return m;
+
+// ----------------------------------------------------------------------------------------------
+// per-lane arithmetic.  Piece i of lane `lane` of compute warp `w` is elements w*512 + i*128 + lane*4 .. +3 of the tile.
+// A frame stores the codes of 32 consecutive elements t in an order of its own: their eight pieces c = 0..7 sit at
+// positions c ^ (t & 7) (4 * Q bits each).  Four elements are held as two packed pairs: the packed fp32 instructions of
+// sm_100 round like the scalar ones and halve the instruction count of decoding and quantising.
+// ----------------------------------------------------------------------------------------------
+struct Piece {
+  uint64_t a, b;  // elements 0, 1 and 2, 3
+};
+__device__ __forceinline__ uint64_t pair(float lo, float hi) {
+  uint64_t d;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(d) : "f"(lo), "f"(hi));
+  return d;
+}
+__device__ __forceinline__ uint64_t pair(uint32_t lo, uint32_t hi) {
+  uint64_t d;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(d) : "r"(lo), "r"(hi));
+  return d;
+}
+__device__ __forceinline__ void unpair(uint64_t p, float& lo, float& hi) { asm("mov.b64 {%0, %1}, %2;" : "=f"(lo), "=f"(hi) : "l"(p)); }
+__device__ __forceinline__ uint64_t add2(uint64_t x, uint64_t y) {
+  uint64_t d;
+  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(x), "l"(y));
+  return d;
+}
+__device__ __forceinline__ uint64_t sub2(uint64_t x, uint64_t y) {
+  uint64_t d;
+  asm("sub.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(x), "l"(y));
+  return d;
+}
+__device__ __forceinline__ uint64_t fma2(uint64_t x, uint64_t y, uint64_t z) {
+  uint64_t d;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(x), "l"(y), "l"(z));
+  return d;
+}
+__device__ __forceinline__ void add4(Piece& x, const Piece& y) {
+  x.a = add2(x.a, y.a);
+  x.b = add2(x.b, y.b);
+}
+// values, mirrors and frames have writers on other SMs and other GPUs: always at the L2
+__device__ __forceinline__ Piece load_piece(const float* p) {
+  Piece v;
+  asm volatile("ld.global.cg.v2.b64 {%0, %1}, [%2];" : "=l"(v.a), "=l"(v.b) : "l"(p));
+  return v;
+}
+__device__ __forceinline__ void store_piece(float* p, const Piece& v) {
+  asm volatile("st.global.v2.b64 [%0], {%1, %2};" ::"l"(p), "l"(v.a), "l"(v.b) : "memory");
+}
+__device__ __forceinline__ void red_add_piece(float* p, const Piece& v) {
+  float x, y, z, w;
+  unpair(v.a, x, y);
+  unpair(v.b, z, w);
+  asm volatile("red.global.add.v4.f32 [%0], {%1, %2, %3, %4};" ::"l"(p), "f"(x), "f"(y), "f"(z), "f"(w) : "memory");
+}
+__device__ __forceinline__ float maxabs(const Piece& v) {
+  float x, y, z, w;
+  unpair(v.a, x, y);
+  unpair(v.b, z, w);
+  return fmaxf(fmaxf(fabsf(x), fabsf(y)), fmaxf(fabsf(z), fabsf(w)));
 }
 
-// ----------------------------------------------------------------------------------------------
-// per-thread arithmetic on 32 consecutive elements held as eight float4 pieces.  Register q holds the elements
-// 4*(q^sw) .. +3 of the thread's 32 (sw = thread & 7, the shared-memory swizzle); a frame stores a thread's codes in
-// the order of its registers, so the sender's and the receiver's thread of the same index agree without shuffling.
-// ----------------------------------------------------------------------------------------------
 __device__ __forceinline__ int floor_log2_dev(float x) { return int((__float_as_uint(x) >> 23) & 0xff) - 127; }
 
 // sign frames: step = 2^floor(log2(2/3 max|x|)), silent below the cut-off (block_code in ../core/codec.cpp)
@@ -299,913 +273,714 @@ __device__ __forceinline__ int block_code_dev(float xmax, uint32_t vmax_bits, in
   else return block_code_int_dev<Q>(xmax, vmax_bits, min_exp, rel_bits);
 }
 
-// the Q code words of thread t and the scale byte of its block, from a frame in a ring slot
+// Where piece i of a lane sits in its warp's part of a frame: the 32-element chunk (0..15) and the position in it.
+__device__ __forceinline__ int piece_chunk(int i, int lane) { return i * 4 + (lane >> 3); }
+__device__ __forceinline__ int piece_pos(int i, int lane) { return (lane & 7) ^ (((i & 1) << 2) + (lane >> 3)); }
+
+// A lane's share of a frame: the codes of its four pieces (the low 4 * Q bits of each word) and their blocks' scale bytes.
+// Frame words were written by a neighbour GPU: they are read from the L2, never from this SM's L1.
+struct FrameRegs {
+  uint32_t w[kPieces];
+  uint32_t codes;
+  __device__ __forceinline__ uint32_t code(int i) const { return (codes >> (8 * i)) & 0xffu; }
+};
 template <int Q>
-__device__ __forceinline__ void load_frame(const uint8_t* fp, int t, int tpb, uint32_t (&w)[Q], uint32_t& code) {
-  const uint8_t* mine = fp + size_t(t) * (4 * Q);
-  if (Q == 8) {
-    const uint4 a = ld_cg_v4(mine), b = ld_cg_v4(mine + 16);
-    w[0] = a.x; w[1] = a.y; w[2] = a.z; w[3] = a.w;
-    w[4 % Q] = b.x; w[5 % Q] = b.y; w[6 % Q] = b.z; w[7 % Q] = b.w;
-  } else if (Q == 4) {
-    const uint4 a = ld_cg_v4(mine);
-    w[0] = a.x; w[1 % Q] = a.y; w[2 % Q] = a.z; w[3 % Q] = a.w;
-  } else if (Q == 2) {
-    const uint2 a = ld_cg_v2(mine);
-    w[0] = a.x; w[1 % Q] = a.y;
-  } else {
-    w[0] = ld_cg_word(mine);
+__device__ __forceinline__ void load_frame(const uint8_t* fp, int warp, int lane, int log2_block, FrameRegs& f) {
+  const uint8_t* mine = fp + warp * (kWarpElems * Q / 8);
+#pragma unroll
+  for (int i = 0; i < kPieces; i++) {
+    const int unit = piece_chunk(i, lane) * 8 + piece_pos(i, lane);  // in pieces of 4 * Q bits
+    if (Q == 8) asm volatile("ld.global.cg.u32 %0, [%1];" : "=r"(f.w[i]) : "l"(mine + unit * 4));
+    else if (Q == 4) asm volatile("{\n\t.reg .u16 h;\n\tld.global.cg.u16 h, [%1];\n\tcvt.u32.u16 %0, h;\n\t}" : "=r"(f.w[i]) : "l"(mine + unit * 2));
+    else if (Q == 2) asm volatile("ld.global.cg.u8 %0, [%1];" : "=r"(f.w[i]) : "l"(mine + unit));
+    else {
+      asm volatile("ld.global.cg.u32 %0, [%1];" : "=r"(f.w[i]) : "l"(mine + piece_chunk(i, lane) * 4));
+      f.w[i] >>= 4 * piece_pos(i, lane);
+    }
   }
-  code = ld_cg_u8(fp + 4 * Q * kWordsPerTile + (t >> tpb));
-}
-
-// acc += the step the frame gives each of the 32 elements
-template <int Q, bool MASKED>
-__device__ __forceinline__ void add_frame(float4 (&acc)[8], const uint32_t (&w)[Q], uint32_t code, int sw, uint32_t vmask) {
-  if (code == 0u || code == 255u) return;
-  const float s = __uint_as_float(code << 23);
-  if (Q == 1) {
-    const uint32_t sb = code << 23;
-#pragma unroll
-    for (int q = 0; q < 8; q++) {
-      const uint32_t wq = w[0] >> (4 * q);
-      const float f0 = __uint_as_float(sb | ((wq << 31) & 0x80000000u)), f1 = __uint_as_float(sb | ((wq << 30) & 0x80000000u));
-      const float f2 = __uint_as_float(sb | ((wq << 29) & 0x80000000u)), f3 = __uint_as_float(sb | ((wq << 28) & 0x80000000u));
-      if (!MASKED) {
-        acc[q].x = __fadd_rn(acc[q].x, f0); acc[q].y = __fadd_rn(acc[q].y, f1);
-        acc[q].z = __fadd_rn(acc[q].z, f2); acc[q].w = __fadd_rn(acc[q].w, f3);
-      } else {
-        const uint32_t vq = vmask >> (4 * (q ^ sw));
-        if (vq & 1u) acc[q].x = __fadd_rn(acc[q].x, f0);
-        if (vq & 2u) acc[q].y = __fadd_rn(acc[q].y, f1);
-        if (vq & 4u) acc[q].z = __fadd_rn(acc[q].z, f2);
-        if (vq & 8u) acc[q].w = __fadd_rn(acc[q].w, f3);
-      }
-    }
+  const uint8_t* scales = fp + 4 * Q * kWordsPerTile;
+  if (log2_block == 5) {  // the warp's sixteen scale bytes at once
+    uint4 c;
+    asm volatile("ld.global.cg.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(c.x), "=r"(c.y), "=r"(c.z), "=r"(c.w) : "l"(scales + warp * 16));
+    const uint32_t sel = uint32_t(lane >> 3) * 0x11u + 0x40u;
+    f.codes = __byte_perm(__byte_perm(c.x, c.y, sel), __byte_perm(c.z, c.w, sel), 0x5410);
   } else {
-    // a code c stands for (c - 2^(Q-1)) steps; 2^23 + c as a float is 0x4B000000 | c
-    const float big = 8388608.f + float(1 << (Q - 1));
-    const float neg_ms = -__fmul_rn(big, s);
+    uint32_t b[kPieces];
 #pragma unroll
-    for (int q = 0; q < 8; q++) {
-      uint32_t z0, z1, z2, z3;
-      if (Q == 8) {
-        const uint32_t wq = w[q % Q];
-        z0 = __byte_perm(wq, 0x4B000000u, 0x7650); z1 = __byte_perm(wq, 0x4B000000u, 0x7651);
-        z2 = __byte_perm(wq, 0x4B000000u, 0x7652); z3 = __byte_perm(wq, 0x4B000000u, 0x7653);
-      } else {
-        constexpr uint32_t m = (1u << Q) - 1u;
-        const uint32_t wq = w[(q * Q / 8) % Q] >> ((q * 4 * Q) & 31);  // 4*Q bits per register
-        z0 = (wq & m) | 0x4B000000u; z1 = ((wq >> Q) & m) | 0x4B000000u;
-        z2 = ((wq >> (2 * Q)) & m) | 0x4B000000u; z3 = ((wq >> (3 * Q)) & m) | 0x4B000000u;
-      }
-      acc[q].x = __fadd_rn(acc[q].x, __fmaf_rn(__uint_as_float(z0), s, neg_ms));
-      acc[q].y = __fadd_rn(acc[q].y, __fmaf_rn(__uint_as_float(z1), s, neg_ms));
-      acc[q].z = __fadd_rn(acc[q].z, __fmaf_rn(__uint_as_float(z2), s, neg_ms));
-      acc[q].w = __fadd_rn(acc[q].w, __fmaf_rn(__uint_as_float(z3), s, neg_ms));
-    }
+    for (int i = 0; i < kPieces; i++)
+      asm volatile("ld.global.cg.u8 %0, [%1];" : "=r"(b[i]) : "l"(scales + ((warp * kWarpElems + piece_chunk(i, lane) * 32) >> log2_block)));
+    f.codes = b[0] | (b[1] << 8) | (b[2] << 16) | (b[3] << 24);
   }
 }
 
-// the codes of v - k for a block with exponent code `code` (non-zero), and the mirror's step
-template <int Q, bool MASKED>
-__device__ __forceinline__ void quantise(const float4 (&v)[8], float4 (&k)[8], uint32_t code, uint32_t (&w)[Q], int sw, uint32_t vmask) {
-  if (Q == 1) {
-    const float sp = __uint_as_float(code << 23), sn = __uint_as_float((code << 23) | 0x80000000u);
-    uint32_t word = 0;
-#pragma unroll
-    for (int q = 0; q < 8; q++) {
-      const bool n0 = !(__fsub_rn(v[q].x, k[q].x) > 0.f), n1 = !(__fsub_rn(v[q].y, k[q].y) > 0.f);
-      const bool n2 = !(__fsub_rn(v[q].z, k[q].z) > 0.f), n3 = !(__fsub_rn(v[q].w, k[q].w) > 0.f);
-      uint32_t nib = (n0 ? 1u : 0u) | (n1 ? 2u : 0u) | (n2 ? 4u : 0u) | (n3 ? 8u : 0u);
-      if (!MASKED) {
-        k[q].x = __fadd_rn(k[q].x, n0 ? sn : sp); k[q].y = __fadd_rn(k[q].y, n1 ? sn : sp);
-        k[q].z = __fadd_rn(k[q].z, n2 ? sn : sp); k[q].w = __fadd_rn(k[q].w, n3 ? sn : sp);
-      } else {
-        const uint32_t vq = (vmask >> (4 * (q ^ sw))) & 0xfu;
-        nib &= vq;
-        if (vq & 1u) k[q].x = __fadd_rn(k[q].x, n0 ? sn : sp);
-        if (vq & 2u) k[q].y = __fadd_rn(k[q].y, n1 ? sn : sp);
-        if (vq & 4u) k[q].z = __fadd_rn(k[q].z, n2 ? sn : sp);
-        if (vq & 8u) k[q].w = __fadd_rn(k[q].w, n3 ? sn : sp);
-      }
-      word |= nib << (4 * q);
-    }
-    w[0] = word;
+// Which of the four elements of piece i exist (bits 0..3).  Only sign frames of the tensor's last tile need it: they have
+// no code for "no step" (integer frames carry the code of zero beyond the tensor's end).
+__device__ __forceinline__ uint32_t valid4(int left, int i) {
+  const int m = left - i * 128;
+  return m >= 4 ? 0xfu : (m <= 0 ? 0u : ((1u << m) - 1u));
+}
+
+// Four sign bits as steps of +-2^(c-127)
+__device__ __forceinline__ Piece sign_steps(uint32_t w, uint32_t c, uint32_t valid) {
+  const uint32_t sb = c << 23;
+  uint32_t f0 = sb | ((w << 31) & 0x80000000u), f1 = sb | ((w << 30) & 0x80000000u);
+  uint32_t f2 = sb | ((w << 29) & 0x80000000u), f3 = sb | ((w << 28) & 0x80000000u);
+  if (valid != 0xfu) {
+    f0 = valid & 1u ? f0 : 0u; f1 = valid & 2u ? f1 : 0u; f2 = valid & 4u ? f2 : 0u; f3 = valid & 8u ? f3 : 0u;
+  }
+  return {pair(f0, f1), pair(f2, f3)};
+}
+
+// The steps a frame gives the four elements of a piece.  Silent blocks (code 0) and the code no encoder emits (255) step
+// by zero.
+template <int Q>
+__device__ __forceinline__ Piece frame_steps(uint32_t w, uint32_t code, uint32_t valid) {
+  const uint32_t c = code == 255u ? 0u : code;
+  if constexpr (Q == 1) {
+    return sign_steps(w, c, valid);
   } else {
-    const float s = __uint_as_float(code << 23), inv = __uint_as_float((254u - code) << 23);
-    const float big = 8388608.f + float(1 << (Q - 1));
-    const float neg_ms = -__fmul_rn(big, s);
-#pragma unroll
-    for (int j = 0; j < Q; j++) w[j] = 0;
-#pragma unroll
-    for (int q = 0; q < 8; q++) {
-      const float z0 = __fmaf_rn(__fsub_rn(v[q].x, k[q].x), inv, big), z1 = __fmaf_rn(__fsub_rn(v[q].y, k[q].y), inv, big);
-      const float z2 = __fmaf_rn(__fsub_rn(v[q].z, k[q].z), inv, big), z3 = __fmaf_rn(__fsub_rn(v[q].w, k[q].w), inv, big);
-      k[q].x = __fadd_rn(k[q].x, __fmaf_rn(z0, s, neg_ms)); k[q].y = __fadd_rn(k[q].y, __fmaf_rn(z1, s, neg_ms));
-      k[q].z = __fadd_rn(k[q].z, __fmaf_rn(z2, s, neg_ms)); k[q].w = __fadd_rn(k[q].w, __fmaf_rn(z3, s, neg_ms));
-      const uint32_t b0 = __float_as_uint(z0), b1 = __float_as_uint(z1), b2 = __float_as_uint(z2), b3 = __float_as_uint(z3);
-      if (Q == 8) {
-        w[q % Q] = __byte_perm(__byte_perm(b0, b1, 0x0040), __byte_perm(b2, b3, 0x0040), 0x5410);
-      } else {
-        constexpr uint32_t m = (1u << Q) - 1u;
-        const uint32_t four = (b0 & m) | ((b1 & m) << Q) | ((b2 & m) << (2 * Q)) | ((b3 & m) << (3 * Q));
-        w[(q * Q / 8) % Q] |= four << ((q * 4 * Q) & 31);
-      }
+    // a code m stands for (m - 2^(Q-1)) steps; 2^23 + m as a float is 0x4B000000 | m
+    const float s = __uint_as_float(c << 23), neg_ms = __fmul_rn(-(8388608.f + float(1 << (Q - 1))), s);
+    uint32_t z0, z1, z2, z3;
+    if (Q == 8) {
+      z0 = __byte_perm(w, 0x4B000000u, 0x7650); z1 = __byte_perm(w, 0x4B000000u, 0x7651);
+      z2 = __byte_perm(w, 0x4B000000u, 0x7652); z3 = __byte_perm(w, 0x4B000000u, 0x7653);
+    } else {
+      constexpr uint32_t m = (1u << Q) - 1u;
+      z0 = (w & m) | 0x4B000000u; z1 = ((w >> Q) & m) | 0x4B000000u;
+      z2 = ((w >> (2 * Q)) & m) | 0x4B000000u; z3 = ((w >> (3 * Q)) & m) | 0x4B000000u;
     }
+    const uint64_t ss = pair(s, s), mm = pair(neg_ms, neg_ms);
+    return {fma2(pair(z0, z1), ss, mm), fma2(pair(z2, z3), ss, mm)};
   }
 }
 
-// largest |v - k| among the 32 elements
-__device__ __forceinline__ float residual_maxabs(const float4 (&v)[8], const float4 (&k)[8]) {
-  float m = 0.f;
-#pragma unroll
-  for (int q = 0; q < 8; q++) {
-    m = fmaxf(fmaxf(m, fabsf(__fsub_rn(v[q].x, k[q].x))), fabsf(__fsub_rn(v[q].y, k[q].y)));
-    m = fmaxf(fmaxf(m, fabsf(__fsub_rn(v[q].z, k[q].z))), fabsf(__fsub_rn(v[q].w, k[q].w)));
+// the codes of v - k (4 * Q bits) for a block with exponent code `code`, and the mirror's step (zero for code 0)
+template <int Q>
+__device__ __forceinline__ uint32_t quantise(const Piece& v, Piece& k, uint32_t code, uint32_t valid) {
+  const Piece x = {sub2(v.a, k.a), sub2(v.b, k.b)};
+  if constexpr (Q == 1) {
+    float x0, x1, x2, x3;
+    unpair(x.a, x0, x1);
+    unpair(x.b, x2, x3);
+    const uint32_t w = ((x0 > 0.f ? 0u : 1u) | (x1 > 0.f ? 0u : 2u) | (x2 > 0.f ? 0u : 4u) | (x3 > 0.f ? 0u : 8u)) & valid;
+    add4(k, sign_steps(w, code, valid));
+    return w;
+  } else {
+    const float s = __uint_as_float(code << 23), inv = code ? __uint_as_float((254u - code) << 23) : 0.f;
+    const float big = 8388608.f + float(1 << (Q - 1)), neg_ms = __fmul_rn(-big, s);
+    const uint64_t ii = pair(inv, inv), bb = pair(big, big), ss = pair(s, s), mm = pair(neg_ms, neg_ms);
+    const uint64_t za = fma2(x.a, ii, bb), zb = fma2(x.b, ii, bb);
+    k.a = add2(k.a, fma2(za, ss, mm));
+    k.b = add2(k.b, fma2(zb, ss, mm));
+    const uint32_t b0 = uint32_t(za), b1 = uint32_t(za >> 32), b2 = uint32_t(zb), b3 = uint32_t(zb >> 32);
+    if (Q == 8) return __byte_perm(__byte_perm(b0, b1, 0x0040), __byte_perm(b2, b3, 0x0040), 0x5410);
+    constexpr uint32_t m = (1u << Q) - 1u;
+    return (b0 & m) | ((b1 & m) << Q) | ((b2 & m) << (2 * Q)) | ((b3 & m) << (3 * Q));
   }
-  return m;
 }
-// bits of the largest |v| among the 32 elements
-__device__ __forceinline__ uint32_t max_abs_bits(const float4 (&v)[8]) {
-  float m = 0.f;
-#pragma unroll
-  for (int q = 0; q < 8; q++) m = fmaxf(fmaxf(fmaxf(m, fabsf(v[q].x)), fabsf(v[q].y)), fmaxf(fabsf(v[q].z), fabsf(v[q].w)));
-  return __float_as_uint(m);
+
+// Reduces each of the four pieces' values over the eight lanes that share a 32-element chunk, in four shuffles instead of
+// twelve: every step halves what a lane holds.  A lane ends up with the result of piece (lane & 3) of its chunk row.
+template <class T, class Op>
+__device__ __forceinline__ T reduce_pieces(const T (&a)[kPieces], int lane, Op op) {
+  const bool b0 = lane & 1, b1 = lane & 2;
+  const T s0 = b0 ? a[0] : a[1], k0 = b0 ? a[1] : a[0], s1 = b0 ? a[2] : a[3], k1 = b0 ? a[3] : a[2];
+  const T r0 = op(k0, __shfl_xor_sync(0xffffffffu, s0, 1)), r1 = op(k1, __shfl_xor_sync(0xffffffffu, s1, 1));
+  const T s = b1 ? r0 : r1, k = b1 ? r1 : r0;
+  const T r = op(k, __shfl_xor_sync(0xffffffffu, s, 2));
+  return op(r, __shfl_xor_sync(0xffffffffu, r, 4));
 }
 
 }  // namespace
 
-int round_smem_bytes(int groups, int slots, int payload_bytes) { return smem_layout(payload_bytes, groups, slots).total; }
+int round_smem_bytes(int groups, int slots, int payload_bytes) {
+  (void)slots;
+  (void)payload_bytes;
+  return groups * int(sizeof(GroupShared));
+}
 
 // ----------------------------------------------------------------------------------------------
 // the kernel
 // ----------------------------------------------------------------------------------------------
-template <int Q, int kGroups, int kSlots>
-__global__ void __launch_bounds__(kGroups * (kGroupThreads + 32) + 32, 1)
-    round_kernel(const __grid_constant__ RoundParams p) {
-  extern __shared__ __align__(128) uint8_t smem[];
-  const SmemLayout lay = smem_layout(p.payload_bytes, kGroups, kSlots);
-  const int tid = threadIdx.x;
-  const bool is_pub = tid >= kGroups * (kGroupThreads + 32);
-  const bool is_io = !is_pub && tid >= kGroups * kGroupThreads;
-  const int g = is_pub ? 0 : (is_io ? (tid - kGroups * kGroupThreads) >> 5 : tid >> 7);
-  const int lane = tid & 31;
-  uint8_t* slots = smem + lay.off_slots + size_t(g) * kSlots * lay.slot_stride;
-  StepDesc* desc = reinterpret_cast<StepDesc*>(smem + lay.off_desc) + g * kSlots;
-  StepDesc* pubq = reinterpret_cast<StepDesc*>(smem + lay.off_pubq) + g * kPubQueue;
-  uint64_t* full = reinterpret_cast<uint64_t*>(smem + lay.off_bar) + g * (2 * kSlots + 1);
-  uint64_t* done = full + kSlots;
-  uint64_t* gsync = full + 2 * kSlots;
-  uint32_t* words = reinterpret_cast<uint32_t*>(smem + lay.off_words) + g * 16;
-  uint32_t* sflags = words;          // [kSlots]
-  uint32_t* armed = words + 4;       // steps armed so far
-  uint32_t* abort_flag = words + 5;
-  uint32_t* pub_ready = words + 6;   // steps whose stores have completed (I/O warp -> publisher)
-  uint32_t* pub_done = words + 7;    // steps published (publisher -> I/O warp)
-  uint32_t* pub_exit = words + 8;    // the group's I/O warp has nothing more to publish
-  uint32_t* yield_seen = reinterpret_cast<uint32_t*>(smem + lay.off_words) + 9;  // group 0's word: an update is waiting
-  float* s_red = reinterpret_cast<float*>(smem + lay.off_red) + g * 16;
+namespace {
 
-  if (tid == 0) {
-    for (int i = 0; i < kGroups; i++) {
-      uint64_t* b = reinterpret_cast<uint64_t*>(smem + lay.off_bar) + i * (2 * kSlots + 1);
-      for (int s = 0; s < kSlots; s++) {
-        mbar_init(b + s, 1);           // full: the I/O warp's arrive (+ the copies' bytes)
-        mbar_init(b + kSlots + s, 4);  // done: one arrive per compute warp
-      }
-      mbar_init(b + 2 * kSlots, 4);    // group sync of the compute warps
-      uint32_t* wd = reinterpret_cast<uint32_t*>(smem + lay.off_words) + i * 16;
-      for (int j = 0; j < 16; j++) wd[j] = 0;
+// Lane 0 of a compute warp: may the warp work on the group's tile number c?  All eight warps get the same answer: the
+// first one to come by moves the claim past c, unless the service warp has closed it.  The wait covers a service warp
+// that is looking for work; the limit only covers one that never comes back.
+__device__ __forceinline__ bool claim_tile(GroupShared& sh, uint32_t c) {
+  uint64_t t_start = 0;
+  for (uint32_t it = 0; it < (1u << 28); it++) {
+    if (int32_t(ld_shared_acquire(&sh.armed) - c) > 0) {
+      const uint32_t cl = *reinterpret_cast<volatile uint32_t*>(&sh.claim);
+      if ((cl & ~kClaimStop) > c) return true;
+      if (cl & kClaimStop) return false;
+      if (atomicCAS(&sh.claim, cl, c + 1u) == cl) return true;
+      continue;
     }
-    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-    fence_async_smem();
+    if (*reinterpret_cast<volatile uint32_t*>(&sh.claim) & kClaimStop) return false;
+    if ((it & 63) == 63) {
+      const uint64_t now = globaltimer_ns();
+      if (t_start == 0) t_start = now;
+      if (now - t_start > 2000ull * 1000 * 1000) return false;
+    }
+    __nanosleep(20);
   }
-  __syncthreads();  // the only CTA-wide barrier: from here on the groups, and the two kinds of warp, run on their own
+  return false;
+}
 
-  const int L = p.n_links;
-  const int pb = p.payload_bytes;
-  const int tpb = p.log2_block - 5;  // log2(threads per block of the quantiser)
-  const uint64_t limit_ns = p.wait_ns;
-  uint64_t* const launch_words = p.status + (p.parity ? kDsLaunch1 : kDsLaunch0);
+// The frames of a tile, as the service warp listed them: address | link, in ring order and sequence order.
+__device__ __forceinline__ const uint8_t* frame_at(uint64_t e) { return reinterpret_cast<const uint8_t*>(e & ~15ull); }
 
-  if (is_pub) {
-    // =========================================================================================
-    // publisher warp: sequence flags and credits of the steps whose stores have completed, for every group of the
-    // CTA.  Lane r serves out-ring r and in-ring r.
-    // =========================================================================================
-    uint32_t published[kGroups];
+// acc = the sum of the steps of the tile's frames (`only_link` < 0: of all of them).  Two frames are fetched at a time.
+template <int Q>
+__device__ __forceinline__ void decode_frames(const RoundParams& p, const uint64_t* list, int count, int only_link, int warp, int lane,
+                                              int left, Piece (&acc)[kPieces]) {
 #pragma unroll
-    for (int i = 0; i < kGroups; i++) published[i] = 0;
-    const uint64_t t_start = globaltimer_ns();
-    for (uint32_t it = 0;; it++) {
-      ST_CRUMB(3, 20);
-      // An update that is waiting for SMs: the I/O warps read this copy of the flag before they hand out a tile.
-      if (p.yield_flag != nullptr && lane == 0 && ld_cg_u32(p.yield_flag) != 0u) st_shared_volatile(yield_seen, 1u);
-      uint32_t ready[kGroups];
-      bool any = false, all_exit = true;
+  for (int i = 0; i < kPieces; i++) acc[i] = {0ull, 0ull};
+  for (int j = 0; j < count; j += 2) {
+    const uint64_t ea = list[j], eb = j + 1 < count ? list[j + 1] : 0ull;
+    const bool ua = only_link < 0 || int(ea & 15u) == only_link, ub = eb != 0 && (only_link < 0 || int(eb & 15u) == only_link);
+    FrameRegs a, b;
+    if (ua) load_frame<Q>(frame_at(ea), warp, lane, p.log2_block, a);
+    if (ub) load_frame<Q>(frame_at(eb), warp, lane, p.log2_block, b);
+    if (ua) {
 #pragma unroll
-      for (int i = 0; i < kGroups; i++) {
-        uint32_t* wd = reinterpret_cast<uint32_t*>(smem + lay.off_words) + i * 16;
-        // These words change under the warp's feet: lane 0 reads them and every lane takes lane 0's answer, so that
-        // the warp decides as one.
-        const uint32_t ex = __shfl_sync(0xffffffffu, ld_shared_volatile(wd + 8), 0);  // read before the counter: an exit
-        all_exit &= ex != 0;                                                           // flag is set after the last hand-over
-        ready[i] = __shfl_sync(0xffffffffu, ld_shared_volatile(wd + 6), 0);
-        any |= ready[i] != published[i];
-      }
-      if (any) {
-        ST_CRUMB(3, 21);
-        __threadfence_block();
-        __threadfence_system();  // the payloads are performed before the flags that announce them
-        ST_CRUMB(3, 22);
+      for (int i = 0; i < kPieces; i++) add4(acc[i], frame_steps<Q>(a.w[i], a.code(i), Q == 1 ? valid4(left, i) : 0xfu));
+    }
+    if (ub) {
 #pragma unroll
-        for (int i = 0; i < kGroups; i++) {
-          const StepDesc* q = reinterpret_cast<const StepDesc*>(smem + lay.off_pubq) + i * kPubQueue;
-          for (; published[i] != ready[i]; published[i]++) {
-            const StepDesc e = q[published[i] & (kPubQueue - 1)];
-            if (e.sent && lane < p.n_out && p.out[lane].link == e.link) {
-              const uint32_t slot_no = ctrl_byte(e.out_lo, e.out_hi, lane) & 63u;
-              const uint32_t seq = ld_cg_u32(p.out[lane].tx_seq + e.tile) + 1u;
-              st_relaxed_sys(p.out[lane].flags_remote + size_t(slot_no) * p.n_tiles + e.tile, seq);
-              st_cg_u32(p.out[lane].tx_seq + e.tile, seq);
-            }
-            if ((e.flags & kDescLast) && lane < p.n_in) {
-              const uint32_t avail = ctrl_byte(e.in_lo, e.in_hi, lane) >> 6;
-              if (avail) {
-                const uint32_t seq = ld_cg_u32(p.in[lane].rx_seq + e.tile) + avail;
-                st_cg_u32(p.in[lane].rx_seq + e.tile, seq);
-                st_relaxed_sys(p.in[lane].credit_remote + e.tile, seq);
-              }
-            }
-          }
-          __syncwarp();
-          __threadfence();  // the sequence counters are read by other warps once the hand-back below is seen
-          if (lane == 0) st_shared_volatile(reinterpret_cast<uint32_t*>(smem + lay.off_words) + i * 16 + 7, published[i]);
-        }
-      } else {
-        if (all_exit) break;
-        __nanosleep(100);
-        if ((it & 1023u) == 1023u && globaltimer_ns() - t_start > 4000ull * 1000 * 1000) break;  // the I/O warps are gone
+      for (int i = 0; i < kPieces; i++) add4(acc[i], frame_steps<Q>(b.w[i], b.code(i), Q == 1 ? valid4(left, i) : 0xfu));
+    }
+  }
+}
+
+// One lane's codes of its four pieces into the ring slots of link l's neighbours.  They go through shared memory, so
+// that a warp's part leaves as one contiguous run of 16-byte stores per ring.
+template <int Q>
+__device__ __forceinline__ void send_codes(const uint64_t* list, int count, int log2_block, int l, int warp, int lane,
+                                           const uint32_t (&w)[kPieces], bool loud, uint32_t code, uint32_t* stage) {
+  uint4 run = make_uint4(0u, 0u, 0u, 0u);
+  if (loud) {
+    if (Q == 1) {
+      uint32_t word[kPieces];
+#pragma unroll
+      for (int i = 0; i < kPieces; i++) word[i] = w[i] << (4 * piece_pos(i, lane));
+      const uint32_t chunk = reduce_pieces(word, lane, [](uint32_t a, uint32_t b) { return a | b; });
+      if ((lane & 4) == 0) stage[piece_chunk(lane & 3, lane)] = chunk;
+    } else {
+#pragma unroll
+      for (int i = 0; i < kPieces; i++) {
+        const int unit = piece_chunk(i, lane) * 8 + piece_pos(i, lane);
+        if (Q == 8) stage[unit] = w[i];
+        else if (Q == 4) reinterpret_cast<uint16_t*>(stage)[unit] = uint16_t(w[i]);
+        else reinterpret_cast<uint8_t*>(stage)[unit] = uint8_t(w[i]);
       }
     }
-    ST_CRUMB(3, 23);
-    return;
+    __syncwarp();
+    if (lane < 4 * Q) run = reinterpret_cast<const uint4*>(stage)[lane];
+    __syncwarp();
   }
+  // the scale byte of a block: the lane that holds the block's first chunk
+  const int chunk = warp * 16 + piece_chunk(lane & 3, lane), per_block = log2_block - 5;
+  const bool mine = (lane & 4) == 0 && (chunk & ((1 << per_block) - 1)) == 0;
+  for (int j = 0; j < count; j++) {
+    if (int(list[j] & 15u) != l) continue;
+    uint8_t* pay = reinterpret_cast<uint8_t*>(list[j] & ~15ull);
+    if (loud && lane < 4 * Q) *reinterpret_cast<uint4*>(pay + warp * (kWarpElems * Q / 8) + lane * 16) = run;
+    if (mine) pay[4 * Q * kWordsPerTile + (chunk >> per_block)] = uint8_t(code);
+  }
+}
 
-  if (!is_io) {
-    // =========================================================================================
-    // compute warps
-    // =========================================================================================
-    const int t = tid & 127;          // thread in group = 32-element chunk of the tile
-    const int wig = (tid >> 5) & 3;   // warp in group
-    const int sw = t & 7;             // XOR swizzle of this thread's eight 16-byte pieces
-    const int64_t n = p.n;
-    float res_max0 = 0.f, res_max1 = 0.f, res_max2 = 0.f;
-    uint32_t gphase = 0;
-    float4 v[8];
-    uint32_t vmax_mine = 0;
-#ifdef ST_ROUND_TIMING
-    long long tm_wait = 0, tm_total0 = clock64(), tm_steps = 0, tm_a = 0, tm_b = 0, tm_c = 0, tm_d = 0, tm_e = 0, st_lap_ = 0;
-#endif
-
-    for (uint32_t c = 0;; c++) {
-      const int s = int(c % kSlots);
-      uint8_t* slot = slots + size_t(s) * lay.slot_stride;
-      ST_CRUMB(4 + g, 30);
-      ST_T0();
-      // The step's descriptor first: it says which frames arrived, and their loads go out before the wait for the
-      // tile, so that the two latencies overlap.
-      const bool armed_ok = __all_sync(0xffffffffu, wait_armed(armed, c, abort_flag));  // the warp decides as one
-      __threadfence_block();
-      const StepDesc d = desc[s];
-      if (armed_ok && (d.flags & kDescExit)) break;
-      const int tile = d.tile, l = d.link;
-      float4* slot_v = reinterpret_cast<float4*>(slot) + t * 8;
-      float4* slot_k = reinterpret_cast<float4*>(slot + kTileBytes) + t * 8;
-      const int64_t left = n - (int64_t(tile) * kTile + int64_t(t) * 32);  // elements of this thread's chunk that exist
-      const bool full_chunk = left >= 32;
-      const uint32_t vmask = left >= 32 ? 0xffffffffu : (left <= 0 ? 0u : ((1u << int(left)) - 1u));
-      const bool masked = (Q == 1) && !full_chunk;
-      bool failed = false;
-
-      // ---- frames, in ring order and sequence order.  `only_link` < 0 takes every ring.
-      int it_r = -1, it_f = 0, it_avail = 0, it_only = -1;
-      uint32_t it_ib = 0;
-      auto first_frame = [&](int only_link) {
-        it_r = -1; it_f = 0; it_avail = 0; it_only = only_link;
-      };
-      auto next_frame = [&]() -> const uint8_t* {
-        while (true) {
-          if (it_r >= 0 && it_f < it_avail) {
-            const int slot_no = (int(it_ib & 63u) + it_f) & (p.ring_slots - 1);
-            it_f++;
-            return p.in[it_r].payload + (size_t(slot_no) * p.n_tiles + tile) * pb;
-          }
-          it_r++;
-          if (it_r >= p.n_in) return nullptr;
-          it_ib = ctrl_byte(d.in_lo, d.in_hi, it_r);
-          it_avail = (it_only >= 0 && p.in[it_r].link != it_only) ? 0 : int(it_ib >> 6);
-          it_f = 0;
-        }
-      };
-      // Frames are fetched four at a time, so that four load latencies overlap, and applied in order.
-      constexpr int kBatch = 4;
-      uint32_t bw[kBatch][Q], bc[kBatch];
-      int bn = 0;
-      auto load_batch = [&]() {
-        bn = 0;
-#pragma unroll
-        for (int i = 0; i < kBatch; i++) {
-          const uint8_t* fp = bn == i ? next_frame() : nullptr;
-          if (fp) {
-            load_frame<Q>(fp, t, tpb, bw[i], bc[i]);
-            bn = i + 1;
-          }
-        }
-      };
-      // acc = the sum of the frames' steps; the first batch may have been fetched already
-      auto decode_frames = [&](float4 (&acc)[8]) {
-#pragma unroll
-        for (int q = 0; q < 8; q++) acc[q] = make_float4(0.f, 0.f, 0.f, 0.f);
-        while (bn > 0) {
-#pragma unroll
-          for (int i = 0; i < kBatch; i++) {
-            if (i < bn) {
-              if (masked) add_frame<Q, true>(acc, bw[i], bc[i], sw, vmask); else add_frame<Q, false>(acc, bw[i], bc[i], sw, vmask);
-            }
-          }
-          if (bn == kBatch) load_batch(); else bn = 0;
-        }
-      };
-
-      const bool rx_first = armed_ok && (d.flags & kDescFirst) && (d.flags & kDescRxAny);
-      if (rx_first) {
-        first_frame(-1);
-        load_batch();
+// kOneLink: one link (a leaf of the tree, a member of a mesh group); what arrived for the values is what arrived on it.
+template <int Q, bool kOneLink>
+__device__ __forceinline__ void compute_warp(const RoundParams& p, GroupShared& sh, int warp, int lane) {
+  const int L = kOneLink ? 1 : p.n_links, lb = p.log2_block;
+  float res_max0 = 0.f, res_max1 = 0.f, res_max2 = 0.f;
+  uint32_t exchanges = 0;
+  for (uint32_t c = 0;; c++) {
+    const uint32_t go = lane == 0 ? (claim_tile(sh, c) ? 1u : 0u) : 0u;
+    if (!__shfl_sync(0xffffffffu, go, 0)) break;
+    const uint32_t entry = c % kBank;
+    const TileDesc d = sh.desc[entry];
+    if (warp == 0 && lane == 0) {
+      // The next tile on its way into the L2.  One tile ahead is best: a window of 25 M elements that receives and sends
+      // takes 92 us so, 115 us with two tiles ahead and 153 us with four.
+      const uint32_t ahead = c + 1u;
+      if (int32_t(ld_shared_acquire(&sh.armed) - ahead) > 0) {
+        const TileDesc& e = sh.desc[ahead % kBank];
+        if (!(e.flags & kDescNoValues)) bulk_prefetch_l2(p.values + size_t(e.tile) * kTile, kTile * 4);
+        for (int l = 0; l < L; l++) bulk_prefetch_l2(p.mirror[l] + size_t(e.tile) * kTile, kTile * 4);
+        for (int j = 0; j < e.n_frames; j++) bulk_prefetch_l2(frame_at(sh.frames[ahead % kBank][j]), uint32_t(p.payload_bytes));
       }
-      ST_CRUMB(4 + g, 31);
-      const bool step_ok = __all_sync(0xffffffffu, armed_ok && mbar_wait_bounded(full + s, (c / kSlots) & 1u, limit_ns));
-      ST_CRUMB(4 + g, 32);
-      if (wig == 0) ST_STAMP(c, 1);
-      ST_ACC(tm_wait);
-#ifdef ST_ROUND_TIMING
-      tm_steps++;
-#endif
-      if (!step_ok) {
-        // Nothing of this step is stored: the warp reports the failure and leaves; the I/O warp then stops the group.
-        if (lane == 0) atomicOr(&sflags[s], kFlagFailed);
-        __syncwarp();
-        if (lane == 0) mbar_arrive(done + s);
-        break;
-      }
-
-#ifdef ST_ROUND_TIMING
-      st_lap_ = clock64();
-#endif
-      if (d.flags & kDescFirst) {
+    }
+    const int in_tile = warp * kWarpElems + lane * 4;
+    const size_t off = size_t(d.tile) * kTile + in_tile;
+    const int left = int(min(int64_t(kTile), p.n - int64_t(d.tile) * kTile)) - in_tile;  // (used by sign frames only)
+    float* const vp = p.values + off;
+    Piece v[kPieces], k[kPieces];
+    const uint64_t* frames = sh.frames[entry];
+    const bool load_v = (d.flags & kDescNoValues) == 0;
+    int applied = -1;  // the link whose mirror has been given what arrived on it
+    if (d.n_frames <= 1) {
+      // the common case: everything is fetched at once, and the one frame's steps never have to be kept
 #pragma unroll
-        for (int q = 0; q < 8; q++) v[q] = (d.flags & kDescNoValues) ? make_float4(0.f, 0.f, 0.f, 0.f) : slot_v[q ^ sw];
-        if (rx_first) {
-          float4 acc[8];
-          decode_frames(acc);
+      for (int i = 0; i < kPieces; i++) v[i] = load_v ? load_piece(vp + i * 128) : Piece{0ull, 0ull};
 #pragma unroll
-          for (int q = 0; q < 8; q++) {
-            v[q].x = __fadd_rn(v[q].x, acc[q].x); v[q].y = __fadd_rn(v[q].y, acc[q].y);
-            v[q].z = __fadd_rn(v[q].z, acc[q].z); v[q].w = __fadd_rn(v[q].w, acc[q].w);
-            slot_v[q ^ sw] = acc[q];  // leaves as a reduce-add into the values
-          }
+      for (int i = 0; i < kPieces; i++) k[i] = load_piece(p.mirror[0] + off + i * 128);
+      if (d.n_frames == 1) {
+        const uint64_t e = frames[0];
+        const bool for0 = kOneLink || (e & 15u) == 0;
+        FrameRegs f;
+        load_frame<Q>(frame_at(e), warp, lane, lb, f);
+#pragma unroll
+        for (int i = 0; i < kPieces; i++) {
+          const Piece s = frame_steps<Q>(f.w[i], f.code(i), Q == 1 ? valid4(left, i) : 0xfu);
+          if (f.code(i)) red_add_piece(vp + i * 128, s);
+          add4(v[i], s);
+          if (for0) add4(k[i], s);
         }
-        vmax_mine = max_abs_bits(v);
+        if (for0) applied = 0;
       }
-
-      ST_LAP(tm_a);
-      float4 k[8];
+    } else {
+      Piece acc[kPieces];
+      decode_frames<Q>(p, frames, d.n_frames, -1, warp, lane, left, acc);
 #pragma unroll
-      for (int q = 0; q < 8; q++) k[q] = slot_k[q ^ sw];
+      for (int i = 0; i < kPieces; i++) {
+        v[i] = load_v ? load_piece(vp + i * 128) : Piece{0ull, 0ull};
+        k[i] = load_piece(p.mirror[0] + off + i * 128);
+      }
+#pragma unroll
+      for (int i = 0; i < kPieces; i++) {
+        red_add_piece(vp + i * 128, acc[i]);
+        add4(v[i], acc[i]);
+        if (kOneLink) add4(k[i], acc[i]);
+      }
+      if (kOneLink) applied = 0;
+    }
+    uint32_t finished = kDoneWarp;
+    bool failed = false;
+    for (int l = 0; l < L; l++) {
+      float* const kp = p.mirror[l] + off;
+      if (!kOneLink && l > 0) {
+#pragma unroll
+        for (int i = 0; i < kPieces; i++) k[i] = load_piece(kp + i * 128);
+      }
       bool changed = false;
-      if (d.flags & kDescRxLink) {
-        float4 acc[8];
-        if (L == 1) {
-          // one link: what arrived for the values is what arrived on this link, and the slot still holds it
+      if (d.flags & (kDescRxLink << l)) {
+        if (!kOneLink && applied != l) {
+          const uint32_t only = (d.flags >> (kDescFrameShift + 5 * l)) & 31u;
+          if (only) {
+            FrameRegs f;
+            load_frame<Q>(frame_at(frames[only - 1u]), warp, lane, lb, f);
 #pragma unroll
-          for (int q = 0; q < 8; q++) acc[q] = slot_v[q ^ sw];
-        } else {
-          first_frame(l);
-          load_batch();
-          decode_frames(acc);
-        }
+            for (int i = 0; i < kPieces; i++) add4(k[i], frame_steps<Q>(f.w[i], f.code(i), Q == 1 ? valid4(left, i) : 0xfu));
+          } else {
+            Piece acc[kPieces];
+            decode_frames<Q>(p, frames, d.n_frames, l, warp, lane, left, acc);
 #pragma unroll
-        for (int q = 0; q < 8; q++) {
-          k[q].x = __fadd_rn(k[q].x, acc[q].x); k[q].y = __fadd_rn(k[q].y, acc[q].y);
-          k[q].z = __fadd_rn(k[q].z, acc[q].z); k[q].w = __fadd_rn(k[q].w, acc[q].w);
+            for (int i = 0; i < kPieces; i++) add4(k[i], acc[i]);
+          }
         }
         changed = true;
       }
-
-      ST_LAP(tm_b);
-      // ---- quantise values - mirror for link l
-      const bool want = (d.flags & kDescTxWant) != 0;  // (a step that only receives says nothing back, whatever rounding left)
-      float xm = residual_maxabs(v, k);
-      if (!want) xm = 0.f;
-      if (l == 0) res_max0 = fmaxf(res_max0, xm); else if (l == 1) res_max1 = fmaxf(res_max1, xm); else res_max2 = fmaxf(res_max2, xm);
-      uint32_t vm = vmax_mine;
-      // blocks larger than 32 elements: maximum over lanes (up to 1024), then over the group's warps
-      for (int sft = 0; sft < tpb && sft < 5; sft++) {
-        xm = fmaxf(xm, __shfl_xor_sync(0xffffffffu, xm, 1 << sft));
-        vm = max(vm, __shfl_xor_sync(0xffffffffu, vm, 1 << sft));
-      }
-      if (tpb > 5) {
-        float* red = s_red + (c & 1u) * 8;  // two buffers: a warp may be one step ahead of the slowest one
-        if (lane == 0) {
-          red[wig] = xm;
-          red[4 + wig] = __uint_as_float(vm);
+      if (d.flags & (kDescTxWant << l)) {  // (a visit that only receives says nothing back, whatever rounding left)
+        float xs[kPieces], vs[kPieces];
+#pragma unroll
+        for (int i = 0; i < kPieces; i++) {
+          xs[i] = maxabs({sub2(v[i].a, k[i].a), sub2(v[i].b, k[i].b)});
+          vs[i] = maxabs(v[i]);
         }
-        __syncwarp();
-        if (lane == 0) mbar_arrive(gsync);
-        if (!__all_sync(0xffffffffu, mbar_wait_bounded(gsync, gphase, limit_ns))) failed = true;
-        gphase ^= 1u;
-        const float a0 = red[0], a1 = red[1], a2 = red[2], a3 = red[3];
-        const uint32_t b0 = __float_as_uint(red[4]), b1 = __float_as_uint(red[5]);
-        const uint32_t b2 = __float_as_uint(red[6]), b3 = __float_as_uint(red[7]);
-        if (tpb == 6) {  // 2048: warps {0,1} and {2,3}
-          xm = wig < 2 ? fmaxf(a0, a1) : fmaxf(a2, a3);
-          vm = wig < 2 ? max(b0, b1) : max(b2, b3);
-        } else {         // 4096: the whole tile
-          xm = fmaxf(fmaxf(a0, a1), fmaxf(a2, a3));
-          vm = max(max(b0, b1), max(b2, b3));
-        }
-      }
-      const int code = block_code_dev<Q>(xm, vm, p.min_exp, p.rel_bits);
-      ST_LAP(tm_c);
-      if ((d.flags & kDescTxOk) != 0) {
-        uint8_t* pay = slot + 2 * kTileBytes;
-        if (code) {
-          uint32_t w[Q];
-          if (masked) quantise<Q, true>(v, k, uint32_t(code), w, sw, vmask); else quantise<Q, false>(v, k, uint32_t(code), w, sw, vmask);
-          changed = true;
-          if (Q == 8) {
-            reinterpret_cast<uint4*>(pay)[t * 2] = make_uint4(w[0], w[1 % Q], w[2 % Q], w[3 % Q]);
-            reinterpret_cast<uint4*>(pay)[t * 2 + 1] = make_uint4(w[4 % Q], w[5 % Q], w[6 % Q], w[7 % Q]);
-          } else if (Q == 4) {
-            reinterpret_cast<uint4*>(pay)[t] = make_uint4(w[0], w[1 % Q], w[2 % Q], w[3 % Q]);
-          } else if (Q == 2) {
-            reinterpret_cast<uint2*>(pay)[t] = make_uint2(w[0], w[1 % Q]);
-          } else {
-            reinterpret_cast<uint32_t*>(pay)[t] = w[0];
+        auto larger = [](float a, float b) { return fmaxf(a, b); };
+        float xm = reduce_pieces(xs, lane, larger), vm = reduce_pieces(vs, lane, larger);
+        if (kOneLink || l == 0) res_max0 = fmaxf(res_max0, xm); else if (l == 1) res_max1 = fmaxf(res_max1, xm); else res_max2 = fmaxf(res_max2, xm);
+        // blocks of more than 32 elements: over the chunks of a piece row, the piece rows, the warps
+        if (lb >= 6) {
+          xm = fmaxf(xm, __shfl_xor_sync(0xffffffffu, xm, 8)); vm = fmaxf(vm, __shfl_xor_sync(0xffffffffu, vm, 8));
+          if (lb >= 7) { xm = fmaxf(xm, __shfl_xor_sync(0xffffffffu, xm, 16)); vm = fmaxf(vm, __shfl_xor_sync(0xffffffffu, vm, 16)); }
+          if (lb >= 8) { xm = fmaxf(xm, __shfl_xor_sync(0xffffffffu, xm, 1)); vm = fmaxf(vm, __shfl_xor_sync(0xffffffffu, vm, 1)); }
+          if (lb >= 9) { xm = fmaxf(xm, __shfl_xor_sync(0xffffffffu, xm, 2)); vm = fmaxf(vm, __shfl_xor_sync(0xffffffffu, vm, 2)); }
+          if (lb >= 10) {
+            float(*red)[kComputeWarps] = sh.red[exchanges & 1u];
+            if (lane == 0) {
+              red[0][warp] = xm;
+              red[1][warp] = vm;
+              mbar_arrive(&sh.gsync);
+            }
+            if (!__all_sync(0xffffffffu, mbar_wait_bounded(&sh.gsync, exchanges & 1u, p.wait_ns))) {
+              failed = true;
+              break;
+            }
+            exchanges++;
+            const int w0 = warp & ~((1 << (lb - 9)) - 1);
+            for (int j = 0; j < (1 << (lb - 9)); j++) {
+              xm = fmaxf(xm, red[0][w0 + j]);
+              vm = fmaxf(vm, red[1][w0 + j]);
+            }
           }
         }
-        if ((t & ((1 << tpb) - 1)) == 0) pay[4 * Q * kWordsPerTile + (t >> tpb)] = uint8_t(code);
+        const uint32_t code = uint32_t(block_code_dev<Q>(xm, __float_as_uint(vm), p.min_exp, p.rel_bits));
+        const bool loud = __any_sync(0xffffffffu, code != 0);
+        if (loud) finished += 1u << (kDoneNonsilentShift + 4 * l);
+        if (d.flags & (kDescTxOk << l)) {
+          uint32_t w[kPieces];
+          if (loud) {
+#pragma unroll
+            for (int i = 0; i < kPieces; i++)
+              w[i] = quantise<Q>(v[i], k[i], __shfl_sync(0xffffffffu, code, (lane & ~3) | i), Q == 1 ? valid4(left, i) : 0xfu);
+            changed = true;
+          }
+          send_codes<Q>(sh.slots[entry], d.n_slots, lb, l, warp, lane, w, loud, code, sh.stage[warp]);
+        }
       }
-      ST_LAP(tm_d);
       if (changed) {
 #pragma unroll
-        for (int q = 0; q < 8; q++) slot_k[q ^ sw] = k[q];
-      }
-      fence_async_smem();  // what this thread wrote into the slot is about to be read by bulk stores
-      {
-        const uint32_t mine = (changed ? kFlagChanged : 0u) | (code ? kFlagNonsilent : 0u) | (failed ? kFlagFailed : 0u);
-        const uint32_t warp_bits = __reduce_or_sync(0xffffffffu, mine);
-        if (lane == 0 && warp_bits) atomicOr(&sflags[s], warp_bits);
-      }
-      __syncwarp();
-      if (lane == 0) mbar_arrive(done + s);
-      if (wig == 0) ST_STAMP(c, 2);
-      ST_LAP(tm_e);
-      if (failed) break;
-    }
-
-#ifdef ST_ROUND_TIMING
-    if (blockIdx.x == 0 && tid == 0)
-      printf("compute: total %lld cycles, waiting for steps %lld, steps %lld; values+decode %lld, mirror+rx %lld, stats %lld, quantise %lld, store+arrive %lld\n",
-             clock64() - tm_total0, tm_wait, tm_steps, tm_a, tm_b, tm_c, tm_d, tm_e);
-#endif
-    ST_CRUMB(4 + g, 33);
-    // ---- statistics: the largest outstanding residual per link
-    {
-      float a0 = res_max0, a1 = res_max1, a2 = res_max2;
-      for (int o = 16; o > 0; o >>= 1) {
-        a0 = fmaxf(a0, __shfl_xor_sync(0xffffffffu, a0, o));
-        a1 = fmaxf(a1, __shfl_xor_sync(0xffffffffu, a1, o));
-        a2 = fmaxf(a2, __shfl_xor_sync(0xffffffffu, a2, o));
-      }
-      if (lane == 0) {  // non-negative floats order like their bit patterns
-        unsigned long long* rm = reinterpret_cast<unsigned long long*>(launch_words + kDlResMax);
-        if (a0 != 0.f) atomicMax(rm + 0, (unsigned long long)__float_as_uint(a0));
-        if (a1 != 0.f) atomicMax(rm + 1, (unsigned long long)__float_as_uint(a1));
-        if (a2 != 0.f) atomicMax(rm + 2, (unsigned long long)__float_as_uint(a2));
+        for (int i = 0; i < kPieces; i++) store_piece(kp + i * 128, k[i]);
       }
     }
-    return;
+    if (failed) finished |= kDoneFailed;
+    __syncwarp();  // what the lanes stored comes before what lane 0 says about it
+    if (lane == 0) red_shared_release_add(&sh.done[entry], finished);
+    if (failed) break;
   }
+  // ---- statistics: the largest outstanding residual per link
+  for (int o = 16; o > 0; o >>= 1) {
+    res_max0 = fmaxf(res_max0, __shfl_xor_sync(0xffffffffu, res_max0, o));
+    res_max1 = fmaxf(res_max1, __shfl_xor_sync(0xffffffffu, res_max1, o));
+    res_max2 = fmaxf(res_max2, __shfl_xor_sync(0xffffffffu, res_max2, o));
+  }
+  if (lane == 0) {  // non-negative floats order like their bit patterns
+    unsigned long long* rm = reinterpret_cast<unsigned long long*>(p.status + (p.parity ? kDsLaunch1 : kDsLaunch0) + kDlResMax);
+    if (res_max0 != 0.f) atomicMax(rm + 0, (unsigned long long)__float_as_uint(res_max0));
+    if (res_max1 != 0.f) atomicMax(rm + 1, (unsigned long long)__float_as_uint(res_max1));
+    if (res_max2 != 0.f) atomicMax(rm + 2, (unsigned long long)__float_as_uint(res_max2));
+  }
+}
 
-  // ===========================================================================================
-  // I/O warp.  All 32 lanes run the same control flow; lane 0 issues copies, stores and flags.
-  // ===========================================================================================
-  // The group's tiles: a run of `chunk` consecutive tiles, or (chunk == 0) every gstride-th tile of the tensor.
-  // (of the launch's window of the tensor, tiles tile_begin .. tile_begin + tile_count - 1)
-  const int gidx = int(blockIdx.x) * kGroups + g;
+// The service warp.  A lane looks after one ring pair (in-ring r and out-ring r) of one tile: with R rings, rounded up to
+// a power of two above one, 32 / R tiles are looked at together, and every look costs two round trips to the L2 whatever R is.
+// All 32 lanes run the same control flow; decisions taken from words that change under the warp's feet are taken by one
+// lane, or on a ballot.
+__device__ __forceinline__ void service_warp(const RoundParams& p, GroupShared& sh, int g, int n_groups, int lane) {
+  // The group's tiles: a run of `chunk` consecutive tiles, or (chunk == 0) every gstride-th tile of the launch's window.
+  const int gidx = int(blockIdx.x) * n_groups + g;
   const int gid0 = p.chunk > 0 ? gidx * p.chunk : gidx;
-  const int gstride = p.chunk > 0 ? 1 : int(gridDim.x) * kGroups;
+  const int gstride = p.chunk > 0 ? 1 : int(gridDim.x) * n_groups;
   const int my_count = p.chunk > 0 ? max(0, min(p.chunk, p.tile_count - gid0))
                                    : (p.tile_count > gid0 ? (p.tile_count - gid0 + gstride - 1) / gstride : 0);
   const int gid = p.tile_begin + gid0;
   const uint32_t smask = uint32_t(p.ring_slots) - 1u;
-  uint32_t issued = 0, retired = 0;
-  unsigned long long n_done = 0, n_tx = 0, n_rx = 0, n_blocked = 0, n_pending = 0, n_sweeps = 0;
-  bool aborted = false, tile_pending = false, yielded = false;
-#ifdef ST_ROUND_TIMING
-  long long tm_done = 0, tm_read = 0, tm_pubwait = 0, tm_pub = 0, tm_scout = 0, tm_issue = 0, tm_store = 0, tm_pf = 0, tm_io0 = clock64();
-#endif
+  const uint64_t limit_ns = p.wait_ns;
+  uint64_t* const launch_words = p.status + (p.parity ? kDsLaunch1 : kDsLaunch0);
+  const unsigned long long sent_before = blockIdx.x == 0 && g == 0 && lane == 0 ? p.status[kDsFramesSent] : 0ull;  // for the trace
+
+  // ---- this lane's ring pair and its place among the tiles looked at together
+  int log2_rings = 1;                             // (16 tiles at most, so that the next look fits into the bank in time)
+  while ((1 << log2_rings) < max(p.n_in, p.n_out)) log2_rings++;
+  const int at_once = 32 >> log2_rings;           // tiles of one look
+  const int r = lane >> (5 - log2_rings), t = lane & (at_once - 1);
+  uint32_t same_tile = 0;                         // the lanes of this lane's tile, one per ring, in ring order
+  for (int i = 0; i < (1 << log2_rings); i++) same_tile |= 1u << (i * at_once + t);
+  const uint32_t below = (1u << lane) - 1u;
+  const bool is_in = r < p.n_in && p.do_rx, is_out = r < p.n_out && p.do_tx;
+  InRing in{};
+  OutRing out{};
+  if (r < p.n_in) in = p.in[r];
+  if (r < p.n_out) out = p.out[r];
+
+  bool handed_on = false;   // the next window's launch has been let in
+  uint32_t n_done = 0, n_tx = 0, n_rx = 0, n_blocked = 0, n_pending = 0, n_sweeps = 0;  // per lane, added up at the end
+  uint32_t armed = 0, finished = 0, published = 0;  // tiles armed, finished by the compute warps, published so far
+  bool aborted = false, yielded = false;
 
   if (p.zero_other && blockIdx.x == 0 && g == 0 && lane == 0) {
     uint64_t* other = p.status + (p.parity ? kDsLaunch0 : kDsLaunch1);  // the next cycle's half
     for (int i = 0; i < 8; i++) other[i] = 0;
   }
-
-  // Steps whose stores have completed are handed to the publisher warp; `pushed` counts the steps queued so far.
-  uint32_t pushed = 0, handed = 0;
-  auto hand_over = [&](uint32_t upto) {
-    if (lane == 0 && upto != handed) {
-      __threadfence_block();
-      st_shared_volatile(pub_ready, upto);
-    }
-    handed = upto;
-  };
-  // bounded wait until the publisher has published `upto` steps
-  auto wait_published = [&](uint32_t upto) -> bool {
-    const uint64_t t0 = globaltimer_ns();
-    bool ok = false;
-    for (uint32_t it = 0; it < (1u << 26); it++) {
-      if (int32_t(ld_shared_volatile(pub_done) - upto) >= 0) {
-        ok = true;
-        break;
-      }
-      if ((it & 15) == 15 && globaltimer_ns() - t0 > 2 * limit_ns + 2000000ull) break;
-      __nanosleep(50);
-    }
-    return __all_sync(0xffffffffu, ok);  // the warp decides as one
+  auto update_waiting = [&]() -> bool {
+    const uint32_t y = p.yield_flag != nullptr && lane == 0 ? ld_cg_u32(p.yield_flag) : 0u;
+    return __any_sync(0xffffffffu, y != 0);
   };
 
-  // a finished step: its stores go out and its slot becomes free
-  auto retire = [&](uint32_t c) -> bool {
-    const int s = int(c % kSlots);
-    bool ok;
-    {
-      ST_T0();
-      ST_CRUMB(g, 4);
-      ok = __all_sync(0xffffffffu, mbar_wait_bounded(done + s, (c / kSlots) & 1u, 2 * limit_ns));
-      ST_ACC(tm_done);
-    }
-    ST_STAMP(c, 3);
-    const uint32_t f = ok ? __shfl_sync(0xffffffffu, ld_shared_volatile(sflags + s), 0) : kFlagFailed;
-    if (f & kFlagFailed) return false;
-    if (pushed - __shfl_sync(0xffffffffu, ld_shared_volatile(pub_done), 0) >= uint32_t(kPubQueue)) {  // (the publisher has fallen behind: its fence takes tens of microseconds under load)
-      bulk_wait_all();
-      __syncwarp();
-      hand_over(pushed);
-      if (!wait_published(pushed)) return false;
-    }
-    ST_T0();
-    {
-      // the step's stores, one per lane, issued by as few instructions as possible: lane 0 the reduce-add of what was
-      // received into the values; lane 1 the stepped mirror, lanes 2.. the frame into the ring of out-ring lane-2.
-      // Every lane that issued commits and later waits for its own bulk group.
-      const StepDesc d = desc[s];
-      uint8_t* slot = slots + size_t(s) * lay.slot_stride;
-      const bool sent = (d.flags & kDescTxOk) != 0 && (f & kFlagNonsilent) != 0;
-      if (lane == 0 && (d.flags & kDescFirst) && (d.flags & kDescRxAny))
-        bulk_reduce_add_f32(p.values + size_t(d.tile) * kTile, slot, kTileBytes);
-      {
-        void* dst = nullptr;
-        const uint8_t* src = nullptr;
-        uint32_t bytes = 0;
-        if (lane == 1) {
-          if (f & kFlagChanged) {
-            dst = p.mirror[d.link] + size_t(d.tile) * kTile;
-            src = slot + kTileBytes;
-            bytes = kTileBytes;
-          }
-        } else if (lane >= 2 && lane - 2 < p.n_out && sent && p.out[lane - 2].link == d.link) {
-          const uint32_t slot_no = ctrl_byte(d.out_lo, d.out_hi, lane - 2) & 63u;
-          dst = p.out[lane - 2].payload_remote + (size_t(slot_no) * p.n_tiles + d.tile) * pb;
-          src = slot + 2 * kTileBytes;
-          bytes = uint32_t(pb);
-        }
-        if (bytes) bulk_s2g(dst, src, bytes);
-      }
-      bulk_commit();
-    }
-    if (lane == 0) {
-      const StepDesc d = desc[s];
-      const bool sent = (d.flags & kDescTxOk) != 0 && (f & kFlagNonsilent) != 0;
-      if (sent)
-        for (int r = 0; r < p.n_out; r++) n_tx += p.out[r].link == d.link ? 1 : 0;
-      StepDesc e = d;
-      e.sent = sent ? 1u : 0u;
-      pubq[pushed & (kPubQueue - 1)] = e;
-      if (f & kFlagNonsilent) {
-        tile_pending = true;  // more may be left to say (or nothing could be said at all)
-        if (!sent && p.do_tx) n_blocked++;
-      }
-      if (d.flags & kDescLast) {
-        if (tile_pending) {
-          st_cg_u32(p.tile_state + d.tile, 1u);
-          n_pending++;
-        }
-        tile_pending = false;
-        n_done++;
-        for (int r = 0; r < p.n_in; r++) n_rx += ctrl_byte(d.in_lo, d.in_hi, r) >> 6;
-      }
-    }
-    {
-      ST_T0();
-      ST_CRUMB(g, 5);
-      bulk_wait_read_all();  // every lane for its own stores: the slot may be refilled
-      ST_ACC(tm_read);
-    }
-    pushed++;
-    __syncwarp();
-    ST_STAMP(c, 4);
-    ST_ACC(tm_store);
-    return true;
-  };
-
-  ST_CRUMB(g, 1);
   for (int sweep = 0; sweep < p.sweeps && !aborted && !yielded && my_count > 0; sweep++) {
-    const unsigned long long done_before = n_done;
-    int scan_pos = 0;
-    uint32_t pend = 0;                 // lanes whose scouted tile still has to be handed out
-    int sc_tile = 0;                   // what this lane found for its tile
-    uint32_t sc_in_lo = 0, sc_in_hi = 0, sc_out_lo = 0, sc_out_hi = 0, sc_dirty = 0;
-    int cur_tile = -1, cur_a = 0;      // the tile whose steps are being handed out
-    uint32_t cur_in_lo = 0, cur_in_hi = 0, cur_out_lo = 0, cur_out_hi = 0, cur_dirty = 0;
-    bool exhausted = my_count == 0;
-
+    const uint32_t armed_before = armed;
+    int looked = 0;           // tiles of the group looked at in this sweep
+    uint32_t idle = 0;
+    uint64_t t_last = globaltimer_ns();
     while (true) {
-      ST_CRUMB(g, 2);
-      if (!exhausted && issued - retired < uint32_t(kSlots)) {
-        if (cur_tile < 0 && __shfl_sync(0xffffffffu, ld_shared_volatile(yield_seen), 0) != 0u) {
-          // An update is waiting for the SMs this kernel holds: hand out nothing more.  Tiles that were looked at but
-          // not handed out get their change marks back, everything else is untouched.
-          if (((pend >> lane) & 1u) && sc_dirty) st_cg_u32(p.tile_state + sc_tile, 1u);
-          pend = 0;
-          exhausted = true;
+      // ---- look at more tiles while the compute warps have less than kAhead in hand and the bank has room for them
+      if (looked < my_count && !yielded && armed - finished < uint32_t(kAhead) && armed - published + uint32_t(at_once) <= uint32_t(kBank)) {
+        ST_CRUMB(g, 2);
+        const uint32_t y = p.yield_flag != nullptr && lane == 0 ? ld_cg_u32(p.yield_flag) : 0u;
+        const int j = looked + t;
+        const bool valid = j < my_count;
+        const int tile = gid + j * gstride;
+        looked += at_once;
+        uint32_t dirty = 0, rx = 0, tx = 0, credit = 0, avail = 0;
+        if (valid) {
+          // The change mark is cleared before the tile's values are read (the tile is armed after this exchange has
+          // returned), and whoever changes the values sets it after the change: a change that this visit does not see
+          // leaves its mark for the next one.
+          if (r == 0) dirty = atomicExch(p.tile_state + tile, 0u);
+          if (is_in) rx = ld_cg_u32(in.rx_seq + tile);
+          if (is_out) {
+            tx = ld_cg_u32(out.tx_seq + tile);
+            credit = ld_relaxed_sys(out.credit + tile);  // (a slot is only stored to once its credit has been seen)
+          }
+          if (is_in) {
+            const uint32_t* fl = in.flags + tile;
+            const uint32_t f0 = ld_relaxed_sys(fl + size_t(rx & smask) * p.n_tiles), f1 = ld_relaxed_sys(fl + size_t((rx + 1u) & smask) * p.n_tiles),
+                           f2 = ld_relaxed_sys(fl + size_t((rx + 2u) & smask) * p.n_tiles);
+            avail = f0 != rx + 1u ? 0u : (f1 != rx + 2u ? 1u : (f2 != rx + 3u ? 2u : 3u));
+            // the flag of the last frame once more, as the acquire that the frames' contents are read behind (the looks
+            // above went out together; an acquire holds up every access after it)
+            if (avail) (void)ld_acquire_sys(fl + size_t((rx + avail - 1u) & smask) * p.n_tiles);
+          }
+        }
+        dirty = __shfl_sync(0xffffffffu, dirty, t);
+        const bool room = is_out && (tx - credit) < uint32_t(p.ring_slots);
+        const uint32_t in1 = __ballot_sync(0xffffffffu, avail >= 1), in2 = __ballot_sync(0xffffffffu, avail >= 2), in3 = __ballot_sync(0xffffffffu, avail >= 3);
+        const bool any_in = (in1 & same_tile) != 0, work = valid && (dirty != 0 || any_in);
+        if (__any_sync(0xffffffffu, y != 0)) {  // an update is waiting for SMs: hand out nothing more
+          if (dirty && r == 0) st_cg_u32(p.tile_state + tile, 1u);
           yielded = true;
           continue;
         }
-        if (cur_tile < 0) {
-          if (pend == 0) {
-            if (scan_pos >= my_count) {
-              exhausted = true;
-              continue;
-            }
-            // ---- look at 32 tiles at once, one per lane
-            ST_T0();
-            const int j = scan_pos + lane;
-            const bool valid = j < my_count;
-            sc_tile = gid + j * gstride;
-            sc_in_lo = sc_in_hi = sc_out_lo = sc_out_hi = sc_dirty = 0;
-            bool work = false;
-            if (valid) {
-              uint32_t dirty = ld_cg_u32(p.tile_state + sc_tile);
-              bool any = false;
-              if (p.do_rx) {
-                for (int r = 0; r < p.n_in; r++) {
-                  const uint32_t e = ld_cg_u32(p.in[r].rx_seq + sc_tile);
-                  uint32_t avail = 0;
-                  while (avail < uint32_t(kRxMax)) {
-                    const uint32_t fl = ld_acquire_sys(p.in[r].flags + size_t((e + avail) & smask) * p.n_tiles + sc_tile);
-                    if (fl != e + avail + 1u) break;
-                    avail++;
-                  }
-                  const uint32_t byte = (avail << 6) | (e & smask);
-                  if (r < 4) sc_in_lo |= byte << (r * 8); else sc_in_hi |= byte << ((r - 4) * 8);
-                  any |= avail != 0;
-                }
-              }
-              if (p.do_tx) {
-                for (int r = 0; r < p.n_out; r++) {
-                  const uint32_t tx = ld_cg_u32(p.out[r].tx_seq + sc_tile);
-                  const uint32_t cr = ld_acquire_sys(p.out[r].credit + sc_tile);
-                  const uint32_t room = (tx - cr) < uint32_t(p.ring_slots) ? 1u : 0u;
-                  const uint32_t byte = (room << 6) | (tx & smask);
-                  if (r < 4) sc_out_lo |= byte << (r * 8); else sc_out_hi |= byte << ((r - 4) * 8);
-                }
-              }
-              // The change mark is cleared before the tile's values are read (the copy is issued after this
-              // exchange has returned), and whoever changes the values sets it after the change: a change
-              // that this visit does not see leaves its mark for the next one.
-              if (dirty) dirty = atomicExch(p.tile_state + sc_tile, 0u);
-              sc_dirty = dirty;
-              work = dirty != 0 || any;
-            }
-            pend = __ballot_sync(0xffffffffu, work);
-            scan_pos += 32;
-            ST_ACC(tm_scout);
-            continue;
+        const uint32_t work_tiles = __ballot_sync(0xffffffffu, work && r == 0);  // bit t: the t-th tile of this look
+        if (work_tiles == 0) continue;
+        // A frame that arrived on link l changes the values and l's mirror alike: it leaves nothing to say on l, and
+        // what rounding makes of it (or a cut-off that moved with the values) is not worth a frame back.  The link
+        // gets a frame when the tile changed here (its mark) or when another link brought something to pass on.
+        uint32_t flags = 0;
+        bool goes_out = false;
+        for (int l = 0; l < p.n_links; l++) {
+          const uint32_t here = __ballot_sync(0xffffffffu, avail != 0 && in.link == l) & same_tile;
+          const uint32_t outs = __ballot_sync(0xffffffffu, is_out && out.link == l) & same_tile;
+          const uint32_t full = __ballot_sync(0xffffffffu, is_out && out.link == l && !room) & same_tile;
+          const bool want = dirty != 0 || (in1 & same_tile & ~here) != 0;
+          const bool ok = want && outs != 0 && full == 0;
+          if (here) {
+            const uint32_t first = same_tile & ((here & (0u - here)) - 1u);
+            if (__popc(in1 & here) == 1 && (in2 & here) == 0)
+              flags |= uint32_t(1 + __popc(in1 & first) + __popc(in2 & first) + __popc(in3 & first)) << (kDescFrameShift + 5 * l);
           }
-          const int src = __ffs(pend) - 1;
-          pend &= pend - 1;
-          cur_tile = __shfl_sync(0xffffffffu, sc_tile, src);
-          cur_in_lo = __shfl_sync(0xffffffffu, sc_in_lo, src);
-          cur_in_hi = __shfl_sync(0xffffffffu, sc_in_hi, src);
-          cur_out_lo = __shfl_sync(0xffffffffu, sc_out_lo, src);
-          cur_out_hi = __shfl_sync(0xffffffffu, sc_out_hi, src);
-          cur_dirty = __shfl_sync(0xffffffffu, sc_dirty, src);
-          cur_a = 0;
+          flags |= (ok ? kDescTxOk << l : 0u) | (here ? kDescRxLink << l : 0u) | (want ? kDescTxWant << l : 0u);
+          goes_out |= ok && is_out && out.link == l;
         }
-        // ---- hand out step (cur_tile, link cur_a)
-        ST_T0();
-        __syncwarp();
-        ST_ACC(tm_pf);
         // A tile of a one-link replica that carries no mark is here only to receive: nothing is said on the link, so
-        // the values themselves are not needed (a third of the step's loads).
-        const bool no_values = L == 1 && cur_dirty == 0;
-        if (lane == 0) {
-          const int s = int(issued % kSlots);
-          uint8_t* slot = slots + size_t(s) * lay.slot_stride;
-          const int l = cur_a;
-          bool tx_any = false, tx_room = true, rx_link = false;
-          for (int r = 0; r < p.n_out; r++) {
-            if (p.out[r].link != l) continue;
-            tx_any = true;
-            tx_room &= (ctrl_byte(cur_out_lo, cur_out_hi, r) >> 6) != 0;
+        // the values themselves are not needed.
+        if (p.n_links == 1 && dirty == 0) flags |= kDescNoValues;
+        const uint32_t sends = __ballot_sync(0xffffffffu, goes_out) & same_tile;
+        const uint32_t pos = armed + __popc(work_tiles & ((1u << t) - 1u)), entry = pos % kBank;
+        if (work) {
+          if (r == 0) {
+            sh.desc[entry] = TileDesc{tile, flags, int(__popc(in1 & same_tile) + __popc(in2 & same_tile) + __popc(in3 & same_tile)), int(__popc(sends))};
+            sh.done[entry] = 0;
+            sh.dirty[entry] = dirty;
           }
-          // A frame that arrived on link l changes the values and l's mirror alike: it leaves nothing to say on l, and
-          // what rounding makes of it (or a cut-off that moved with the values) is not worth a frame back.  The link
-          // gets a frame when the tile changed here (its mark) or when another link brought something to pass on.
-          bool rx_other = false;
-          for (int r = 0; r < p.n_in; r++) {
-            if ((ctrl_byte(cur_in_lo, cur_in_hi, r) >> 6) == 0) continue;
-            if (p.in[r].link == l) rx_link = true; else rx_other = true;
+          if (pos == finished) {  // (the compute warps see to the later ones)
+            if (r == 0) {
+              if (!(flags & kDescNoValues)) bulk_prefetch_l2(p.values + size_t(tile) * kTile, kTile * 4);
+              for (int l = 0; l < p.n_links; l++) bulk_prefetch_l2(p.mirror[l] + size_t(tile) * kTile, kTile * 4);
+            }
+            for (uint32_t f = 0; f < avail; f++)
+              bulk_prefetch_l2(in.payload + (size_t((rx + f) & smask) * p.n_tiles + tile) * p.payload_bytes, uint32_t(p.payload_bytes));
           }
-          const bool tx_want = cur_dirty != 0 || rx_other;
-          const bool rx_any = ((cur_in_lo | cur_in_hi) & 0xc0c0c0c0u) != 0;
-          StepDesc d;
-          d.tile = cur_tile;
-          d.link = l;
-          d.flags = (cur_a == 0 ? kDescFirst : 0u) | (rx_any ? kDescRxAny : 0u) | (tx_any && tx_room && tx_want && p.do_tx ? kDescTxOk : 0u) |
-                    (rx_link ? kDescRxLink : 0u) | (tx_want ? kDescTxWant : 0u) | (no_values ? kDescNoValues : 0u) | (cur_a == L - 1 ? kDescLast : 0u);
-          d.sent = 0;
-          d.in_lo = cur_in_lo; d.in_hi = cur_in_hi; d.out_lo = cur_out_lo; d.out_hi = cur_out_hi;
-          desc[s] = d;
-          sflags[s] = 0;
-          __threadfence_block();
-          st_shared_volatile(armed, issued + 1u);  // the compute warps may read the descriptor from here on
-          uint32_t bytes = (cur_a == 0 && !no_values ? 2u : 1u) * uint32_t(kTileBytes);
-          if (cur_tile == p.stall_tile) bytes += 16;  // test hook: this barrier never completes
-          mbar_expect_tx(full + s, bytes);
+          const uint32_t before = same_tile & below;
+          uint64_t* list = &sh.frames[entry][__popc(in1 & before) + __popc(in2 & before) + __popc(in3 & before)];
+          for (uint32_t f = 0; f < avail; f++)
+            list[f] = reinterpret_cast<uint64_t>(in.payload + (size_t((rx + f) & smask) * p.n_tiles + tile) * p.payload_bytes) | uint32_t(in.link);
+          if (goes_out)
+            sh.slots[entry][__popc(sends & before)] =
+                reinterpret_cast<uint64_t>(out.payload_remote + (size_t(tx & smask) * p.n_tiles + tile) * p.payload_bytes) | uint32_t(out.link);
+          sh.rx[entry][r] = avail ? rx + avail : 0u;
+          sh.tx[entry][r] = goes_out ? tx + 1u : 0u;
+          sh.moved[entry][r] = uint8_t(avail | (goes_out ? 4u : 0u));
         }
+        // test hook: this tile is never handed to the compute warps, so the wait for it below runs out
+        const uint32_t stalled = __ballot_sync(0xffffffffu, work && tile == p.stall_tile && r == 0);
+        const uint32_t handed = stalled ? armed + __popc(work_tiles & ((1u << (__ffs(stalled) - 1)) - 1u)) : armed + __popc(work_tiles);
         __syncwarp();
-        {
-          // the step's copies, one per lane, issued by one instruction: lane 0 the link's mirror, lane 1 the values
-          const int s = int(issued % kSlots);
-          uint8_t* slot = slots + size_t(s) * lay.slot_stride;
-          if (lane == 0 || (lane == 1 && cur_a == 0 && !no_values)) {
-            const float* src = (lane == 0 ? p.mirror[cur_a] : p.values) + size_t(cur_tile) * kTile;
-            bulk_g2s(slot + (lane == 0 ? kTileBytes : 0), src, kTileBytes, full + s);
-          }
-        }
-        ST_STAMP(issued, 0);
-        issued++;
-        cur_a++;
-        if (cur_a == L) cur_tile = -1;
-        __syncwarp();
-        ST_ACC(tm_issue);
+        if (lane == 0) st_shared_release(&sh.armed, handed);
+        if (armed == finished) t_last = globaltimer_ns();
+        armed += __popc(work_tiles);
+        if (stalled) looked = my_count;
+        idle = 0;
         continue;
       }
-      // Nothing can be handed out right now: the steps whose stores have had time to land (all but the two most
-      // recent) go to the publisher warp.
-      if (pushed - handed > 2) {
-        ST_T0();
-        ST_CRUMB(g, 6);
-        bulk_wait_all_but_2();  // every lane for its own stores
-        hand_over(pushed - 2);
-        ST_ACC(tm_pubwait);
+      // ---- the next window's launch may move in on SMs that run dry: its tiles are others than this launch's
+      if (!handed_on && looked >= my_count && armed - finished <= 2u) {
+        asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+        handed_on = true;
       }
-      if (retired < issued) {
-        if (!retire(retired)) {
-          aborted = true;
-          break;
+      // ---- watch the compute warps
+      ST_CRUMB(g, 4);
+      const uint32_t at = finished + uint32_t(lane);
+      const uint32_t w = int32_t(armed - at) > 0 ? ld_shared_acquire(&sh.done[at % kBank]) : 0u;
+      const bool fail = __any_sync(0xffffffffu, w >= kDoneFailed);
+      const uint32_t ready = __ballot_sync(0xffffffffu, (w & kDoneWarps) == uint32_t(kComputeWarps) && w < kDoneFailed);
+      const uint32_t more = ready == 0xffffffffu ? 32u : uint32_t(__ffs(~ready) - 1);
+      if (more) {
+        finished += more;
+        t_last = globaltimer_ns();
+      }
+      const bool last = finished == armed && (looked >= my_count || yielded || aborted);
+      // ---- publish: when nothing is in hand, and earlier when half a bank has piled up, so that a neighbour does not
+      // wait for the end of a long launch.  Not more often: a system-scope fence takes 1.5 us on a quiet GPU and 3.9 us as
+      // soon as 37 or more SMs have one under way (measured: 2815 and 7400 cycles), and a fence that finds others under
+      // way waits for those first.  A fence behind every tile made the last one of a launch take 8 us.
+      if (finished != published && (finished == armed || finished - published >= uint32_t(kBank / 2))) {
+        asm volatile("fence.acq_rel.sys;" ::: "memory");  // the payloads are performed before the flags that announce them
+        for (; published != finished; published += min(finished - published, uint32_t(at_once))) {
+          if (int32_t(finished - published) <= t) continue;
+          const uint32_t entry = (published + uint32_t(t)) % kBank;
+          const TileDesc d = sh.desc[entry];
+          const uint32_t done = sh.done[entry], moved = sh.moved[entry][r];
+          if ((moved & 4u) && ((done >> (kDoneNonsilentShift + 4 * out.link)) & 0xfu)) {
+            const uint32_t seq = sh.tx[entry][r];
+            st_relaxed_sys(out.flags_remote + size_t((seq - 1u) & smask) * p.n_tiles + d.tile, seq);
+            st_cg_u32(out.tx_seq + d.tile, seq);
+            n_tx++;
+          }
+          if (moved & 3u) {
+            const uint32_t seq = sh.rx[entry][r];
+            st_cg_u32(in.rx_seq + d.tile, seq);
+            st_relaxed_sys(in.credit_remote + d.tile, seq);
+            n_rx += moved & 3u;
+          }
+          if (r == 0) {
+            bool left = false;
+            for (int l = 0; l < p.n_links; l++) {
+              if (((done >> (kDoneNonsilentShift + 4 * l)) & 0xfu) == 0) continue;
+              left = true;  // more may be left to say (or nothing could be said at all)
+              if (!(d.flags & (kDescTxOk << l)) && p.do_tx) n_blocked++;
+            }
+            if (left) {
+              st_cg_u32(p.tile_state + d.tile, 1u);
+              n_pending++;
+            }
+            n_done++;
+          }
         }
-        retired++;
+        __syncwarp();
         continue;
       }
-      break;  // every tile looked at, every step retired
+      if (last) break;
+      if (more) continue;
+      idle++;
+      const bool late = __any_sync(0xffffffffu, fail || globaltimer_ns() - t_last > 2 * limit_ns);
+      if (late) {
+        if (aborted) break;  // the tiles that had been started did not finish either
+        aborted = true;
+      } else if (yielded || aborted || (idle & 7u) != 0 || !update_waiting()) {
+        __nanosleep(40);
+        continue;
+      } else {
+        yielded = true;
+      }
+      // An update is waiting for the SMs this kernel holds, or a wait ran out: no more tiles are started.  Those that
+      // were looked at but not started get their change marks back, everything else about them is untouched.
+      uint32_t started = 0;
+      if (lane == 0) started = atomicOr(&sh.claim, kClaimStop) & ~kClaimStop;
+      started = __shfl_sync(0xffffffffu, started, 0);
+      for (uint32_t c = started + uint32_t(lane); int32_t(armed - c) > 0; c += 32)
+        if (sh.dirty[c % kBank]) st_cg_u32(p.tile_state + sh.desc[c % kBank].tile, 1u);
+      armed = started;
+      t_last = globaltimer_ns();
     }
-    if (aborted) break;
-    // ---- end of the sweep: every store has landed and is published before the tiles are looked at again
-    ST_CRUMB(g, 7);
-    bulk_wait_all();
-    __syncwarp();
-    hand_over(pushed);
-    {
-      ST_T0();
-      ST_CRUMB(g, 8);
-      if (!wait_published(pushed)) aborted = true;  // the next sweep reads the counters the publisher advances
-      ST_ACC(tm_pub);
-    }
-    ST_CRUMB(g, 9);
-    __syncwarp();
     if (aborted) break;
     n_sweeps++;
-    if (n_done == done_before && sweep + 1 < p.sweeps) __nanosleep(1000);
+    if (armed == armed_before && sweep + 1 < p.sweeps) __nanosleep(1000);
   }
-
+  if (lane == 0) atomicOr(&sh.claim, kClaimStop);  // the compute warps leave
   if (aborted) {
-    // Stop the group.  The compute warps leave on the abort flag (or on the exit descriptor); copies that are still
-    // on their way get a bounded chance to land before the CTA's shared memory is released; what was stored is
-    // published; every tile of the group is marked for another visit.
-    if (lane == 0) st_shared_volatile(abort_flag, 1u);
-    __syncwarp();
-    for (uint32_t c = retired; c < issued; c++)
-      (void)__all_sync(0xffffffffu, mbar_wait_bounded(full + int(c % kSlots), (c / kSlots) & 1u, limit_ns));
-    bulk_wait_all();
-    __syncwarp();
-    hand_over(pushed);
-    (void)wait_published(pushed);
     for (int j = lane; j < my_count; j += 32) st_cg_u32(p.tile_state + gid + j * gstride, 1u);
     if (lane == 0) {
       atomicOr(reinterpret_cast<unsigned long long*>(p.status + kDsErrors), (unsigned long long)kErrBarrierTimeout);
       atomicAdd(reinterpret_cast<unsigned long long*>(p.status + kDsWaitTimeouts), 1ull);
     }
   }
-#ifdef ST_ROUND_TIMING
-  if (blockIdx.x == 0 && g == 0 && lane == 0)
-    printf("io: total %lld cycles, wait done %lld, wait read %lld, wait stores %lld, fence+publish %lld, scout %lld, prefetch %lld, issue(incl prefetch) %lld, retire(incl read wait) %lld, steps %u\n",
-           clock64() - tm_io0, tm_done, tm_read, tm_pubwait, tm_pub, tm_scout, tm_pf, tm_issue, tm_store, issued);
-#endif
+  // A launch that was let in early ends after the one before it, so that what follows in the stream finds both complete.
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+  n_done = __reduce_add_sync(0xffffffffu, n_done);
+  n_tx = __reduce_add_sync(0xffffffffu, n_tx);
+  n_rx = __reduce_add_sync(0xffffffffu, n_rx);
+  n_blocked = __reduce_add_sync(0xffffffffu, n_blocked);
+  n_pending = __reduce_add_sync(0xffffffffu, n_pending);
   if (lane == 0) {
-    // tell the compute warps that the launch is over (the slot of step `issued` is free: all earlier steps are retired
-    // or abandoned)
-    const int s = int(issued % kSlots);
-    StepDesc d;
-    d.tile = 0; d.link = 0; d.flags = kDescExit; d.sent = 0;
-    d.in_lo = d.in_hi = d.out_lo = d.out_hi = 0;
-    if (!aborted) {  // (after an abort the compute warps leave on the abort flag)
-      desc[s] = d;
-      __threadfence_block();
-      st_shared_volatile(armed, issued + 1u);
-      mbar_arrive(full + s);
-    }
-    st_shared_volatile(pub_exit, 1u);
     ST_CRUMB(g, 10);
-    if (yielded) atomicAdd(reinterpret_cast<unsigned long long*>(p.status + kDsYields), 1ull);
-    if (n_done) atomicAdd(reinterpret_cast<unsigned long long*>(p.status + kDsTilesProcessed), n_done);
-    if (n_tx) atomicAdd(reinterpret_cast<unsigned long long*>(p.status + kDsFramesSent), n_tx);
-    if (n_rx) atomicAdd(reinterpret_cast<unsigned long long*>(p.status + kDsFramesRecv), n_rx);
-    if (n_blocked) atomicAdd(reinterpret_cast<unsigned long long*>(p.status + kDsBlockedNoCredit), n_blocked);
-    if (n_done) atomicAdd(reinterpret_cast<unsigned long long*>(launch_words + kDlWork), n_done);
-    if (n_pending) atomicAdd(reinterpret_cast<unsigned long long*>(launch_words + kDlPending), n_pending);
+    auto count = [&](uint64_t* w, unsigned long long by) {
+      if (by) atomicAdd(reinterpret_cast<unsigned long long*>(w), by);
+    };
+    count(p.status + kDsYields, yielded ? 1 : 0);
+    count(p.status + kDsTilesProcessed, n_done);
+    count(p.status + kDsFramesSent, n_tx);
+    count(p.status + kDsFramesRecv, n_rx);
+    count(p.status + kDsBlockedNoCredit, n_blocked);
+    count(launch_words + kDlWork, n_done);
+    count(launch_words + kDlPending, n_pending);
     if (blockIdx.x == 0 && g == 0) {
-      const unsigned long long r = atomicAdd(reinterpret_cast<unsigned long long*>(p.status + kDsSweeps), n_sweeps);
+      count(p.status + kDsSweeps, n_sweeps);
       uint64_t* rec = p.status + kDsTrace + (uint64_t(p.round) % kTraceEntries) * kTraceWords;  // trace ring, read by stats()
       rec[0] = globaltimer_ns();
       rec[1] = uint64_t(p.round);
       rec[2] = n_done;
-      rec[3] = p.status[kDsFramesSent];
-      (void)r;
+      rec[3] = sent_before + n_tx;
     }
   }
+}
+
+}  // namespace
+
+template <int Q, int kGroups, bool kOneLink>
+__global__ void __launch_bounds__(kGroups * kGroupThreads, 1) round_kernel(const __grid_constant__ RoundParams p) {
+  __shared__ GroupShared shared[kGroups];
+  const int g = int(threadIdx.x) / kGroupThreads, warp = (int(threadIdx.x) % kGroupThreads) >> 5, lane = threadIdx.x & 31;
+  if (threadIdx.x < kGroups) {
+    GroupShared& sh = shared[threadIdx.x];
+    sh.armed = 0;
+    sh.claim = 0;
+    mbar_init(&sh.gsync, kComputeWarps);
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+  }
+  __syncthreads();  // the only CTA-wide barrier: from here on the groups, and the two kinds of warp, run on their own
+  if (warp == kComputeWarps) service_warp(p, shared[g], g, kGroups, lane);
+  else compute_warp<Q, kOneLink>(p, shared[g], warp, lane);
 }
 
 // ----------------------------------------------------------------------------------------------
 // Taking frames back.  When a neighbour is lost, the frames it never acknowledged (sequence numbers from its last
 // credit up to what was sent) are still in its ring, which stays mapped here; their steps come off the mirror again,
 // so that what they said counts as not yet told (the TCP edges do the same with a frame whose write fails).
-// One CTA per tile, thread t its 32 elements, the same element order as the round kernel.
+// One CTA per tile, warp w its 512 elements, the same lane layout as the round kernel.
 // ----------------------------------------------------------------------------------------------
 template <int Q>
-__global__ void __launch_bounds__(kGroupThreads) unsend_kernel(float* __restrict__ mirror, const uint8_t* __restrict__ payload,
-                                                               uint32_t* __restrict__ tx_seq, const uint32_t* __restrict__ credit,
-                                                               int n_tiles, int ring_slots, int pb, int log2_block, int64_t n,
-                                                               unsigned long long* __restrict__ taken_back) {
-  const int tile = blockIdx.x, t = threadIdx.x, sw = t & 7, tpb = log2_block - 5;
+__global__ void __launch_bounds__(kComputeWarps * 32) unsend_kernel(float* __restrict__ mirror, const uint8_t* __restrict__ payload,
+                                                                    uint32_t* __restrict__ tx_seq, const uint32_t* __restrict__ credit,
+                                                                    int n_tiles, int ring_slots, int pb, int log2_block, int64_t n,
+                                                                    unsigned long long* __restrict__ taken_back) {
+  const int tile = blockIdx.x, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const uint32_t c = ld_acquire_sys(credit + tile), tx = ld_cg_u32(tx_seq + tile);
   const uint32_t count = tx - c;
   if (count == 0 || count > uint32_t(ring_slots)) return;
-  const int64_t left = n - (int64_t(tile) * kTile + int64_t(t) * 32);
-  const uint32_t vmask = left >= 32 ? 0xffffffffu : (left <= 0 ? 0u : ((1u << int(left)) - 1u));
-  const bool masked = (Q == 1) && left < 32;
-  float4 acc[8];
+  const int in_tile = warp * kWarpElems + lane * 4, left = int(min(int64_t(kTile), n - int64_t(tile) * kTile)) - in_tile;
+  Piece acc[kPieces];
 #pragma unroll
-  for (int q = 0; q < 8; q++) acc[q] = make_float4(0.f, 0.f, 0.f, 0.f);
+  for (int i = 0; i < kPieces; i++) acc[i] = {0ull, 0ull};
   for (uint32_t f = 0; f < count; f++) {
-    const uint8_t* fp = payload + (size_t((c + f) & uint32_t(ring_slots - 1)) * n_tiles + tile) * pb;
-    uint32_t w[Q], code;
-    load_frame<Q>(fp, t, tpb, w, code);
-    if (masked) add_frame<Q, true>(acc, w, code, sw, vmask); else add_frame<Q, false>(acc, w, code, sw, vmask);
-  }
-  float4* k4 = reinterpret_cast<float4*>(mirror + size_t(tile) * kTile) + t * 8;
+    FrameRegs fr;
+    load_frame<Q>(payload + (size_t((c + f) & uint32_t(ring_slots - 1)) * n_tiles + tile) * pb, warp, lane, log2_block, fr);
 #pragma unroll
-  for (int q = 0; q < 8; q++) {
-    float4 k = k4[q ^ sw];
-    k.x = __fsub_rn(k.x, acc[q].x); k.y = __fsub_rn(k.y, acc[q].y); k.z = __fsub_rn(k.z, acc[q].z); k.w = __fsub_rn(k.w, acc[q].w);
-    k4[q ^ sw] = k;
+    for (int i = 0; i < kPieces; i++) add4(acc[i], frame_steps<Q>(fr.w[i], fr.code(i), Q == 1 ? valid4(left, i) : 0xfu));
+  }
+  float* const kp = mirror + size_t(tile) * kTile + in_tile;
+#pragma unroll
+  for (int i = 0; i < kPieces; i++) {
+    const Piece k = load_piece(kp + i * 128);
+    store_piece(kp + i * 128, {sub2(k.a, acc[i].a), sub2(k.b, acc[i].b)});
   }
   __syncthreads();
-  if (t == 0) {
+  if (threadIdx.x == 0) {
     st_cg_u32(tx_seq + tile, c);
     atomicAdd(taken_back, (unsigned long long)count);
   }
@@ -1216,10 +991,10 @@ int launch_unsend(float* mirror, const uint8_t* payload_remote, uint32_t* tx_seq
   cudaStream_t s = static_cast<cudaStream_t>(stream_v);
   unsigned long long* tb = reinterpret_cast<unsigned long long*>(taken_back);
   switch (bits) {
-    case 1: unsend_kernel<1><<<n_tiles, kGroupThreads, 0, s>>>(mirror, payload_remote, tx_seq, credit, n_tiles, ring_slots, payload_bytes, log2_block, n, tb); break;
-    case 2: unsend_kernel<2><<<n_tiles, kGroupThreads, 0, s>>>(mirror, payload_remote, tx_seq, credit, n_tiles, ring_slots, payload_bytes, log2_block, n, tb); break;
-    case 4: unsend_kernel<4><<<n_tiles, kGroupThreads, 0, s>>>(mirror, payload_remote, tx_seq, credit, n_tiles, ring_slots, payload_bytes, log2_block, n, tb); break;
-    case 8: unsend_kernel<8><<<n_tiles, kGroupThreads, 0, s>>>(mirror, payload_remote, tx_seq, credit, n_tiles, ring_slots, payload_bytes, log2_block, n, tb); break;
+    case 1: unsend_kernel<1><<<n_tiles, kComputeWarps * 32, 0, s>>>(mirror, payload_remote, tx_seq, credit, n_tiles, ring_slots, payload_bytes, log2_block, n, tb); break;
+    case 2: unsend_kernel<2><<<n_tiles, kComputeWarps * 32, 0, s>>>(mirror, payload_remote, tx_seq, credit, n_tiles, ring_slots, payload_bytes, log2_block, n, tb); break;
+    case 4: unsend_kernel<4><<<n_tiles, kComputeWarps * 32, 0, s>>>(mirror, payload_remote, tx_seq, credit, n_tiles, ring_slots, payload_bytes, log2_block, n, tb); break;
+    case 8: unsend_kernel<8><<<n_tiles, kComputeWarps * 32, 0, s>>>(mirror, payload_remote, tx_seq, credit, n_tiles, ring_slots, payload_bytes, log2_block, n, tb); break;
     default: return int(cudaErrorInvalidValue);
   }
   return int(cudaGetLastError());
@@ -1228,29 +1003,33 @@ int launch_unsend(float* mirror, const uint8_t* payload_remote, uint32_t* tx_seq
 // ----------------------------------------------------------------------------------------------
 // launcher
 // ----------------------------------------------------------------------------------------------
-template <int Q, int G, int S>
+template <int Q, int kGroups>
 static int launch_round_t(const RoundParams& p, int ctas, cudaStream_t stream) {
-  const int smem = smem_layout(p.payload_bytes, G, S).total;
-  static int configured_for = -1;  // per instantiation
-  if (configured_for < smem) {
-    cudaError_t e = cudaFuncSetAttribute(round_kernel<Q, G, S>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-    if (e != cudaSuccess) return int(e);
-    configured_for = smem;
-  }
-  round_kernel<Q, G, S><<<ctas, G * (kGroupThreads + 32) + 32, smem, stream>>>(p);
-  return int(cudaGetLastError());
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = dim3(ctas);
+  cfg.blockDim = dim3(kGroups * kGroupThreads);
+  cfg.stream = stream;
+  // Every window but a cycle's first may start while the window before it is running out: the two have no tile in common.
+  // (The first one clears counters that the launch before it may still add to.)
+  cudaLaunchAttribute early{};
+  early.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  early.val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = &early;
+  cfg.numAttrs = p.follows_window ? 1 : 0;
+  return int(p.n_links == 1 ? cudaLaunchKernelEx(&cfg, round_kernel<Q, kGroups, true>, p) : cudaLaunchKernelEx(&cfg, round_kernel<Q, kGroups, false>, p));
 }
+
+// Groups of a CTA.  A replica with one ring pair, or with one per link, is bound by HBM and by the length of a tile's
+// chain of operations: two groups with 96 registers a thread are enough and were 2 to 8 % faster than three with 72.
+// Several rings on one link (a mesh group) mean several frames to decode per tile, which more warps hide: 51 against
+// 55 us for seven rings and 4 Mi elements.  Shape 0 asks for three whatever the rings.
+int round_groups(int shape, int n_links, int n_in) { return shape == 0 || (n_links == 1 && n_in > 1) ? 3 : 2; }
 
 template <int Q>
 static int launch_round_q(const RoundParams& p, int shape, int ctas, cudaStream_t stream) {
-  switch (shape) {
-    case 0: return launch_round_t<Q, 3, 2>(p, ctas, stream);
-    case 1: return launch_round_t<Q, 2, 3>(p, ctas, stream);
-    default: return int(cudaErrorInvalidValue);
-  }
+  if (shape != 0 && shape != 1) return int(cudaErrorInvalidValue);
+  return round_groups(shape, p.n_links, p.n_in) == 3 ? launch_round_t<Q, 3>(p, ctas, stream) : launch_round_t<Q, 2>(p, ctas, stream);
 }
-
-int round_shape_groups(int shape) { return shape == 0 ? 3 : 2; }
 
 int launch_round(const RoundParams& p, int shape, int ctas, void* stream_v) {
   cudaStream_t stream = static_cast<cudaStream_t>(stream_v);

@@ -74,6 +74,7 @@ struct RoundParams {
   int32_t tile_begin, tile_count; // the window of the tensor this launch covers
   int32_t parity;                // which half of the per-cycle counters this launch uses (a cycle = one pass over all windows)
   int32_t zero_other;            // first launch of a cycle: clear the other half for the cycle after this one
+  int32_t follows_window;        // the launch before this one in the stream is the window before this one, of the same cycle
   int32_t do_rx, do_tx;          // receiver-only / sender-only launches
   int32_t sweeps;                // passes over the tensor in this launch (>= 1)
   uint32_t wait_ns;              // upper bound of every wait on one of the kernel's own copies
@@ -124,10 +125,10 @@ enum StatusWord : int {
 };
 
 // Launchers.  `stream` is a cudaStream_t passed as void*.  Return a cudaError_t as int.
-// `shape` picks the CTA's make-up: 0 = 3 groups x 2 staging slots, 1 = 2 groups x 3 slots (one CTA per SM either way).
-// A group is 4 compute warps and one I/O warp; a CTA has one more warp that publishes flags and credits.
+// `shape` picks the CTA's make-up: 1 = two or three groups by the replica's rings, 0 = three groups (one CTA per SM
+// either way).  A group is eight compute warps and one service warp.
 int launch_round(const RoundParams& p, int shape, int ctas, void* stream);
-int round_shape_groups(int shape);
+int round_groups(int shape, int n_links, int n_in);
 // Takes back the frames of one out-ring that the receiver never acknowledged: their steps are subtracted from the
 // link's mirror and the ring's send counters fall back to the credits.  *taken_back (device) counts the tile-frames.
 int launch_unsend(float* mirror, const uint8_t* payload_remote, uint32_t* tx_seq, const uint32_t* credit, int n_tiles, int ring_slots,
