@@ -39,6 +39,8 @@ class _Range:
 
 
 def _check(t: torch.Tensor, n: int, device: torch.device, what: str) -> torch.Tensor:
+    if isinstance(t, torch.Tensor) and t.dtype is torch.float32 and t.numel() == n and t.device == device and t.is_contiguous():
+        return t
     if not isinstance(t, torch.Tensor):
         raise TypeError(f"{what}: expected a torch.Tensor, got {type(t).__name__}")
     if t.dtype != torch.float32:
@@ -65,22 +67,34 @@ class SharedTensor:
     # --- reference API ---------------------------------------------------------------------
     def copyToTensor(self, t: torch.Tensor) -> torch.Tensor:
         """``t <- values`` (src/sharedtensor.c:435-446).  Per-element consistent snapshot."""
-        with _Range(self.cfg.nvtx, "sharedtensor.copyToTensor"):
-            self._b.copy_to(_check(t, self._n, self._b.device, "copyToTensor"))
+        b = self._b
+        if self.cfg.nvtx:
+            with _Range(True, "sharedtensor.copyToTensor"):
+                b.copy_to(_check(t, self._n, b.device, "copyToTensor"))
+        else:
+            b.copy_to(_check(t, self._n, b.device, "copyToTensor"))
         return t
 
     def addFromTensor(self, delta: torch.Tensor) -> None:
         """``values += delta`` locally; the change reaches every other replica asynchronously
         (src/sharedtensor.c:334-344, 448-453)."""
-        with _Range(self.cfg.nvtx, "sharedtensor.addFromTensor"):
-            self._b.add(_check(delta, self._n, self._b.device, "addFromTensor"))
+        b = self._b
+        if self.cfg.nvtx:
+            with _Range(True, "sharedtensor.addFromTensor"):
+                b.add(_check(delta, self._n, b.device, "addFromTensor"))
+        else:
+            b.add(_check(delta, self._n, b.device, "addFromTensor"))
 
     # --- additions -------------------------------------------------------------------------
     def pushUpdate(self, new: torch.Tensor, old: torch.Tensor) -> None:
         """``values += new - old`` in one pass (the README's ``addFromTensor(new:csub(current))``)."""
-        dev = self._b.device
-        with _Range(self.cfg.nvtx, "sharedtensor.pushUpdate"):
-            self._b.sub_add(_check(new, self._n, dev, "pushUpdate(new)"), _check(old, self._n, dev, "pushUpdate(old)"))
+        b = self._b
+        n, dev = self._n, b.device
+        if self.cfg.nvtx:
+            with _Range(True, "sharedtensor.pushUpdate"):
+                b.sub_add(_check(new, n, dev, "pushUpdate(new)"), _check(old, n, dev, "pushUpdate(old)"))
+        else:
+            b.sub_add(_check(new, n, dev, "pushUpdate(new)"), _check(old, n, dev, "pushUpdate(old)"))
 
     def copyToTensorBF16(self, t: torch.Tensor) -> torch.Tensor:
         """``t <- bf16(values)`` in one pass (GPU replicas; bf16 compute over fp32 master weights)."""

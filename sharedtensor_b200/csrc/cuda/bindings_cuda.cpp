@@ -44,19 +44,19 @@ PYBIND11_MODULE(_cuda, m) {
 
   // ---- raw kernels ----
   m.def("snapshot_f32", [](uintptr_t v, uintptr_t out, int64_t n, uintptr_t s) {
-    ck(launch_snapshot_f32(ptr<float>(v), ptr<float>(out), n, strm(s)), "snapshot_f32");
+    ck(launch_snapshot_f32(ptr<float>(v), ptr<float>(out), n, UpdateMarks{}, strm(s)), "snapshot_f32");
   });
   m.def("snapshot_bf16", [](uintptr_t v, uintptr_t out, int64_t n, uintptr_t s) {
-    ck(launch_snapshot_bf16(ptr<float>(v), ptr<void>(out), n, strm(s)), "snapshot_bf16");
+    ck(launch_snapshot_bf16(ptr<float>(v), ptr<void>(out), n, UpdateMarks{}, strm(s)), "snapshot_bf16");
   });
   m.def("add", [](uintptr_t v, uintptr_t d, int64_t n, bool atomic, uintptr_t s) {
-    ck(launch_add(ptr<float>(v), ptr<float>(d), n, atomic, strm(s)), "add");
+    ck(launch_add(ptr<float>(v), ptr<float>(d), n, atomic, UpdateMarks{}, strm(s)), "add");
   });
   m.def("sub_add", [](uintptr_t v, uintptr_t a, uintptr_t b, int64_t n, bool atomic, uintptr_t s) {
-    ck(launch_sub_add(ptr<float>(v), ptr<float>(a), ptr<float>(b), n, atomic, strm(s)), "sub_add");
+    ck(launch_sub_add(ptr<float>(v), ptr<float>(a), ptr<float>(b), n, atomic, UpdateMarks{}, strm(s)), "sub_add");
   });
   m.def("add_scaled_bf16", [](uintptr_t v, uintptr_t g, float alpha, int64_t n, bool atomic, uintptr_t s) {
-    ck(launch_add_scaled_bf16(ptr<float>(v), ptr<void>(g), alpha, n, atomic, strm(s)), "add_scaled_bf16");
+    ck(launch_add_scaled_bf16(ptr<float>(v), ptr<void>(g), alpha, n, atomic, UpdateMarks{}, strm(s)), "add_scaled_bf16");
   });
   m.def("round_smem_bytes", &round_smem_bytes);
   m.def("table_scales_scratch_doubles", &table_scales_scratch_doubles);

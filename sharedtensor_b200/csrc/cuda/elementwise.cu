@@ -44,197 +44,206 @@ inline bool aligned16(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 
 }  // namespace
 
 // ---------------------------------------------------------------------------------------------
-// snapshot
+// snapshot, add / sub_add / add_scaled_bf16
+//
+// All of these are bound by HBM for large tensors and by calls and launches for small ones, so each is ONE launch: the
+// ragged end is handled inside, the updates set the change marks themselves and the last CTA takes back the request for
+// SMs (see GpuReplica::ask_for_sms).  A CTA takes one 4096-element tile at a time, four 16-byte accesses per thread in
+// flight and eight CTAs per SM.  User tensors that are not 16-byte aligned go element by element, eight coalesced accesses
+// per thread in flight.
 // ---------------------------------------------------------------------------------------------
-__global__ void __launch_bounds__(kEwThreads) snapshot_f32_vec(const float4* __restrict__ src, float4* __restrict__ dst, int64_t n4) {
-  int64_t i = int64_t(blockIdx.x) * kEwThreads + threadIdx.x;
-  const int64_t stride = int64_t(gridDim.x) * kEwThreads;
-  // four independent 16-byte loads in flight per thread
-  for (; i + 3 * stride < n4; i += 4 * stride) {
-    float4 a = src[i], b = src[i + stride], c = src[i + 2 * stride], d = src[i + 3 * stride];
-    __stcs(dst + i, a);
-    __stcs(dst + i + stride, b);
-    __stcs(dst + i + 2 * stride, c);
-    __stcs(dst + i + 3 * stride, d);
-  }
-  for (; i < n4; i += stride) __stcs(dst + i, src[i]);
-}
-__global__ void snapshot_f32_scalar(const float* __restrict__ src, float* __restrict__ dst, int64_t begin, int64_t n) {
-  int64_t i = begin + int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
-  const int64_t stride = int64_t(gridDim.x) * blockDim.x;
-  for (; i < n; i += stride) dst[i] = src[i];
-}
-__global__ void __launch_bounds__(kEwThreads) snapshot_bf16_vec(const float4* __restrict__ src, uint2* __restrict__ dst, int64_t n4) {
-  int64_t i = int64_t(blockIdx.x) * kEwThreads + threadIdx.x;
-  const int64_t stride = int64_t(gridDim.x) * kEwThreads;
-  for (; i < n4; i += stride) {
-    float4 a = src[i];
-    __nv_bfloat162 lo = __floats2bfloat162_rn(a.x, a.y), hi = __floats2bfloat162_rn(a.z, a.w);
-    uint2 o;
-    o.x = *reinterpret_cast<uint32_t*>(&lo);
-    o.y = *reinterpret_cast<uint32_t*>(&hi);
-    dst[i] = o;
-  }
-}
-__global__ void snapshot_bf16_scalar(const float* __restrict__ src, __nv_bfloat16* __restrict__ dst, int64_t begin, int64_t n) {
-  int64_t i = begin + int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
-  const int64_t stride = int64_t(gridDim.x) * blockDim.x;
-  for (; i < n; i += stride) dst[i] = __float2bfloat16_rn(src[i]);
-}
+namespace {
 
-int launch_snapshot_f32(const float* values, float* out, int64_t n, void* stream_v) {
-  cudaStream_t s = static_cast<cudaStream_t>(stream_v);
-  int64_t n4 = aligned16(out) && aligned16(values) ? n / 4 : 0;
-  if (n4) snapshot_f32_vec<<<ew_blocks(n4 / 4 + 1), kEwThreads, 0, s>>>(reinterpret_cast<const float4*>(values), reinterpret_cast<float4*>(out), n4);
-  if (n4 * 4 < n) snapshot_f32_scalar<<<ew_blocks(n - n4 * 4), kEwThreads, 0, s>>>(values, out, n4 * 4, n);
-  return int(cudaGetLastError());
-}
-int launch_snapshot_bf16(const float* values, void* out, int64_t n, void* stream_v) {
-  cudaStream_t s = static_cast<cudaStream_t>(stream_v);
-  bool al = aligned16(values) && (reinterpret_cast<uintptr_t>(out) & 7) == 0;
-  int64_t n4 = al ? n / 4 : 0;
-  if (n4) snapshot_bf16_vec<<<ew_blocks(n4), kEwThreads, 0, s>>>(reinterpret_cast<const float4*>(values), reinterpret_cast<uint2*>(out), n4);
-  if (n4 * 4 < n) snapshot_bf16_scalar<<<ew_blocks(n - n4 * 4), kEwThreads, 0, s>>>(values, static_cast<__nv_bfloat16*>(out), n4 * 4, n);
-  return int(cudaGetLastError());
-}
+constexpr int kVecs = kTile / 4 / kEwThreads;  // 16-byte pieces of a thread
+constexpr int kElems = 8;                      // single elements of a thread in flight
 
-// ---------------------------------------------------------------------------------------------
-// add / sub_add
-// ---------------------------------------------------------------------------------------------
-template <bool SUB, bool ATOMIC>
-__global__ void __launch_bounds__(kEwThreads) add_vec(float4* __restrict__ values, const float4* __restrict__ a, const float4* __restrict__ b,
-                                                      int64_t n4) {
-  int64_t i = int64_t(blockIdx.x) * kEwThreads + threadIdx.x;
-  const int64_t stride = int64_t(gridDim.x) * kEwThreads;
-  // four independent 16-byte streams per thread and iteration
-  for (; i + 3 * stride < n4; i += 4 * stride) {
-    float4 d[4], v[4];
-#pragma unroll
-    for (int u = 0; u < 4; u++) d[u] = ldg_stream(a + i + u * stride);
-    if (SUB) {
-#pragma unroll
-      for (int u = 0; u < 4; u++) {
-        float4 o = ldg_stream(b + i + u * stride);
-        d[u].x -= o.x; d[u].y -= o.y; d[u].z -= o.z; d[u].w -= o.w;
-      }
+// What is left to do when a CTA's part of an update or of a snapshot is done.
+__device__ __forceinline__ void finish(const UpdateMarks& m, int64_t n_tiles) {
+  if (m.tile_state != nullptr) {
+    // Marks after the data: the CTA's reductions come before the barrier, the barrier before the fence (which is
+    // cumulative), the fence before the marks.
+    __syncthreads();
+    if (threadIdx.x < 32) {
+      __threadfence();
+      for (int64_t t = blockIdx.x + int64_t(threadIdx.x) * gridDim.x; t < n_tiles; t += 32 * int64_t(gridDim.x)) __stcg(m.tile_state + t, 1u);
     }
-    if (ATOMIC) {
+  }
+  if (m.yield_word != nullptr && threadIdx.x == 0) {
+    if (atomicAdd(m.ticket, 1u) == gridDim.x - 1) {
+      *m.ticket = 0u;
+      *reinterpret_cast<volatile uint32_t*>(m.yield_word) = 0u;
+    }
+  }
+}
+
+inline int tile_blocks(int64_t n, int per_sm = 8) {
+  const int64_t tiles = (n + kTile - 1) / kTile;
+  return int(tiles < 148 * per_sm ? tiles : 148 * per_sm);
+}
+
+struct Bf16x4 {
+  uint32_t lo, hi;
+};
+__device__ __forceinline__ Bf16x4 to_bf16(float4 v) {
+  __nv_bfloat162 lo = __floats2bfloat162_rn(v.x, v.y), hi = __floats2bfloat162_rn(v.z, v.w);
+  return {*reinterpret_cast<uint32_t*>(&lo), *reinterpret_cast<uint32_t*>(&hi)};
+}
+__device__ __forceinline__ float4 from_bf16(uint2 raw) {
+  const float2 a = __bfloat1622float2(*reinterpret_cast<__nv_bfloat162*>(&raw.x)), b = __bfloat1622float2(*reinterpret_cast<__nv_bfloat162*>(&raw.y));
+  return make_float4(a.x, a.y, b.x, b.y);
+}
+
+template <class T, bool VEC>
+__global__ void __launch_bounds__(kEwThreads, 8) snapshot_kernel(const float* __restrict__ src, T* __restrict__ dst, int64_t n, UpdateMarks m) {
+  constexpr bool kBf16 = sizeof(T) == 2;
+  const int64_t n_tiles = (n + kTile - 1) / kTile;
+  for (int64_t tile = blockIdx.x; tile < n_tiles; tile += gridDim.x) {
+    if (VEC && (tile + 1) * kTile <= n) {
+      const float4* s4 = reinterpret_cast<const float4*>(src + tile * kTile) + threadIdx.x;
+      float4 v[kVecs];
 #pragma unroll
-      for (int u = 0; u < 4; u++) red_add_v4(reinterpret_cast<float*>(values + i + u * stride), d[u]);
+      for (int i = 0; i < kVecs; i++) v[i] = s4[i * kEwThreads];
+#pragma unroll
+      for (int i = 0; i < kVecs; i++) {
+        if constexpr (kBf16) {
+          const Bf16x4 o = to_bf16(v[i]);
+          __stcs(reinterpret_cast<uint2*>(dst + tile * kTile) + threadIdx.x + i * kEwThreads, make_uint2(o.lo, o.hi));
+        } else {
+          __stcs(reinterpret_cast<float4*>(dst + tile * kTile) + threadIdx.x + i * kEwThreads, v[i]);
+        }
+      }
     } else {
+      const int left = int(min(int64_t(kTile), n - tile * kTile));
+      for (int e0 = threadIdx.x; e0 < left; e0 += kElems * kEwThreads) {
+        float v[kElems];
 #pragma unroll
-      for (int u = 0; u < 4; u++) v[u] = values[i + u * stride];
+        for (int i = 0; i < kElems; i++)
+          if (e0 + i * kEwThreads < left) v[i] = src[tile * kTile + e0 + i * kEwThreads];
 #pragma unroll
-      for (int u = 0; u < 4; u++) {
-        v[u].x += d[u].x; v[u].y += d[u].y; v[u].z += d[u].z; v[u].w += d[u].w;
-        values[i + u * stride] = v[u];
+        for (int i = 0; i < kElems; i++) {
+          if (e0 + i * kEwThreads >= left) continue;
+          if constexpr (kBf16) dst[tile * kTile + e0 + i * kEwThreads] = __float2bfloat16_rn(v[i]);
+          else dst[tile * kTile + e0 + i * kEwThreads] = v[i];
+        }
       }
     }
   }
-  for (; i < n4; i += stride) {
-    float4 d0 = ldg_stream(a + i);
-    if (SUB) {
-      float4 o0 = ldg_stream(b + i);
-      d0.x -= o0.x; d0.y -= o0.y; d0.z -= o0.z; d0.w -= o0.w;
-    }
-    if (ATOMIC) {
-      red_add_v4(reinterpret_cast<float*>(values + i), d0);
-    } else {
-      float4 v0 = values[i];
-      v0.x += d0.x; v0.y += d0.y; v0.z += d0.z; v0.w += d0.w;
-      values[i] = v0;
-    }
-  }
-}
-template <bool SUB, bool ATOMIC>
-__global__ void add_scalar(float* __restrict__ values, const float* __restrict__ a, const float* __restrict__ b, int64_t begin, int64_t n) {
-  int64_t i = int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
-  const int64_t stride = int64_t(gridDim.x) * blockDim.x;
-  for (i += begin; i < n; i += stride) {
-    float d = SUB ? a[i] - b[i] : a[i];
-    if (ATOMIC)
-      atomicAdd(values + i, d);
-    else
-      values[i] += d;
-  }
+  finish(m, n_tiles);
 }
 
-template <bool SUB>
-static int launch_add_t(float* values, const float* a, const float* b, int64_t n, int atomic, cudaStream_t s) {
-  bool al = aligned16(values) && aligned16(a) && (!SUB || aligned16(b));
-  int64_t n4 = al ? n / 4 : 0;
-  if (n4) {
-    int blocks = ew_blocks(n4 / 4 + 1);
-    if (atomic)
-      add_vec<SUB, true><<<blocks, kEwThreads, 0, s>>>(reinterpret_cast<float4*>(values), reinterpret_cast<const float4*>(a),
-                                                       reinterpret_cast<const float4*>(b), n4);
-    else
-      add_vec<SUB, false><<<blocks, kEwThreads, 0, s>>>(reinterpret_cast<float4*>(values), reinterpret_cast<const float4*>(a),
-                                                        reinterpret_cast<const float4*>(b), n4);
+enum Update { kAdd, kSubAdd, kScaledBf16 };
+constexpr int update_ctas(int kind) { return kind == kSubAdd ? 5 : 8; }  // per SM: two operands take more registers
+
+// values += a | values += a - b | values += alpha * a (bf16: the optimiser step of plain SGD fused with addFromTensor, so
+// that bf16 training never materialises an fp32 delta)
+template <int KIND, bool ATOMIC, bool VEC>
+__global__ void __launch_bounds__(kEwThreads, update_ctas(KIND)) update_kernel(float* __restrict__ values, const void* __restrict__ a_v, const float* __restrict__ b,
+                                                               float alpha, int64_t n, UpdateMarks m) {
+  const int64_t n_tiles = (n + kTile - 1) / kTile;
+  for (int64_t tile = blockIdx.x; tile < n_tiles; tile += gridDim.x) {
+    const int64_t base = tile * kTile;
+    if (VEC && base + kTile <= n) {
+      float4 d[kVecs];
+      if constexpr (KIND == kScaledBf16) {
+        const uint2* g = reinterpret_cast<const uint2*>(static_cast<const __nv_bfloat16*>(a_v) + base) + threadIdx.x;
+        uint2 raw[kVecs];
+#pragma unroll
+        for (int i = 0; i < kVecs; i++) raw[i] = __ldcs(g + i * kEwThreads);
+#pragma unroll
+        for (int i = 0; i < kVecs; i++) {
+          d[i] = from_bf16(raw[i]);
+          d[i].x *= alpha; d[i].y *= alpha; d[i].z *= alpha; d[i].w *= alpha;
+        }
+      } else {
+        const float4* a = reinterpret_cast<const float4*>(static_cast<const float*>(a_v) + base) + threadIdx.x;
+#pragma unroll
+        for (int i = 0; i < kVecs; i++) d[i] = ldg_stream(a + i * kEwThreads);
+        if constexpr (KIND == kSubAdd) {
+#pragma unroll
+          for (int i = 0; i < kVecs; i++) {
+            const float4 o = ldg_stream(reinterpret_cast<const float4*>(b + base) + threadIdx.x + i * kEwThreads);
+            d[i].x -= o.x; d[i].y -= o.y; d[i].z -= o.z; d[i].w -= o.w;
+          }
+        }
+      }
+#pragma unroll
+      for (int i = 0; i < kVecs; i++) {
+        float4* v4 = reinterpret_cast<float4*>(values + base) + threadIdx.x + i * kEwThreads;
+        if (ATOMIC) {
+          red_add_v4(reinterpret_cast<float*>(v4), d[i]);
+        } else {
+          float4 v = *v4;
+          v.x += d[i].x; v.y += d[i].y; v.z += d[i].z; v.w += d[i].w;
+          *v4 = v;
+        }
+      }
+    } else {
+      const int left = int(min(int64_t(kTile), n - base));
+      for (int e0 = threadIdx.x; e0 < left; e0 += kElems * kEwThreads) {
+        float d[kElems];
+#pragma unroll
+        for (int i = 0; i < kElems; i++) {
+          const int e = e0 + i * kEwThreads;
+          if (e >= left) continue;
+          if constexpr (KIND == kScaledBf16) d[i] = alpha * __bfloat162float(static_cast<const __nv_bfloat16*>(a_v)[base + e]);
+          else d[i] = static_cast<const float*>(a_v)[base + e];
+        }
+        if constexpr (KIND == kSubAdd) {
+#pragma unroll
+          for (int i = 0; i < kElems; i++)
+            if (e0 + i * kEwThreads < left) d[i] -= b[base + e0 + i * kEwThreads];
+        }
+#pragma unroll
+        for (int i = 0; i < kElems; i++) {
+          const int e = e0 + i * kEwThreads;
+          if (e >= left) continue;
+          if (ATOMIC) atomicAdd(values + base + e, d[i]);
+          else values[base + e] += d[i];
+        }
+      }
+    }
   }
-  if (n4 * 4 < n) {
-    int blocks = ew_blocks(n - n4 * 4);
-    if (atomic)
-      add_scalar<SUB, true><<<blocks, kEwThreads, 0, s>>>(values, a, b, n4 * 4, n);
-    else
-      add_scalar<SUB, false><<<blocks, kEwThreads, 0, s>>>(values, a, b, n4 * 4, n);
+  finish(m, n_tiles);
+}
+
+template <int KIND>
+int launch_update(float* values, const void* a, const float* b, float alpha, int64_t n, int atomic, const UpdateMarks& m, void* stream) {
+  cudaStream_t s = static_cast<cudaStream_t>(stream);
+  const bool vec = aligned16(values) && (KIND == kScaledBf16 ? (reinterpret_cast<uintptr_t>(a) & 7) == 0 : aligned16(a)) && (KIND != kSubAdd || aligned16(b));
+  const int blocks = tile_blocks(n, update_ctas(KIND));
+  if (atomic) {
+    if (vec) update_kernel<KIND, true, true><<<blocks, kEwThreads, 0, s>>>(values, a, b, alpha, n, m);
+    else update_kernel<KIND, true, false><<<blocks, kEwThreads, 0, s>>>(values, a, b, alpha, n, m);
+  } else {
+    if (vec) update_kernel<KIND, false, true><<<blocks, kEwThreads, 0, s>>>(values, a, b, alpha, n, m);
+    else update_kernel<KIND, false, false><<<blocks, kEwThreads, 0, s>>>(values, a, b, alpha, n, m);
   }
   return int(cudaGetLastError());
 }
 
-int launch_add(float* values, const float* delta, int64_t n, int atomic, void* stream) {
-  return launch_add_t<false>(values, delta, nullptr, n, atomic, static_cast<cudaStream_t>(stream));
-}
-int launch_sub_add(float* values, const float* neu, const float* old, int64_t n, int atomic, void* stream) {
-  return launch_add_t<true>(values, neu, old, n, atomic, static_cast<cudaStream_t>(stream));
-}
+}  // namespace
 
-// values += alpha * g for a bf16 gradient: the optimiser step of plain SGD fused with addFromTensor, so
-// that bf16 training never materialises an fp32 delta.
-template <bool ATOMIC>
-__global__ void __launch_bounds__(kEwThreads) add_scaled_bf16_vec(float4* __restrict__ values, const uint2* __restrict__ g, float alpha,
-                                                                  int64_t n4) {
-  int64_t i = int64_t(blockIdx.x) * kEwThreads + threadIdx.x;
-  const int64_t stride = int64_t(gridDim.x) * kEwThreads;
-  for (; i < n4; i += stride) {
-    uint2 raw = g[i];
-    __nv_bfloat162 lo = *reinterpret_cast<__nv_bfloat162*>(&raw.x), hi = *reinterpret_cast<__nv_bfloat162*>(&raw.y);
-    float2 a = __bfloat1622float2(lo), b = __bfloat1622float2(hi);
-    if (ATOMIC) {
-      red_add_v4(reinterpret_cast<float*>(values + i), make_float4(alpha * a.x, alpha * a.y, alpha * b.x, alpha * b.y));
-    } else {
-      float4 v = values[i];
-      v.x += alpha * a.x;
-      v.y += alpha * a.y;
-      v.z += alpha * b.x;
-      v.w += alpha * b.y;
-      values[i] = v;
-    }
-  }
-}
-template <bool ATOMIC>
-__global__ void add_scaled_bf16_scalar(float* __restrict__ values, const __nv_bfloat16* __restrict__ g, float alpha, int64_t begin,
-                                       int64_t n) {
-  int64_t i = int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
-  const int64_t stride = int64_t(gridDim.x) * blockDim.x;
-  for (i += begin; i < n; i += stride) {
-    if (ATOMIC) atomicAdd(values + i, alpha * __bfloat162float(g[i]));
-    else values[i] += alpha * __bfloat162float(g[i]);
-  }
-}
-int launch_add_scaled_bf16(float* values, const void* g_bf16, float alpha, int64_t n, int atomic, void* stream_v) {
-  cudaStream_t s = static_cast<cudaStream_t>(stream_v);
-  bool al = aligned16(values) && (reinterpret_cast<uintptr_t>(g_bf16) & 7) == 0;
-  int64_t n4 = al ? n / 4 : 0;
-  if (n4) {
-    if (atomic) add_scaled_bf16_vec<true><<<ew_blocks(n4), kEwThreads, 0, s>>>(reinterpret_cast<float4*>(values), static_cast<const uint2*>(g_bf16), alpha, n4);
-    else add_scaled_bf16_vec<false><<<ew_blocks(n4), kEwThreads, 0, s>>>(reinterpret_cast<float4*>(values), static_cast<const uint2*>(g_bf16), alpha, n4);
-  }
-  if (n4 * 4 < n) {
-    if (atomic) add_scaled_bf16_scalar<true><<<ew_blocks(n - n4 * 4), kEwThreads, 0, s>>>(values, static_cast<const __nv_bfloat16*>(g_bf16), alpha, n4 * 4, n);
-    else add_scaled_bf16_scalar<false><<<ew_blocks(n - n4 * 4), kEwThreads, 0, s>>>(values, static_cast<const __nv_bfloat16*>(g_bf16), alpha, n4 * 4, n);
-  }
+int launch_snapshot_f32(const float* values, float* out, int64_t n, const UpdateMarks& m, void* stream) {
+  cudaStream_t s = static_cast<cudaStream_t>(stream);
+  if (aligned16(values) && aligned16(out)) snapshot_kernel<float, true><<<tile_blocks(n), kEwThreads, 0, s>>>(values, out, n, m);
+  else snapshot_kernel<float, false><<<tile_blocks(n), kEwThreads, 0, s>>>(values, out, n, m);
   return int(cudaGetLastError());
+}
+int launch_snapshot_bf16(const float* values, void* out, int64_t n, const UpdateMarks& m, void* stream) {
+  cudaStream_t s = static_cast<cudaStream_t>(stream);
+  __nv_bfloat16* o = static_cast<__nv_bfloat16*>(out);
+  if (aligned16(values) && (reinterpret_cast<uintptr_t>(out) & 7) == 0) snapshot_kernel<__nv_bfloat16, true><<<tile_blocks(n), kEwThreads, 0, s>>>(values, o, n, m);
+  else snapshot_kernel<__nv_bfloat16, false><<<tile_blocks(n), kEwThreads, 0, s>>>(values, o, n, m);
+  return int(cudaGetLastError());
+}
+int launch_add(float* values, const float* delta, int64_t n, int atomic, const UpdateMarks& m, void* stream) {
+  return launch_update<kAdd>(values, delta, nullptr, 1.f, n, atomic, m, stream);
+}
+int launch_sub_add(float* values, const float* neu, const float* old, int64_t n, int atomic, const UpdateMarks& m, void* stream) {
+  return launch_update<kSubAdd>(values, neu, old, 1.f, n, atomic, m, stream);
+}
+int launch_add_scaled_bf16(float* values, const void* g_bf16, float alpha, int64_t n, int atomic, const UpdateMarks& m, void* stream) {
+  return launch_update<kScaledBf16>(values, g_bf16, nullptr, alpha, n, atomic, m, stream);
 }
 
 __global__ void fill_state_kernel(uint32_t* s, int n, uint32_t v) {

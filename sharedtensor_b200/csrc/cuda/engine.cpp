@@ -81,8 +81,8 @@ GpuReplica::GpuReplica(int device, int64_t n, const GpuConfig& cfg) : device_(de
   check(cudaMalloc(reinterpret_cast<void**>(&tile_state_), size_t(n_tiles_) * 4), "cudaMalloc tile_state");
   check(cudaMalloc(reinterpret_cast<void**>(&status_), kDsTotalWords * 8), "cudaMalloc status");
   check(cudaMallocHost(reinterpret_cast<void**>(&status_host_), (kDsTotalWords + 16) * 8), "cudaMallocHost status");
-  check(cudaMalloc(reinterpret_cast<void**>(&yield_flag_), 4), "cudaMalloc yield flag");
-  check(cudaMemsetAsync(yield_flag_, 0, 4, s), "memset");
+  check(cudaMalloc(reinterpret_cast<void**>(&yield_flag_), 4 + 4 * kTickets), "cudaMalloc yield flag");
+  check(cudaMemsetAsync(yield_flag_, 0, 4 + 4 * kTickets, s), "memset");
   check(launch_fill_state(tile_state_, n_tiles_, 1u, comm_), "fill_state");
   check(cudaMemsetAsync(status_, 0, kDsTotalWords * 8, s), "memset");
   std::memset(status_host_, 0, (kDsTotalWords + 16) * 8);
@@ -350,6 +350,7 @@ void GpuReplica::rebuild_params() {
   }
   params_.n_in = r;
   params_.n_out = r;
+  ring_peers_.store(r);
 }
 
 // ---------------------------------------------------------------------------------------------
@@ -434,72 +435,67 @@ void GpuReplica::load_values(const float* src, void* user_stream) {
   local_update();
 }
 
-// Around an update, in the order of the caller's stream: a word that asks the round kernel to give up its SMs (it
-// holds all of them, for as long as a pass over the tensor takes), then the update, then the change marks, then the
-// word is cleared.  The update itself never waits for a round; it only wants somewhere to run.
-void GpuReplica::ask_for_sms(void* user_stream, bool on) {
-  if (!cfg_.yield_to_updates) return;
-  if (!stream_write_u32(user_stream, yield_flag_, on ? 1u : 0u)) check(launch_set_word(yield_flag_, on ? 1u : 0u, user_stream), "set_word");
+// Before an update (or a snapshot, which sits on the training loop's critical path like an update does), in the order of
+// the caller's stream: a word that asks the round kernel to give up its SMs (it holds all of them, for as long as a window
+// of the tensor takes).  The update itself never waits for a round; it only wants somewhere to run.  Its kernel sets the
+// change marks behind the data and its last CTA clears the word.  A replica without a ring peer runs no rounds and needs
+// no word (a peer that is attached before the update gets to run costs it the wait for one window).
+UpdateMarks GpuReplica::ask_for_sms(void* user_stream, bool marks) {
+  UpdateMarks m;
+  if (marks) m.tile_state = tile_state_;
+  if (cfg_.yield_to_updates && ring_peers_.load(std::memory_order_relaxed) > 0) {
+    m.yield_word = yield_flag_;
+    m.ticket = yield_flag_ + 1 + next_ticket_.fetch_add(1, std::memory_order_relaxed) % kTickets;
+    if (!stream_write_u32(user_stream, yield_flag_, 1u)) check(launch_set_word(yield_flag_, 1u, user_stream), "set_word");
+  }
+  return m;
 }
 
 void GpuReplica::add(const float* delta, void* user_stream) {
   DeviceGuard g(device_);
   std::lock_guard<std::mutex> gate(gate_mu_);
-  ask_for_sms(user_stream, true);
-  check(launch_add(values(), delta, n_, 1, user_stream), "add kernel");
-  check(launch_fill_state(tile_state_, n_tiles_, 1u, user_stream), "fill_state");  // marks after the data, in stream order
-  ask_for_sms(user_stream, false);
-  epoch_++;
-  launches_ += 2;
-  local_update();
+  check(launch_add(values(), delta, n_, 1, ask_for_sms(user_stream, true), user_stream), "add kernel");
+  updated();
 }
 
 void GpuReplica::sub_add(const float* neu, const float* old, void* user_stream) {
   DeviceGuard g(device_);
   std::lock_guard<std::mutex> gate(gate_mu_);
-  ask_for_sms(user_stream, true);
-  check(launch_sub_add(values(), neu, old, n_, 1, user_stream), "sub_add kernel");
-  check(launch_fill_state(tile_state_, n_tiles_, 1u, user_stream), "fill_state");
-  ask_for_sms(user_stream, false);
-  epoch_++;
-  launches_ += 2;
-  local_update();
+  check(launch_sub_add(values(), neu, old, n_, 1, ask_for_sms(user_stream, true), user_stream), "sub_add kernel");
+  updated();
 }
 
 void GpuReplica::add_scaled_bf16(const void* g, float alpha, void* user_stream) {
   DeviceGuard gd(device_);
   std::lock_guard<std::mutex> gate(gate_mu_);
-  ask_for_sms(user_stream, true);
-  check(launch_add_scaled_bf16(values(), g, alpha, n_, 1, user_stream), "add_scaled_bf16 kernel");
-  check(launch_fill_state(tile_state_, n_tiles_, 1u, user_stream), "fill_state");
-  ask_for_sms(user_stream, false);
+  check(launch_add_scaled_bf16(values(), g, alpha, n_, 1, ask_for_sms(user_stream, true), user_stream), "add_scaled_bf16 kernel");
+  updated();
+}
+
+void GpuReplica::updated() {
   epoch_++;
-  launches_ += 2;
+  launches_ += 1;
   local_update();
 }
 
 void GpuReplica::add_gate_held(const float* delta) {
   DeviceGuard g(device_);
-  check(launch_add(values(), delta, n_, 1, comm_), "add kernel");
-  check(launch_fill_state(tile_state_, n_tiles_, 1u, comm_), "fill_state");
+  UpdateMarks m;
+  m.tile_state = tile_state_;
+  check(launch_add(values(), delta, n_, 1, m, comm_), "add kernel");
   epoch_++;
-  launches_ += 2;
+  launches_ += 1;
 }
 
-// A snapshot sits on the training loop's critical path like an update does: it asks for the SMs too.
 void GpuReplica::snapshot(float* out, void* user_stream) {
   DeviceGuard g(device_);
-  ask_for_sms(user_stream, true);
-  check(launch_snapshot_f32(values(), out, n_, user_stream), "snapshot kernel");
-  ask_for_sms(user_stream, false);
+  check(launch_snapshot_f32(values(), out, n_, ask_for_sms(user_stream, false), user_stream), "snapshot kernel");
   launches_ += 1;
 }
 
 void GpuReplica::snapshot_bf16(void* out, void* user_stream) {
   DeviceGuard g(device_);
-  ask_for_sms(user_stream, true);
-  check(launch_snapshot_bf16(values(), out, n_, user_stream), "snapshot kernel");
-  ask_for_sms(user_stream, false);
+  check(launch_snapshot_bf16(values(), out, n_, ask_for_sms(user_stream, false), user_stream), "snapshot kernel");
   launches_ += 1;
 }
 

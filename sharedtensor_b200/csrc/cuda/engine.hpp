@@ -162,7 +162,8 @@ class GpuReplica {
   int window_tiles() const;
   int n_windows() const;
   void fill_guards(const VmmBlock& b, size_t used_bytes);
-  void ask_for_sms(void* user_stream, bool on);
+  UpdateMarks ask_for_sms(void* user_stream, bool marks);
+  void updated();
   void check(int cuda_err, const char* what);
   void engine_loop();
   void order_after_user(void* user_stream);
@@ -179,7 +180,12 @@ class GpuReplica {
   std::vector<Peer> peers_;
   uint32_t* tile_state_ = nullptr;     // change mark per tile
   uint64_t* status_ = nullptr;         // DevStatus layout
-  uint32_t* yield_flag_ = nullptr;     // non-zero while an update wants the SMs the round kernel holds
+  // non-zero while an update wants the SMs the round kernel holds; behind it the words in which the CTAs of updates count
+  // themselves off (more of them than a GPU runs kernels at once)
+  static constexpr uint32_t kTickets = 255;
+  uint32_t* yield_flag_ = nullptr;
+  std::atomic<uint32_t> next_ticket_{0};
+  std::atomic<int> ring_peers_{0};
   uint32_t* dbg_host_ = nullptr;       // mapped host memory for the debug build's progress marks
   uint64_t* status_host_ = nullptr;    // pinned
   uint32_t* tcp_words_dev_ = nullptr;  // ceil(n/32) words, staging of TCP frames

@@ -610,7 +610,7 @@ class GpuNode {
     }
     cudaStream_t cs = static_cast<cudaStream_t>(rep_->comm_stream());
     cudaMemsetAsync(carry, 0, size_t(n_) * 4, cs);
-    launch_sub_add(carry, rep_->values(), rep_->mirror(orphan_link_), n_, 0, rep_->comm_stream());
+    launch_sub_add(carry, rep_->values(), rep_->mirror(orphan_link_), n_, 0, UpdateMarks{}, rep_->comm_stream());
     rep_->sync();
     return carry;
   }

@@ -136,13 +136,19 @@ int launch_unsend(float* mirror, const uint8_t* payload_remote, uint32_t* tx_seq
 int round_smem_bytes(int groups, int slots, int payload_bytes);
 
 // Element-wise kernels (copyToTensor / addFromTensor / pushUpdate; src/sharedtensor.c:435-446, 334-344).
-int launch_snapshot_f32(const float* values, float* out, int64_t n, void* stream);
-int launch_snapshot_bf16(const float* values, void* out_bf16, int64_t n, void* stream);
+// What an update or a snapshot does besides its data; null pointers: nothing.
+struct UpdateMarks {
+  uint32_t* tile_state = nullptr;  // the change marks of the tiles, set behind the data
+  uint32_t* yield_word = nullptr;  // the request for SMs, taken back by the last CTA
+  uint32_t* ticket = nullptr;      // a zeroed word of this launch's own (left zero again): counts the CTAs that are done
+};
+int launch_snapshot_f32(const float* values, float* out, int64_t n, const UpdateMarks& m, void* stream);
+int launch_snapshot_bf16(const float* values, void* out_bf16, int64_t n, const UpdateMarks& m, void* stream);
 // atomic != 0: every element is added with a reduction at the L2, so the add commutes with whatever else adds into
 // `values` at the same time (the round kernel, other streams).
-int launch_add(float* values, const float* delta, int64_t n, int atomic, void* stream);
-int launch_sub_add(float* values, const float* neu, const float* old, int64_t n, int atomic, void* stream);
-int launch_add_scaled_bf16(float* values, const void* g_bf16, float alpha, int64_t n, int atomic, void* stream);
+int launch_add(float* values, const float* delta, int64_t n, int atomic, const UpdateMarks& m, void* stream);
+int launch_sub_add(float* values, const float* neu, const float* old, int64_t n, int atomic, const UpdateMarks& m, void* stream);
+int launch_add_scaled_bf16(float* values, const void* g_bf16, float alpha, int64_t n, int atomic, const UpdateMarks& m, void* stream);
 // Marks every tile as changed.  Launched behind an update on the same stream, so the marks become visible after the data.
 int launch_fill_state(uint32_t* tile_state, int n_tiles, uint32_t value, void* stream);
 int launch_set_word(uint32_t* word, uint32_t value, void* stream);  // one thread; stands in for a stream memory write

@@ -35,8 +35,12 @@ def _gpu_config(cfg: Config):
     return g
 
 
+# The stream's address without a Stream object around it: 0.1 us instead of 2.2 us a call.
+_raw_stream = getattr(torch._C, "_cuda_getCurrentRawStream", None)
+
+
 def _stream(device: torch.device) -> int:
-    return torch.cuda.current_stream(device).cuda_stream
+    return _raw_stream(device.index) if _raw_stream is not None else torch.cuda.current_stream(device).cuda_stream
 
 
 class GpuBackend:
