@@ -69,16 +69,14 @@ __device__ __forceinline__ void finish(const UpdateMarks& m, int64_t n_tiles) {
     }
   }
   if (m.yield_word != nullptr && threadIdx.x == 0) {
-    if (atomicAdd(m.ticket, 1u) == gridDim.x - 1) {
-      *m.ticket = 0u;
-      *reinterpret_cast<volatile uint32_t*>(m.yield_word) = 0u;
-    }
+    // (a counter that wraps: whatever it held before, one of the grid's CTAs takes the request back)
+    if (atomicInc(m.ticket, gridDim.x - 1) >= gridDim.x - 1) *reinterpret_cast<volatile uint32_t*>(m.yield_word) = 0u;
   }
 }
 
 inline int tile_blocks(int64_t n, int per_sm = 8) {
   const int64_t tiles = (n + kTile - 1) / kTile;
-  return int(tiles < 148 * per_sm ? tiles : 148 * per_sm);
+  return int(tiles < 1 ? 1 : (tiles < 148 * per_sm ? tiles : 148 * per_sm));
 }
 
 struct Bf16x4 {
@@ -93,10 +91,31 @@ __device__ __forceinline__ float4 from_bf16(uint2 raw) {
   return make_float4(a.x, a.y, b.x, b.y);
 }
 
+// These kernels follow each other and other small kernels closely: each may be launched while the one before it in the
+// stream runs out, and waits for it before it touches memory.
+__device__ __forceinline__ void wait_for_stream() {
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+}
+template <class... P, class... A>
+int launch_early(void (*kernel)(P...), int blocks, void* stream, A... args) {
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = dim3(blocks);
+  cfg.blockDim = dim3(kEwThreads);
+  cfg.stream = static_cast<cudaStream_t>(stream);
+  cudaLaunchAttribute early{};
+  early.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  early.val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = &early;
+  cfg.numAttrs = 1;
+  return int(cudaLaunchKernelEx(&cfg, kernel, P(args)...));
+}
+
 template <class T, bool VEC>
 __global__ void __launch_bounds__(kEwThreads, 8) snapshot_kernel(const float* __restrict__ src, T* __restrict__ dst, int64_t n, UpdateMarks m) {
   constexpr bool kBf16 = sizeof(T) == 2;
   const int64_t n_tiles = (n + kTile - 1) / kTile;
+  wait_for_stream();
   for (int64_t tile = blockIdx.x; tile < n_tiles; tile += gridDim.x) {
     if (VEC && (tile + 1) * kTile <= n) {
       const float4* s4 = reinterpret_cast<const float4*>(src + tile * kTile) + threadIdx.x;
@@ -140,6 +159,7 @@ template <int KIND, bool ATOMIC, bool VEC>
 __global__ void __launch_bounds__(kEwThreads, update_ctas(KIND)) update_kernel(float* __restrict__ values, const void* __restrict__ a_v, const float* __restrict__ b,
                                                                float alpha, int64_t n, UpdateMarks m) {
   const int64_t n_tiles = (n + kTile - 1) / kTile;
+  wait_for_stream();
   for (int64_t tile = blockIdx.x; tile < n_tiles; tile += gridDim.x) {
     const int64_t base = tile * kTile;
     if (VEC && base + kTile <= n) {
@@ -208,33 +228,22 @@ __global__ void __launch_bounds__(kEwThreads, update_ctas(KIND)) update_kernel(f
 
 template <int KIND>
 int launch_update(float* values, const void* a, const float* b, float alpha, int64_t n, int atomic, const UpdateMarks& m, void* stream) {
-  cudaStream_t s = static_cast<cudaStream_t>(stream);
   const bool vec = aligned16(values) && (KIND == kScaledBf16 ? (reinterpret_cast<uintptr_t>(a) & 7) == 0 : aligned16(a)) && (KIND != kSubAdd || aligned16(b));
-  const int blocks = tile_blocks(n, update_ctas(KIND));
-  if (atomic) {
-    if (vec) update_kernel<KIND, true, true><<<blocks, kEwThreads, 0, s>>>(values, a, b, alpha, n, m);
-    else update_kernel<KIND, true, false><<<blocks, kEwThreads, 0, s>>>(values, a, b, alpha, n, m);
-  } else {
-    if (vec) update_kernel<KIND, false, true><<<blocks, kEwThreads, 0, s>>>(values, a, b, alpha, n, m);
-    else update_kernel<KIND, false, false><<<blocks, kEwThreads, 0, s>>>(values, a, b, alpha, n, m);
-  }
-  return int(cudaGetLastError());
+  const auto kernel = atomic ? (vec ? update_kernel<KIND, true, true> : update_kernel<KIND, true, false>)
+                             : (vec ? update_kernel<KIND, false, true> : update_kernel<KIND, false, false>);
+  return launch_early(kernel, tile_blocks(n, update_ctas(KIND)), stream, values, a, b, alpha, n, m);
 }
 
 }  // namespace
 
 int launch_snapshot_f32(const float* values, float* out, int64_t n, const UpdateMarks& m, void* stream) {
-  cudaStream_t s = static_cast<cudaStream_t>(stream);
-  if (aligned16(values) && aligned16(out)) snapshot_kernel<float, true><<<tile_blocks(n), kEwThreads, 0, s>>>(values, out, n, m);
-  else snapshot_kernel<float, false><<<tile_blocks(n), kEwThreads, 0, s>>>(values, out, n, m);
-  return int(cudaGetLastError());
+  const bool vec = aligned16(values) && aligned16(out);
+  return launch_early(vec ? snapshot_kernel<float, true> : snapshot_kernel<float, false>, tile_blocks(n), stream, values, out, n, m);
 }
 int launch_snapshot_bf16(const float* values, void* out, int64_t n, const UpdateMarks& m, void* stream) {
-  cudaStream_t s = static_cast<cudaStream_t>(stream);
-  __nv_bfloat16* o = static_cast<__nv_bfloat16*>(out);
-  if (aligned16(values) && (reinterpret_cast<uintptr_t>(out) & 7) == 0) snapshot_kernel<__nv_bfloat16, true><<<tile_blocks(n), kEwThreads, 0, s>>>(values, o, n, m);
-  else snapshot_kernel<__nv_bfloat16, false><<<tile_blocks(n), kEwThreads, 0, s>>>(values, o, n, m);
-  return int(cudaGetLastError());
+  const bool vec = aligned16(values) && (reinterpret_cast<uintptr_t>(out) & 7) == 0;
+  return launch_early(vec ? snapshot_kernel<__nv_bfloat16, true> : snapshot_kernel<__nv_bfloat16, false>, tile_blocks(n), stream, values,
+                      static_cast<__nv_bfloat16*>(out), n, m);
 }
 int launch_add(float* values, const float* delta, int64_t n, int atomic, const UpdateMarks& m, void* stream) {
   return launch_update<kAdd>(values, delta, nullptr, 1.f, n, atomic, m, stream);

@@ -439,11 +439,12 @@ void GpuReplica::load_values(const float* src, void* user_stream) {
 // the caller's stream: a word that asks the round kernel to give up its SMs (it holds all of them, for as long as a window
 // of the tensor takes).  The update itself never waits for a round; it only wants somewhere to run.  Its kernel sets the
 // change marks behind the data and its last CTA clears the word.  A replica without a ring peer runs no rounds and needs
-// no word (a peer that is attached before the update gets to run costs it the wait for one window).
+// no word (a peer that is attached before the update gets to run costs it the wait for one window), and an update on the
+// rounds' own stream finds none running.
 UpdateMarks GpuReplica::ask_for_sms(void* user_stream, bool marks) {
   UpdateMarks m;
   if (marks) m.tile_state = tile_state_;
-  if (cfg_.yield_to_updates && ring_peers_.load(std::memory_order_relaxed) > 0) {
+  if (cfg_.yield_to_updates && user_stream != comm_ && ring_peers_.load(std::memory_order_relaxed) > 0) {
     m.yield_word = yield_flag_;
     m.ticket = yield_flag_ + 1 + next_ticket_.fetch_add(1, std::memory_order_relaxed) % kTickets;
     if (!stream_write_u32(user_stream, yield_flag_, 1u)) check(launch_set_word(yield_flag_, 1u, user_stream), "set_word");

@@ -140,7 +140,7 @@ int round_smem_bytes(int groups, int slots, int payload_bytes);
 struct UpdateMarks {
   uint32_t* tile_state = nullptr;  // the change marks of the tiles, set behind the data
   uint32_t* yield_word = nullptr;  // the request for SMs, taken back by the last CTA
-  uint32_t* ticket = nullptr;      // a zeroed word of this launch's own (left zero again): counts the CTAs that are done
+  uint32_t* ticket = nullptr;      // a word of this launch's own that starts at zero and ends there: counts the CTAs that are done
 };
 int launch_snapshot_f32(const float* values, float* out, int64_t n, const UpdateMarks& m, void* stream);
 int launch_snapshot_bf16(const float* values, void* out_bf16, int64_t n, const UpdateMarks& m, void* stream);
