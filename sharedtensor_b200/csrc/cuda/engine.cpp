@@ -162,6 +162,7 @@ GpuReplica::~GpuReplica() {
   for (void* e : ev_round_) cudaEventDestroy(E(e));
   for (void* e : ev_kernel_) cudaEventDestroy(E(e));
   if (stat_) cudaStreamDestroy(S(stat_));
+  if (flush_) cudaStreamDestroy(S(flush_));
   if (ev_user_) cudaEventDestroy(E(ev_user_));
   if (ev_comm_) cudaEventDestroy(E(ev_comm_));
   if (comm_) cudaStreamDestroy(S(comm_));
@@ -252,6 +253,7 @@ int GpuReplica::attach_peer(int link, int local_block, void* remote_base) {
       // whatever the link still had to say must be looked at again
       launch_fill_state(tile_state_, n_tiles_, 1u, comm_);
       rebuild_params();
+      check(load_round(params_, cfg_.shape), "round kernel");  // the neighbour's first frames are not to wait for that
       return i;
     }
   }
@@ -772,6 +774,55 @@ void GpuReplica::idle_pause(uint64_t us) {
   wake_pending_ = false;
 }
 
+// Frames (per tile and ring) that no neighbour has acknowledged yet.
+uint32_t GpuReplica::unacknowledged() {
+  uint32_t* const count = reinterpret_cast<uint32_t*>(status_host_ + kDsTotalWords + 12);
+  if (!flush_) {
+    cudaStream_t st;
+    check(cudaStreamCreateWithFlags(&st, cudaStreamNonBlocking), "cudaStreamCreate");
+    flush_ = st;
+  }
+  {
+    std::lock_guard<std::mutex> lk(mu_);
+    *count = 0;
+    check(launch_count_unacknowledged(params_, count, flush_), "count_unacknowledged kernel");
+    // the edges cannot be taken down while the kernel looks at them
+    check(cudaStreamSynchronize(S(flush_)), "cudaStreamSynchronize");
+  }
+  return *reinterpret_cast<volatile uint32_t*>(count);
+}
+
+// Three passes of the engine thread in a row, begun after the caller's updates have run, that find nothing to do; for as
+// long as a neighbour may need to take in what it was sent and pass it on (two busy passes at HBM rate) no pass that did;
+// and every frame acknowledged (a neighbour may be gone, or have no engine running: after a tenth of a second of quiet the
+// frames count as delivered, they are in its memory).
+bool GpuReplica::flush(void* user_stream, int timeout_ms) {
+  DeviceGuard g(device_);
+  std::lock_guard<std::mutex> one(flush_mu_);
+  check(cudaStreamSynchronize(S(user_stream)), "cudaStreamSynchronize");
+  const uint64_t start = steady_ns(), limit = uint64_t(timeout_ms < 0 ? 0 : timeout_ms) * 1000000ull;
+  const uint64_t quiet_ns = 100000ull + uint64_t(n_padded_) * 2 * 18 / 6000;   // 18 bytes an element and pass, 6000 bytes a ns
+  const uint64_t before = engine_launched_.load(), passes = 3ull * uint64_t(n_windows());
+  uint64_t woken = 0;
+  while (engine_on_.load()) {
+    const uint64_t busy = last_busy_launch_.load(), looked = engine_looked_.load(), now = steady_ns();
+    const uint64_t since = last_busy_ns_.load();
+    const uint64_t quiet = now - (since > start ? since : start);
+    if (looked >= (busy > before ? busy : before) + passes && quiet >= quiet_ns && (quiet >= quiet_ns + 100000000ull || unacknowledged() == 0)) return true;
+    if (ring_peers_.load() == 0) return true;  // the last neighbour has gone
+    if (now - start > limit) break;
+    if (woken == 0 || now - woken > 2000000ull) {
+      const std::string err = last_error();
+      if (!err.empty()) throw std::runtime_error("sharedtensor GPU engine: " + err);
+      wake(false);  // the engine keeps looking often
+      woken = now;
+    }
+    if (now - start < 2000000ull) std::this_thread::yield();
+    else ::usleep(50);
+  }
+  return false;
+}
+
 void GpuReplica::engine_loop() {
   cudaSetDevice(device_);
   ::prctl(PR_SET_TIMERSLACK, 1000UL, 0, 0, 0);  // 1 us instead of the default 50 us: the idle pauses start at 10 us
@@ -782,6 +833,7 @@ void GpuReplica::engine_loop() {
   uint64_t* work_host = status_host_ + kDsTotalWords;  // behind the part status() uses
   uint64_t work_seen = 0;
   uint64_t r = 0;
+  engine_looked_.store(engine_launched_.load());  // (launches of an earlier run of this thread that were not looked back on)
   uint64_t idle_rounds = 0;
   uint64_t quiet_launches = 0;   // launches in a row that found nothing to do
   while (!engine_stop_.load()) {
@@ -794,6 +846,7 @@ void GpuReplica::engine_loop() {
         // thread, which only starts the next launch and reads how much the last one found to do.
         windows = n_windows();
         launch(true, true, auto_sweeps());
+        engine_launched_.fetch_add(1);
         cudaEventRecord(E(ev_kernel_[r % depth]), S(comm_));
         cudaStreamWaitEvent(S(stat_), E(ev_kernel_[r % depth]), 0);
         cudaMemcpyAsync(work_host + (r % depth), status_ + kDsTilesProcessed, 8, cudaMemcpyDeviceToHost, S(stat_));
@@ -814,6 +867,15 @@ void GpuReplica::engine_loop() {
       const uint64_t now = work_host[(r - depth) % depth];
       work = now > work_seen ? now - work_seen : 0;
       work_seen = now > work_seen ? now : work_seen;
+    }
+    if (r >= depth) {
+      // what flush() watches: how many launches have been looked back on, and the last of them that found work
+      const uint64_t looked = engine_looked_.load() + 1;
+      if (work != 0) {
+        last_busy_ns_.store(steady_ns());
+        last_busy_launch_.store(looked);
+      }
+      engine_looked_.store(looked);
     }
     if (work != 0) epoch_++;
     quiet_launches = work == 0 ? quiet_launches + 1 : 0;

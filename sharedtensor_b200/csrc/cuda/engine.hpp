@@ -122,6 +122,10 @@ class GpuReplica {
   void start_engine();
   void stop_engine();
   bool engine_running() const { return engine_on_.load(); }
+  // With the engine running: waits until the work queued on `user_stream` is done and the rounds have gone quiet; false
+  // when they have not within the time given.
+  bool flush(void* user_stream, int timeout_ms);
+  int ring_peers() const { return ring_peers_.load(); }
   // Ends the engine thread's idle pause at once.  `from_neighbour` marks a doorbell that came over a socket; the
   // return value says whether the engine had been idle (the caller then passes the doorbell on).
   bool wake(bool from_neighbour = false);
@@ -164,6 +168,7 @@ class GpuReplica {
   void fill_guards(const VmmBlock& b, size_t used_bytes);
   UpdateMarks ask_for_sms(void* user_stream, bool marks);
   void updated();
+  uint32_t unacknowledged();
   void check(int cuda_err, const char* what);
   void engine_loop();
   void order_after_user(void* user_stream);
@@ -205,11 +210,15 @@ class GpuReplica {
   std::vector<void*> ev_round_;       // per launch in flight: its work count has been read back
   std::vector<void*> ev_kernel_;      // per launch in flight: the kernel has finished (comm stream)
   void* stat_ = nullptr;               // cudaStream_t: reads work counts back beside the comm stream, so that launches follow each other without a copy in between
+  void* flush_ = nullptr;              // cudaStream_t: flush() counts unacknowledged frames beside the rounds (made on first use)
+  std::mutex flush_mu_;                // one flush at a time; taken before mu_
   mutable std::mutex mu_;
   std::mutex gate_mu_;                 // taken before mu_ by every update from outside the rounds
   std::mutex engine_mu_;               // serialises start_engine / stop_engine
   std::thread engine_;
   std::atomic<bool> engine_on_{false}, engine_stop_{false};
+  std::atomic<uint64_t> engine_launched_{0}, engine_looked_{0};       // launches of the engine thread, and those looked back on
+  std::atomic<uint64_t> last_busy_launch_{0}, last_busy_ns_{0};       // the last of the latter that found work, and when that was seen
   std::atomic<uint64_t> last_wake_ns_{0};  // when wake() was last called (steady clock)
   std::atomic<bool> idle_{false};      // the engine has seen several rounds without work and pauses between rounds
   std::mutex wake_mu_;

@@ -1000,6 +1000,19 @@ int launch_unsend(float* mirror, const uint8_t* payload_remote, uint32_t* tx_seq
   return int(cudaGetLastError());
 }
 
+__global__ void __launch_bounds__(256) unacknowledged_kernel(const __grid_constant__ RoundParams p, uint32_t* __restrict__ count) {
+  uint32_t n = 0;
+  for (int tile = blockIdx.x * 256 + threadIdx.x; tile < p.n_tiles; tile += gridDim.x * 256)
+    for (int r = 0; r < p.n_out; r++) n += ld_cg_u32(p.out[r].tx_seq + tile) - ld_relaxed_sys(p.out[r].credit + tile);
+  n = __reduce_add_sync(0xffffffffu, n);
+  if ((threadIdx.x & 31) == 0 && n) atomicAdd_system(count, n);
+}
+int launch_count_unacknowledged(const RoundParams& p, uint32_t* count, void* stream) {
+  const int blocks = (p.n_tiles + 255) / 256;
+  unacknowledged_kernel<<<blocks < 32 ? blocks : 32, 256, 0, static_cast<cudaStream_t>(stream)>>>(p, count);
+  return int(cudaGetLastError());
+}
+
 // ----------------------------------------------------------------------------------------------
 // launcher
 // ----------------------------------------------------------------------------------------------
@@ -1019,6 +1032,12 @@ static int launch_round_t(const RoundParams& p, int ctas, cudaStream_t stream) {
   return int(p.n_links == 1 ? cudaLaunchKernelEx(&cfg, round_kernel<Q, kGroups, true>, p) : cudaLaunchKernelEx(&cfg, round_kernel<Q, kGroups, false>, p));
 }
 
+template <int Q, int kGroups>
+static int load_round_t(const RoundParams& p) {
+  cudaFuncAttributes a;
+  return int(p.n_links == 1 ? cudaFuncGetAttributes(&a, round_kernel<Q, kGroups, true>) : cudaFuncGetAttributes(&a, round_kernel<Q, kGroups, false>));
+}
+
 // Groups of a CTA.  A replica with one ring pair, or with one per link, is bound by HBM and by the length of a tile's
 // chain of operations: two groups with 96 registers a thread are enough and were 2 to 8 % faster than three with 72.
 // Several rings on one link (a mesh group) mean several frames to decode per tile, which more warps hide: 51 against
@@ -1029,6 +1048,20 @@ template <int Q>
 static int launch_round_q(const RoundParams& p, int shape, int ctas, cudaStream_t stream) {
   if (shape != 0 && shape != 1) return int(cudaErrorInvalidValue);
   return round_groups(shape, p.n_links, p.n_in) == 3 ? launch_round_t<Q, 3>(p, ctas, stream) : launch_round_t<Q, 2>(p, ctas, stream);
+}
+
+template <int Q>
+static int load_round_q(const RoundParams& p, int shape) {
+  return round_groups(shape, p.n_links, p.n_in) == 3 ? load_round_t<Q, 3>(p) : load_round_t<Q, 2>(p);
+}
+
+int load_round(const RoundParams& p, int shape) {
+  switch (p.bits) {
+    case 1: return load_round_q<1>(p, shape);
+    case 2: return load_round_q<2>(p, shape);
+    case 4: return load_round_q<4>(p, shape);
+    default: return load_round_q<8>(p, shape);
+  }
 }
 
 int launch_round(const RoundParams& p, int shape, int ctas, void* stream_v) {

@@ -128,11 +128,16 @@ enum StatusWord : int {
 // `shape` picks the CTA's make-up: 1 = two or three groups by the replica's rings, 0 = three groups (one CTA per SM
 // either way).  A group is eight compute warps and one service warp.
 int launch_round(const RoundParams& p, int shape, int ctas, void* stream);
+// Loads the kernel that launch_round would run (code is otherwise loaded on a kernel's first launch, which takes up to some
+// tens of milliseconds).
+int load_round(const RoundParams& p, int shape);
 int round_groups(int shape, int n_links, int n_in);
 // Takes back the frames of one out-ring that the receiver never acknowledged: their steps are subtracted from the
 // link's mirror and the ring's send counters fall back to the credits.  *taken_back (device) counts the tile-frames.
 int launch_unsend(float* mirror, const uint8_t* payload_remote, uint32_t* tx_seq, const uint32_t* credit, int n_tiles, int ring_slots,
                   int payload_bytes, int log2_block, int bits, int64_t n, uint64_t* taken_back, void* stream);
+// Adds to *count (pinned host memory) the frames that have been sent and not yet acknowledged, over all rings and tiles.
+int launch_count_unacknowledged(const RoundParams& p, uint32_t* count, void* stream);
 int round_smem_bytes(int groups, int slots, int payload_bytes);
 
 // Element-wise kernels (copyToTensor / addFromTensor / pushUpdate; src/sharedtensor.c:435-446, 334-344).

@@ -90,9 +90,11 @@ class GpuBackend:
     def flush(self, timeout_s: float) -> bool:
         import time
 
+        t0 = time.time()
+        if self.rep.engine_running() and self.rep.ring_peers() > 0 and self.rep.flush(_stream(self.device), int(timeout_s * 1000)):
+            return True
         names = _native.cuda().status_names()
         i_work, i_pend = names.index("last_work_count"), names.index("pending_tiles")
-        t0 = time.time()
         quiet = 0
         while time.time() - t0 < timeout_s:
             if not self.rep.engine_running():
