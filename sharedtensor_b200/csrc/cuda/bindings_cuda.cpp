@@ -108,6 +108,11 @@ PYBIND11_MODULE(_cuda, m) {
       .def_readwrite("chunk_tiles", &GpuConfig::chunk_tiles)
       .def_readwrite("window_tiles", &GpuConfig::window_tiles);
 
+  py::class_<TablePlan>(m, "TablePlan")
+      .def(py::init<int, const std::vector<int64_t>&, const std::vector<int64_t>&>())
+      .def("tensors", &TablePlan::tensors)
+      .def("scales", [](TablePlan& t, uintptr_t arena, uintptr_t s) { py::gil_scoped_release rel; return t.scales(ptr<float>(arena), strm(s)); });
+
   py::class_<GpuReplica>(m, "GpuReplica")
       .def(py::init<int, int64_t, const GpuConfig&>())
       .def("size", &GpuReplica::size)
@@ -143,6 +148,8 @@ PYBIND11_MODULE(_cuda, m) {
       .def("add_scaled_bf16", [](GpuReplica& r, uintptr_t g, float alpha, uintptr_t s) { r.add_scaled_bf16(ptr<void>(g), alpha, strm(s)); })
       .def("snapshot", [](GpuReplica& r, uintptr_t out, uintptr_t s) { r.snapshot(ptr<float>(out), strm(s)); })
       .def("snapshot_bf16", [](GpuReplica& r, uintptr_t out, uintptr_t s) { r.snapshot_bf16(ptr<void>(out), strm(s)); })
+      .def("table_add", [](GpuReplica& r, const TablePlan& t, const std::vector<uintptr_t>& p, uintptr_t s) { r.table_add(t, p, strm(s)); })
+      .def("table_copy", [](GpuReplica& r, const TablePlan& t, const std::vector<uintptr_t>& p, uintptr_t s) { r.table_copy(t, p, strm(s)); })
       .def("copy_mirror_from_values", &GpuReplica::copy_mirror_from_values)
       .def("round", &GpuReplica::round, py::arg("do_rx") = true, py::arg("do_tx") = true, py::arg("sweeps") = 1)
       .def("set_test_stall_tile", &GpuReplica::set_test_stall_tile)

@@ -475,6 +475,23 @@ void GpuReplica::add_scaled_bf16(const void* g, float alpha, void* user_stream) 
   updated();
 }
 
+void GpuReplica::table_add(const TablePlan& plan, const std::vector<uintptr_t>& tensors, void* user_stream) {
+  if (int(tensors.size()) != plan.tensors()) throw std::invalid_argument("the table has another number of tensors");
+  if (tensors.empty()) return;
+  DeviceGuard g(device_);
+  std::lock_guard<std::mutex> gate(gate_mu_);
+  plan.add(values(), tensors, ask_for_sms(user_stream, true), user_stream);
+  updated();
+}
+
+void GpuReplica::table_copy(const TablePlan& plan, const std::vector<uintptr_t>& tensors, void* user_stream) {
+  if (int(tensors.size()) != plan.tensors()) throw std::invalid_argument("the table has another number of tensors");
+  if (tensors.empty()) return;
+  DeviceGuard g(device_);
+  plan.copy(values(), tensors, ask_for_sms(user_stream, false), user_stream);
+  launches_ += 1;
+}
+
 void GpuReplica::updated() {
   epoch_++;
   launches_ += 1;

@@ -24,6 +24,7 @@
 #include <vector>
 
 #include "round.h"
+#include "table.hpp"
 #include "vmm.hpp"
 
 namespace st {
@@ -100,6 +101,9 @@ class GpuReplica {
   void gate_unlock() { gate_mu_.unlock(); }
   void add_gate_held(const float* delta);   // values += delta on the comm stream; the caller holds the gate
   void snapshot(float* out, void* user_stream);
+  // The values are the arena of a table: the caller's tensors (one address each) are added into it / filled from it.
+  void table_add(const TablePlan& plan, const std::vector<uintptr_t>& tensors, void* user_stream);
+  void table_copy(const TablePlan& plan, const std::vector<uintptr_t>& tensors, void* user_stream);
   void snapshot_bf16(void* out, void* user_stream);
   void copy_mirror_from_values(int link);                 // mirror <- values (neighbour is given a snapshot)
   void push_snapshot(int link, float* remote_values);     // neighbour's values <- values, mirror <- values

@@ -1,0 +1,272 @@
+// Kernels over a table of tensors (see table.hpp).  A table of a model has a few large tensors and many small ones: a copy
+// launch per tensor cost 2.1 ms of launches and gaps for the 148 tensors of GPT-2 small, whose bytes take 0.4 ms.
+#include <cuda_runtime.h>
+
+#include <algorithm>
+#include <cstring>
+#include <stdexcept>
+#include <string>
+
+#include "table.hpp"
+
+namespace st {
+
+struct Chunk {
+  uint32_t tensor;
+  uint32_t count;    // elements
+  int64_t start;     // element of the tensor
+  int64_t arena;     // element of the arena
+};
+struct SumChunk {
+  int64_t begin;     // elements of the arena
+  uint32_t count;
+  uint32_t segment;
+};
+struct SumSegment {
+  uint32_t first, chunks;  // its chunks
+  int64_t count;           // its elements
+};
+
+namespace {
+
+constexpr int kThreads = 256;
+constexpr int kChunk = 4096;          // a CTA's step: four 16-byte accesses per thread
+constexpr int kSumChunk = 1 << 14;    // of the sums
+constexpr int kPtrs = 256;            // tensors of one launch: their addresses travel as kernel parameters
+
+struct Pointers {
+  float* p[kPtrs];
+};
+
+void ck(cudaError_t e, const char* what) {
+  if (e != cudaSuccess) throw std::runtime_error(std::string("table of tensors: ") + what + ": " + cudaGetErrorString(e));
+}
+
+// ADD: arena += tensors (reductions at the L2), then the change marks of the arena tiles it touched, as an update does.
+// Otherwise tensors = arena.  Chunks are walked in arena order, every CTA takes every gridDim-th.
+template <bool ADD>
+__global__ void __launch_bounds__(kThreads, 8) table_kernel(float* __restrict__ arena, const Chunk* __restrict__ chunks, uint32_t n_chunks,
+                                                            uint32_t first_tensor, const __grid_constant__ Pointers ptrs, UpdateMarks m) {
+  for (uint32_t c = blockIdx.x; c < n_chunks; c += gridDim.x) {
+    const Chunk ch = chunks[c];
+    float* const t = ptrs.p[ch.tensor - first_tensor] + ch.start;
+    float* const a = arena + ch.arena;
+    if (ch.count == kChunk && (reinterpret_cast<uintptr_t>(t) & 15) == 0) {
+      const float4* src = reinterpret_cast<const float4*>(ADD ? t : a) + threadIdx.x;
+      float4 v[4];
+#pragma unroll
+      for (int i = 0; i < 4; i++) v[i] = __ldcs(src + i * kThreads);
+#pragma unroll
+      for (int i = 0; i < 4; i++) {
+        if (ADD)
+          asm volatile("red.global.add.v4.f32 [%0], {%1, %2, %3, %4};" ::"l"(reinterpret_cast<float4*>(a) + threadIdx.x + i * kThreads), "f"(v[i].x),
+                       "f"(v[i].y), "f"(v[i].z), "f"(v[i].w)
+                       : "memory");
+        else
+          __stcs(reinterpret_cast<float4*>(t) + threadIdx.x + i * kThreads, v[i]);
+      }
+    } else {
+      for (uint32_t e0 = threadIdx.x; e0 < ch.count; e0 += 8 * kThreads) {
+        float v[8];
+#pragma unroll
+        for (int i = 0; i < 8; i++)
+          if (e0 + i * kThreads < ch.count) v[i] = (ADD ? t : a)[e0 + i * kThreads];
+#pragma unroll
+        for (int i = 0; i < 8; i++) {
+          if (e0 + i * kThreads >= ch.count) continue;
+          if (ADD) atomicAdd(a + e0 + i * kThreads, v[i]);
+          else t[e0 + i * kThreads] = v[i];
+        }
+      }
+    }
+  }
+  if (ADD && m.tile_state != nullptr) {
+    __syncthreads();
+    if (threadIdx.x < 32) {
+      __threadfence();  // marks after the data
+      for (uint32_t c = blockIdx.x + threadIdx.x * gridDim.x; c < n_chunks; c += 32 * gridDim.x) {
+        const Chunk ch = chunks[c];
+        __stcg(m.tile_state + ch.arena / kTile, 1u);
+        __stcg(m.tile_state + (ch.arena + ch.count - 1) / kTile, 1u);
+      }
+    }
+  }
+  if (m.yield_word != nullptr && threadIdx.x == 0)
+    if (atomicInc(m.ticket, gridDim.x - 1) >= gridDim.x - 1) *reinterpret_cast<volatile uint32_t*>(m.yield_word) = 0u;
+}
+
+// Sums of squares in double precision.  A CTA takes every gridDim-th chunk and leaves a partial sum; whoever finishes a
+// segment's last chunk adds the segment's partial sums up in their fixed order, so that the result does not depend on who
+// that is, and writes it to the host.  One launch instead of three.
+__global__ void __launch_bounds__(kThreads, 8) table_sums_kernel(const float* __restrict__ arena, const SumChunk* __restrict__ chunks, uint32_t n_chunks,
+                                                                 const SumSegment* __restrict__ segments, double* __restrict__ partials,
+                                                                 uint32_t* __restrict__ counters, double* __restrict__ out, int n_seg) {
+  __shared__ double red[kThreads / 32];
+  __shared__ bool s_last;
+  const bool aligned = (reinterpret_cast<uintptr_t>(arena) & 15) == 0;
+  for (uint32_t c = blockIdx.x; c < n_chunks; c += gridDim.x) {
+    const SumChunk ch = chunks[c];
+    double s0 = 0.0, s1 = 0.0;
+    uint32_t at = 0;
+    if (aligned) {
+      const float4* x = reinterpret_cast<const float4*>(arena + ch.begin);  // (segments start on multiples of four)
+      const uint32_t n4 = ch.count / 4;
+      uint32_t i = threadIdx.x;
+      for (; i + 3 * kThreads < n4; i += 4 * kThreads) {
+        float4 v[4];
+#pragma unroll
+        for (int u = 0; u < 4; u++) v[u] = __ldcs(x + i + u * kThreads);
+#pragma unroll
+        for (int u = 0; u < 4; u++) {
+          s0 += double(v[u].x) * double(v[u].x) + double(v[u].y) * double(v[u].y);
+          s1 += double(v[u].z) * double(v[u].z) + double(v[u].w) * double(v[u].w);
+        }
+      }
+      for (; i < n4; i += kThreads) {
+        const float4 v = __ldcs(x + i);
+        s0 += double(v.x) * double(v.x) + double(v.y) * double(v.y);
+        s1 += double(v.z) * double(v.z) + double(v.w) * double(v.w);
+      }
+      at = n4 * 4;
+    }
+    for (uint32_t i = at + threadIdx.x; i < ch.count; i += kThreads) s0 += double(arena[ch.begin + i]) * double(arena[ch.begin + i]);
+    double acc = s0 + s1;
+    for (int o = 16; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
+    if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = acc;
+    __syncthreads();
+    const SumSegment sg = segments[ch.segment];
+    if (threadIdx.x == 0) {
+      double t = 0.0;
+      for (int w = 0; w < kThreads / 32; w++) t += red[w];
+      __stcg(partials + c, t);
+      __threadfence();
+      s_last = atomicAdd(counters + ch.segment, 1u) == sg.chunks - 1;
+    }
+    __syncthreads();
+    if (s_last && threadIdx.x < 32) {
+      __threadfence();
+      double t = 0.0;
+      for (uint32_t i = threadIdx.x; i < sg.chunks; i += 32) t += __ldcg(partials + sg.first + i);
+      for (int o = 16; o > 0; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
+      if (threadIdx.x == 0) {
+        counters[ch.segment] = 0u;
+        int e = -128;
+        if (t > 0.0) {
+          int ex;
+          frexp(sqrt(t / double(sg.count)), &ex);
+          e = ex - 1 < -126 ? -128 : min(ex - 1, 127);
+        }
+        out[ch.segment] = t;
+        out[n_seg + ch.segment] = double(e);
+      }
+    }
+    __syncthreads();  // red and s_last are reused by the next chunk
+  }
+}
+
+int blocks_for(uint32_t chunks) { return int(chunks < 148u * 8u ? chunks : 148u * 8u); }
+
+struct OnDevice {
+  int prev = -1;
+  explicit OnDevice(int dev) {
+    cudaGetDevice(&prev);
+    if (prev != dev) cudaSetDevice(dev);
+    else prev = -1;
+  }
+  ~OnDevice() {
+    if (prev >= 0) cudaSetDevice(prev);
+  }
+};
+
+}  // namespace
+
+TablePlan::TablePlan(int device, const std::vector<int64_t>& offsets, const std::vector<int64_t>& sizes) : device_(device), n_(int(sizes.size())) {
+  if (offsets.size() != sizes.size() + 1) throw std::invalid_argument("a table has one more offset than tensors");
+  std::vector<Chunk> chunks;
+  std::vector<SumChunk> sum_chunks;
+  std::vector<SumSegment> segments;
+  for (int k = 0; k < n_; k++) {
+    if ((offsets[k] & 3) != 0 || sizes[k] < 0 || offsets[k + 1] < offsets[k] + sizes[k]) throw std::invalid_argument("offsets and sizes of a table contradict each other");
+    first_chunk_.push_back(uint32_t(chunks.size()));
+    for (int64_t at = 0; at < sizes[k]; at += kChunk)
+      chunks.push_back({uint32_t(k), uint32_t(std::min<int64_t>(kChunk, sizes[k] - at)), at, offsets[k] + at});
+    const int64_t len = offsets[k + 1] - offsets[k];
+    segments.push_back({uint32_t(sum_chunks.size()), uint32_t((len + kSumChunk - 1) / kSumChunk), len});
+    for (int64_t at = 0; at < len; at += kSumChunk)
+      sum_chunks.push_back({offsets[k] + at, uint32_t(std::min<int64_t>(kSumChunk, len - at)), uint32_t(k)});
+  }
+  first_chunk_.push_back(uint32_t(chunks.size()));
+  n_chunks_ = uint32_t(chunks.size());
+  n_sum_chunks_ = uint32_t(sum_chunks.size());
+  // one block of device memory, laid out on the host and copied in one go
+  auto padded = [](size_t v) { return (v + 255) / 256 * 256; };
+  const size_t o_sum = padded(chunks.size() * sizeof(Chunk)), o_seg = o_sum + padded(sum_chunks.size() * sizeof(SumChunk)),
+               o_cnt = o_seg + padded(segments.size() * sizeof(SumSegment)), o_par = o_cnt + padded(size_t(n_) * 4), bytes = o_par + padded(sum_chunks.size() * 8) + 256;
+  std::vector<uint8_t> host(o_par, 0);
+  if (!chunks.empty()) std::memcpy(host.data(), chunks.data(), chunks.size() * sizeof(Chunk));
+  if (!sum_chunks.empty()) std::memcpy(host.data() + o_sum, sum_chunks.data(), sum_chunks.size() * sizeof(SumChunk));
+  if (!segments.empty()) std::memcpy(host.data() + o_seg, segments.data(), segments.size() * sizeof(SumSegment));
+  OnDevice on(device_);
+  ck(cudaMalloc(&dev_, bytes), "cudaMalloc");
+  ck(cudaMallocHost(reinterpret_cast<void**>(&host_), (size_t(n_) * 2 + 1) * 8), "cudaMallocHost");
+  ck(cudaMemcpy(dev_, host.data(), o_par, cudaMemcpyHostToDevice), "cudaMemcpy");
+  uint8_t* d = static_cast<uint8_t*>(dev_);
+  chunks_ = reinterpret_cast<Chunk*>(d);
+  sum_chunks_ = reinterpret_cast<SumChunk*>(d + o_sum);
+  sum_segments_ = reinterpret_cast<SumSegment*>(d + o_seg);
+  counters_ = reinterpret_cast<uint32_t*>(d + o_cnt);
+  partials_ = reinterpret_cast<double*>(d + o_par);
+}
+
+TablePlan::~TablePlan() {
+  OnDevice on(device_);
+  cudaFree(dev_);
+  if (host_) cudaFreeHost(host_);
+}
+
+// The request for SMs is taken back by the last of several launches, the marks are set by each.
+template <bool ADD>
+static void launch_table(float* arena, const std::vector<uintptr_t>& ptrs, const Chunk* chunks, const std::vector<uint32_t>& first_chunk, UpdateMarks m,
+                         void* stream) {
+  const int n = int(ptrs.size());
+  UpdateMarks inner = m;
+  inner.yield_word = nullptr;
+  for (int k0 = 0; k0 < n; k0 += kPtrs) {
+    const int k1 = std::min(n, k0 + kPtrs);
+    Pointers p;
+    for (int k = k0; k < k1; k++) p.p[k - k0] = reinterpret_cast<float*>(ptrs[k]);
+    const uint32_t c0 = first_chunk[k0], count = first_chunk[k1] - c0;
+    if (count == 0 && (k1 < n || m.yield_word == nullptr)) continue;
+    table_kernel<ADD><<<count ? blocks_for(count) : 1, kThreads, 0, static_cast<cudaStream_t>(stream)>>>(arena, chunks + c0, count, uint32_t(k0), p,
+                                                                                                         k1 == n ? m : inner);
+    ck(cudaGetLastError(), "kernel launch");
+  }
+}
+
+void TablePlan::add(float* arena, const std::vector<uintptr_t>& ptrs, const UpdateMarks& m, void* stream) const {
+  launch_table<true>(arena, ptrs, chunks_, first_chunk_, m, stream);
+}
+
+void TablePlan::copy(const float* arena, const std::vector<uintptr_t>& ptrs, const UpdateMarks& m, void* stream) const {
+  launch_table<false>(const_cast<float*>(arena), ptrs, chunks_, first_chunk_, m, stream);
+}
+
+std::pair<std::vector<double>, std::vector<int>> TablePlan::scales(const float* arena, void* stream) {
+  OnDevice on(device_);
+  std::lock_guard<std::mutex> lk(mu_);
+  for (int k = 0; k < n_; k++) {  // (segments without elements)
+    host_[k] = 0.0;
+    host_[n_ + k] = -128.0;
+  }
+  if (n_sum_chunks_) {
+    table_sums_kernel<<<blocks_for(n_sum_chunks_), kThreads, 0, static_cast<cudaStream_t>(stream)>>>(arena, sum_chunks_, n_sum_chunks_, sum_segments_, partials_,
+                                                                                                    counters_, host_, n_);
+    ck(cudaGetLastError(), "kernel launch");
+    ck(cudaStreamSynchronize(static_cast<cudaStream_t>(stream)), "cudaStreamSynchronize");
+  }
+  std::vector<int> exps(n_);
+  for (int k = 0; k < n_; k++) exps[k] = int(host_[n_ + k]);
+  return {std::vector<double>(host_, host_ + n_), std::move(exps)};
+}
+
+}  // namespace st

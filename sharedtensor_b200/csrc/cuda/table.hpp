@@ -1,0 +1,44 @@
+// A table of tensors inside one shared arena: what is laid out once per table and the launches over it (host-visible, no
+// CUDA syntax).  The tensors themselves stay where the caller has them: one kernel adds all of them into the arena, or
+// fills all of them from it, and one kernel reads the arena for the per-tensor magnitudes.
+#pragma once
+#include <cstdint>
+#include <mutex>
+#include <utility>
+#include <vector>
+
+#include "round.h"
+
+namespace st {
+
+class TablePlan {
+ public:
+  // Tensor k covers elements offsets[k] .. offsets[k] + sizes[k] - 1 of the arena; its segment ends where the next one
+  // starts (offsets has one more entry, the arena's size).  Offsets are multiples of 4.
+  TablePlan(int device, const std::vector<int64_t>& offsets, const std::vector<int64_t>& sizes);
+  ~TablePlan();
+  TablePlan(const TablePlan&) = delete;
+
+  int tensors() const { return n_; }
+  // arena[k] += *ptrs[k], a reduction at the L2, for every tensor; *ptrs[k] = arena[k].  fp32 tensors of this device,
+  // tensors() addresses.
+  void add(float* arena, const std::vector<uintptr_t>& ptrs, const UpdateMarks& m, void* stream) const;
+  void copy(const float* arena, const std::vector<uintptr_t>& ptrs, const UpdateMarks& m, void* stream) const;
+  // Per segment the sum of squares and floor(log2(rms)) (-128: all zero) of `arena`; waits for the stream.
+  std::pair<std::vector<double>, std::vector<int>> scales(const float* arena, void* stream);
+
+ private:
+  int device_, n_;
+  uint32_t n_chunks_ = 0, n_sum_chunks_ = 0;
+  void* dev_ = nullptr;                 // everything below, one allocation
+  struct Chunk* chunks_ = nullptr;      // pieces of at most kChunk elements of the tensors, in arena order
+  std::vector<uint32_t> first_chunk_;   // of each tensor
+  struct SumChunk* sum_chunks_ = nullptr;  // the same over whole segments, for the sums
+  struct SumSegment* sum_segments_ = nullptr;
+  double* partials_ = nullptr;
+  uint32_t* counters_ = nullptr;        // chunks of a segment that are done (zero between launches)
+  double* host_ = nullptr;              // pinned: sums, then exponents
+  std::mutex mu_;                       // scales() uses partials_, counters_ and host_
+};
+
+}  // namespace st

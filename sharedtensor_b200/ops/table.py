@@ -11,7 +11,8 @@ from typing import Mapping
 
 import torch
 
-from ..api import SharedTensor, createOrFetch
+from ..api import SharedTensor, _Range, createOrFetch
+from ..parallel.gpu_backend import _stream
 
 
 class TableLayout:
@@ -51,15 +52,57 @@ class SharedTable:
         self.shared = shared
         self.layout = layout
         self._scratch: torch.Tensor | None = None
+        self._items = [(k, layout.shapes[k]) for k in layout.names]
+        self._plan = None            # GPU replicas: the native layout of the table
+        self._native_plan()
+
+    # ---- GPU replicas: all tensors in one kernel
+    def _native_plan(self):
+        """(replica, plan) of a GPU replica, else None."""
+        rep = getattr(self.shared._b, "rep", None)
+        if rep is None or not self._items:
+            return None
+        if self._plan is None:
+            from .. import _native
+
+            sizes = [shape.numel() for _, shape in self._items]
+            self._plan = _native.cuda().TablePlan(self.shared.device.index, self.layout.segment_offsets(), sizes)
+        return rep, self._plan
+
+    def _addresses(self, tensors: Mapping[str, torch.Tensor], written: bool) -> list[int] | None:
+        """The tensors' addresses, or None if one of them needs a conversion, a broadcast or autograd on the way."""
+        index, tracked = self.shared.device.index, written and torch.is_grad_enabled()
+        f32, strided = torch.float32, torch.strided
+        out = []
+        for k, shape in self._items:
+            t = tensors[k]
+            if (t.dtype is not f32 or t.layout is not strided or t.shape != shape or t.get_device() != index or not t.is_contiguous()
+                    or (tracked and t.requires_grad)):
+                return None
+            out.append(t.data_ptr())
+        if written and len(set(out)) < len(out):
+            return None  # names that share a tensor: one after the other
+        return out
 
     # ---- dict-of-tensors interface
     def copyToTensors(self, out: Mapping[str, torch.Tensor]) -> None:
+        native = self._native_plan()
+        if native is not None and (addresses := self._addresses(out, True)) is not None:
+            with _Range(self.shared.cfg.nvtx, "sharedtensor.copyToTensor"):
+                native[0].table_copy(native[1], addresses, _stream(self.shared.device))
+            torch.autograd.graph.increment_version([out[k] for k in self.layout.names])
+            return
         flat = self._flat()
         self.shared.copyToTensor(flat)
         for k, v in self.layout.views(flat).items():
             out[k].copy_(v)
 
     def addFromTensors(self, deltas: Mapping[str, torch.Tensor]) -> None:
+        native = self._native_plan()
+        if native is not None and (addresses := self._addresses(deltas, False)) is not None:
+            with _Range(self.shared.cfg.nvtx, "sharedtensor.addFromTensor"):
+                native[0].table_add(native[1], addresses, _stream(self.shared.device))
+            return
         flat = self._flat()
         flat.zero_()
         self.layout.pack(deltas, flat)
@@ -87,6 +130,11 @@ class SharedTable:
     # ---- per-tensor magnitudes
     def scales(self, flat: torch.Tensor | None = None) -> dict[str, dict]:
         """Per-tensor sum of squares and floor(log2(rms)) of the current values (or of ``flat``)."""
+        native = self._native_plan()
+        if native is not None and (flat is None or flat.get_device() == self.shared.device.index):
+            arena = native[0].values_ptr() if flat is None else flat.data_ptr()
+            sums_l, exps_l = native[1].scales(arena, _stream(self.shared.device))
+            return {k: {"sumsq": s, "rms_exp": e} for k, s, e in zip(self.layout.names, sums_l, exps_l)}
         src = flat
         if src is None:
             src = self._flat()

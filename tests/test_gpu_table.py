@@ -1,0 +1,57 @@
+"""The kernels over a table of tensors against PyTorch."""
+import math
+
+import pytest
+import torch
+
+import sharedtensor
+
+pytestmark = pytest.mark.gpu
+
+
+def _table(sizes, offset=0, seed=0):
+    g = torch.Generator(device="cuda").manual_seed(seed)
+    return {f"t{i}": torch.randn(n + offset, generator=g, device="cuda")[offset:] * 2.0 ** -(i % 7) for i, n in enumerate(sizes)}
+
+
+@pytest.mark.parametrize("sizes,offset", [
+    ([1], 0), ([3, 1, 5], 1), ([4095, 4096, 4097, 31, 33], 0), ([4097, 8192], 3), ([16384 * 3 + 5, 2, 16384], 0),
+    ([7] * 300, 0), ([100_003, 1, 2_000_001], 2)])
+def test_table_of_tensors(free_port, sizes, offset):
+    """One tensor, tensors around the chunk sizes, misaligned ones, and more tensors than one launch takes."""
+    init = _table(sizes)
+    tab = sharedtensor.createOrFetchTable("127.0.0.1", free_port, init)
+    try:
+        deltas = _table(sizes, seed=1)
+        store = {k: torch.zeros(v.numel() + offset, device="cuda") for k, v in init.items()}
+        out = {k: v[offset:] for k, v in store.items()}
+        for _ in range(2):
+            tab.addFromTensors({k: torch.cat([torch.zeros(offset, device="cuda"), v])[offset:] for k, v in deltas.items()})
+            tab.copyToTensors(out)
+        for k in init:
+            assert torch.equal(out[k], (init[k] + deltas[k]) + deltas[k]), k
+            assert not store[k][:offset].any()
+        flat = tab.copyToFlat(tab.new_flat())
+        assert float(flat.double().abs().sum()) == pytest.approx(sum(float(v.double().abs().sum()) for v in out.values()), rel=1e-12)
+        for got in (tab.scales(), tab.scales(flat)):
+            for k, v in out.items():
+                sumsq = float(v.double().square().sum())
+                padded = (v.numel() + 31) // 32 * 32
+                assert got[k]["sumsq"] == pytest.approx(sumsq, rel=1e-12), k
+                assert got[k]["rms_exp"] == math.floor(math.log2(math.sqrt(sumsq / padded))), k
+    finally:
+        tab.close()
+
+
+def test_table_tensors_that_need_a_conversion(free_port):
+    init = {"a": torch.randn(40, 30, device="cuda"), "b": torch.randn(7, device="cuda")}
+    tab = sharedtensor.createOrFetchTable("127.0.0.1", free_port, init)
+    try:
+        tab.addFromTensors({"a": torch.ones(30, 40, device="cuda").t(), "b": torch.ones(7, dtype=torch.float64)})
+        out = {"a": torch.empty(30, 40, device="cuda").t(), "b": torch.empty(7, dtype=torch.bfloat16, device="cuda")}
+        tab.copyToTensors(out)
+        assert torch.equal(out["a"], init["a"] + 1) and torch.equal(out["b"], (init["b"] + 1).to(torch.bfloat16))
+        with pytest.raises(RuntimeError):
+            tab.addFromTensors({"a": torch.ones(3, device="cuda"), "b": torch.ones(7, device="cuda")})
+    finally:
+        tab.close()
