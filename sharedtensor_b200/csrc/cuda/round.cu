@@ -31,6 +31,7 @@
 // matter), so codes, scales, mirrors and values are bit-identical to the host codec (../core/codec.cpp).
 #include <cuda_runtime.h>
 
+#include <atomic>
 #include <cstdint>
 
 #include "round.h"
@@ -144,7 +145,6 @@ struct __align__(16) TileDesc {
 constexpr uint32_t kDescNoValues = 2;       // the visit only receives: the values are not loaded, what arrived goes into them as a reduction
 constexpr uint32_t kDescTxOk = 1u << 4;     // << link: every out-ring of the link has room
 constexpr uint32_t kDescRxLink = 1u << 8;   // << link: at least one frame arrived on the link
-constexpr int kDescFrameShift = 16;         // + 5 * link: 1 + the place in the frame list of the only frame that arrived on the link (0: none or several)
 constexpr uint32_t kDescTxWant = 1u << 12;  // << link: the link may have something to hear: the tile changed here, or frames arrived on another link
 // what a compute warp adds to a tile's `done` word when it has finished its part
 constexpr uint32_t kDoneWarp = 1, kDoneWarps = 0xff;
@@ -432,27 +432,57 @@ __device__ __forceinline__ bool claim_tile(GroupShared& sh, uint32_t c) {
 // The frames of a tile, as the service warp listed them: address | link, in ring order and sequence order.
 __device__ __forceinline__ const uint8_t* frame_at(uint64_t e) { return reinterpret_cast<const uint8_t*>(e & ~15ull); }
 
-// acc = the sum of the steps of the tile's frames (`only_link` < 0: of all of them).  Two frames are fetched at a time.
-template <int Q>
-__device__ __forceinline__ void decode_frames(const RoundParams& p, const uint64_t* list, int count, int only_link, int warp, int lane,
-                                              int left, Piece (&acc)[kPieces]) {
+__device__ __forceinline__ void get_stash(const float* stash, int link, Piece (&x)[kPieces]) {
 #pragma unroll
-  for (int i = 0; i < kPieces; i++) acc[i] = {0ull, 0ull};
-  for (int j = 0; j < count; j += 2) {
-    const uint64_t ea = list[j], eb = j + 1 < count ? list[j + 1] : 0ull;
-    const bool ua = only_link < 0 || int(ea & 15u) == only_link, ub = eb != 0 && (only_link < 0 || int(eb & 15u) == only_link);
-    FrameRegs a, b;
-    if (ua) load_frame<Q>(frame_at(ea), warp, lane, p.log2_block, a);
-    if (ub) load_frame<Q>(frame_at(eb), warp, lane, p.log2_block, b);
-    if (ua) {
-#pragma unroll
-      for (int i = 0; i < kPieces; i++) add4(acc[i], frame_steps<Q>(a.w[i], a.code(i), Q == 1 ? valid4(left, i) : 0xfu));
-    }
-    if (ub) {
-#pragma unroll
-      for (int i = 0; i < kPieces; i++) add4(acc[i], frame_steps<Q>(b.w[i], b.code(i), Q == 1 ? valid4(left, i) : 0xfu));
-    }
+  for (int i = 0; i < kPieces; i++) {
+    const ulonglong2 y = *reinterpret_cast<const ulonglong2*>(stash + link * kTile + i * 128);
+    x[i] = {y.x, y.y};
   }
+}
+
+// total = the sum of the steps of the tile's frames, in list order; kStash: what came on each link is summed up besides, and
+// left in this lane's part of the link's stash (shared memory; a frame is decoded once, however many links hear of it: a hub
+// with three links and six frames per tile took 224 us per 16 M elements when it decoded them for the values and again for
+// each mirror, 170 us so).  The loop stays rolled: unrolled by four frames it was slower for every number of rings, the code
+// of a tile's visit then no longer fits the instruction cache.
+template <int Q, bool kStash>
+__device__ __forceinline__ void decode_frames(const uint64_t* list, int count, int log2_block, int warp, int lane, int left, float* stash,
+                                              Piece (&total)[kPieces]) {
+  constexpr int kDeep = kStash ? 0 : 1;  // frames on their way while one is decoded (the stash variant has no registers left for it)
+  Piece mine[kPieces];
+  int cur = -1;
+  uint32_t seen = 0;
+#pragma unroll
+  for (int i = 0; i < kPieces; i++) total[i] = {0ull, 0ull};
+  auto put = [&](int link) {
+#pragma unroll
+    for (int i = 0; i < kPieces; i++) *reinterpret_cast<ulonglong2*>(stash + link * kTile + i * 128) = make_ulonglong2(mine[i].a, mine[i].b);
+  };
+  FrameRegs f[kDeep + 1];
+  if (kDeep > 0) load_frame<Q>(frame_at(list[0]), warp, lane, log2_block, f[0]);
+#pragma unroll 1
+  for (int j = 0; j < count; j++) {
+    if (kDeep == 0 || j + kDeep < count) load_frame<Q>(frame_at(list[j + kDeep]), warp, lane, log2_block, f[kDeep]);
+    if (kStash) {
+      const int link = int(list[j] & 15u);
+      if (link != cur) {
+        if (cur >= 0) put(cur);
+#pragma unroll
+        for (int i = 0; i < kPieces; i++) mine[i] = {0ull, 0ull};
+        if ((seen >> link) & 1u) get_stash(stash, link, mine);
+        cur = link;
+        seen |= 1u << link;
+      }
+    }
+#pragma unroll
+    for (int i = 0; i < kPieces; i++) {
+      const Piece st = frame_steps<Q>(f[0].w[i], f[0].code(i), Q == 1 ? valid4(left, i) : 0xfu);
+      add4(total[i], st);
+      if (kStash) add4(mine[i], st);
+    }
+    if (kDeep > 0) f[0] = f[kDeep];
+  }
+  if (kStash && cur >= 0) put(cur);
 }
 
 // One lane's codes of its four pieces into the ring slots of link l's neighbours.  They go through shared memory, so
@@ -494,7 +524,7 @@ __device__ __forceinline__ void send_codes(const uint64_t* list, int count, int 
 
 // kOneLink: one link (a leaf of the tree, a member of a mesh group); what arrived for the values is what arrived on it.
 template <int Q, bool kOneLink>
-__device__ __forceinline__ void compute_warp(const RoundParams& p, GroupShared& sh, int warp, int lane) {
+__device__ __forceinline__ void compute_warp(const RoundParams& p, GroupShared& sh, float* group_stash, int warp, int lane) {
   const int L = kOneLink ? 1 : p.n_links, lb = p.log2_block;
   float res_max0 = 0.f, res_max1 = 0.f, res_max2 = 0.f;
   uint32_t exchanges = 0;
@@ -544,7 +574,7 @@ __device__ __forceinline__ void compute_warp(const RoundParams& p, GroupShared& 
       }
     } else {
       Piece acc[kPieces];
-      decode_frames<Q>(p, frames, d.n_frames, -1, warp, lane, left, acc);
+      decode_frames<Q, !kOneLink>(frames, d.n_frames, lb, warp, lane, left, group_stash + in_tile, acc);
 #pragma unroll
       for (int i = 0; i < kPieces; i++) {
         v[i] = load_v ? load_piece(vp + i * 128) : Piece{0ull, 0ull};
@@ -569,15 +599,14 @@ __device__ __forceinline__ void compute_warp(const RoundParams& p, GroupShared& 
       bool changed = false;
       if (d.flags & (kDescRxLink << l)) {
         if (!kOneLink && applied != l) {
-          const uint32_t only = (d.flags >> (kDescFrameShift + 5 * l)) & 31u;
-          if (only) {
+          if (d.n_frames == 1) {
             FrameRegs f;
-            load_frame<Q>(frame_at(frames[only - 1u]), warp, lane, lb, f);
+            load_frame<Q>(frame_at(frames[0]), warp, lane, lb, f);
 #pragma unroll
             for (int i = 0; i < kPieces; i++) add4(k[i], frame_steps<Q>(f.w[i], f.code(i), Q == 1 ? valid4(left, i) : 0xfu));
           } else {
             Piece acc[kPieces];
-            decode_frames<Q>(p, frames, d.n_frames, l, warp, lane, left, acc);
+            get_stash(group_stash + in_tile, l, acc);
 #pragma unroll
             for (int i = 0; i < kPieces; i++) add4(k[i], acc[i]);
           }
@@ -663,7 +692,8 @@ __device__ __forceinline__ void compute_warp(const RoundParams& p, GroupShared& 
 // lane, or on a ballot.
 __device__ __forceinline__ void service_warp(const RoundParams& p, GroupShared& sh, int g, int n_groups, int lane) {
   // The group's tiles: a run of `chunk` consecutive tiles, or (chunk == 0) every gstride-th tile of the launch's window.
-  const int gidx = int(blockIdx.x) * n_groups + g;
+  // The groups of a CTA are a grid apart, so that the odd tiles of the last turn fall on all SMs alike.
+  const int gidx = p.chunk > 0 ? int(blockIdx.x) * n_groups + g : g * int(gridDim.x) + int(blockIdx.x);
   const int gid0 = p.chunk > 0 ? gidx * p.chunk : gidx;
   const int gstride = p.chunk > 0 ? 1 : int(gridDim.x) * n_groups;
   const int my_count = p.chunk > 0 ? max(0, min(p.chunk, p.tile_count - gid0))
@@ -759,11 +789,6 @@ __device__ __forceinline__ void service_warp(const RoundParams& p, GroupShared& 
           const uint32_t full = __ballot_sync(0xffffffffu, is_out && out.link == l && !room) & same_tile;
           const bool want = dirty != 0 || (in1 & same_tile & ~here) != 0;
           const bool ok = want && outs != 0 && full == 0;
-          if (here) {
-            const uint32_t first = same_tile & ((here & (0u - here)) - 1u);
-            if (__popc(in1 & here) == 1 && (in2 & here) == 0)
-              flags |= uint32_t(1 + __popc(in1 & first) + __popc(in2 & first) + __popc(in3 & first)) << (kDescFrameShift + 5 * l);
-          }
           flags |= (ok ? kDescTxOk << l : 0u) | (here ? kDescRxLink << l : 0u) | (want ? kDescTxWant << l : 0u);
           goes_out |= ok && is_out && out.link == l;
         }
@@ -935,6 +960,7 @@ __device__ __forceinline__ void service_warp(const RoundParams& p, GroupShared& 
 template <int Q, int kGroups, bool kOneLink>
 __global__ void __launch_bounds__(kGroups * kGroupThreads, 1) round_kernel(const __grid_constant__ RoundParams p) {
   __shared__ GroupShared shared[kGroups];
+  extern __shared__ __align__(16) float stash[];  // several links: [group][link][element of the tile]
   const int g = int(threadIdx.x) / kGroupThreads, warp = (int(threadIdx.x) % kGroupThreads) >> 5, lane = threadIdx.x & 31;
   if (threadIdx.x < kGroups) {
     GroupShared& sh = shared[threadIdx.x];
@@ -945,7 +971,7 @@ __global__ void __launch_bounds__(kGroups * kGroupThreads, 1) round_kernel(const
   }
   __syncthreads();  // the only CTA-wide barrier: from here on the groups, and the two kinds of warp, run on their own
   if (warp == kComputeWarps) service_warp(p, shared[g], g, kGroups, lane);
-  else compute_warp<Q, kOneLink>(p, shared[g], warp, lane);
+  else compute_warp<Q, kOneLink>(p, shared[g], stash + (kOneLink ? 0 : g * kMaxLinks * kTile), warp, lane);
 }
 
 // ----------------------------------------------------------------------------------------------
@@ -1016,11 +1042,35 @@ int launch_count_unacknowledged(const RoundParams& p, uint32_t* count, void* str
 // ----------------------------------------------------------------------------------------------
 // launcher
 // ----------------------------------------------------------------------------------------------
+template <int kGroups>
+static constexpr int stash_bytes(bool one_link) { return one_link ? 0 : kGroups * kMaxLinks * kTile * 4; }
+
+// Loads the kernel and, once per device, gives it its shared memory.
+template <int Q, int kGroups, bool kOneLink>
+static int load_round_l() {
+  static std::atomic<uint64_t> loaded{0};
+  int dev = 0;
+  cudaGetDevice(&dev);
+  if ((loaded.load(std::memory_order_relaxed) >> (dev & 63)) & 1u) return 0;
+  cudaFuncAttributes a;
+  cudaError_t e = cudaFuncGetAttributes(&a, round_kernel<Q, kGroups, kOneLink>);
+  if (e == cudaSuccess && !kOneLink)
+    e = cudaFuncSetAttribute(round_kernel<Q, kGroups, kOneLink>, cudaFuncAttributeMaxDynamicSharedMemorySize, stash_bytes<kGroups>(false));
+  if (e == cudaSuccess) loaded.fetch_or(1ull << (dev & 63), std::memory_order_relaxed);
+  return int(e);
+}
+template <int Q, int kGroups>
+static int load_round_t(const RoundParams& p) {
+  return p.n_links == 1 ? load_round_l<Q, kGroups, true>() : load_round_l<Q, kGroups, false>();
+}
+
 template <int Q, int kGroups>
 static int launch_round_t(const RoundParams& p, int ctas, cudaStream_t stream) {
+  if (const int e = load_round_t<Q, kGroups>(p)) return e;
   cudaLaunchConfig_t cfg{};
   cfg.gridDim = dim3(ctas);
   cfg.blockDim = dim3(kGroups * kGroupThreads);
+  cfg.dynamicSmemBytes = stash_bytes<kGroups>(p.n_links == 1);
   cfg.stream = stream;
   // Every window but a cycle's first may start while the window before it is running out: the two have no tile in common.
   // (The first one clears counters that the launch before it may still add to.)
@@ -1030,12 +1080,6 @@ static int launch_round_t(const RoundParams& p, int ctas, cudaStream_t stream) {
   cfg.attrs = &early;
   cfg.numAttrs = p.follows_window ? 1 : 0;
   return int(p.n_links == 1 ? cudaLaunchKernelEx(&cfg, round_kernel<Q, kGroups, true>, p) : cudaLaunchKernelEx(&cfg, round_kernel<Q, kGroups, false>, p));
-}
-
-template <int Q, int kGroups>
-static int load_round_t(const RoundParams& p) {
-  cudaFuncAttributes a;
-  return int(p.n_links == 1 ? cudaFuncGetAttributes(&a, round_kernel<Q, kGroups, true>) : cudaFuncGetAttributes(&a, round_kernel<Q, kGroups, false>));
 }
 
 // Groups of a CTA.  A replica with one ring pair, or with one per link, is bound by HBM and by the length of a tile's

@@ -31,7 +31,8 @@ namespace {
 
 constexpr int kThreads = 256;
 constexpr int kChunk = 4096;          // a CTA's step: four 16-byte accesses per thread
-constexpr int kSumChunk = 1 << 14;    // of the sums
+constexpr int64_t kSumRange = 2048;   // the sums: elements of the arena that a CTA takes at least
+constexpr int kSumCtas = 148 * 8;
 constexpr int kPtrs = 256;            // tensors of one launch: their addresses travel as kernel parameters
 
 struct Pointers {
@@ -95,16 +96,18 @@ __global__ void __launch_bounds__(kThreads, 8) table_kernel(float* __restrict__ 
     if (atomicInc(m.ticket, gridDim.x - 1) >= gridDim.x - 1) *reinterpret_cast<volatile uint32_t*>(m.yield_word) = 0u;
 }
 
-// Sums of squares in double precision.  A CTA takes every gridDim-th chunk and leaves a partial sum; whoever finishes a
+// Sums of squares in double precision.  The arena is cut into equal ranges, one per CTA, and those into chunks where a
+// segment ends: nobody waits for a last wave, and a CTA reduces over its threads once per chunk.  Whoever finishes a
 // segment's last chunk adds the segment's partial sums up in their fixed order, so that the result does not depend on who
 // that is, and writes it to the host.  One launch instead of three.
-__global__ void __launch_bounds__(kThreads, 8) table_sums_kernel(const float* __restrict__ arena, const SumChunk* __restrict__ chunks, uint32_t n_chunks,
-                                                                 const SumSegment* __restrict__ segments, double* __restrict__ partials,
+__global__ void __launch_bounds__(kThreads, 8) table_sums_kernel(const float* __restrict__ arena, const SumChunk* __restrict__ chunks,
+                                                                 const uint32_t* __restrict__ first_chunk, const SumSegment* __restrict__ segments, double* __restrict__ partials,
                                                                  uint32_t* __restrict__ counters, double* __restrict__ out, int n_seg) {
   __shared__ double red[kThreads / 32];
   __shared__ bool s_last;
   const bool aligned = (reinterpret_cast<uintptr_t>(arena) & 15) == 0;
-  for (uint32_t c = blockIdx.x; c < n_chunks; c += gridDim.x) {
+  const uint32_t c1 = first_chunk[blockIdx.x + 1];
+  for (uint32_t c = first_chunk[blockIdx.x]; c < c1; c++) {
     const SumChunk ch = chunks[c];
     double s0 = 0.0, s1 = 0.0;
     uint32_t at = 0;
@@ -185,27 +188,35 @@ TablePlan::TablePlan(int device, const std::vector<int64_t>& offsets, const std:
   std::vector<Chunk> chunks;
   std::vector<SumChunk> sum_chunks;
   std::vector<SumSegment> segments;
+  std::vector<uint32_t> sum_first{0};
+  const int64_t range = std::max(kSumRange, ((offsets.back() + kSumCtas - 1) / kSumCtas + 1023) / 1024 * 1024);
   for (int k = 0; k < n_; k++) {
     if ((offsets[k] & 3) != 0 || sizes[k] < 0 || offsets[k + 1] < offsets[k] + sizes[k]) throw std::invalid_argument("offsets and sizes of a table contradict each other");
     first_chunk_.push_back(uint32_t(chunks.size()));
     for (int64_t at = 0; at < sizes[k]; at += kChunk)
       chunks.push_back({uint32_t(k), uint32_t(std::min<int64_t>(kChunk, sizes[k] - at)), at, offsets[k] + at});
     const int64_t len = offsets[k + 1] - offsets[k];
-    segments.push_back({uint32_t(sum_chunks.size()), uint32_t((len + kSumChunk - 1) / kSumChunk), len});
-    for (int64_t at = 0; at < len; at += kSumChunk)
-      sum_chunks.push_back({offsets[k] + at, uint32_t(std::min<int64_t>(kSumChunk, len - at)), uint32_t(k)});
+    segments.push_back({uint32_t(sum_chunks.size()), 0u, len});
+    for (int64_t at = offsets[k]; at < offsets[k + 1];) {
+      const int64_t end = std::min(offsets[k + 1], (at / range + 1) * range);
+      for (int64_t r = int64_t(sum_first.size()); r <= at / range; r++) sum_first.push_back(uint32_t(sum_chunks.size()));
+      sum_chunks.push_back({at, uint32_t(end - at), uint32_t(k)});
+      segments.back().chunks++;
+      at = end;
+    }
   }
+  sum_first.push_back(uint32_t(sum_chunks.size()));
+  n_sum_ctas_ = sum_chunks.empty() ? 0 : int(sum_first.size()) - 1;
   first_chunk_.push_back(uint32_t(chunks.size()));
-  n_chunks_ = uint32_t(chunks.size());
-  n_sum_chunks_ = uint32_t(sum_chunks.size());
   // one block of device memory, laid out on the host and copied in one go
   auto padded = [](size_t v) { return (v + 255) / 256 * 256; };
   const size_t o_sum = padded(chunks.size() * sizeof(Chunk)), o_seg = o_sum + padded(sum_chunks.size() * sizeof(SumChunk)),
-               o_cnt = o_seg + padded(segments.size() * sizeof(SumSegment)), o_par = o_cnt + padded(size_t(n_) * 4), bytes = o_par + padded(sum_chunks.size() * 8) + 256;
+               o_fst = o_seg + padded(segments.size() * sizeof(SumSegment)), o_cnt = o_fst + padded(sum_first.size() * 4), o_par = o_cnt + padded(size_t(n_) * 4), bytes = o_par + padded(sum_chunks.size() * 8) + 256;
   std::vector<uint8_t> host(o_par, 0);
   if (!chunks.empty()) std::memcpy(host.data(), chunks.data(), chunks.size() * sizeof(Chunk));
   if (!sum_chunks.empty()) std::memcpy(host.data() + o_sum, sum_chunks.data(), sum_chunks.size() * sizeof(SumChunk));
   if (!segments.empty()) std::memcpy(host.data() + o_seg, segments.data(), segments.size() * sizeof(SumSegment));
+  std::memcpy(host.data() + o_fst, sum_first.data(), sum_first.size() * 4);
   OnDevice on(device_);
   ck(cudaMalloc(&dev_, bytes), "cudaMalloc");
   ck(cudaMallocHost(reinterpret_cast<void**>(&host_), (size_t(n_) * 2 + 1) * 8), "cudaMallocHost");
@@ -214,6 +225,7 @@ TablePlan::TablePlan(int device, const std::vector<int64_t>& offsets, const std:
   chunks_ = reinterpret_cast<Chunk*>(d);
   sum_chunks_ = reinterpret_cast<SumChunk*>(d + o_sum);
   sum_segments_ = reinterpret_cast<SumSegment*>(d + o_seg);
+  sum_first_ = reinterpret_cast<uint32_t*>(d + o_fst);
   counters_ = reinterpret_cast<uint32_t*>(d + o_cnt);
   partials_ = reinterpret_cast<double*>(d + o_par);
 }
@@ -258,9 +270,9 @@ std::pair<std::vector<double>, std::vector<int>> TablePlan::scales(const float* 
     host_[k] = 0.0;
     host_[n_ + k] = -128.0;
   }
-  if (n_sum_chunks_) {
-    table_sums_kernel<<<blocks_for(n_sum_chunks_), kThreads, 0, static_cast<cudaStream_t>(stream)>>>(arena, sum_chunks_, n_sum_chunks_, sum_segments_, partials_,
-                                                                                                    counters_, host_, n_);
+  if (n_sum_ctas_) {
+    table_sums_kernel<<<n_sum_ctas_, kThreads, 0, static_cast<cudaStream_t>(stream)>>>(arena, sum_chunks_, sum_first_, sum_segments_, partials_, counters_,
+                                                                                      host_, n_);
     ck(cudaGetLastError(), "kernel launch");
     ck(cudaStreamSynchronize(static_cast<cudaStream_t>(stream)), "cudaStreamSynchronize");
   }

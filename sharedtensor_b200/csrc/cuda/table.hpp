@@ -29,12 +29,13 @@ class TablePlan {
 
  private:
   int device_, n_;
-  uint32_t n_chunks_ = 0, n_sum_chunks_ = 0;
+  int n_sum_ctas_ = 0;
   void* dev_ = nullptr;                 // everything below, one allocation
   struct Chunk* chunks_ = nullptr;      // pieces of at most kChunk elements of the tensors, in arena order
   std::vector<uint32_t> first_chunk_;   // of each tensor
   struct SumChunk* sum_chunks_ = nullptr;  // the same over whole segments, for the sums
   struct SumSegment* sum_segments_ = nullptr;
+  uint32_t* sum_first_ = nullptr;       // the first chunk of each CTA, and their number
   double* partials_ = nullptr;
   uint32_t* counters_ = nullptr;        // chunks of a segment that are done (zero between launches)
   double* host_ = nullptr;              // pinned: sums, then exponents
