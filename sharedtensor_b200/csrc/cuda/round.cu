@@ -112,6 +112,27 @@ __device__ __forceinline__ bool mbar_try_wait(uint64_t* bar, uint32_t parity) {
       : "memory");
   return ok != 0;
 }
+__device__ __forceinline__ bool mbar_test(uint64_t* bar, uint32_t parity) {  // never blocks
+  uint32_t ok;
+  asm volatile(
+      "{\n\t.reg .pred p;\n\t"
+      "mbarrier.test_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
+      "selp.u32 %0, 1, 0, p;\n\t}"
+      : "=r"(ok)
+      : "r"(smem_u32(bar)), "r"(parity)
+      : "memory");
+  return ok != 0;
+}
+__device__ __forceinline__ void mbar_expect_tx(uint64_t* bar, uint32_t bytes) {
+  asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(smem_u32(bar)), "r"(bytes) : "memory");
+}
+// global -> this CTA's shared memory, completion counted in bytes on `bar`.  Source is always this GPU's own memory; size
+// and both addresses are multiples of 16.
+__device__ __forceinline__ void bulk_g2s(void* dst_smem, const void* src_gmem, uint32_t bytes, uint64_t* bar) {
+  asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(smem_u32(dst_smem)), "l"(src_gmem),
+               "r"(bytes), "r"(smem_u32(bar))
+               : "memory");
+}
 // global -> L2, this GPU's own memory; size and address are multiples of 16
 __device__ __forceinline__ void bulk_prefetch_l2(const void* src_gmem, uint32_t bytes) {
   asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(src_gmem), "r"(bytes) : "memory");
@@ -139,8 +160,9 @@ __device__ __forceinline__ bool mbar_wait_bounded(uint64_t* bar, uint32_t parity
 struct __align__(16) TileDesc {
   int32_t tile;
   uint32_t flags;
-  int32_t n_frames;  // entries of the tile's frame list
-  int32_t n_slots;   // entries of the tile's slot list
+  uint16_t n_frames;  // entries of the tile's frame list
+  uint16_t n_slots;   // entries of the tile's slot list
+  uint32_t stage;     // two frames or more: the number of the tile among those whose frames are staged
 };
 constexpr uint32_t kDescNoValues = 2;       // the visit only receives: the values are not loaded, what arrived goes into them as a reduction
 constexpr uint32_t kDescTxOk = 1u << 4;     // << link: every out-ring of the link has room
@@ -158,6 +180,7 @@ struct GroupShared {
   uint64_t frames[kBank][kMaxRings * kRxMax + 1];  // per tile: the frames that arrived (address | link), in ring and sequence order
   uint64_t slots[kBank][kMaxRings + 1];            // per tile: the ring slots a frame goes into (address | link)
   uint32_t done[kBank];
+  uint64_t full[2], empty[2];  // of the two frame stages
   uint32_t armed;        // tiles armed so far in this launch (bank entry = number % kBank)
   uint32_t claim;        // tiles the compute warps have started so far | kClaimStop: no new ones
   uint32_t pad[2];
@@ -313,6 +336,23 @@ __device__ __forceinline__ void load_frame(const uint8_t* fp, int warp, int lane
   }
 }
 
+// the same from a frame staged in shared memory
+template <int Q>
+__device__ __forceinline__ void load_staged(const uint8_t* fp, int warp, int lane, int log2_block, FrameRegs& f) {
+  const uint8_t* mine = fp + warp * (kWarpElems * Q / 8);
+  const uint8_t* scales = fp + 4 * Q * kWordsPerTile;
+  f.codes = 0;
+#pragma unroll
+  for (int i = 0; i < kPieces; i++) {
+    const int unit = piece_chunk(i, lane) * 8 + piece_pos(i, lane);
+    if (Q == 8) f.w[i] = reinterpret_cast<const uint32_t*>(mine)[unit];
+    else if (Q == 4) f.w[i] = reinterpret_cast<const uint16_t*>(mine)[unit];
+    else if (Q == 2) f.w[i] = mine[unit];
+    else f.w[i] = reinterpret_cast<const uint32_t*>(mine)[piece_chunk(i, lane)] >> (4 * piece_pos(i, lane));
+    f.codes |= uint32_t(scales[(warp * kWarpElems + piece_chunk(i, lane) * 32) >> log2_block]) << (8 * i);
+  }
+}
+
 // Which of the four elements of piece i exist (bits 0..3).  Only sign frames of the tensor's last tile need it: they have
 // no code for "no step" (integer frames carry the code of zero beyond the tensor's end).
 __device__ __forceinline__ uint32_t valid4(int left, int i) {
@@ -440,15 +480,25 @@ __device__ __forceinline__ void get_stash(const float* stash, int link, Piece (&
   }
 }
 
+// What kind of replica a kernel is for: a leaf of the tree (one link, one ring in), a member of a mesh group (one link,
+// several rings in), an inner node (several links).
+enum Kind { kLeaf, kMember, kInner };
+// Frames of a tile that are staged in shared memory, and the room for one.  A member of a mesh of eight decodes seven frames
+// per tile: out of shared memory, two tiles ahead, a pass over 4 Mi elements takes 42 us, with loads from the L2 48 us.  The
+// other kinds fetch their frames themselves: a leaf seldom has more than one, an inner node no registers to spare (a pass of
+// a hub and its leaves over 16 M elements takes 522 us so, 542 us with stages).
+template <int Q>
+constexpr int kFrameRoom = Q * 512 + 128;
+template <int kKind>
+constexpr int kStaged = kKind == kMember ? 8 : 0;
+
 // total = the sum of the steps of the tile's frames, in list order; kStash: what came on each link is summed up besides, and
 // left in this lane's part of the link's stash (shared memory; a frame is decoded once, however many links hear of it: a hub
 // with three links and six frames per tile took 224 us per 16 M elements when it decoded them for the values and again for
-// each mirror, 170 us so).  The loop stays rolled: unrolled by four frames it was slower for every number of rings, the code
-// of a tile's visit then no longer fits the instruction cache.
-template <int Q, bool kStash>
-__device__ __forceinline__ void decode_frames(const uint64_t* list, int count, uint32_t live, int log2_block, int warp, int lane, int left, float* stash,
-                                              Piece (&total)[kPieces]) {
-  constexpr int kDeep = kStash ? 0 : 1;  // frames on their way while one is decoded (the stash variant has no registers left for it)
+// each mirror, 170 us so).  The loop stays rolled: the code of a tile's visit has to fit the instruction cache.
+template <int Q, bool kStash, int kIn>
+__device__ __forceinline__ void decode_frames(const uint64_t* list, const uint8_t* staged, int count, uint32_t live, uint64_t* empty, int log2_block,
+                                              int warp, int lane, int left, float* stash, Piece (&total)[kPieces]) {
   Piece mine[kPieces];
   int cur = -1;
   uint32_t seen = 0;
@@ -458,11 +508,13 @@ __device__ __forceinline__ void decode_frames(const uint64_t* list, int count, u
 #pragma unroll
     for (int i = 0; i < kPieces; i++) *reinterpret_cast<ulonglong2*>(stash + link * kTile + i * 128) = make_ulonglong2(mine[i].a, mine[i].b);
   };
-  FrameRegs f[kDeep + 1] = {};
-  if (kDeep > 0 && live) load_frame<Q>(frame_at(list[0]), warp, lane, log2_block, f[0]);
 #pragma unroll 1
   for (int j = 0; j < count; j++) {
-    if (live && (kDeep == 0 || j + kDeep < count)) load_frame<Q>(frame_at(list[j + kDeep]), warp, lane, log2_block, f[kDeep]);
+    FrameRegs f{};
+    if (live) {
+      if (j < kIn) load_staged<Q>(staged + j * kFrameRoom<Q>, warp, lane, log2_block, f);
+      else load_frame<Q>(frame_at(list[j]), warp, lane, log2_block, f);
+    }
     if (kStash) {
       const int link = live ? int(list[j] & 15u) : 0;
       if (link != cur) {
@@ -476,13 +528,15 @@ __device__ __forceinline__ void decode_frames(const uint64_t* list, int count, u
     }
 #pragma unroll
     for (int i = 0; i < kPieces; i++) {
-      const Piece st = frame_steps<Q>(f[0].w[i], f[0].code(i), Q == 1 ? valid4(left, i) : 0xfu);
+      const Piece st = frame_steps<Q>(f.w[i], f.code(i), Q == 1 ? valid4(left, i) : 0xfu);
       add4(total[i], st);
       if (kStash) add4(mine[i], st);
     }
-    if (kDeep > 0) f[0] = f[kDeep];
   }
   if (kStash && cur >= 0) put(cur);
+  if (kIn == 0) return;
+  __syncwarp();
+  if (live && lane == 0) mbar_arrive(empty);  // the stage may be filled again when all warps have been here
 }
 
 // One lane's codes of its four pieces into the ring slots of link l's neighbours.  They go through shared memory, so
@@ -522,9 +576,10 @@ __device__ __forceinline__ void send_codes(const uint64_t* list, int count, int 
   }
 }
 
-// kOneLink: one link (a leaf of the tree, a member of a mesh group); what arrived for the values is what arrived on it.
-template <int Q, bool kOneLink>
-__device__ __forceinline__ void compute_warp(const RoundParams& p, GroupShared& sh, float* group_stash, int warp, int lane) {
+template <int Q, int kKind>
+__device__ __forceinline__ void compute_warp(const RoundParams& p, GroupShared& sh, float* group_stash, const uint8_t* stages, int warp, int lane) {
+  constexpr bool kOneLink = kKind != kInner;  // what arrived for the values is what arrived on the link
+  constexpr int kIn = kStaged<kKind>;
   const int L = kOneLink ? 1 : p.n_links, lb = p.log2_block;
   float res_max0 = 0.f, res_max1 = 0.f, res_max2 = 0.f;
   uint32_t exchanges = 0;
@@ -534,7 +589,7 @@ __device__ __forceinline__ void compute_warp(const RoundParams& p, GroupShared& 
   asm volatile("" : "+r"(live));  // (the compiler is not to make a copy of the code for it)
 #pragma unroll 1
   for (uint32_t c = 0;;) {
-    TileDesc d{0, int32_t(kDescTxOk | kDescRxLink | kDescTxWant), p.n_in > 1 ? 2 : 1, 0};
+    TileDesc d{0, kDescTxOk | kDescRxLink | kDescTxWant, uint16_t(p.n_in > 1 ? 2 : 1), 0, 0};
     uint32_t entry = 0;
     if (live) {
       const uint32_t go = lane == 0 ? (claim_tile(sh, c) ? 1u : 0u) : 0u;
@@ -551,7 +606,8 @@ __device__ __forceinline__ void compute_warp(const RoundParams& p, GroupShared& 
         const TileDesc& e = sh.desc[ahead % kBank];
         if (!(e.flags & kDescNoValues)) bulk_prefetch_l2(p.values + size_t(e.tile) * kTile, kTile * 4);
         for (int l = 0; l < L; l++) bulk_prefetch_l2(p.mirror[l] + size_t(e.tile) * kTile, kTile * 4);
-        for (int j = 0; j < e.n_frames; j++) bulk_prefetch_l2(frame_at(sh.frames[ahead % kBank][j]), uint32_t(p.payload_bytes));
+        if (kIn == 0 || e.n_frames == 1)
+          for (int j = 0; j < e.n_frames; j++) bulk_prefetch_l2(frame_at(sh.frames[ahead % kBank][j]), uint32_t(p.payload_bytes));
       }
     }
     const int in_tile = warp * kWarpElems + lane * 4;
@@ -583,13 +639,24 @@ __device__ __forceinline__ void compute_warp(const RoundParams& p, GroupShared& 
         if (for0) applied = 0;
       }
     } else {
-      Piece acc[kPieces];
-      decode_frames<Q, !kOneLink>(frames, d.n_frames, live, lb, warp, lane, left, group_stash + in_tile, acc);
+      // (one link: values and mirror on their way while the frames are decoded)
+      auto fetch = [&]() {
 #pragma unroll
-      for (int i = 0; i < kPieces; i++) {
-        v[i] = load_v ? load_piece(vp + i * 128) : Piece{0ull, 0ull};
-        k[i] = live ? load_piece(p.mirror[0] + off + i * 128) : Piece{0ull, 0ull};
+        for (int i = 0; i < kPieces; i++) {
+          v[i] = load_v ? load_piece(vp + i * 128) : Piece{0ull, 0ull};
+          k[i] = live ? load_piece(p.mirror[0] + off + i * 128) : Piece{0ull, 0ull};
+        }
+      };
+      if (kOneLink) fetch();
+      const uint32_t st = d.stage & 1u;
+      if (kIn > 0 && live && !__all_sync(0xffffffffu, mbar_wait_bounded(&sh.full[st], (d.stage >> 1) & 1u, 2ull * p.wait_ns))) {
+        if (lane == 0) red_shared_release_add(&sh.done[entry], kDoneWarp | kDoneFailed);  // nothing of the tile is stored
+        break;
       }
+      Piece acc[kPieces];
+      decode_frames<Q, !kOneLink, kIn>(frames, stages + st * (kIn * kFrameRoom<Q>), d.n_frames, live, &sh.empty[st], lb, warp, lane, left,
+                                       group_stash + in_tile, acc);
+      if (!kOneLink) fetch();
 #pragma unroll
       for (int i = 0; i < kPieces; i++) {
         if (live) red_add_piece(vp + i * 128, acc[i]);
@@ -702,7 +769,7 @@ __device__ __forceinline__ void compute_warp(const RoundParams& p, GroupShared& 
 // a power of two above one, 32 / R tiles are looked at together, and every look costs two round trips to the L2 whatever R is.
 // All 32 lanes run the same control flow; decisions taken from words that change under the warp's feet are taken by one
 // lane, or on a ballot.
-__device__ __forceinline__ void service_warp(const RoundParams& p, GroupShared& sh, int g, int n_groups, int lane) {
+__device__ __forceinline__ void service_warp(const RoundParams& p, GroupShared& sh, uint8_t* stages, int staged_frames, int frame_room, int g, int n_groups, int lane) {
   // The group's tiles: a run of `chunk` consecutive tiles, or (chunk == 0) every gstride-th tile of the launch's window.
   // The groups of a CTA are a grid apart, so that the odd tiles of the last turn fall on all SMs alike.
   const int gidx = p.chunk > 0 ? int(blockIdx.x) * n_groups + g : g * int(gridDim.x) + int(blockIdx.x);
@@ -733,6 +800,8 @@ __device__ __forceinline__ void service_warp(const RoundParams& p, GroupShared& 
   bool handed_on = false;   // the next window's launch has been let in
   uint32_t n_done = 0, n_tx = 0, n_rx = 0, n_blocked = 0, n_pending = 0, n_sweeps = 0;  // per lane, added up at the end
   uint32_t armed = 0, finished = 0, published = 0;  // tiles armed, finished by the compute warps, published so far
+  uint32_t handed = 0, staged = 0;                  // tiles the compute warps may start, and those of them whose frames have been seen to
+  uint32_t stage_no = 0, stage_issued = 0;          // tiles with two frames or more found so far, and those staged
   bool aborted = false, yielded = false;
 
   if (p.zero_other && blockIdx.x == 0 && g == 0 && lane == 0) {
@@ -750,6 +819,26 @@ __device__ __forceinline__ void service_warp(const RoundParams& p, GroupShared& 
     uint32_t idle = 0;
     uint64_t t_last = globaltimer_ns();
     while (true) {
+      // ---- the frames of the next tiles that have several on their way into shared memory, as stages become free
+      while (staged_frames > 0 && staged != handed) {
+        const TileDesc d = sh.desc[staged % kBank];
+        if (d.n_frames > 1) {
+          const uint32_t u = stage_issued & 1u;
+          uint32_t free = 1;
+          if (stage_issued >= 2 && lane == 0) free = mbar_test(&sh.empty[u], (stage_issued / 2 - 1u) & 1u) ? 1u : 0u;
+          if (!__shfl_sync(0xffffffffu, free, 0)) break;
+          const int count = min(int(d.n_frames), staged_frames);
+          if (lane == 0) mbar_expect_tx(&sh.full[u], uint32_t(count) * uint32_t(p.payload_bytes));
+          __syncwarp();
+          if (lane < count) {
+            asm volatile("fence.proxy.async;" ::: "memory");  // the frames came by ordinary stores, their flags have been acquired
+            bulk_g2s(stages + (int(u) * staged_frames + lane) * frame_room, frame_at(sh.frames[staged % kBank][lane]), uint32_t(p.payload_bytes), &sh.full[u]);
+          }
+          __syncwarp();
+          stage_issued++;
+        }
+        staged++;
+      }
       // ---- look at more tiles while the compute warps have less than kAhead in hand and the bank has room for them
       if (looked < my_count && !yielded && armed - finished < uint32_t(kAhead) && armed - published + uint32_t(at_once) <= uint32_t(kBank)) {
         ST_CRUMB(g, 2);
@@ -827,10 +916,12 @@ __device__ __forceinline__ void service_warp(const RoundParams& p, GroupShared& 
         // the values themselves are not needed.
         if (p.n_links == 1 && dirty == 0) flags |= kDescNoValues;
         const uint32_t sends = __ballot_sync(0xffffffffu, goes_out) & same_tile;
+        const int n_frames = __popc(in1 & same_tile) + __popc(in2 & same_tile) + __popc(in3 & same_tile);
+        const uint32_t several = __ballot_sync(0xffffffffu, work && r == 0 && n_frames > 1);
         const uint32_t pos = armed + __popc(work_tiles & ((1u << t) - 1u)), entry = pos % kBank;
         if (work) {
           if (r == 0) {
-            sh.desc[entry] = TileDesc{tile, flags, int(__popc(in1 & same_tile) + __popc(in2 & same_tile) + __popc(in3 & same_tile)), int(__popc(sends))};
+            sh.desc[entry] = TileDesc{tile, flags, uint16_t(n_frames), uint16_t(__popc(sends)), stage_no + __popc(several & ((1u << t) - 1u))};
             sh.done[entry] = 0;
             sh.dirty[entry] = dirty;
           }
@@ -839,7 +930,7 @@ __device__ __forceinline__ void service_warp(const RoundParams& p, GroupShared& 
               if (!(flags & kDescNoValues)) bulk_prefetch_l2(p.values + size_t(tile) * kTile, kTile * 4);
               for (int l = 0; l < p.n_links; l++) bulk_prefetch_l2(p.mirror[l] + size_t(tile) * kTile, kTile * 4);
             }
-            for (uint32_t f = 0; f < avail; f++)
+            for (uint32_t f = 0; f < avail && (staged_frames == 0 || n_frames == 1); f++)
               bulk_prefetch_l2(in.payload + (size_t((rx + f) & smask) * p.n_tiles + tile) * p.payload_bytes, uint32_t(p.payload_bytes));
           }
           const uint32_t before = same_tile & below;
@@ -855,11 +946,12 @@ __device__ __forceinline__ void service_warp(const RoundParams& p, GroupShared& 
         }
         // test hook: this tile is never handed to the compute warps, so the wait for it below runs out
         const uint32_t stalled = __ballot_sync(0xffffffffu, work && tile == p.stall_tile && r == 0);
-        const uint32_t handed = stalled ? armed + __popc(work_tiles & ((1u << (__ffs(stalled) - 1)) - 1u)) : armed + __popc(work_tiles);
+        handed = stalled ? armed + __popc(work_tiles & ((1u << (__ffs(stalled) - 1)) - 1u)) : armed + __popc(work_tiles);
         __syncwarp();
         if (lane == 0) st_shared_release(&sh.armed, handed);
         if (armed == finished) t_last = globaltimer_ns();
         armed += __popc(work_tiles);
+        stage_no += __popc(several);
         if (stalled) looked = my_count;
         idle = 0;
         continue;
@@ -942,6 +1034,8 @@ __device__ __forceinline__ void service_warp(const RoundParams& p, GroupShared& 
       for (uint32_t c = started + uint32_t(lane); int32_t(armed - c) > 0; c += 32)
         if (sh.dirty[c % kBank]) st_cg_u32(p.tile_state + sh.desc[c % kBank].tile, 1u);
       armed = started;
+      if (int32_t(handed - started) > 0) handed = started;
+      if (int32_t(staged - handed) > 0) staged = handed;
       t_last = globaltimer_ns();
     }
     if (aborted) break;
@@ -949,6 +1043,9 @@ __device__ __forceinline__ void service_warp(const RoundParams& p, GroupShared& 
     if (armed == armed_before && sweep + 1 < p.sweeps) __nanosleep(1000);
   }
   if (lane == 0) atomicOr(&sh.claim, kClaimStop);  // the compute warps leave
+  // copies of tiles that nobody started get a bounded chance to land before the CTA's shared memory is released
+  for (uint32_t q = stage_issued > 2 ? stage_issued - 2 : 0; q < stage_issued; q++)
+    (void)__all_sync(0xffffffffu, mbar_wait_bounded(&sh.full[q & 1u], (q >> 1) & 1u, limit_ns));
   if (aborted) {
     for (int j = lane; j < my_count; j += 32) st_cg_u32(p.tile_state + gid + j * gstride, 1u);
     if (lane == 0) {
@@ -988,22 +1085,30 @@ __device__ __forceinline__ void service_warp(const RoundParams& p, GroupShared& 
 
 }  // namespace
 
-template <int Q, int kGroups, bool kOneLink>
+template <int Q, int kGroups, int kKind>
 __global__ void __launch_bounds__(kGroups * kGroupThreads, 1) round_kernel(const __grid_constant__ RoundParams p) {
   __shared__ GroupShared shared[kGroups];
-  extern __shared__ __align__(16) float stash[];  // several links: [group][link][element of the tile]
+  extern __shared__ __align__(128) uint8_t dynamic[];  // [group][two stages of frames], and for an inner node [group][link][element of the tile]
+  constexpr int kIn = kStaged<kKind>, kStageBytes = 2 * kIn * kFrameRoom<Q>;
   const int g = int(threadIdx.x) / kGroupThreads, warp = (int(threadIdx.x) % kGroupThreads) >> 5, lane = threadIdx.x & 31;
   if (threadIdx.x < kGroups) {
     GroupShared& sh = shared[threadIdx.x];
     sh.armed = 0;
     sh.claim = 0;
     mbar_init(&sh.gsync, kComputeWarps);
+    for (int u = 0; u < 2; u++) {
+      mbar_init(&sh.full[u], 1);
+      mbar_init(&sh.empty[u], kComputeWarps);
+    }
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
   }
   if (!p.follows_window) asm volatile("griddepcontrol.wait;" ::: "memory");
   __syncthreads();  // the only CTA-wide barrier: from here on the groups, and the two kinds of warp, run on their own
-  if (warp == kComputeWarps) service_warp(p, shared[g], g, kGroups, lane);
-  else compute_warp<Q, kOneLink>(p, shared[g], stash + (kOneLink ? 0 : g * kMaxLinks * kTile), warp, lane);
+  uint8_t* const stages = dynamic + g * kStageBytes;
+  float* const stash = reinterpret_cast<float*>(dynamic + kGroups * kStageBytes) + (kKind == kInner ? g * kMaxLinks * kTile : 0);
+  if (warp == kComputeWarps) service_warp(p, shared[g], stages, kIn, kFrameRoom<Q>, g, kGroups, lane);
+  else compute_warp<Q, kKind>(p, shared[g], stash, stages, warp, lane);
 }
 
 // ----------------------------------------------------------------------------------------------
@@ -1074,35 +1179,28 @@ int launch_count_unacknowledged(const RoundParams& p, uint32_t* count, void* str
 // ----------------------------------------------------------------------------------------------
 // launcher
 // ----------------------------------------------------------------------------------------------
-template <int kGroups>
-static constexpr int stash_bytes(bool one_link) { return one_link ? 0 : kGroups * kMaxLinks * kTile * 4; }
+template <int Q, int kGroups, int kKind>
+constexpr int kDynamicBytes = kGroups * (2 * kStaged<kKind> * kFrameRoom<Q> + (kKind == kInner ? kMaxLinks * kTile * 4 : 0));
 
 // Loads the kernel and, once per device, gives it its shared memory.
-template <int Q, int kGroups, bool kOneLink>
+template <int Q, int kGroups, int kKind>
 static int load_round_l() {
   static std::atomic<uint64_t> loaded{0};
   int dev = 0;
   cudaGetDevice(&dev);
   if ((loaded.load(std::memory_order_relaxed) >> (dev & 63)) & 1u) return 0;
-  cudaFuncAttributes a;
-  cudaError_t e = cudaFuncGetAttributes(&a, round_kernel<Q, kGroups, kOneLink>);
-  if (e == cudaSuccess && !kOneLink)
-    e = cudaFuncSetAttribute(round_kernel<Q, kGroups, kOneLink>, cudaFuncAttributeMaxDynamicSharedMemorySize, stash_bytes<kGroups>(false));
+  const cudaError_t e = cudaFuncSetAttribute(round_kernel<Q, kGroups, kKind>, cudaFuncAttributeMaxDynamicSharedMemorySize, kDynamicBytes<Q, kGroups, kKind>);
   if (e == cudaSuccess) loaded.fetch_or(1ull << (dev & 63), std::memory_order_relaxed);
   return int(e);
 }
-template <int Q, int kGroups>
-static int load_round_t(const RoundParams& p) {
-  return p.n_links == 1 ? load_round_l<Q, kGroups, true>() : load_round_l<Q, kGroups, false>();
-}
 
-template <int Q, int kGroups>
-static int launch_round_t(const RoundParams& p, int ctas, cudaStream_t stream) {
-  if (const int e = load_round_t<Q, kGroups>(p)) return e;
+template <int Q, int kGroups, int kKind>
+static int launch_round_l(const RoundParams& p, int ctas, cudaStream_t stream) {
+  if (const int e = load_round_l<Q, kGroups, kKind>()) return e;
   cudaLaunchConfig_t cfg{};
   cfg.gridDim = dim3(ctas);
   cfg.blockDim = dim3(kGroups * kGroupThreads);
-  cfg.dynamicSmemBytes = stash_bytes<kGroups>(p.n_links == 1);
+  cfg.dynamicSmemBytes = kDynamicBytes<Q, kGroups, kKind>;
   cfg.stream = stream;
   // The launch may move in while the kernel before it in the stream is running out (and is cheaper to issue so: 2.4 instead
   // of 2.9 us).  A window that follows another of its cycle starts at once: the two have no tile in common.  Any other launch
@@ -1112,39 +1210,20 @@ static int launch_round_t(const RoundParams& p, int ctas, cudaStream_t stream) {
   early.val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = &early;
   cfg.numAttrs = 1;
-  return int(p.n_links == 1 ? cudaLaunchKernelEx(&cfg, round_kernel<Q, kGroups, true>, p) : cudaLaunchKernelEx(&cfg, round_kernel<Q, kGroups, false>, p));
+  return int(cudaLaunchKernelEx(&cfg, round_kernel<Q, kGroups, kKind>, p));
 }
 
-// Groups of a CTA.  A replica with one ring pair, or with one per link, is bound by HBM and by the length of a tile's
-// chain of operations: two groups with 96 registers a thread are enough and were 2 to 8 % faster than three with 72.
-// Several rings on one link (a mesh group) mean several frames to decode per tile, which more warps hide: 51 against
-// 55 us for seven rings and 4 Mi elements.  Shape 0 asks for three whatever the rings.
-int round_groups(int shape, int n_links, int n_in) { return shape == 0 || (n_links == 1 && n_in > 1) ? 3 : 2; }
-
+// `ctas` == 0: only loads the kernel
 template <int Q>
 static int launch_round_q(const RoundParams& p, int shape, int ctas, cudaStream_t stream) {
   if (shape != 0 && shape != 1) return int(cudaErrorInvalidValue);
-  return round_groups(shape, p.n_links, p.n_in) == 3 ? launch_round_t<Q, 3>(p, ctas, stream) : launch_round_t<Q, 2>(p, ctas, stream);
+  if (p.n_links > 1) return ctas ? launch_round_l<Q, 2, kInner>(p, ctas, stream) : load_round_l<Q, 2, kInner>();
+  if (p.n_in > 1) return ctas ? launch_round_l<Q, 2, kMember>(p, ctas, stream) : load_round_l<Q, 2, kMember>();
+  if (round_groups(shape, p.n_links, p.n_in) == 3) return ctas ? launch_round_l<Q, 3, kLeaf>(p, ctas, stream) : load_round_l<Q, 3, kLeaf>();
+  return ctas ? launch_round_l<Q, 2, kLeaf>(p, ctas, stream) : load_round_l<Q, 2, kLeaf>();
 }
 
-template <int Q>
-static int load_round_q(const RoundParams& p, int shape) {
-  return round_groups(shape, p.n_links, p.n_in) == 3 ? load_round_t<Q, 3>(p) : load_round_t<Q, 2>(p);
-}
-
-int load_round(const RoundParams& p, int shape) {
-  switch (p.bits) {
-    case 1: return load_round_q<1>(p, shape);
-    case 2: return load_round_q<2>(p, shape);
-    case 4: return load_round_q<4>(p, shape);
-    default: return load_round_q<8>(p, shape);
-  }
-}
-
-int launch_round(const RoundParams& p, int shape, int ctas, void* stream_v) {
-  cudaStream_t stream = static_cast<cudaStream_t>(stream_v);
-  if (p.n_links < 1 || p.n_links > kMaxLinks || p.sweeps < 1 || ctas < 1) return int(cudaErrorInvalidValue);
-  if (p.ring_slots < 2 || p.ring_slots > 64 || (p.ring_slots & (p.ring_slots - 1))) return int(cudaErrorInvalidValue);
+static int launch_round_any(const RoundParams& p, int shape, int ctas, cudaStream_t stream) {
   switch (p.bits) {
     case 1: return launch_round_q<1>(p, shape, ctas, stream);
     case 2: return launch_round_q<2>(p, shape, ctas, stream);
@@ -1152,6 +1231,17 @@ int launch_round(const RoundParams& p, int shape, int ctas, void* stream_v) {
     case 8: return launch_round_q<8>(p, shape, ctas, stream);
     default: return int(cudaErrorInvalidValue);
   }
+}
+
+// Groups of a CTA: two with 96 registers a thread; for a leaf shape 0 asks for three with 72.
+int round_groups(int shape, int n_links, int n_in) { return shape == 0 && n_links == 1 && n_in <= 1 ? 3 : 2; }
+
+int load_round(const RoundParams& p, int shape) { return launch_round_any(p, shape, 0, nullptr); }
+
+int launch_round(const RoundParams& p, int shape, int ctas, void* stream_v) {
+  if (p.n_links < 1 || p.n_links > kMaxLinks || p.sweeps < 1 || ctas < 1) return int(cudaErrorInvalidValue);
+  if (p.ring_slots < 2 || p.ring_slots > 64 || (p.ring_slots & (p.ring_slots - 1))) return int(cudaErrorInvalidValue);
+  return launch_round_any(p, shape, ctas, static_cast<cudaStream_t>(stream_v));
 }
 
 }  // namespace st

@@ -125,7 +125,7 @@ enum StatusWord : int {
 };
 
 // Launchers.  `stream` is a cudaStream_t passed as void*.  Return a cudaError_t as int.
-// `shape` picks the CTA's make-up: 1 = two or three groups by the replica's rings, 0 = three groups (one CTA per SM
+// `shape` picks the CTA's make-up: 1 = two groups, 0 = three groups where there is one link with one ring (one CTA per SM
 // either way).  A group is eight compute warps and one service warp.
 int launch_round(const RoundParams& p, int shape, int ctas, void* stream);
 // Loads the kernel that launch_round would run (code is otherwise loaded on a kernel's first launch, which takes up to some
