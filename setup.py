@@ -1,5 +1,5 @@
 """Packaging (the counterpart of the reference's rockspec, sharedtensor-scm-1.rockspec:19-26, which builds its one C
-file): ``pip install .`` compiles the two native modules in-tree with the same commands as
+file): ``pip install .`` compiles the native modules in-tree with the same commands as
 ``python -m sharedtensor_b200._build`` (g++ for the host core, nvcc for sm_100a) and installs them with the package.
 """
 from pathlib import Path
@@ -17,6 +17,7 @@ class BuildNative(build_py):
         spec.loader.exec_module(mod)
         mod.build_core()
         mod.build_cuda()
+        mod.build_tensors()
         super().run()
 
 

@@ -1,13 +1,15 @@
 """In-tree build of the native extensions.
 
-Two shared objects are produced next to this file:
+Three shared objects are produced next to this file:
 
 * ``_core``  – host-only C++ (codec, tree join, TCP edges, CPU replica node); built with g++.
 * ``_cuda``  – sm_100a kernels, the peer-memory transport and the GPU engine; built with nvcc for
   ``compute_100a/sm_100a`` only, CUDA runtime linked statically so the module also imports on a
   machine without a GPU or driver.
 
-``python -m sharedtensor_b200._build`` builds both; ``ensure_built()`` rebuilds what is stale.
+* ``_tensors`` – the look over a dict of torch tensors; the only one that uses torch's headers and libraries.
+
+``python -m sharedtensor_b200._build`` builds them; ``ensure_built()`` rebuilds what is stale.
 """
 from __future__ import annotations
 
@@ -111,13 +113,30 @@ def build_cuda(force: bool = False, verbose: bool = False, ptxas_v: bool = False
     return target
 
 
+def build_tensors(force: bool = False, verbose: bool = False) -> Path:
+    import importlib.util
+
+    target, src = target_path("_tensors"), CSRC / "core/tensors.cpp"
+    if not force and not _stale(target, [src]):
+        return target
+    OBJ.mkdir(exist_ok=True)
+    torch_dir = Path(importlib.util.find_spec("torch").submodule_search_locations[0])
+    obj, inc, lib = OBJ / "core_tensors.cpp.o", torch_dir / "include", torch_dir / "lib"
+    _run([CXX, "-std=c++17", "-O2", "-fPIC", "-fvisibility=hidden", f"-isystem{inc}", f"-isystem{inc / 'torch/csrc/api/include'}",
+          "-isystem/usr/local/cuda/include", f"-I{sysconfig.get_paths()['include']}", "-c", str(src), "-o", str(obj)], verbose)
+    _run([CXX, "-shared", "-o", str(target), str(obj), f"-L{lib}", "-ltorch_python", "-ltorch_cpu", "-lc10"], verbose)
+    return target
+
+
 def ensure_built(verbose: bool = False) -> None:
     build_core(verbose=verbose)
     build_cuda(verbose=verbose)
+    build_tensors(verbose=verbose)
 
 
 if __name__ == "__main__":
     force = "--force" in sys.argv
     build_core(force=force, verbose=True)
     build_cuda(force=force, verbose=True, ptxas_v="--ptxas-v" in sys.argv)
-    print("built:", target_path("_core").name, target_path("_cuda").name)
+    build_tensors(force=force, verbose=True)
+    print("built:", target_path("_core").name, target_path("_cuda").name, target_path("_tensors").name)

@@ -21,7 +21,7 @@ def _load(name: str):
         except ImportError:
             from . import _build
 
-            (_build.build_core if name == "_core" else _build.build_cuda)()
+            {"_core": _build.build_core, "_cuda": _build.build_cuda, "_tensors": _build.build_tensors}[name]()
             importlib.invalidate_caches()
             mod = importlib.import_module(f"sharedtensor_b200.{name}")
         _mods[name] = mod
@@ -34,3 +34,9 @@ def core():
 
 def cuda():
     return _load("_cuda")
+
+
+def tensors():
+    import torch  # noqa: F401  (its libraries have to be loaded first)
+
+    return _load("_tensors")

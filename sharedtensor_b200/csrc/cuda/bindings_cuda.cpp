@@ -5,6 +5,9 @@
 
 #include <cuda_runtime_api.h>
 
+#include <cstring>
+#include <string_view>
+
 #include "../core/codec.hpp"
 #include "engine.hpp"
 #include "round.h"
@@ -18,6 +21,12 @@ static T* ptr(uintptr_t p) {
   return reinterpret_cast<T*>(p);
 }
 static void* strm(uintptr_t s) { return reinterpret_cast<void*>(s); }
+static std::vector<uintptr_t> unpack(const py::bytes& b) {  // packed addresses
+  const std::string_view v = b;
+  std::vector<uintptr_t> out(v.size() / sizeof(uintptr_t));
+  std::memcpy(out.data(), v.data(), out.size() * sizeof(uintptr_t));
+  return out;
+}
 static void ck(int e, const char* what) {
   if (e != 0) throw std::runtime_error(std::string(what) + ": " + cudaGetErrorString(cudaError_t(e)));
 }
@@ -148,8 +157,8 @@ PYBIND11_MODULE(_cuda, m) {
       .def("add_scaled_bf16", [](GpuReplica& r, uintptr_t g, float alpha, uintptr_t s) { r.add_scaled_bf16(ptr<void>(g), alpha, strm(s)); })
       .def("snapshot", [](GpuReplica& r, uintptr_t out, uintptr_t s) { r.snapshot(ptr<float>(out), strm(s)); })
       .def("snapshot_bf16", [](GpuReplica& r, uintptr_t out, uintptr_t s) { r.snapshot_bf16(ptr<void>(out), strm(s)); })
-      .def("table_add", [](GpuReplica& r, const TablePlan& t, const std::vector<uintptr_t>& p, uintptr_t s) { r.table_add(t, p, strm(s)); })
-      .def("table_copy", [](GpuReplica& r, const TablePlan& t, const std::vector<uintptr_t>& p, uintptr_t s) { r.table_copy(t, p, strm(s)); })
+      .def("table_add", [](GpuReplica& r, const TablePlan& t, const py::bytes& p, uintptr_t s) { r.table_add(t, unpack(p), strm(s)); })
+      .def("table_copy", [](GpuReplica& r, const TablePlan& t, const py::bytes& p, uintptr_t s) { r.table_copy(t, unpack(p), strm(s)); })
       .def("copy_mirror_from_values", &GpuReplica::copy_mirror_from_values)
       .def("round", &GpuReplica::round, py::arg("do_rx") = true, py::arg("do_tx") = true, py::arg("sweeps") = 1)
       .def("set_test_stall_tile", &GpuReplica::set_test_stall_tile)

@@ -52,7 +52,6 @@ class SharedTable:
         self.shared = shared
         self.layout = layout
         self._scratch: torch.Tensor | None = None
-        self._items = [(k, layout.shapes[k]) for k in layout.names]
         self._plan = None            # GPU replicas: the native layout of the table
         self._native_plan()
 
@@ -60,29 +59,16 @@ class SharedTable:
     def _native_plan(self):
         """(replica, plan) of a GPU replica, else None."""
         rep = getattr(self.shared._b, "rep", None)
-        if rep is None or not self._items:
+        if rep is None or not self.layout.names:
             return None
         if self._plan is None:
             from .. import _native
 
-            sizes = [shape.numel() for _, shape in self._items]
-            self._plan = _native.cuda().TablePlan(self.shared.device.index, self.layout.segment_offsets(), sizes)
+            shapes = list(self.layout.shapes.values())
+            self._plan = _native.cuda().TablePlan(self.shared.device.index, self.layout.segment_offsets(), [s.numel() for s in shapes])
+            # the look over a dict of tensors: their addresses, or None if one of them needs a conversion on the way
+            self._addresses = _native.tensors().TensorList(self.layout.names, shapes, self.shared.device.index).addresses
         return rep, self._plan
-
-    def _addresses(self, tensors: Mapping[str, torch.Tensor], written: bool) -> list[int] | None:
-        """The tensors' addresses, or None if one of them needs a conversion, a broadcast or autograd on the way."""
-        index, tracked = self.shared.device.index, written and torch.is_grad_enabled()
-        f32, strided = torch.float32, torch.strided
-        out = []
-        for k, shape in self._items:
-            t = tensors[k]
-            if (t.dtype is not f32 or t.layout is not strided or t.shape != shape or t.get_device() != index or not t.is_contiguous()
-                    or (tracked and t.requires_grad)):
-                return None
-            out.append(t.data_ptr())
-        if written and len(set(out)) < len(out):
-            return None  # names that share a tensor: one after the other
-        return out
 
     # ---- dict-of-tensors interface
     def copyToTensors(self, out: Mapping[str, torch.Tensor]) -> None:
@@ -90,7 +76,6 @@ class SharedTable:
         if native is not None and (addresses := self._addresses(out, True)) is not None:
             with _Range(self.shared.cfg.nvtx, "sharedtensor.copyToTensor"):
                 native[0].table_copy(native[1], addresses, _stream(self.shared.device))
-            torch.autograd.graph.increment_version([out[k] for k in self.layout.names])
             return
         flat = self._flat()
         self.shared.copyToTensor(flat)
