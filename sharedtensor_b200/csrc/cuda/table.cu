@@ -52,33 +52,41 @@ __global__ void __launch_bounds__(kThreads, 8) table_kernel(float* __restrict__ 
     const Chunk ch = chunks[c];
     float* const t = ptrs.p[ch.tensor - first_tensor] + ch.start;
     float* const a = arena + ch.arena;
-    if (ch.count == kChunk && (reinterpret_cast<uintptr_t>(t) & 15) == 0) {
-      const float4* src = reinterpret_cast<const float4*>(ADD ? t : a) + threadIdx.x;
-      float4 v[4];
+    // Whole vectors on the side that is added to or written (the arena's chunks are aligned, a tensor may start anywhere);
+    // the side that is read takes four accesses where it is not aligned with the other, three of which the L1 serves.
+    const uint32_t head = ADD ? 0u : min(ch.count, uint32_t((4 - reinterpret_cast<uintptr_t>(t) / 4 % 4) % 4));
+    const uint32_t n4 = (ch.count - head) / 4;
+    const float* const src = (ADD ? t : a) + head;
+    float* const dst = (ADD ? a : t) + head;
+    const bool vec = (reinterpret_cast<uintptr_t>(src) & 15) == 0;
+    float4 v[4];
 #pragma unroll
-      for (int i = 0; i < 4; i++) v[i] = __ldcs(src + i * kThreads);
-#pragma unroll
-      for (int i = 0; i < 4; i++) {
-        if (ADD)
-          asm volatile("red.global.add.v4.f32 [%0], {%1, %2, %3, %4};" ::"l"(reinterpret_cast<float4*>(a) + threadIdx.x + i * kThreads), "f"(v[i].x),
-                       "f"(v[i].y), "f"(v[i].z), "f"(v[i].w)
-                       : "memory");
-        else
-          __stcs(reinterpret_cast<float4*>(t) + threadIdx.x + i * kThreads, v[i]);
+    for (int i = 0; i < 4; i++) {
+      const uint32_t at = threadIdx.x + i * kThreads;
+      if (at >= n4) continue;
+      if (vec) {
+        v[i] = __ldcs(reinterpret_cast<const float4*>(src) + at);
+      } else {
+        const float* p = src + 4 * at;
+        v[i] = make_float4(p[0], p[1], p[2], p[3]);
       }
-    } else {
-      for (uint32_t e0 = threadIdx.x; e0 < ch.count; e0 += 8 * kThreads) {
-        float v[8];
+    }
 #pragma unroll
-        for (int i = 0; i < 8; i++)
-          if (e0 + i * kThreads < ch.count) v[i] = (ADD ? t : a)[e0 + i * kThreads];
-#pragma unroll
-        for (int i = 0; i < 8; i++) {
-          if (e0 + i * kThreads >= ch.count) continue;
-          if (ADD) atomicAdd(a + e0 + i * kThreads, v[i]);
-          else t[e0 + i * kThreads] = v[i];
-        }
-      }
+    for (int i = 0; i < 4; i++) {
+      const uint32_t at = threadIdx.x + i * kThreads;
+      if (at >= n4) continue;
+      if (ADD)
+        asm volatile("red.global.add.v4.f32 [%0], {%1, %2, %3, %4};" ::"l"(reinterpret_cast<float4*>(dst) + at), "f"(v[i].x), "f"(v[i].y), "f"(v[i].z),
+                     "f"(v[i].w)
+                     : "memory");
+      else
+        __stcs(reinterpret_cast<float4*>(dst) + at, v[i]);
+    }
+    // the elements before the first vector and behind the last
+    const uint32_t e = threadIdx.x < head ? threadIdx.x : threadIdx.x + 4 * n4;
+    if (threadIdx.x < ch.count - 4 * n4) {
+      if (ADD) atomicAdd(a + e, t[e]);
+      else t[e] = a[e];
     }
   }
   if (ADD && m.tile_state != nullptr) {
