@@ -120,6 +120,11 @@ PYBIND11_MODULE(_cuda, m) {
   py::class_<TablePlan>(m, "TablePlan")
       .def(py::init<int, const std::vector<int64_t>&, const std::vector<int64_t>&>())
       .def("tensors", &TablePlan::tensors)
+      .def("device_bytes", &TablePlan::device_bytes)
+      .def("pinned_bytes", &TablePlan::pinned_bytes)
+      .def("bind", [](TablePlan& t, const py::object& device, const py::object& pinned, uintptr_t s) {  // two tensors, kept alive with the plan
+        t.bind(ptr<void>(device.attr("data_ptr")().cast<uintptr_t>()), ptr<void>(pinned.attr("data_ptr")().cast<uintptr_t>()), strm(s));
+      }, py::keep_alive<1, 2>(), py::keep_alive<1, 3>())
       .def("scales", [](TablePlan& t, uintptr_t arena, uintptr_t s) { py::gil_scoped_release rel; return t.scales(ptr<float>(arena), strm(s)); });
 
   py::class_<GpuReplica>(m, "GpuReplica")

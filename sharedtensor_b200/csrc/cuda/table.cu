@@ -12,10 +12,9 @@
 namespace st {
 
 struct Chunk {
+  int64_t arena;     // element of the arena
   uint32_t tensor;
   uint32_t count;    // elements
-  int64_t start;     // element of the tensor
-  int64_t arena;     // element of the arena
 };
 struct SumChunk {
   int64_t begin;     // elements of the arena
@@ -30,13 +29,13 @@ struct SumSegment {
 namespace {
 
 constexpr int kThreads = 256;
-constexpr int kChunk = 4096;          // a CTA's step: four 16-byte accesses per thread
+constexpr uint32_t kChunk = 4096;     // a CTA's step: four 16-byte accesses per thread
 constexpr int64_t kSumRange = 2048;   // the sums: elements of the arena that a CTA takes at least
 constexpr int kSumCtas = 148 * 8;
 constexpr int kPtrs = 256;            // tensors of one launch: their addresses travel as kernel parameters
 
 struct Pointers {
-  float* p[kPtrs];
+  float* p[kPtrs];                    // less the tensor's offset, so that an arena element's number finds its tensor element
 };
 
 void ck(cudaError_t e, const char* what) {
@@ -50,7 +49,7 @@ __global__ void __launch_bounds__(kThreads, 8) table_kernel(float* __restrict__ 
                                                             uint32_t first_tensor, const __grid_constant__ Pointers ptrs, UpdateMarks m) {
   for (uint32_t c = blockIdx.x; c < n_chunks; c += gridDim.x) {
     const Chunk ch = chunks[c];
-    float* const t = ptrs.p[ch.tensor - first_tensor] + ch.start;
+    float* const t = ptrs.p[ch.tensor - first_tensor] + ch.arena;
     float* const a = arena + ch.arena;
     // Whole vectors on the side that is added to or written (the arena's chunks are aligned, a tensor may start anywhere);
     // the side that is read takes four accesses where it is not aligned with the other, three of which the L1 serves.
@@ -191,18 +190,18 @@ struct OnDevice {
 
 }  // namespace
 
-TablePlan::TablePlan(int device, const std::vector<int64_t>& offsets, const std::vector<int64_t>& sizes) : device_(device), n_(int(sizes.size())) {
+TablePlan::TablePlan(int device, const std::vector<int64_t>& offsets, const std::vector<int64_t>& sizes)
+    : device_(device), n_(int(sizes.size())), offsets_(offsets) {
   if (offsets.size() != sizes.size() + 1) throw std::invalid_argument("a table has one more offset than tensors");
-  std::vector<Chunk> chunks;
+  uint32_t n_chunks = 0;
   std::vector<SumChunk> sum_chunks;
   std::vector<SumSegment> segments;
   std::vector<uint32_t> sum_first{0};
   const int64_t range = std::max(kSumRange, ((offsets.back() + kSumCtas - 1) / kSumCtas + 1023) / 1024 * 1024);
   for (int k = 0; k < n_; k++) {
     if ((offsets[k] & 3) != 0 || sizes[k] < 0 || offsets[k + 1] < offsets[k] + sizes[k]) throw std::invalid_argument("offsets and sizes of a table contradict each other");
-    first_chunk_.push_back(uint32_t(chunks.size()));
-    for (int64_t at = 0; at < sizes[k]; at += kChunk)
-      chunks.push_back({uint32_t(k), uint32_t(std::min<int64_t>(kChunk, sizes[k] - at)), at, offsets[k] + at});
+    first_chunk_.push_back(n_chunks);
+    n_chunks += uint32_t((sizes[k] + kChunk - 1) / kChunk);
     const int64_t len = offsets[k + 1] - offsets[k];
     segments.push_back({uint32_t(sum_chunks.size()), 0u, len});
     for (int64_t at = offsets[k]; at < offsets[k + 1];) {
@@ -215,46 +214,56 @@ TablePlan::TablePlan(int device, const std::vector<int64_t>& offsets, const std:
   }
   sum_first.push_back(uint32_t(sum_chunks.size()));
   n_sum_ctas_ = sum_chunks.empty() ? 0 : int(sum_first.size()) - 1;
-  first_chunk_.push_back(uint32_t(chunks.size()));
+  first_chunk_.push_back(n_chunks);
   // one block of device memory, laid out on the host and copied in one go
   auto padded = [](size_t v) { return (v + 255) / 256 * 256; };
-  const size_t o_sum = padded(chunks.size() * sizeof(Chunk)), o_seg = o_sum + padded(sum_chunks.size() * sizeof(SumChunk)),
-               o_fst = o_seg + padded(segments.size() * sizeof(SumSegment)), o_cnt = o_fst + padded(sum_first.size() * 4), o_par = o_cnt + padded(size_t(n_) * 4), bytes = o_par + padded(sum_chunks.size() * 8) + 256;
-  std::vector<uint8_t> host(o_par, 0);
-  if (!chunks.empty()) std::memcpy(host.data(), chunks.data(), chunks.size() * sizeof(Chunk));
-  if (!sum_chunks.empty()) std::memcpy(host.data() + o_sum, sum_chunks.data(), sum_chunks.size() * sizeof(SumChunk));
-  if (!segments.empty()) std::memcpy(host.data() + o_seg, segments.data(), segments.size() * sizeof(SumSegment));
-  std::memcpy(host.data() + o_fst, sum_first.data(), sum_first.size() * 4);
+  o_sum_ = padded(size_t(n_chunks) * sizeof(Chunk));
+  o_seg_ = o_sum_ + padded(sum_chunks.size() * sizeof(SumChunk));
+  o_fst_ = o_seg_ + padded(segments.size() * sizeof(SumSegment));
+  o_cnt_ = o_fst_ + padded(sum_first.size() * 4);
+  o_par_ = o_cnt_ + padded(size_t(n_) * 4);
+  bytes_ = o_par_ + padded(sum_chunks.size() * 8) + 256;
+  layout_.resize(o_par_);
+  Chunk* c = reinterpret_cast<Chunk*>(layout_.data());
+  for (int k = 0; k < n_; k++)
+    for (int64_t at = 0; at < sizes[k]; at += kChunk) *c++ = {offsets[k] + at, uint32_t(k), uint32_t(std::min<int64_t>(kChunk, sizes[k] - at))};
+  if (!sum_chunks.empty()) std::memcpy(layout_.data() + o_sum_, sum_chunks.data(), sum_chunks.size() * sizeof(SumChunk));
+  if (!segments.empty()) std::memcpy(layout_.data() + o_seg_, segments.data(), segments.size() * sizeof(SumSegment));
+  std::memcpy(layout_.data() + o_fst_, sum_first.data(), sum_first.size() * 4);
+}
+
+void TablePlan::bind(void* device_memory, void* pinned, void* stream) {
   OnDevice on(device_);
-  ck(cudaMalloc(&dev_, bytes), "cudaMalloc");
-  ck(cudaMallocHost(reinterpret_cast<void**>(&host_), (size_t(n_) * 2 + 1) * 8), "cudaMallocHost");
-  ck(cudaMemcpy(dev_, host.data(), o_par, cudaMemcpyHostToDevice), "cudaMemcpy");
-  uint8_t* d = static_cast<uint8_t*>(dev_);
+  uint8_t* d = static_cast<uint8_t*>(device_memory);
+  ck(cudaMemcpyAsync(d, layout_.data(), layout_.size(), cudaMemcpyHostToDevice, static_cast<cudaStream_t>(stream)), "cudaMemcpyAsync");
+  ck(cudaStreamSynchronize(static_cast<cudaStream_t>(stream)), "cudaStreamSynchronize");  // (used from any stream from here on)
+  std::vector<uint8_t>().swap(layout_);
   chunks_ = reinterpret_cast<Chunk*>(d);
-  sum_chunks_ = reinterpret_cast<SumChunk*>(d + o_sum);
-  sum_segments_ = reinterpret_cast<SumSegment*>(d + o_seg);
-  sum_first_ = reinterpret_cast<uint32_t*>(d + o_fst);
-  counters_ = reinterpret_cast<uint32_t*>(d + o_cnt);
-  partials_ = reinterpret_cast<double*>(d + o_par);
+  sum_chunks_ = reinterpret_cast<SumChunk*>(d + o_sum_);
+  sum_segments_ = reinterpret_cast<SumSegment*>(d + o_seg_);
+  sum_first_ = reinterpret_cast<uint32_t*>(d + o_fst_);
+  counters_ = reinterpret_cast<uint32_t*>(d + o_cnt_);
+  partials_ = reinterpret_cast<double*>(d + o_par_);
+  host_ = static_cast<double*>(pinned);
 }
 
 TablePlan::~TablePlan() {
+  if (chunks_ == nullptr) return;
   OnDevice on(device_);
-  cudaFree(dev_);
-  if (host_) cudaFreeHost(host_);
+  cudaDeviceSynchronize();  // kernels that use the memory may be under way on any stream
 }
 
 // The request for SMs is taken back by the last of several launches, the marks are set by each.
 template <bool ADD>
-static void launch_table(float* arena, const std::vector<uintptr_t>& ptrs, const Chunk* chunks, const std::vector<uint32_t>& first_chunk, UpdateMarks m,
-                         void* stream) {
+static void launch_table(float* arena, const std::vector<uintptr_t>& ptrs, const std::vector<int64_t>& offsets, const Chunk* chunks,
+                         const std::vector<uint32_t>& first_chunk, UpdateMarks m, void* stream) {
   const int n = int(ptrs.size());
   UpdateMarks inner = m;
   inner.yield_word = nullptr;
   for (int k0 = 0; k0 < n; k0 += kPtrs) {
     const int k1 = std::min(n, k0 + kPtrs);
     Pointers p;
-    for (int k = k0; k < k1; k++) p.p[k - k0] = reinterpret_cast<float*>(ptrs[k]);
+    for (int k = k0; k < k1; k++) p.p[k - k0] = reinterpret_cast<float*>(ptrs[k] - uintptr_t(offsets[k]) * 4);
     const uint32_t c0 = first_chunk[k0], count = first_chunk[k1] - c0;
     if (count == 0 && (k1 < n || m.yield_word == nullptr)) continue;
     table_kernel<ADD><<<count ? blocks_for(count) : 1, kThreads, 0, static_cast<cudaStream_t>(stream)>>>(arena, chunks + c0, count, uint32_t(k0), p,
@@ -264,11 +273,11 @@ static void launch_table(float* arena, const std::vector<uintptr_t>& ptrs, const
 }
 
 void TablePlan::add(float* arena, const std::vector<uintptr_t>& ptrs, const UpdateMarks& m, void* stream) const {
-  launch_table<true>(arena, ptrs, chunks_, first_chunk_, m, stream);
+  launch_table<true>(arena, ptrs, offsets_, chunks_, first_chunk_, m, stream);
 }
 
 void TablePlan::copy(const float* arena, const std::vector<uintptr_t>& ptrs, const UpdateMarks& m, void* stream) const {
-  launch_table<false>(const_cast<float*>(arena), ptrs, chunks_, first_chunk_, m, stream);
+  launch_table<false>(const_cast<float*>(arena), ptrs, offsets_, chunks_, first_chunk_, m, stream);
 }
 
 std::pair<std::vector<double>, std::vector<int>> TablePlan::scales(const float* arena, void* stream) {

@@ -20,6 +20,10 @@ class TablePlan {
   TablePlan(const TablePlan&) = delete;
 
   int tensors() const { return n_; }
+  // The caller's memory for the layout (device) and the magnitudes (pinned), to be given to bind() before anything else.
+  size_t device_bytes() const { return bytes_; }
+  size_t pinned_bytes() const { return (size_t(n_) * 2 + 1) * 8; }
+  void bind(void* device_memory, void* pinned, void* stream);
   // arena[k] += *ptrs[k], a reduction at the L2, for every tensor; *ptrs[k] = arena[k].  fp32 tensors of this device,
   // tensors() addresses.
   void add(float* arena, const std::vector<uintptr_t>& ptrs, const UpdateMarks& m, void* stream) const;
@@ -30,10 +34,12 @@ class TablePlan {
  private:
   int device_, n_;
   int n_sum_ctas_ = 0;
-  void* dev_ = nullptr;                 // everything below, one allocation
-  struct Chunk* chunks_ = nullptr;      // pieces of at most kChunk elements of the tensors, in arena order
+  std::vector<int64_t> offsets_;
+  std::vector<uint8_t> layout_;         // what bind() copies
+  size_t o_sum_ = 0, o_seg_ = 0, o_fst_ = 0, o_cnt_ = 0, o_par_ = 0, bytes_ = 0;
+  struct Chunk* chunks_ = nullptr;      // pieces of at most 4096 elements of the tensors, in arena order
   std::vector<uint32_t> first_chunk_;   // of each tensor
-  struct SumChunk* sum_chunks_ = nullptr;  // the same over whole segments, for the sums
+  struct SumChunk* sum_chunks_ = nullptr;  // pieces of the segments, for the sums
   struct SumSegment* sum_segments_ = nullptr;
   uint32_t* sum_first_ = nullptr;       // the first chunk of each CTA, and their number
   double* partials_ = nullptr;

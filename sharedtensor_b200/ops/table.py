@@ -65,7 +65,12 @@ class SharedTable:
             from .. import _native
 
             shapes = list(self.layout.shapes.values())
-            self._plan = _native.cuda().TablePlan(self.shared.device.index, self.layout.segment_offsets(), [s.numel() for s in shapes])
+            dev = self.shared.device
+            plan = _native.cuda().TablePlan(dev.index, self.layout.segment_offsets(), [s.numel() for s in shapes])
+            # (memory of torch's allocators: a cudaMalloc and a cudaMallocHost here took 1 ms and more)
+            plan.bind(torch.empty(plan.device_bytes(), dtype=torch.uint8, device=dev),
+                      torch.empty(plan.pinned_bytes(), dtype=torch.uint8, pin_memory=True), _stream(dev))
+            self._plan = plan
             # the look over a dict of tensors: their addresses, or None if one of them needs a conversion on the way
             self._addresses = _native.tensors().TensorList(self.layout.names, shapes, self.shared.device.index).addresses
         return rep, self._plan
