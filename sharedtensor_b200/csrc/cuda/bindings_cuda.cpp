@@ -67,7 +67,6 @@ PYBIND11_MODULE(_cuda, m) {
   m.def("add_scaled_bf16", [](uintptr_t v, uintptr_t g, float alpha, int64_t n, bool atomic, uintptr_t s) {
     ck(launch_add_scaled_bf16(ptr<float>(v), ptr<void>(g), alpha, n, atomic, UpdateMarks{}, strm(s)), "add_scaled_bf16");
   });
-  m.def("round_smem_bytes", &round_smem_bytes);
   m.def("table_scales_scratch_doubles", &table_scales_scratch_doubles);
   m.def("table_scales", [](uintptr_t x, uintptr_t offsets, int n_seg, int64_t n_total, uintptr_t scratch, uintptr_t out_sumsq,
                            uintptr_t out_exp, uintptr_t s) {

@@ -434,12 +434,6 @@ __device__ __forceinline__ T reduce_pieces(const T (&a)[kPieces], int lane, Op o
 
 }  // namespace
 
-int round_smem_bytes(int groups, int slots, int payload_bytes) {
-  (void)slots;
-  (void)payload_bytes;
-  return groups * int(sizeof(GroupShared));
-}
-
 // ----------------------------------------------------------------------------------------------
 // the kernel
 // ----------------------------------------------------------------------------------------------

@@ -18,10 +18,10 @@
 //
 // One launch of the round kernel makes up to `sweeps` passes over the tensor.  In a pass every group of
 // the grid looks at its own tiles' flags and credits, and for each tile that has something to do
-//   - stages values and mirrors with TMA bulk copies,
-//   - decodes the frames that arrived, accumulates them into the values (a bulk reduce-add, so that
-//     updates made by other streams at the same time are kept) and into the mirror of the link they
-//     came from (reference hot loops src/sharedtensor.c:106-111, 124-127),
+//   - loads values, mirrors and the frames that arrived into registers (a mesh member's frames by way of shared memory),
+//   - decodes the frames, accumulates them into the values (a reduction at the L2, so that updates made by other streams
+//     at the same time are kept) and into the mirror of the link they came from (reference hot loops
+//     src/sharedtensor.c:106-111, 124-127),
 //   - quantises values - mirror for every link, steps the mirror and pushes the packed codes and
 //     scales straight into the neighbours' ring slots (156-177),
 //   - and, once the stores have landed, publishes sequence flags to the receivers and credits to the
@@ -77,8 +77,8 @@ struct RoundParams {
   int32_t follows_window;        // the launch before this one in the stream is the window before this one, of the same cycle
   int32_t do_rx, do_tx;          // receiver-only / sender-only launches
   int32_t sweeps;                // passes over the tensor in this launch (>= 1)
-  uint32_t wait_ns;              // upper bound of every wait on one of the kernel's own copies
-  int32_t stall_tile;            // test hook: the copy barrier of this tile expects more bytes than are copied (-1: none)
+  uint32_t wait_ns;              // upper bound of every wait on the kernel's own warps and copies
+  int32_t stall_tile;            // test hook: this tile is never handed to the compute warps, so a wait runs out (-1: none)
   int32_t chunk;                 // > 0: a group owns this many consecutive tiles; 0: every (groups in the grid)-th tile
   const uint32_t* yield_flag;    // non-zero while an update is waiting for SMs: groups hand out no more tiles and leave
   uint32_t* dbg;                 // debug builds: progress marks in mapped host memory, 8 words per CTA (else null)
@@ -138,7 +138,6 @@ int launch_unsend(float* mirror, const uint8_t* payload_remote, uint32_t* tx_seq
                   int payload_bytes, int log2_block, int bits, int64_t n, uint64_t* taken_back, void* stream);
 // Adds to *count (pinned host memory) the frames that have been sent and not yet acknowledged, over all rings and tiles.
 int launch_count_unacknowledged(const RoundParams& p, uint32_t* count, void* stream);
-int round_smem_bytes(int groups, int slots, int payload_bytes);
 
 // Element-wise kernels (copyToTensor / addFromTensor / pushUpdate; src/sharedtensor.c:435-446, 334-344).
 // What an update or a snapshot does besides its data; null pointers: nothing.
