@@ -588,6 +588,7 @@ __device__ __forceinline__ void compute_warp(const RoundParams& p, GroupShared& 
     if (live) {
       const uint32_t go = lane == 0 ? (claim_tile(sh, c) ? 1u : 0u) : 0u;
       if (!__shfl_sync(0xffffffffu, go, 0)) break;
+      __syncwarp();  // a shuffle orders no memory: what lane 0 has acquired is there for all lanes from here on
       entry = c % kBank;
       d = sh.desc[entry];
       c++;
@@ -702,6 +703,7 @@ __device__ __forceinline__ void compute_warp(const RoundParams& p, GroupShared& 
           if (lb >= 9) { xm = fmaxf(xm, __shfl_xor_sync(0xffffffffu, xm, 2)); vm = fmaxf(vm, __shfl_xor_sync(0xffffffffu, vm, 2)); }
           if (lb >= 10 && live) {
             float(*red)[kComputeWarps] = sh.red[exchanges & 1u];
+            __syncwarp();  // every lane has read the exchange before last, whose words are written again behind this one
             if (lane == 0) {
               red[0][warp] = xm;
               red[1][warp] = vm;
@@ -963,6 +965,7 @@ __device__ __forceinline__ void service_warp(const RoundParams& p, GroupShared& 
       const uint32_t ready = __ballot_sync(0xffffffffu, (w & kDoneWarps) == uint32_t(kComputeWarps) && w < kDoneFailed);
       const uint32_t more = ready == 0xffffffffu ? 32u : uint32_t(__ffs(~ready) - 1);
       if (more) {
+        __syncwarp();  // (nor does a ballot) what each lane has acquired of its tile comes before the fence and the flags of any lane
         finished += more;
         t_last = globaltimer_ns();
       }

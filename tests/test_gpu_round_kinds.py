@@ -1,0 +1,110 @@
+"""Members of mesh groups and inner nodes of a tree, pass by pass and bit for bit against the host model."""
+import pytest
+import torch
+
+from sharedtensor_b200 import _native
+from sharedtensor_b200.parallel.local_wiring import connect_local, connect_mesh
+
+from replica_model import Oracle
+
+pytestmark = pytest.mark.gpu
+
+
+class Group:
+    """Replicas on one GPU and a host model of each.  `rings[i]`: the neighbours of replica i in ring order, with the link
+    the ring belongs to."""
+
+    def __init__(self, topology, members, n, bits, block, **options):
+        cu, core = _native.cuda(), _native.core()
+        cfg = cu.GpuConfig()
+        cfg.bits, cfg.block = bits, block
+        for k, v in options.items():
+            setattr(cfg, k, v)
+        self.n = n
+        self.reps = [cu.GpuReplica(0, n, cfg) for _ in range(members)]
+        if topology == "mesh":
+            connect_mesh(self.reps)
+            self.rings = [[(j, 0) for j in range(members) if j != i] for i in range(members)]
+        else:  # a star: replica 0 is the inner node
+            for leaf in self.reps[1:]:
+                connect_local(self.reps[0], leaf)
+            self.rings = [[(j, j - 1) for j in range(1, members)]] + [[(0, 0)] for _ in range(1, members)]
+        links = [1 + max(link for _, link in r) for r in self.rings]
+        self.models = [Oracle(core, n, block, k, bits) for k in links]
+        self.inbox = {(i, j): [] for i in range(members) for j, _ in self.rings[i]}
+        init = torch.randn(n)
+        stream = torch.cuda.current_stream().cuda_stream
+        for r, m in zip(self.reps, self.models):  # a common start that every edge knows
+            r.load_values(init.cuda().data_ptr(), stream)
+            m.v, m.k = init.clone(), [init.clone() for _ in m.k]
+            for link in range(len(m.k)):
+                r.copy_mirror_from_values(link)
+        torch.cuda.synchronize()
+
+    def add(self, i, d):
+        self.models[i].v += d
+        self.models[i].mark()
+        self.reps[i].add(d.cuda().data_ptr(), torch.cuda.current_stream().cuda_stream)
+        torch.cuda.synchronize()
+
+    def visit(self, i):
+        self.reps[i].round()
+        self.reps[i].sync()
+        arrived = {}
+        for j, link in self.rings[i]:
+            arrived.setdefault(link, []).extend(self.inbox[(i, j)])
+            self.inbox[(i, j)] = []
+        for link, frame in self.models[i].visit(arrived).items():
+            for j, l in self.rings[i]:
+                if l == link:
+                    self.inbox[(j, i)].append(frame)
+
+    def check(self, i, where):
+        r, m = self.reps[i], self.models[i]
+        got = torch.empty(self.n, device="cuda")
+        r.snapshot(got.data_ptr(), torch.cuda.current_stream().cuda_stream)
+        torch.cuda.synchronize()
+        assert torch.equal(got.cpu(), m.v), f"values of replica {i} differ {where}"
+        for link, k in enumerate(m.k):
+            _native.cuda().memcpy_d2d(got.data_ptr(), r.mirror_ptr(link), self.n * 4)
+            torch.cuda.synchronize()
+            assert torch.equal(got.cpu(), k), f"mirror {link} of replica {i} differs {where}"
+
+    def done(self):
+        for r in self.reps:
+            assert r.status()[5] == 0, "no error bits"
+            assert r.check_guards() == 0
+
+
+@pytest.mark.parametrize("block", [32, 256, 1024, 4096])
+@pytest.mark.parametrize("bits", [1, 2, 4, 8])
+@pytest.mark.parametrize("topology,members", [("mesh", 3), ("mesh", 8), ("star", 3), ("star", 4)])
+def test_round_bit_exact_in_a_group(topology, members, bits, block):
+    """Replica 0 makes every third pass only, so that it finds up to three frames in each ring (up to twenty-one for a
+    tile, more than a member stages in shared memory)."""
+    torch.manual_seed(members * 100 + bits * 10 + block)
+    g = Group(topology, members, 2 * 4096 + 333, bits, block)
+    for it in range(10):
+        if it in (0, 4):
+            for i in range(members):
+                g.add(i, torch.randn(g.n) * 10.0 ** -(i % 3))
+        for i in range(members):
+            if i == 0 and it % 3:
+                continue
+            g.visit(i)
+            g.check(i, f"in pass {it}")
+    g.done()
+
+
+@pytest.mark.parametrize("topology,members", [("mesh", 2), ("mesh", 4), ("star", 4)])
+def test_round_bit_exact_with_many_tiles_per_group(topology, members):
+    """One CTA for 151 tiles: its two groups go through their 32 descriptors more than twice in a pass."""
+    torch.manual_seed(members)
+    g = Group(topology, members, 150 * 4096 + 7, 8, 32, comm_ctas=1)
+    for i in range(members):
+        g.add(i, torch.randn(g.n))
+    for it in range(4):
+        for i in range(members):
+            g.visit(i)
+            g.check(i, f"in pass {it}")
+    g.done()
