@@ -165,7 +165,7 @@ PYBIND11_MODULE(_cuda, m) {
       .def("table_copy", [](GpuReplica& r, const TablePlan& t, const py::bytes& p, uintptr_t s) { r.table_copy(t, unpack(p), strm(s)); })
       .def("copy_mirror_from_values", &GpuReplica::copy_mirror_from_values)
       .def("round", &GpuReplica::round, py::arg("do_rx") = true, py::arg("do_tx") = true, py::arg("sweeps") = 1)
-      .def("set_test_stall_tile", &GpuReplica::set_test_stall_tile)
+      .def("set_test_stall_tile", &GpuReplica::set_test_stall_tile, py::arg("tile"), py::arg("warp") = -1)
       .def("check_guards", [](GpuReplica& r) { py::gil_scoped_release rel; return r.check_guards(); })
       .def("bits", &GpuReplica::bits)
       .def("debug_crumbs", &GpuReplica::debug_crumbs)

@@ -126,6 +126,7 @@ GpuReplica::GpuReplica(int device, int64_t n, const GpuConfig& cfg) : device_(de
   params_.sweeps = 1;
   params_.wait_ns = uint32_t(cfg.poll_deadline_us < 1 ? 1 : (cfg.poll_deadline_us > 2000000 ? 2000000 : cfg.poll_deadline_us)) * 1000u;
   params_.stall_tile = -1;
+  params_.stall_warp = -1;
   params_.yield_flag = cfg_.yield_to_updates ? yield_flag_ : nullptr;
   params_.dbg = nullptr;
   if (::getenv("SHAREDTENSOR_DEBUG_CRUMBS")) {
@@ -417,9 +418,10 @@ int GpuReplica::check_guards() {
   return bad;
 }
 
-void GpuReplica::set_test_stall_tile(int tile) {
+void GpuReplica::set_test_stall_tile(int tile, int warp) {
   std::lock_guard<std::mutex> lk(mu_);
   params_.stall_tile = tile;
+  params_.stall_warp = warp;
 }
 
 void GpuReplica::load_values(const float* src, void* user_stream) {

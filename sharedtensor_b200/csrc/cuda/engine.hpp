@@ -110,7 +110,7 @@ class GpuReplica {
   void round(bool do_rx = true, bool do_tx = true, int sweeps = 1);
   // Test hook: while set (>= 0), the round kernel's copy barrier of this tile expects more bytes than are copied,
   // so the bounded wait of the group that owns the tile runs out.
-  void set_test_stall_tile(int tile);
+  void set_test_stall_tile(int tile, int warp);
   // Compares the canaries around the values, every mirror and every edge block; returns the number of damaged ones.
   int check_guards();
   // TCP links: a link with a mirror and no ring peers; its tensor-scale frames (the reference's wire format) are

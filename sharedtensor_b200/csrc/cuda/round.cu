@@ -24,8 +24,10 @@
 // Small tensors: latency.  A launch over one tile takes 10 us in the kernel, of which the look at the tile takes 2, the
 // tile 3 and the fence 2; some hundred tiles take 23 us, of which the fence takes 5 to 8 (see the publication below).
 //
-// Nothing in here waits for another GPU.  The waits are on this group's own warps, and every one is bounded: when a
-// wait runs out the group records an error in the status block, marks its tiles for another visit and leaves.
+// Nothing in here waits for another GPU.  The waits are on this group's own warps and copies, and every one is bounded.
+// When one runs out, no visit is left half done: the warps go by the same answer, frames that are not in their stage are
+// read from the ring, and a block whose maximum is not known is not spoken of while everything that arrived is taken in and
+// acknowledged.  The group records an error in the status block, marks its tiles for another visit and leaves.
 //
 // Arithmetic is written with explicit round-to-nearest operations; block statistics are maxima (order does not
 // matter), so codes, scales, mirrors and values are bit-identical to the host codec (../core/codec.cpp).
@@ -143,15 +145,16 @@ __device__ __forceinline__ uint64_t globaltimer_ns() {
   return t;
 }
 
-// Bounded wait on one of this CTA's own barriers; false when `limit_ns` has passed.
+// Bounded wait on one of this CTA's own barriers; false when `limit_ns` has passed.  The clock runs on while another process
+// has the GPU, so the wait also takes a number of looks, the last of them after the clock was read.
 __device__ __forceinline__ bool mbar_wait_bounded(uint64_t* bar, uint32_t parity, uint64_t limit_ns) {
   if (mbar_try_wait(bar, parity)) return true;
   const uint64_t t0 = globaltimer_ns();
   for (uint32_t it = 0; it < (1u << 26); it++) {
     if (mbar_try_wait(bar, parity)) return true;
-    if ((it & 15) == 15 && globaltimer_ns() - t0 > limit_ns) return false;
+    if ((it & 15) == 15 && it > 48 && globaltimer_ns() - t0 > limit_ns) break;
   }
-  return false;
+  return mbar_test(bar, parity);
 }
 
 // ----------------------------------------------------------------------------------------------
@@ -171,9 +174,9 @@ constexpr uint32_t kDescTxWant = 1u << 12;  // << link: the link may have someth
 // what a compute warp adds to a tile's `done` word when it has finished its part
 constexpr uint32_t kDoneWarp = 1, kDoneWarps = 0xff;
 constexpr int kDoneNonsilentShift = 8;      // + 4 * link: warps that found something to say on the link
-constexpr uint32_t kDoneFailed = 1u << 24;  // a wait ran out: nothing of the warp's part was stored
+constexpr uint32_t kDoneFailed = 1u << 24;  // a wait ran out: what arrived has been taken in, links that were to hear something may not have
 
-constexpr uint32_t kClaimStop = 0x80000000u;
+constexpr uint32_t kStop = 0x80000000u;     // a count of steps that has been closed, see claim_tile()
 
 struct GroupShared {
   TileDesc desc[kBank];
@@ -182,8 +185,9 @@ struct GroupShared {
   uint32_t done[kBank];
   uint64_t full[2], empty[2];  // of the two frame stages
   uint32_t armed;        // tiles armed so far in this launch (bank entry = number % kBank)
-  uint32_t claim;        // tiles the compute warps have started so far | kClaimStop: no new ones
-  uint32_t pad[2];
+  uint32_t claim;        // tiles the compute warps have started so far | kStop: no new ones
+  uint32_t exchanged;    // exchanges the compute warps have gone through so far | kStop: one ran out
+  uint32_t pad;
   uint64_t gsync;        // the compute warps among themselves (blocks of more than 512 elements)
   float red[2][2][kComputeWarps];  // two buffers: a warp may be one step ahead of the slowest one
   alignas(16) uint32_t stage[kComputeWarps][kWarpElems / 4];  // the codes of a warp's part on their way into the ring slots
@@ -439,26 +443,33 @@ __device__ __forceinline__ T reduce_pieces(const T (&a)[kPieces], int lane, Op o
 // ----------------------------------------------------------------------------------------------
 namespace {
 
-// Lane 0 of a compute warp: may the warp work on the group's tile number c?  All eight warps get the same answer: the
-// first one to come by moves the claim past c, unless the service warp has closed it.  The wait covers a service warp
-// that is looking for work; the limit only covers one that never comes back.
+// The eight compute warps take the steps of a launch (tiles, exchanges) in order, and each step is taken by all of them or by
+// none, so that no warp has stored its part of a visit that another gave up.  A count of the steps taken says which: the
+// first warp to come by moves it past step c, or closes it (kStop) because its wait ran out; the others follow.
+
+// Lane 0 of a compute warp: does the group work on its tile number c?  No when the service warp has closed the claim.  The
+// wait covers a service warp that is looking for work; the limit only covers one that never comes back.
 __device__ __forceinline__ bool claim_tile(GroupShared& sh, uint32_t c) {
   uint64_t t_start = 0;
+  bool give_up = false;
+#pragma unroll 1
   for (uint32_t it = 0; it < (1u << 28); it++) {
-    if (int32_t(ld_shared_acquire(&sh.armed) - c) > 0) {
-      const uint32_t cl = *reinterpret_cast<volatile uint32_t*>(&sh.claim);
-      if ((cl & ~kClaimStop) > c) return true;
-      if (cl & kClaimStop) return false;
-      if (atomicCAS(&sh.claim, cl, c + 1u) == cl) return true;
+    const bool armed = int32_t(ld_shared_acquire(&sh.armed) - c) > 0;
+    const uint32_t cl = *reinterpret_cast<volatile uint32_t*>(&sh.claim);
+    if ((cl & ~kStop) > c) {
+      if (armed) return true;  // (not armed: the word has been read before another warp saw it armed)
+    } else if (cl & kStop) {
+      return false;
+    } else if (armed || give_up) {
+      if (atomicCAS(&sh.claim, cl, armed ? c + 1u : cl | kStop) == cl) return armed;
       continue;
     }
-    if (*reinterpret_cast<volatile uint32_t*>(&sh.claim) & kClaimStop) return false;
     if ((it & 63) == 63) {
       const uint64_t now = globaltimer_ns();
       if (t_start == 0) t_start = now;
-      if (now - t_start > 2000ull * 1000 * 1000) return false;
+      give_up = now - t_start > 2000ull * 1000 * 1000;
     }
-    __nanosleep(20);
+    if (!armed) __nanosleep(20);
   }
   return false;
 }
@@ -491,7 +502,7 @@ constexpr int kStaged = kKind == kMember ? 8 : 0;
 // with three links and six frames per tile took 224 us per 16 M elements when it decoded them for the values and again for
 // each mirror, 170 us so).  The loop stays rolled: the code of a tile's visit has to fit the instruction cache.
 template <int Q, bool kStash, int kIn>
-__device__ __forceinline__ void decode_frames(const uint64_t* list, const uint8_t* staged, int count, uint32_t live, uint64_t* empty, int log2_block,
+__device__ __forceinline__ void decode_frames(const uint64_t* list, const uint8_t* staged, bool in_stage, int count, uint32_t live, uint64_t* empty, int log2_block,
                                               int warp, int lane, int left, float* stash, Piece (&total)[kPieces]) {
   Piece mine[kPieces];
   int cur = -1;
@@ -506,7 +517,7 @@ __device__ __forceinline__ void decode_frames(const uint64_t* list, const uint8_
   for (int j = 0; j < count; j++) {
     FrameRegs f{};
     if (live) {
-      if (j < kIn) load_staged<Q>(staged + j * kFrameRoom<Q>, warp, lane, log2_block, f);
+      if (in_stage && j < kIn) load_staged<Q>(staged + j * kFrameRoom<Q>, warp, lane, log2_block, f);
       else load_frame<Q>(frame_at(list[j]), warp, lane, log2_block, f);
     }
     if (kStash) {
@@ -530,7 +541,7 @@ __device__ __forceinline__ void decode_frames(const uint64_t* list, const uint8_
   if (kStash && cur >= 0) put(cur);
   if (kIn == 0) return;
   __syncwarp();
-  if (live && lane == 0) mbar_arrive(empty);  // the stage may be filled again when all warps have been here
+  if (live && in_stage && lane == 0) mbar_arrive(empty);  // the stage may be filled again when all warps have read it
 }
 
 // One lane's codes of its four pieces into the ring slots of link l's neighbours.  They go through shared memory, so
@@ -570,6 +581,42 @@ __device__ __forceinline__ void send_codes(const uint64_t* list, int count, int 
   }
 }
 
+// Test hook: this warp's waits for the tile count as having run out.
+__device__ __forceinline__ bool held(const RoundParams& p, int tile, int warp) {
+  return tile == p.stall_tile && p.stall_warp >= 0 && (p.stall_warp & (kComputeWarps - 1)) == warp;
+}
+
+// The maxima of a block of 1024 elements and more, over the warps that share it: {-1, -1} if the eight did not come together
+// in time for exchange number e.
+__device__ __forceinline__ float2 exchange(const RoundParams& p, GroupShared& sh, uint32_t e, int tile, int warp, int lane, float xm, float vm) {
+  const bool hold = held(p, tile, warp);
+  float(*red)[kComputeWarps] = sh.red[e & 1u];
+  __syncwarp();  // every lane has read the exchange before last, whose words are written again behind this one
+  if (lane == 0 && !(hold && p.stall_warp < kComputeWarps)) {
+    red[0][warp] = xm;
+    red[1][warp] = vm;
+    mbar_arrive(&sh.gsync);
+  }
+  const bool there = __all_sync(0xffffffffu, !hold && mbar_wait_bounded(&sh.gsync, e & 1u, p.wait_ns));
+  bool go = false;
+  if (lane == 0) {
+    const uint32_t seen = atomicCAS(&sh.exchanged, e, there ? e + 1u : e | kStop);
+    go = seen == e ? there : (seen & ~kStop) > e;
+  }
+  if (!__any_sync(0xffffffffu, go)) return make_float2(-1.f, -1.f);
+  if (!there) (void)mbar_wait_bounded(&sh.gsync, e & 1u, p.wait_ns);  // (another warp has seen it complete)
+  const int share = 1 << (p.log2_block - 9), w0 = warp & ~(share - 1);
+  for (int j = 0; j < share; j++) {
+    xm = fmaxf(xm, red[0][w0 + j]);
+    vm = fmaxf(vm, red[1][w0 + j]);
+  }
+  return make_float2(xm, vm);
+}
+// (out of the way of smaller blocks where the visit has few registers to save around a call)
+__device__ __noinline__ float2 exchange_apart(const RoundParams& p, GroupShared& sh, uint32_t e, int tile, int warp, int lane, float xm, float vm) {
+  return exchange(p, sh, e, tile, warp, lane, xm, vm);
+}
+
 template <int Q, int kKind>
 __device__ __forceinline__ void compute_warp(const RoundParams& p, GroupShared& sh, float* group_stash, const uint8_t* stages, int warp, int lane) {
   constexpr bool kOneLink = kKind != kInner;  // what arrived for the values is what arrived on the link
@@ -577,6 +624,7 @@ __device__ __forceinline__ void compute_warp(const RoundParams& p, GroupShared& 
   const int L = kOneLink ? 1 : p.n_links, lb = p.log2_block;
   float res_max0 = 0.f, res_max1 = 0.f, res_max2 = 0.f;
   uint32_t exchanges = 0;
+  bool unstaged = false;  // the warp has stopped using the stages
   // While the service warp looks for work, the compute warps go once through the code of a visit with nothing in hand: the
   // instruction cache is cold at the start of a launch, and the first tile took 5 us longer than the others for that.
   uint32_t live = 0;
@@ -644,12 +692,14 @@ __device__ __forceinline__ void compute_warp(const RoundParams& p, GroupShared& 
       };
       if (kOneLink) fetch();
       const uint32_t st = d.stage & 1u;
-      if (kIn > 0 && live && !__all_sync(0xffffffffu, mbar_wait_bounded(&sh.full[st], (d.stage >> 1) & 1u, 2ull * p.wait_ns))) {
-        if (lane == 0) red_shared_release_add(&sh.done[entry], kDoneWarp | kDoneFailed);  // nothing of the tile is stored
-        break;
+      if (kIn > 0 && live) {
+        // A warp whose stage is not filled in time reads the frames from the ring, where they stay until the tile is
+        // published.  It does not report the stage as read, so that neither stage is filled again under another warp's
+        // hands once its turn has come, and uses no stage any more.
+        if (!unstaged) unstaged = !__all_sync(0xffffffffu, !held(p, d.tile, warp) && mbar_wait_bounded(&sh.full[st], (d.stage >> 1) & 1u, 2ull * p.wait_ns));
       }
       Piece acc[kPieces];
-      decode_frames<Q, !kOneLink, kIn>(frames, stages + st * (kIn * kFrameRoom<Q>), d.n_frames, live, &sh.empty[st], lb, warp, lane, left,
+      decode_frames<Q, !kOneLink, kIn>(frames, stages + st * (kIn * kFrameRoom<Q>), !unstaged, d.n_frames, live, &sh.empty[st], lb, warp, lane, left,
                                        group_stash + in_tile, acc);
       if (!kOneLink) fetch();
 #pragma unroll
@@ -702,23 +752,21 @@ __device__ __forceinline__ void compute_warp(const RoundParams& p, GroupShared& 
           if (lb >= 8) { xm = fmaxf(xm, __shfl_xor_sync(0xffffffffu, xm, 1)); vm = fmaxf(vm, __shfl_xor_sync(0xffffffffu, vm, 1)); }
           if (lb >= 9) { xm = fmaxf(xm, __shfl_xor_sync(0xffffffffu, xm, 2)); vm = fmaxf(vm, __shfl_xor_sync(0xffffffffu, vm, 2)); }
           if (lb >= 10 && live) {
-            float(*red)[kComputeWarps] = sh.red[exchanges & 1u];
-            __syncwarp();  // every lane has read the exchange before last, whose words are written again behind this one
-            if (lane == 0) {
-              red[0][warp] = xm;
-              red[1][warp] = vm;
-              mbar_arrive(&sh.gsync);
-            }
-            if (!__all_sync(0xffffffffu, mbar_wait_bounded(&sh.gsync, exchanges & 1u, p.wait_ns))) {
+            float2 m = make_float2(-1.f, -1.f);
+            if (!failed) m = kOneLink ? exchange_apart(p, sh, exchanges, d.tile, warp, lane, xm, vm) : exchange(p, sh, exchanges, d.tile, warp, lane, xm, vm);
+            if (__any_sync(0xffffffffu, m.x < 0.f)) {
+              // Without the block's maximum nothing can be said on the link; what arrived is taken in all the same.  (From
+              // here on no warp comes to the barrier any more: nobody is counted for an exchange it was late for.)
               failed = true;
-              break;
+              if (changed) {
+#pragma unroll
+                for (int i = 0; i < kPieces; i++) store_piece(kp + i * 128, k[i]);
+              }
+              continue;
             }
             exchanges++;
-            const int w0 = warp & ~((1 << (lb - 9)) - 1);
-            for (int j = 0; j < (1 << (lb - 9)); j++) {
-              xm = fmaxf(xm, red[0][w0 + j]);
-              vm = fmaxf(vm, red[1][w0 + j]);
-            }
+            xm = m.x;
+            vm = m.y;
           }
         }
         const uint32_t code = uint32_t(block_code_dev<Q>(xm, __float_as_uint(vm), p.min_exp, p.rel_bits));
@@ -740,7 +788,7 @@ __device__ __forceinline__ void compute_warp(const RoundParams& p, GroupShared& 
         for (int i = 0; i < kPieces; i++) store_piece(kp + i * 128, k[i]);
       }
     }
-    if (failed) finished |= kDoneFailed;
+    if (failed || unstaged) finished |= kDoneFailed;
     __syncwarp();  // what the lanes stored comes before what lane 0 says about it
     if (lane == 0 && live) red_shared_release_add(&sh.done[entry], finished);
     if (failed) break;
@@ -799,6 +847,7 @@ __device__ __forceinline__ void service_warp(const RoundParams& p, GroupShared& 
   uint32_t handed = 0, staged = 0;                  // tiles the compute warps may start, and those of them whose frames have been seen to
   uint32_t stage_no = 0, stage_issued = 0;          // tiles with two frames or more found so far, and those staged
   bool aborted = false, yielded = false;
+  bool ran_out = false;                             // a wait of a compute warp did
 
   if (p.zero_other && blockIdx.x == 0 && g == 0 && lane == 0) {
     uint64_t* other = p.status + (p.parity ? kDsLaunch0 : kDsLaunch1);  // the next cycle's half
@@ -816,7 +865,7 @@ __device__ __forceinline__ void service_warp(const RoundParams& p, GroupShared& 
     uint64_t t_last = globaltimer_ns();
     while (true) {
       // ---- the frames of the next tiles that have several on their way into shared memory, as stages become free
-      while (staged_frames > 0 && staged != handed) {
+      while (staged_frames > 0 && staged != handed && !ran_out) {
         const TileDesc d = sh.desc[staged % kBank];
         if (d.n_frames > 1) {
           const uint32_t u = stage_issued & 1u;
@@ -836,7 +885,7 @@ __device__ __forceinline__ void service_warp(const RoundParams& p, GroupShared& 
         staged++;
       }
       // ---- look at more tiles while the compute warps have less than kAhead in hand and the bank has room for them
-      if (looked < my_count && !yielded && armed - finished < uint32_t(kAhead) && armed - published + uint32_t(at_once) <= uint32_t(kBank)) {
+      if (looked < my_count && !yielded && !aborted && !ran_out && armed - finished < uint32_t(kAhead) && armed - published + uint32_t(at_once) <= uint32_t(kBank)) {
         ST_CRUMB(g, 2);
         const uint32_t y = p.yield_flag != nullptr && lane == 0 ? ld_cg_u32(p.yield_flag) : 0u;
         const int j = looked + t;
@@ -941,7 +990,7 @@ __device__ __forceinline__ void service_warp(const RoundParams& p, GroupShared& 
           sh.moved[entry][r] = uint8_t(avail | (goes_out ? 4u : 0u));
         }
         // test hook: this tile is never handed to the compute warps, so the wait for it below runs out
-        const uint32_t stalled = __ballot_sync(0xffffffffu, work && tile == p.stall_tile && r == 0);
+        const uint32_t stalled = __ballot_sync(0xffffffffu, work && tile == p.stall_tile && p.stall_warp < 0 && r == 0);
         handed = stalled ? armed + __popc(work_tiles & ((1u << (__ffs(stalled) - 1)) - 1u)) : armed + __popc(work_tiles);
         __syncwarp();
         if (lane == 0) st_shared_release(&sh.armed, handed);
@@ -961,15 +1010,16 @@ __device__ __forceinline__ void service_warp(const RoundParams& p, GroupShared& 
       ST_CRUMB(g, 4);
       const uint32_t at = finished + uint32_t(lane);
       const uint32_t w = int32_t(armed - at) > 0 ? ld_shared_acquire(&sh.done[at % kBank]) : 0u;
-      const bool fail = __any_sync(0xffffffffu, w >= kDoneFailed);
-      const uint32_t ready = __ballot_sync(0xffffffffu, (w & kDoneWarps) == uint32_t(kComputeWarps) && w < kDoneFailed);
+      ran_out |= __any_sync(0xffffffffu, w >= kDoneFailed);
+      const uint32_t ready = __ballot_sync(0xffffffffu, (w & kDoneWarps) == uint32_t(kComputeWarps));
       const uint32_t more = ready == 0xffffffffu ? 32u : uint32_t(__ffs(~ready) - 1);
       if (more) {
         __syncwarp();  // (nor does a ballot) what each lane has acquired of its tile comes before the fence and the flags of any lane
         finished += more;
         t_last = globaltimer_ns();
+        idle = 0;
       }
-      const bool last = finished == armed && (looked >= my_count || yielded || aborted);
+      const bool last = finished == armed && (looked >= my_count || yielded || aborted || ran_out);
       // ---- publish: when nothing is in hand, and earlier when half a bank has piled up, so that a neighbour does not
       // wait for the end of a long launch.  Not more often: a system-scope fence takes 1.5 us on a quiet GPU and 3.9 us as
       // soon as 37 or more SMs have one under way (measured: 2815 and 7400 cycles), and a fence that finds others under
@@ -994,7 +1044,7 @@ __device__ __forceinline__ void service_warp(const RoundParams& p, GroupShared& 
             n_rx += moved & 3u;
           }
           if (r == 0) {
-            bool left = false;
+            bool left = done >= kDoneFailed;
             for (int l = 0; l < p.n_links; l++) {
               if (((done >> (kDoneNonsilentShift + 4 * l)) & 0xfu) == 0) continue;
               left = true;  // more may be left to say (or nothing could be said at all)
@@ -1013,8 +1063,10 @@ __device__ __forceinline__ void service_warp(const RoundParams& p, GroupShared& 
       if (last) break;
       if (more) continue;
       idle++;
-      const bool late = __any_sync(0xffffffffu, fail || globaltimer_ns() - t_last > 2 * limit_ns);
-      if (late) {
+      // (The time by the clock and in looks, like the waits of the compute warps.  The second time it is longer than all the
+      // waits of a compute warp in one tile: one on a stage, one per link on an exchange.)
+      const bool late = __any_sync(0xffffffffu, idle > 2048u && globaltimer_ns() - t_last > (aborted ? 8 : 2) * limit_ns);
+      if (late || (ran_out && !aborted)) {
         if (aborted) break;  // the tiles that had been started did not finish either
         aborted = true;
       } else if (yielded || aborted || (idle & 7u) != 0 || !update_waiting()) {
@@ -1026,7 +1078,7 @@ __device__ __forceinline__ void service_warp(const RoundParams& p, GroupShared& 
       // An update is waiting for the SMs this kernel holds, or a wait ran out: no more tiles are started.  Those that
       // were looked at but not started get their change marks back, everything else about them is untouched.
       uint32_t started = 0;
-      if (lane == 0) started = atomicOr(&sh.claim, kClaimStop) & ~kClaimStop;
+      if (lane == 0) started = atomicOr(&sh.claim, kStop) & ~kStop;
       started = __shfl_sync(0xffffffffu, started, 0);
       for (uint32_t c = started + uint32_t(lane); int32_t(armed - c) > 0; c += 32)
         if (sh.dirty[c % kBank]) st_cg_u32(p.tile_state + sh.desc[c % kBank].tile, 1u);
@@ -1035,15 +1087,15 @@ __device__ __forceinline__ void service_warp(const RoundParams& p, GroupShared& 
       if (int32_t(staged - handed) > 0) staged = handed;
       t_last = globaltimer_ns();
     }
-    if (aborted) break;
+    if (aborted || ran_out) break;
     n_sweeps++;
     if (armed == armed_before && sweep + 1 < p.sweeps) __nanosleep(1000);
   }
-  if (lane == 0) atomicOr(&sh.claim, kClaimStop);  // the compute warps leave
+  if (lane == 0) atomicOr(&sh.claim, kStop);  // the compute warps leave
   // copies of tiles that nobody started get a bounded chance to land before the CTA's shared memory is released
   for (uint32_t q = stage_issued > 2 ? stage_issued - 2 : 0; q < stage_issued; q++)
     (void)__all_sync(0xffffffffu, mbar_wait_bounded(&sh.full[q & 1u], (q >> 1) & 1u, limit_ns));
-  if (aborted) {
+  if (aborted || ran_out) {
     for (int j = lane; j < my_count; j += 32) st_cg_u32(p.tile_state + gid + j * gstride, 1u);
     if (lane == 0) {
       atomicOr(reinterpret_cast<unsigned long long*>(p.status + kDsErrors), (unsigned long long)kErrBarrierTimeout);
@@ -1092,6 +1144,7 @@ __global__ void __launch_bounds__(kGroups * kGroupThreads, 1) round_kernel(const
     GroupShared& sh = shared[threadIdx.x];
     sh.armed = 0;
     sh.claim = 0;
+    sh.exchanged = 0;
     mbar_init(&sh.gsync, kComputeWarps);
     for (int u = 0; u < 2; u++) {
       mbar_init(&sh.full[u], 1);

@@ -78,7 +78,8 @@ struct RoundParams {
   int32_t do_rx, do_tx;          // receiver-only / sender-only launches
   int32_t sweeps;                // passes over the tensor in this launch (>= 1)
   uint32_t wait_ns;              // upper bound of every wait on the kernel's own warps and copies
-  int32_t stall_tile;            // test hook: this tile is never handed to the compute warps, so a wait runs out (-1: none)
+  int32_t stall_tile;            // test hook: a wait for this tile runs out (-1: none)
+  int32_t stall_warp;            // -1: it is never handed to the compute warps; w: compute warp w does not come to its waits; 8 + w: it comes late
   int32_t chunk;                 // > 0: a group owns this many consecutive tiles; 0: every (groups in the grid)-th tile
   const uint32_t* yield_flag;    // non-zero while an update is waiting for SMs: groups hand out no more tiles and leave
   uint32_t* dbg;                 // debug builds: progress marks in mapped host memory, 8 words per CTA (else null)

@@ -100,11 +100,12 @@ class Oracle:
         pad[:scales.numel()] = scales
         return pad.reshape(-1, spt).ne(0).any(1)
 
-    def visit(self, arrived=None):
+    def visit(self, arrived=None, unheard=None):
         """One pass over the tensor.  `arrived`: {link: [frames]} found in the in-rings.  Returns {link: frame} for the
         links that were told something (frames that say nothing anywhere are left out).  What arrived goes into the
         values and into the mirror of the link it came on; a link then hears about a tile if the tile carries a
-        change mark or if something for it arrived on another link."""
+        change mark or if something for it arrived on another link.  `unheard`: mask of tiles that no link hears about
+        this time (a wait ran out); they keep a mark."""
         arrived = {l: fr for l, fr in sorted((arrived or {}).items()) if fr}
         came = {l: torch.zeros_like(self.dirty) for l in arrived}
         total = torch.zeros(self.n)   # everything that arrived, added up ring by ring and frame by frame, goes into
@@ -126,10 +127,12 @@ class Oracle:
             for j, m in came.items():
                 if j != l:
                     want |= m
+            if unheard is not None:
+                want &= ~unheard
             self.dirty = want.clone()
             frame = self.encode(l)          # leaves in self.dirty the wanted tiles that still had something to say
             still |= self.dirty
             if bool(frame[1].any()):
                 out[l] = frame
-        self.dirty = still
+        self.dirty = still if unheard is None else still | unheard
         return out
