@@ -1,0 +1,42 @@
+// What the engine thread tells a flush: how many launches it has looked back on, and the last of them that found work.
+#pragma once
+#include <algorithm>
+#include <atomic>
+#include <cstdint>
+
+namespace st {
+
+class QuietWatch {
+ public:
+  // ---- engine thread
+  void begin() { looked_.store(launched_.load()); }  // launches of an earlier run that were not looked back on
+  void launched() { launched_.fetch_add(1); }
+  void looked(bool busy, uint64_t now_ns) {
+    const uint64_t n = looked_.load() + 1;
+    if (busy) {
+      busy_ns_.store(now_ns);
+      busy_launch_.store(n);
+    }
+    looked_.store(n);
+  }
+
+  // ---- flush
+  uint64_t launches() const { return launched_.load(); }
+  // The last `count` launches found nothing and were all begun after launch number `before`.  (The launches are read before
+  // the busy one, which is written before them: a busy launch is never counted.)
+  bool quiet_launches(uint64_t before, uint64_t count) const {
+    const uint64_t n = looked_.load(), busy = busy_launch_.load();
+    return n >= std::max(before, busy) + count;
+  }
+  // How long no launch has found work, counted from `start_ns` at the earliest.  The engine thread may have found some since
+  // the caller took the time.
+  uint64_t quiet_for(uint64_t start_ns, uint64_t now_ns) const {
+    const uint64_t since = std::max(start_ns, busy_ns_.load());
+    return now_ns > since ? now_ns - since : 0;
+  }
+
+ private:
+  std::atomic<uint64_t> launched_{0}, looked_{0}, busy_launch_{0}, busy_ns_{0};
+};
+
+}  // namespace st

@@ -116,6 +116,15 @@ PYBIND11_MODULE(_cuda, m) {
       .def_readwrite("chunk_tiles", &GpuConfig::chunk_tiles)
       .def_readwrite("window_tiles", &GpuConfig::window_tiles);
 
+  py::class_<QuietWatch>(m, "QuietWatch")
+      .def(py::init<>())
+      .def("begin", &QuietWatch::begin)
+      .def("launched", &QuietWatch::launched)
+      .def("looked", &QuietWatch::looked)
+      .def("launches", &QuietWatch::launches)
+      .def("quiet_launches", &QuietWatch::quiet_launches)
+      .def("quiet_for", &QuietWatch::quiet_for);
+
   py::class_<TablePlan>(m, "TablePlan")
       .def(py::init<int, const std::vector<int64_t>&, const std::vector<int64_t>&>())
       .def("tensors", &TablePlan::tensors)

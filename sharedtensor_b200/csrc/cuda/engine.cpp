@@ -821,13 +821,13 @@ bool GpuReplica::flush(void* user_stream, int timeout_ms) {
   check(cudaStreamSynchronize(S(user_stream)), "cudaStreamSynchronize");
   const uint64_t start = steady_ns(), limit = uint64_t(timeout_ms < 0 ? 0 : timeout_ms) * 1000000ull;
   const uint64_t quiet_ns = 100000ull + uint64_t(n_padded_) * 2 * 18 / 6000;   // 18 bytes an element and pass, 6000 bytes a ns
-  const uint64_t before = engine_launched_.load(), passes = 3ull * uint64_t(n_windows());
+  const uint64_t before = watch_.launches(), passes = 3ull * uint64_t(n_windows());
   uint64_t woken = 0;
   while (engine_on_.load()) {
-    const uint64_t busy = last_busy_launch_.load(), looked = engine_looked_.load(), now = steady_ns();
-    const uint64_t since = last_busy_ns_.load();
-    const uint64_t quiet = now - (since > start ? since : start);
-    if (looked >= (busy > before ? busy : before) + passes && quiet >= quiet_ns && (quiet >= quiet_ns + 100000000ull || unacknowledged() == 0)) return true;
+    const uint64_t now = steady_ns(), quiet = watch_.quiet_for(start, now);
+    if (quiet >= quiet_ns && watch_.quiet_launches(before, passes) && (quiet >= quiet_ns + 100000000ull || unacknowledged() == 0) &&
+        watch_.quiet_launches(before, passes))  // (still so)
+      return true;
     if (ring_peers_.load() == 0) return true;  // the last neighbour has gone
     if (now - start > limit) break;
     if (woken == 0 || now - woken > 2000000ull) {
@@ -852,7 +852,7 @@ void GpuReplica::engine_loop() {
   uint64_t* work_host = status_host_ + kDsTotalWords;  // behind the part status() uses
   uint64_t work_seen = 0;
   uint64_t r = 0;
-  engine_looked_.store(engine_launched_.load());  // (launches of an earlier run of this thread that were not looked back on)
+  watch_.begin();
   uint64_t idle_rounds = 0;
   uint64_t quiet_launches = 0;   // launches in a row that found nothing to do
   while (!engine_stop_.load()) {
@@ -865,7 +865,7 @@ void GpuReplica::engine_loop() {
         // thread, which only starts the next launch and reads how much the last one found to do.
         windows = n_windows();
         launch(true, true, auto_sweeps());
-        engine_launched_.fetch_add(1);
+        watch_.launched();
         cudaEventRecord(E(ev_kernel_[r % depth]), S(comm_));
         cudaStreamWaitEvent(S(stat_), E(ev_kernel_[r % depth]), 0);
         cudaMemcpyAsync(work_host + (r % depth), status_ + kDsTilesProcessed, 8, cudaMemcpyDeviceToHost, S(stat_));
@@ -887,15 +887,7 @@ void GpuReplica::engine_loop() {
       work = now > work_seen ? now - work_seen : 0;
       work_seen = now > work_seen ? now : work_seen;
     }
-    if (r >= depth) {
-      // what flush() watches: how many launches have been looked back on, and the last of them that found work
-      const uint64_t looked = engine_looked_.load() + 1;
-      if (work != 0) {
-        last_busy_ns_.store(steady_ns());
-        last_busy_launch_.store(looked);
-      }
-      engine_looked_.store(looked);
-    }
+    if (r >= depth) watch_.looked(work != 0, steady_ns());  // what flush() watches
     if (work != 0) epoch_++;
     quiet_launches = work == 0 ? quiet_launches + 1 : 0;
     if (work == 0 && quiet_launches < uint64_t(windows)) continue;  // the other windows of the tensor have not been looked at yet

@@ -23,6 +23,7 @@
 #include <thread>
 #include <vector>
 
+#include "../core/quiet.hpp"
 #include "round.h"
 #include "table.hpp"
 #include "vmm.hpp"
@@ -221,8 +222,7 @@ class GpuReplica {
   std::mutex engine_mu_;               // serialises start_engine / stop_engine
   std::thread engine_;
   std::atomic<bool> engine_on_{false}, engine_stop_{false};
-  std::atomic<uint64_t> engine_launched_{0}, engine_looked_{0};       // launches of the engine thread, and those looked back on
-  std::atomic<uint64_t> last_busy_launch_{0}, last_busy_ns_{0};       // the last of the latter that found work, and when that was seen
+  QuietWatch watch_;                   // launches of the engine thread
   std::atomic<uint64_t> last_wake_ns_{0};  // when wake() was last called (steady clock)
   std::atomic<bool> idle_{false};      // the engine has seen several rounds without work and pauses between rounds
   std::mutex wake_mu_;

@@ -1,0 +1,32 @@
+"""What flush() goes by: launches of the engine thread that found nothing to do, and for how long."""
+from sharedtensor_b200 import _native
+
+
+def _watch(*looked):
+    w = _native.cuda().QuietWatch()
+    w.begin()
+    for args in looked:
+        w.launched()
+        w.looked(*args)
+    return w
+
+
+def test_work_found_after_the_clock_was_read_is_not_a_long_quiet_time():
+    w = _watch((False, 1000), (True, 5000))
+    assert w.quiet_for(500, 4000) == 0, "the launch that found work was looked at after the caller took the time"
+    assert w.quiet_for(6000, 4000) == 0
+    assert w.quiet_for(500, 7000) == 2000
+    assert w.quiet_for(6500, 7000) == 500
+
+
+def test_quiet_launches_begin_after_the_caller_and_after_the_last_busy_one():
+    w = _watch((False, 1), (False, 2), (False, 3))
+    assert w.quiet_launches(0, 3) and not w.quiet_launches(1, 3)
+    w.launched()
+    w.looked(True, 4)
+    assert not w.quiet_launches(0, 1)
+    for t in (5, 6, 7):
+        assert not w.quiet_launches(0, 3)
+        w.launched()
+        w.looked(False, t)
+    assert w.quiet_launches(0, 3) and w.launches() == 7
