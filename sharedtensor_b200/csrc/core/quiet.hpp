@@ -1,4 +1,5 @@
-// What the engine thread tells a flush: how many launches it has looked back on, and the last of them that found work.
+// What the engine thread tells a flush: how many launches it has looked back on, and the last of them that found work or
+// did not get to look.
 #pragma once
 #include <algorithm>
 #include <atomic>
@@ -11,9 +12,11 @@ class QuietWatch {
   // ---- engine thread
   void begin() { looked_.store(launched_.load()); }  // launches of an earlier run that were not looked back on
   void launched() { launched_.fetch_add(1); }
-  void looked(bool busy, uint64_t now_ns) {
+  // `cut_short`: a group left before it had looked at its tiles (an update wanted the SMs, a wait ran out).  That says nothing
+  // about them, so the launch does not count as one that found nothing.
+  void looked(bool found_work, bool cut_short, uint64_t now_ns) {
     const uint64_t n = looked_.load() + 1;
-    if (busy) {
+    if (found_work || cut_short) {
       busy_ns_.store(now_ns);
       busy_launch_.store(n);
     }

@@ -17,6 +17,11 @@ cudaStream_t S(void* p) { return static_cast<cudaStream_t>(p); }
 cudaEvent_t E(void* p) { return static_cast<cudaEvent_t>(p); }
 size_t align_up(size_t v, size_t a) { return (v + a - 1) / a * a; }
 
+// Pinned words behind the copy of the status block: what the engine thread reads back per launch in flight (at most four),
+// and the results of two kernels.
+constexpr int kHostRead = kDsYields - kDsTilesProcessed + 1, kHostUnsend = 4 * kHostRead, kHostUnacknowledged = kHostUnsend + 1,
+              kHostExtraWords = kHostUnacknowledged + 1;
+
 struct DeviceGuard {
   int prev = -1;
   explicit DeviceGuard(int dev) {
@@ -80,12 +85,12 @@ GpuReplica::GpuReplica(int device, int64_t n, const GpuConfig& cfg) : device_(de
   // default stream, which nothing here is ordered against).
   check(cudaMalloc(reinterpret_cast<void**>(&tile_state_), size_t(n_tiles_) * 4), "cudaMalloc tile_state");
   check(cudaMalloc(reinterpret_cast<void**>(&status_), kDsTotalWords * 8), "cudaMalloc status");
-  check(cudaMallocHost(reinterpret_cast<void**>(&status_host_), (kDsTotalWords + 16) * 8), "cudaMallocHost status");
+  check(cudaMallocHost(reinterpret_cast<void**>(&status_host_), (kDsTotalWords + kHostExtraWords) * 8), "cudaMallocHost status");
   check(cudaMalloc(reinterpret_cast<void**>(&yield_flag_), 4 + 4 * kTickets), "cudaMalloc yield flag");
   check(cudaMemsetAsync(yield_flag_, 0, 4 + 4 * kTickets, s), "memset");
   check(launch_fill_state(tile_state_, n_tiles_, 1u, comm_), "fill_state");
   check(cudaMemsetAsync(status_, 0, kDsTotalWords * 8, s), "memset");
-  std::memset(status_host_, 0, (kDsTotalWords + 16) * 8);
+  std::memset(status_host_, 0, (kDsTotalWords + kHostExtraWords) * 8);
   cudaEvent_t e1, e2;
   check(cudaEventCreateWithFlags(&e1, cudaEventDisableTiming), "cudaEventCreate");
   check(cudaEventCreateWithFlags(&e2, cudaEventDisableTiming), "cudaEventCreate");
@@ -276,9 +281,9 @@ uint64_t GpuReplica::unsend_unacknowledged(int peer) {
         "unsend kernel");
   check(launch_fill_state(tile_state_, n_tiles_, 1u, comm_), "fill_state");  // the link has something to hear again
   uint64_t host = 0;
-  check(cudaMemcpyAsync(status_host_ + kDsTotalWords + 8, dev_count, 8, cudaMemcpyDeviceToHost, S(comm_)), "cudaMemcpyAsync");
+  check(cudaMemcpyAsync(status_host_ + kDsTotalWords + kHostUnsend, dev_count, 8, cudaMemcpyDeviceToHost, S(comm_)), "cudaMemcpyAsync");
   check(cudaStreamSynchronize(S(comm_)), "cudaStreamSynchronize");
-  host = status_host_[kDsTotalWords + 8];
+  host = status_host_[kDsTotalWords + kHostUnsend];
   cudaFree(dev_count);
   launches_ += 1;
   return host;
@@ -795,7 +800,7 @@ void GpuReplica::idle_pause(uint64_t us) {
 
 // Frames (per tile and ring) that no neighbour has acknowledged yet.
 uint32_t GpuReplica::unacknowledged() {
-  uint32_t* const count = reinterpret_cast<uint32_t*>(status_host_ + kDsTotalWords + 12);
+  uint32_t* const count = reinterpret_cast<uint32_t*>(status_host_ + kDsTotalWords + kHostUnacknowledged);
   if (!flush_) {
     cudaStream_t st;
     check(cudaStreamCreateWithFlags(&st, cudaStreamNonBlocking), "cudaStreamCreate");
@@ -811,7 +816,8 @@ uint32_t GpuReplica::unacknowledged() {
   return *reinterpret_cast<volatile uint32_t*>(count);
 }
 
-// Three passes of the engine thread in a row, begun after the caller's updates have run, that find nothing to do; for as
+// Three passes of the engine thread in a row, begun after the caller's updates have run, that get to look at all tiles and
+// find nothing to do; for as
 // long as a neighbour may need to take in what it was sent and pass it on (two busy passes at HBM rate) no pass that did;
 // and every frame acknowledged (a neighbour may be gone, or have no engine running: after a tenth of a second of quiet the
 // frames count as delivered, they are in its memory).
@@ -846,11 +852,12 @@ void GpuReplica::engine_loop() {
   cudaSetDevice(device_);
   ::prctl(PR_SET_TIMERSLACK, 1000UL, 0, 0, 0);  // 1 us instead of the default 50 us: the idle pauses start at 10 us
   const size_t depth = ev_round_.size();
-  // One pinned word per launch in flight: tiles handled so far, read once that launch has finished.  The read runs on
+  // A few pinned words per launch in flight: tiles handled, groups that left early, and waits that ran out so far, read once
+  // that launch has finished.  The read runs on
   // a stream of its own behind an event, so that the comm stream goes from one launch straight to the next; a later
   // launch may already have added to the count by then, which only moves work from one difference to the next.
   uint64_t* work_host = status_host_ + kDsTotalWords;  // behind the part status() uses
-  uint64_t work_seen = 0;
+  uint64_t work_seen = 0, cut_seen = 0;
   uint64_t r = 0;
   watch_.begin();
   uint64_t idle_rounds = 0;
@@ -868,7 +875,7 @@ void GpuReplica::engine_loop() {
         watch_.launched();
         cudaEventRecord(E(ev_kernel_[r % depth]), S(comm_));
         cudaStreamWaitEvent(S(stat_), E(ev_kernel_[r % depth]), 0);
-        cudaMemcpyAsync(work_host + (r % depth), status_ + kDsTilesProcessed, 8, cudaMemcpyDeviceToHost, S(stat_));
+        cudaMemcpyAsync(work_host + (r % depth) * kHostRead, status_ + kDsTilesProcessed, kHostRead * 8, cudaMemcpyDeviceToHost, S(stat_));
         cudaEventRecord(E(ev_round_[r % depth]), S(stat_));
         launched = true;
       }
@@ -883,11 +890,13 @@ void GpuReplica::engine_loop() {
     uint64_t work = 1;
     if (r >= depth) {
       cudaEventSynchronize(E(ev_round_[(r - depth) % depth]));
-      const uint64_t now = work_host[(r - depth) % depth];
+      const uint64_t* const words = work_host + ((r - depth) % depth) * kHostRead;
+      const uint64_t now = words[0], cut = words[kDsYields - kDsTilesProcessed] + words[kDsWaitTimeouts - kDsTilesProcessed];
       work = now > work_seen ? now - work_seen : 0;
       work_seen = now > work_seen ? now : work_seen;
+      watch_.looked(work != 0, cut != cut_seen, steady_ns());  // what flush() watches
+      cut_seen = cut;
     }
-    if (r >= depth) watch_.looked(work != 0, steady_ns());  // what flush() watches
     if (work != 0) epoch_++;
     quiet_launches = work == 0 ? quiet_launches + 1 : 0;
     if (work == 0 && quiet_launches < uint64_t(windows)) continue;  // the other windows of the tensor have not been looked at yet

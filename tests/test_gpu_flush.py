@@ -1,4 +1,6 @@
 """flush() on a pair of replicas in one process, engine threads running."""
+import threading
+
 import pytest
 import torch
 
@@ -24,5 +26,46 @@ def test_flush_waits_until_an_update_has_arrived(free_port, n):
             dst.copyToTensor(out)
             assert ((out - expect).norm() / expect.norm()).item() < 1e-5
     finally:
+        b.close()
+        a.close()
+
+
+def test_flush_while_another_thread_reads_all_the_time(free_port):
+    """Every read asks the round kernel for its SMs, so that its launches keep leaving before they have looked at their
+    tiles: flush() does not take that for silence."""
+    n = 20_000_000
+    init = torch.randn(n, device="cuda")
+    a = sharedtensor.createOrFetch("127.0.0.1", free_port, init, rejoin=False)
+    b = sharedtensor.createOrFetch("127.0.0.1", free_port, torch.zeros(n, device="cuda"), rejoin=False)
+    stop = threading.Event()
+
+    def read():
+        mine = torch.empty(n, device="cuda")
+        with torch.cuda.stream(torch.cuda.Stream()):
+            while not stop.is_set():
+                for _ in range(8):
+                    a.copyToTensor(mine)
+                torch.cuda.current_stream().synchronize()
+
+    reader = threading.Thread(target=read)
+    try:
+        assert a.flush(10.0) and b.flush(10.0)
+        reader.start()
+        expect, out = init.clone(), torch.empty_like(init)
+        for i in range(12):
+            d = torch.randn(n, device="cuda") * 1e-2
+            a.addFromTensor(d)
+            expect += d
+            if not a.flush(2.0):
+                continue
+            b.copyToTensor(out)
+            assert ((out - expect).norm() / expect.norm()).item() < 1e-5, i
+        stop.set()
+        reader.join()
+        assert a.flush(10.0) and b.flush(10.0)
+        b.copyToTensor(out)
+        assert ((out - expect).norm() / expect.norm()).item() < 1e-5
+    finally:
+        stop.set()
         b.close()
         a.close()

@@ -12,7 +12,7 @@ def _watch(*looked):
 
 
 def test_work_found_after_the_clock_was_read_is_not_a_long_quiet_time():
-    w = _watch((False, 1000), (True, 5000))
+    w = _watch((False, False, 1000), (True, False, 5000))
     assert w.quiet_for(500, 4000) == 0, "the launch that found work was looked at after the caller took the time"
     assert w.quiet_for(6000, 4000) == 0
     assert w.quiet_for(500, 7000) == 2000
@@ -20,13 +20,22 @@ def test_work_found_after_the_clock_was_read_is_not_a_long_quiet_time():
 
 
 def test_quiet_launches_begin_after_the_caller_and_after_the_last_busy_one():
-    w = _watch((False, 1), (False, 2), (False, 3))
+    w = _watch(*((False, False, t) for t in (1, 2, 3)))
     assert w.quiet_launches(0, 3) and not w.quiet_launches(1, 3)
     w.launched()
-    w.looked(True, 4)
+    w.looked(True, False, 4)
     assert not w.quiet_launches(0, 1)
     for t in (5, 6, 7):
         assert not w.quiet_launches(0, 3)
         w.launched()
-        w.looked(False, t)
+        w.looked(False, False, t)
     assert w.quiet_launches(0, 3) and w.launches() == 7
+
+
+def test_a_launch_that_did_not_get_to_look_does_not_count():
+    """An update that wants the SMs makes groups leave before they have looked at their tiles; a wait that runs out too."""
+    w = _watch(*((False, True, t) for t in (1, 2, 3)))
+    assert not w.quiet_launches(0, 1) and w.quiet_for(0, 10) == 7
+    w.launched()
+    w.looked(False, False, 4)
+    assert w.quiet_launches(0, 1) and not w.quiet_launches(0, 2)
