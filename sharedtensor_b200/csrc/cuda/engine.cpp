@@ -233,7 +233,7 @@ void GpuReplica::free_edge_block(int id) {
   DeviceGuard g(device_);
   std::lock_guard<std::mutex> lk(mu_);
   if (id < 0 || id >= kMaxRings || !blocks_[id].used) return;
-  cudaStreamSynchronize(S(comm_));
+  publish_pending();
   vmm_free(&blocks_[id].mem);
   blocks_[id].used = false;
 }
@@ -319,6 +319,7 @@ void GpuReplica::publish_pending() {
   // Ring numbering is about to change.  Every round ends with its publish kernel, so once the
   // stream has drained nothing refers to the old numbering any more.
   cudaStreamSynchronize(S(comm_));
+  if (flush_) cudaStreamSynchronize(S(flush_));  // (a flush counts frames over the old edges)
 }
 
 void GpuReplica::rebuild_params() {
@@ -801,17 +802,22 @@ void GpuReplica::idle_pause(uint64_t us) {
 // Frames (per tile and ring) that no neighbour has acknowledged yet.
 uint32_t GpuReplica::unacknowledged() {
   uint32_t* const count = reinterpret_cast<uint32_t*>(status_host_ + kDsTotalWords + kHostUnacknowledged);
-  if (!flush_) {
-    cudaStream_t st;
-    check(cudaStreamCreateWithFlags(&st, cudaStreamNonBlocking), "cudaStreamCreate");
-    flush_ = st;
-  }
   {
+    // The engine thread needs the mutex for the pass that takes the acknowledgements in: it is held for the launch only.
+    // (An edge is not taken down while the kernel looks at it, see publish_pending.)
     std::lock_guard<std::mutex> lk(mu_);
+    if (!flush_) {
+      cudaStream_t st;
+      check(cudaStreamCreateWithFlags(&st, cudaStreamNonBlocking), "cudaStreamCreate");
+      flush_ = st;
+    }
     *count = 0;
     check(launch_count_unacknowledged(params_, count, flush_), "count_unacknowledged kernel");
-    // the edges cannot be taken down while the kernel looks at them
-    check(cudaStreamSynchronize(S(flush_)), "cudaStreamSynchronize");
+  }
+  const cudaError_t e = cudaStreamSynchronize(S(flush_));
+  if (e != cudaSuccess) {
+    std::lock_guard<std::mutex> lk(mu_);
+    check(e, "cudaStreamSynchronize");
   }
   return *reinterpret_cast<volatile uint32_t*>(count);
 }
@@ -828,12 +834,19 @@ bool GpuReplica::flush(void* user_stream, int timeout_ms) {
   const uint64_t start = steady_ns(), limit = uint64_t(timeout_ms < 0 ? 0 : timeout_ms) * 1000000ull;
   const uint64_t quiet_ns = 100000ull + uint64_t(n_padded_) * 2 * 18 / 6000;   // 18 bytes an element and pass, 6000 bytes a ns
   const uint64_t before = watch_.launches(), passes = 3ull * uint64_t(n_windows());
-  uint64_t woken = 0;
+  uint64_t woken = 0, asked_at = 0, pause_ns = 20000;
   while (engine_on_.load()) {
     const uint64_t now = steady_ns(), quiet = watch_.quiet_for(start, now);
-    if (quiet >= quiet_ns && watch_.quiet_launches(before, passes) && (quiet >= quiet_ns + 100000000ull || unacknowledged() == 0) &&
-        watch_.quiet_launches(before, passes))  // (still so)
-      return true;
+    if (quiet >= quiet_ns && watch_.quiet_launches(before, passes)) {
+      bool arrived = quiet >= quiet_ns + 100000000ull;
+      if (!arrived && now - asked_at >= pause_ns) {
+        // (asked less and less often: a neighbour that takes its time is not to be slowed down by the question)
+        arrived = unacknowledged() == 0;
+        asked_at = steady_ns();
+        pause_ns = pause_ns < 640000 ? pause_ns * 2 : pause_ns;
+      }
+      if (arrived && watch_.quiet_launches(before, passes)) return true;  // (still so)
+    }
     if (ring_peers_.load() == 0) return true;  // the last neighbour has gone
     if (now - start > limit) break;
     if (woken == 0 || now - woken > 2000000ull) {
