@@ -183,7 +183,7 @@ PYBIND11_MODULE(_cuda, m) {
       .def("stop_engine", [](GpuReplica& r) { py::gil_scoped_release rel; r.stop_engine(); })
       .def("engine_running", &GpuReplica::engine_running)
       .def("ring_peers", &GpuReplica::ring_peers)
-      .def("flush", [](GpuReplica& r, uintptr_t s, int timeout_ms) { py::gil_scoped_release rel; return r.flush(strm(s), timeout_ms); })
+      .def("flush", [](GpuReplica& r, uintptr_t s, int64_t timeout_ms) { py::gil_scoped_release rel; return r.flush(strm(s), timeout_ms); })
       .def("status", [](GpuReplica& r) { py::gil_scoped_release rel; return r.status(); })
       .def("launches", &GpuReplica::launches)
       .def("last_error", &GpuReplica::last_error);

@@ -19,6 +19,7 @@ size_t align_up(size_t v, size_t a) { return (v + a - 1) / a * a; }
 
 // Pinned words behind the copy of the status block: what the engine thread reads back per launch in flight (at most four),
 // and the results of two kernels.
+constexpr int64_t kLongestWaitMs = 1000ll * 3600 * 24 * 365;  // (a year, in nanoseconds, is far from the end of 64 bits)
 constexpr int kHostRead = kDsYields - kDsTilesProcessed + 1, kHostUnsend = 4 * kHostRead, kHostUnacknowledged = kHostUnsend + 1,
               kHostExtraWords = kHostUnacknowledged + 1;
 
@@ -827,11 +828,21 @@ uint32_t GpuReplica::unacknowledged() {
 // long as a neighbour may need to take in what it was sent and pass it on (two busy passes at HBM rate) no pass that did;
 // and every frame acknowledged (a neighbour may be gone, or have no engine running: after a tenth of a second of quiet the
 // frames count as delivered, they are in its memory).
-bool GpuReplica::flush(void* user_stream, int timeout_ms) {
+bool GpuReplica::flush(void* user_stream, int64_t timeout_ms) {
   DeviceGuard g(device_);
-  std::lock_guard<std::mutex> one(flush_mu_);
-  check(cudaStreamSynchronize(S(user_stream)), "cudaStreamSynchronize");
-  const uint64_t start = steady_ns(), limit = uint64_t(timeout_ms < 0 ? 0 : timeout_ms) * 1000000ull;
+  // The limit covers the wait for another thread's flush and for the caller's stream too.
+  const uint64_t entered = steady_ns(), limit = uint64_t(timeout_ms < 0 ? 0 : (timeout_ms > kLongestWaitMs ? kLongestWaitMs : timeout_ms)) * 1000000ull;
+  std::unique_lock<std::timed_mutex> one(flush_mu_, std::defer_lock);
+  if (!one.try_lock_for(std::chrono::nanoseconds(limit))) return false;
+  for (cudaError_t e; (e = cudaStreamQuery(S(user_stream))) != cudaSuccess;) {
+    if (e != cudaErrorNotReady) check(e, "cudaStreamQuery");
+    cudaGetLastError();
+    const uint64_t waited = steady_ns() - entered;
+    if (waited > limit) return false;
+    if (waited < 2000000ull) std::this_thread::yield();
+    else ::usleep(50);
+  }
+  const uint64_t start = steady_ns();
   const uint64_t quiet_ns = 100000ull + uint64_t(n_padded_) * 2 * 18 / 6000;   // 18 bytes an element and pass, 6000 bytes a ns
   const uint64_t before = watch_.launches(), passes = 3ull * uint64_t(n_windows());
   uint64_t woken = 0, asked_at = 0, pause_ns = 20000;
@@ -848,7 +859,7 @@ bool GpuReplica::flush(void* user_stream, int timeout_ms) {
       if (arrived && watch_.quiet_launches(before, passes)) return true;  // (still so)
     }
     if (ring_peers_.load() == 0) return true;  // the last neighbour has gone
-    if (now - start > limit) break;
+    if (now - entered > limit) break;
     if (woken == 0 || now - woken > 2000000ull) {
       const std::string err = last_error();
       if (!err.empty()) throw std::runtime_error("sharedtensor GPU engine: " + err);

@@ -129,7 +129,7 @@ class GpuReplica {
   bool engine_running() const { return engine_on_.load(); }
   // With the engine running: waits until the work queued on `user_stream` is done and the rounds have gone quiet; false
   // when they have not within the time given.
-  bool flush(void* user_stream, int timeout_ms);
+  bool flush(void* user_stream, int64_t timeout_ms);
   int ring_peers() const { return ring_peers_.load(); }
   // Ends the engine thread's idle pause at once.  `from_neighbour` marks a doorbell that came over a socket; the
   // return value says whether the engine had been idle (the caller then passes the doorbell on).
@@ -216,7 +216,7 @@ class GpuReplica {
   std::vector<void*> ev_kernel_;      // per launch in flight: the kernel has finished (comm stream)
   void* stat_ = nullptr;               // cudaStream_t: reads work counts back beside the comm stream, so that launches follow each other without a copy in between
   void* flush_ = nullptr;              // cudaStream_t: flush() counts unacknowledged frames beside the rounds (made on first use)
-  std::mutex flush_mu_;                // one flush at a time; taken before mu_
+  std::timed_mutex flush_mu_;          // one flush at a time; taken before mu_
   mutable std::mutex mu_;
   std::mutex gate_mu_;                 // taken before mu_ by every update from outside the rounds
   std::mutex engine_mu_;               // serialises start_engine / stop_engine

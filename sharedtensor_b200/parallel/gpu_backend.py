@@ -43,6 +43,11 @@ def _stream(device: torch.device) -> int:
     return _raw_stream(device.index) if _raw_stream is not None else torch.cuda.current_stream(device).cuda_stream
 
 
+def _milliseconds(seconds: float) -> int:
+    """For the native waits: anything that can be compared with a time, infinity among it."""
+    return int(min(seconds, 1e9) * 1000) if seconds > 0 else 0
+
+
 class GpuBackend:
     def __init__(self, n: int, cfg: Config, device: torch.device):
         if not torch.cuda.is_available():
@@ -91,7 +96,7 @@ class GpuBackend:
         import time
 
         t0 = time.time()
-        if self.rep.engine_running() and self.rep.ring_peers() > 0 and self.rep.flush(_stream(self.device), int(timeout_s * 1000)):
+        if self.rep.engine_running() and self.rep.ring_peers() > 0 and self.rep.flush(_stream(self.device), _milliseconds(timeout_s)):
             return True
         names = _native.cuda().status_names()
         i_work, i_pend = names.index("last_work_count"), names.index("pending_tiles")

@@ -1,10 +1,12 @@
 """flush() on a pair of replicas in one process, engine threads running."""
 import threading
+import time
 
 import pytest
 import torch
 
 import sharedtensor
+from sharedtensor_b200 import _native
 
 pytestmark = pytest.mark.gpu
 
@@ -67,5 +69,30 @@ def test_flush_while_another_thread_reads_all_the_time(free_port):
         assert ((out - expect).norm() / expect.norm()).item() < 1e-5
     finally:
         stop.set()
+        b.close()
+        a.close()
+
+
+def test_flush_keeps_to_its_timeout(free_port):
+    """Any limit can be given, infinity among them, and it covers what the caller has queued and another thread's flush."""
+    n = 1000
+    a = sharedtensor.createOrFetch("127.0.0.1", free_port, torch.zeros(n, device="cuda"), rejoin=False)
+    b = sharedtensor.createOrFetch("127.0.0.1", free_port, torch.zeros(n, device="cuda"), rejoin=False)
+    try:
+        a.addFromTensor(torch.ones(n, device="cuda"))
+        assert a.flush(float("inf")) and a.flush(1e12)
+        assert not a.flush(0.0) and not a.flush(-1.0) and not a.flush(float("nan"))
+        busy = torch.cuda.Stream()
+        with torch.cuda.stream(busy):
+            _native.cuda().delay(1_000_000_000, busy.cuda_stream)   # a second of queued work
+            t0 = time.time()
+            other = threading.Thread(target=lambda: torch.cuda.set_stream(busy) or a.flush(5.0))
+            other.start()
+            time.sleep(0.05)
+            assert not a.flush(0.1)
+            assert time.time() - t0 < 0.5
+            assert a.flush(5.0)
+            other.join()
+    finally:
         b.close()
         a.close()

@@ -39,3 +39,11 @@ def test_a_launch_that_did_not_get_to_look_does_not_count():
     w.launched()
     w.looked(False, False, 4)
     assert w.quiet_launches(0, 1) and not w.quiet_launches(0, 2)
+
+
+def test_any_timeout_can_be_given():
+    from sharedtensor_b200.parallel.gpu_backend import _milliseconds
+
+    assert _milliseconds(0.25) == 250 and _milliseconds(30) == 30000
+    assert _milliseconds(0.0) == _milliseconds(-1.0) == _milliseconds(float("nan")) == 0
+    assert 0 < _milliseconds(float("inf")) == _milliseconds(1e300) < 2 ** 63
