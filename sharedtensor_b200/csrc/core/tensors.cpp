@@ -7,6 +7,7 @@
 
 #include <algorithm>
 #include <cstdint>
+#include <utility>
 #include <vector>
 
 namespace {
@@ -38,9 +39,14 @@ class TensorList {
       out[k] = reinterpret_cast<uintptr_t>(written ? t.mutable_data_ptr() : const_cast<void*>(t.const_data_ptr()));
     }
     if (written) {
-      std::vector<uintptr_t> sorted(out);
-      std::sort(sorted.begin(), sorted.end());
-      if (std::adjacent_find(sorted.begin(), sorted.end()) != sorted.end()) return py::none();  // names that share a tensor: one after the other
+      // names that share memory, wholly or in part, are written one after the other
+      std::vector<std::pair<uintptr_t, uintptr_t>> spans;
+      spans.reserve(n);
+      for (size_t k = 0; k < n; k++)
+        if (const size_t bytes = THPVariable_Unpack(held[k].ptr()).nbytes()) spans.emplace_back(out[k], out[k] + bytes);
+      std::sort(spans.begin(), spans.end());
+      for (size_t k = 1; k < spans.size(); k++)
+        if (spans[k].first < spans[k - 1].second) return py::none();
       for (size_t k = 0; k < n; k++) THPVariable_Unpack(held[k].ptr()).unsafeGetTensorImpl()->bump_version();
     }
     return py::bytes(reinterpret_cast<const char*>(out.data()), n * sizeof(uintptr_t));

@@ -55,3 +55,26 @@ def test_table_tensors_that_need_a_conversion(free_port):
             tab.addFromTensors({"a": torch.ones(3, device="cuda"), "b": torch.ones(7, device="cuda")})
     finally:
         tab.close()
+
+
+def test_names_that_share_memory_are_filled_one_after_the_other(free_port):
+    """The later name wins where two overlap, as it does when they are copied in turn."""
+    n = 300_000
+    init = {"a": torch.randn(n, device="cuda"), "b": torch.randn(n, device="cuda"), "none": torch.empty(0, device="cuda")}
+    tab = sharedtensor.createOrFetchTable("127.0.0.1", free_port, init)
+    try:
+        for shift in (0, 1, n // 2, n - 1, n):
+            store = torch.zeros(2 * n, device="cuda")
+            want = store.clone()
+            want[:n] = init["a"]
+            want[shift:shift + n] = init["b"]
+            for _ in range(5):
+                store.zero_()
+                tab.copyToTensors({"a": store[:n], "b": store[shift:shift + n], "none": torch.empty(0, device="cuda")})
+                assert torch.equal(store, want), shift
+            # (what is read may overlap as it likes)
+            tab.addFromTensors({"a": store[:n], "b": store[shift:shift + n], "none": torch.empty(0, device="cuda")})
+            init["a"] += store[:n]
+            init["b"] += store[shift:shift + n]
+    finally:
+        tab.close()
