@@ -22,7 +22,7 @@ class TensorList {
   }
 
   // The tensors' addresses as packed 64-bit words, or None if one of them needs a conversion, a broadcast or autograd on the
-  // way.  `written`: the caller is about to overwrite them (their version counters move).
+  // way, or has no memory.  `written`: the caller is about to overwrite them (their version counters move).
   py::object addresses(const py::object& tensors, bool written) const {
     const size_t n = shapes_.size();
     std::vector<uintptr_t> out(n);
@@ -33,9 +33,11 @@ class TensorList {
       PyObject* const o = held[k].ptr();
       if (!THPVariable_Check(o)) return py::none();
       const at::Tensor& t = THPVariable_Unpack(o);
-      if (!t.defined() || t.scalar_type() != at::kFloat || t.layout() != at::kStrided || !t.is_cuda() || t.get_device() != device_ || t.is_neg() ||
+      if (!t.defined() || !t.has_storage() || t.scalar_type() != at::kFloat || t.layout() != at::kStrided || !t.is_cuda() || t.get_device() != device_ || t.is_neg() ||
           t.key_set().has(c10::DispatchKey::Python) || !(t.sizes() == at::IntArrayRef(shapes_[k])) || !t.is_contiguous() || (tracked && t.requires_grad()))
         return py::none();
+      // zeros without memory (forward-mode differentiation makes them), and tensors whose storage has been given up
+      if (t._is_zerotensor() || t.storage().nbytes() < (size_t(t.storage_offset()) + size_t(t.numel())) * sizeof(float)) return py::none();
       out[k] = reinterpret_cast<uintptr_t>(written ? t.mutable_data_ptr() : const_cast<void*>(t.const_data_ptr()));
     }
     if (written) {

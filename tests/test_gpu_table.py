@@ -78,3 +78,20 @@ def test_names_that_share_memory_are_filled_one_after_the_other(free_port):
             init["b"] += store[shift:shift + n]
     finally:
         tab.close()
+
+
+def test_tensors_without_memory(free_port):
+    """Zeros that are not stored anywhere are added like any others; nothing is read from where a storage used to be."""
+    init = {"a": torch.randn(40, 30, device="cuda"), "b": torch.randn(7, device="cuda")}
+    tab = sharedtensor.createOrFetchTable("127.0.0.1", free_port, init)
+    try:
+        tab.addFromTensors({"a": torch._efficientzerotensor((40, 30), device="cuda"), "b": torch.ones(7, device="cuda")})
+        out = {k: torch.empty_like(v) for k, v in init.items()}
+        tab.copyToTensors(out)
+        assert torch.equal(out["a"], init["a"]) and torch.equal(out["b"], init["b"] + 1)
+        gone = torch.ones(40, 30, device="cuda")
+        gone.untyped_storage().resize_(0)
+        assert tab._addresses({"a": gone, "b": out["b"]}, False) is None
+        assert tab._addresses(out, False) is not None
+    finally:
+        tab.close()
