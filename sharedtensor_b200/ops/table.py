@@ -53,13 +53,16 @@ class SharedTable:
         self.layout = layout
         self._scratch: torch.Tensor | None = None
         self._plan = None            # GPU replicas: the native layout of the table
+        # The kernels need tensors that start on whole vectors of an arena of exactly this size.  Any other layout (of a caller's
+        # own) takes the way over a flat tensor, whose size is looked at there.
+        self._native_layout = layout.numel == shared.numel and all(off % 4 == 0 for off in layout.segment_offsets())
         self._native_plan()
 
     # ---- GPU replicas: all tensors in one kernel
     def _native_plan(self):
         """(replica, plan) of a GPU replica, else None."""
         rep = getattr(self.shared._b, "rep", None)
-        if rep is None or not self.layout.names:
+        if rep is None or not self.layout.names or not self._native_layout:
             return None
         if self._plan is None:
             from .. import _native

@@ -95,3 +95,30 @@ def test_tensors_without_memory(free_port):
         assert tab._addresses(out, False) is not None
     finally:
         tab.close()
+
+
+def test_layouts_of_a_callers_own(free_port):
+    """Tensors without padding between them, and a layout that is not the shared tensor's size."""
+    from sharedtensor_b200.ops.table import SharedTable, TableLayout
+
+    shapes = {"a": torch.Size([5]), "b": torch.Size([4097]), "c": torch.Size([2, 3])}
+    lay = TableLayout(shapes, 1)
+    init = torch.randn(lay.numel, device="cuda")
+    st = sharedtensor.createOrFetch("127.0.0.1", free_port, init)
+    try:
+        tab = SharedTable(st, lay)
+        deltas = {k: torch.randn(v, device="cuda") for k, v in shapes.items()}
+        tab.addFromTensors(deltas)
+        out = {k: torch.empty(v, device="cuda") for k, v in shapes.items()}
+        tab.copyToTensors(out)
+        for k, v in lay.views(init).items():
+            assert torch.equal(out[k], v + deltas[k])
+        got = tab.scales()
+        for k, v in out.items():
+            assert got[k]["sumsq"] == pytest.approx(float(v.double().square().sum()), rel=1e-12)
+        other = SharedTable(st, TableLayout({"a": torch.Size([lay.numel + 1])}, 32))
+        for call in (other.addFromTensors, other.copyToTensors):
+            with pytest.raises(ValueError):
+                call({"a": torch.zeros(lay.numel + 1, device="cuda")})
+    finally:
+        st.close()
