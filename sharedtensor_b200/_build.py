@@ -113,11 +113,18 @@ def build_cuda(force: bool = False, verbose: bool = False, ptxas_v: bool = False
     return target
 
 
+def _torch_version() -> str:
+    from importlib import metadata
+
+    return metadata.version("torch")
+
+
 def build_tensors(force: bool = False, verbose: bool = False) -> Path:
     import importlib.util
 
-    target, src = target_path("_tensors"), CSRC / "core/tensors.cpp"
-    if not force and not _stale(target, [src]):
+    # The module only fits the torch it was built against: which one that is lies beside its object file.
+    target, src, built_for = target_path("_tensors"), CSRC / "core/tensors.cpp", OBJ / "tensors.torch"
+    if not force and not _stale(target, [src]) and built_for.exists() and built_for.read_text() == _torch_version():
         return target
     OBJ.mkdir(exist_ok=True)
     torch_dir = Path(importlib.util.find_spec("torch").submodule_search_locations[0])
@@ -125,6 +132,7 @@ def build_tensors(force: bool = False, verbose: bool = False) -> Path:
     _run([CXX, "-std=c++17", "-O2", "-fPIC", "-fvisibility=hidden", f"-isystem{inc}", f"-isystem{inc / 'torch/csrc/api/include'}",
           "-isystem/usr/local/cuda/include", f"-I{sysconfig.get_paths()['include']}", "-c", str(src), "-o", str(obj)], verbose)
     _run([CXX, "-shared", "-o", str(target), str(obj), f"-L{lib}", "-ltorch_python", "-ltorch_cpu", "-lc10"], verbose)
+    built_for.write_text(_torch_version())
     return target
 
 

@@ -7,12 +7,16 @@ segmented reduction kernel reports per-tensor energies and RMS exponents.
 """
 from __future__ import annotations
 
+import logging
 from typing import Mapping
 
 import torch
 
 from ..api import SharedTensor, _Range, createOrFetch
 from ..parallel.gpu_backend import _stream
+
+
+log = logging.getLogger("sharedtensor")
 
 
 class TableLayout:
@@ -75,7 +79,11 @@ class SharedTable:
                       torch.empty(plan.pinned_bytes(), dtype=torch.uint8, pin_memory=True), _stream(dev))
             self._plan = plan
             # the look over a dict of tensors: their addresses, or None if one of them needs a conversion on the way
-            self._addresses = _native.tensors().TensorList(self.layout.names, shapes, self.shared.device.index).addresses
+            try:
+                self._addresses = _native.tensors().TensorList(self.layout.names, shapes, self.shared.device.index).addresses
+            except (ImportError, RuntimeError, OSError) as e:  # it is tied to the installed torch, and has to be built for it
+                log.warning("tables of tensors go through a flat tensor, which is slower: the _tensors module cannot be loaded (%s)", e)
+                self._addresses = lambda tensors, written: None
         return rep, self._plan
 
     # ---- dict-of-tensors interface
@@ -188,4 +196,8 @@ def createOrFetchTable(host: str, port: int, tensors: Mapping[str, torch.Tensor]
     layout = TableLayout({k: v.shape for k, v in tensors.items()}, align)
     flat = layout.pack(tensors)
     shared = createOrFetch(host, port, flat, **options)
-    return SharedTable(shared, layout)
+    try:
+        return SharedTable(shared, layout)
+    except BaseException:
+        shared.close()
+        raise
