@@ -122,3 +122,32 @@ def test_layouts_of_a_callers_own(free_port):
                 call({"a": torch.zeros(lay.numel + 1, device="cuda")})
     finally:
         st.close()
+
+
+def test_every_push_reaches_the_other_replica(free_port):
+    """The push sets the change marks of the arena tiles it touches itself: more tensors than one launch takes, tensors that
+    straddle tiles, the last of them within one chunk; all of them changed, then one at a time."""
+    sizes = [7] * 280 + [5000, 3 * 4096 + 5, 1, 9000, 3000]
+    init = _table(sizes)
+    a = sharedtensor.createOrFetchTable("127.0.0.1", free_port, init, rejoin=False)
+    b = sharedtensor.createOrFetchTable("127.0.0.1", free_port, {k: torch.zeros_like(v) for k, v in init.items()}, rejoin=False)
+    try:
+        names = list(init)
+        expect = {k: v.clone() for k, v in init.items()}
+        out = {k: torch.empty_like(v) for k, v in init.items()}
+        deltas = {k: torch.zeros_like(v) for k, v in init.items()}
+        assert a.flush(10.0) and b.flush(10.0)   # the marks of a new edge are gone
+        for changed in (names, [names[0]], [names[255]], [names[256]], *([k] for k in names[-5:])):
+            for k in names:
+                deltas[k].zero_()
+            for k in changed:
+                deltas[k].copy_(torch.randn_like(deltas[k]))
+                expect[k] += deltas[k]
+            a.addFromTensors(deltas)
+            assert a.flush(10.0) and b.flush(10.0)
+            b.copyToTensors(out)
+            for k in changed:
+                assert ((out[k] - expect[k]).norm() / expect[k].norm()).item() < 1e-5, (k, len(changed))
+    finally:
+        b.close()
+        a.close()
