@@ -2,7 +2,7 @@
 """Runs every hot kernel a few times on a small case (arrays larger than L2) so that a profiler can capture them,
 and prints CUDA-event timings of the same launches.
 
-    python benchmarks/profile_kernels.py [--elements 33554432] [--links 1 | --mesh 8] [--bits 8] [--shape 0]
+    python benchmarks/profile_kernels.py [--elements 33554432] [--links 1 | --mesh 8] [--bits 8]
     ncu --set full --clock-control none -k regex:round_kernel -s 2 -c 1 -o out python benchmarks/profile_kernels.py
 
 Kernels, in launch order after the warm-up iterations: add (addFromTensor), sub_add (pushUpdate), snapshot fp32,
@@ -33,7 +33,6 @@ def main():
     ap.add_argument("--mesh", type=int, default=0, help="members of a fully connected group instead of a star")
     ap.add_argument("--bits", type=int, default=8)
     ap.add_argument("--block", type=int, default=32)
-    ap.add_argument("--shape", type=int, default=-1, help="CTA make-up of the round kernel (default: the library's)")
     ap.add_argument("--chunk", type=int, default=0)
     ap.add_argument("--ctas", type=int, default=0, help="CTAs of the round kernel (0: one per SM)")
     ap.add_argument("--iters", type=int, default=3)
@@ -50,8 +49,6 @@ def main():
     cfg.bits = args.bits
     cfg.block = args.block
     cfg.ring_slots = 2
-    if args.shape >= 0:
-        cfg.shape = args.shape
     cfg.chunk_tiles = args.chunk
     cfg.comm_ctas = args.ctas
     hub = cu.GpuReplica(0, n, cfg)
@@ -126,7 +123,7 @@ def main():
     hbm = json.loads(peaks_file.read_text())["hbm_gbs"] if peaks_file.exists() else 6650.0
     rep = {k: {"ms": round(v, 4), "algorithmic_GBs": round(alg[k] / v / 1e6, 1), "frac_of_measured_hbm": round(alg[k] / v / 1e6 / hbm, 3)}
            for k, v in med.items()}
-    print(json.dumps({"elements": n, "links": n_links, "rings": n_rings, "mesh": args.mesh, "bits": args.bits, "shape": cfg.shape,
+    print(json.dumps({"elements": n, "links": n_links, "rings": n_rings, "mesh": args.mesh, "bits": args.bits,
                       "kernels": rep, "hub_status": dict(zip(cu.status_names(), hub.status()[:12]))}))
 
 

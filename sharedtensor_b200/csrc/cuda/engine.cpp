@@ -260,7 +260,7 @@ int GpuReplica::attach_peer(int link, int local_block, void* remote_base) {
       // whatever the link still had to say must be looked at again
       launch_fill_state(tile_state_, n_tiles_, 1u, comm_);
       rebuild_params();
-      check(load_round(params_, cfg_.shape), "round kernel");  // the neighbour's first frames are not to wait for that
+      check(load_round(params_), "round kernel");  // the neighbour's first frames are not to wait for that
       return i;
     }
   }
@@ -558,7 +558,7 @@ int GpuReplica::n_windows() const {
 
 // How a launch covers its window: the grid, and how many consecutive tiles a group owns (0: every n-th tile).
 void GpuReplica::grid_for_launch(int tiles, int* grid, int* chunk, int* tiles_per_group) const {
-  const int groups_per_cta = round_groups(cfg_.shape, params_.n_links, params_.n_in);
+  const int groups_per_cta = kRoundGroups;
   if (cfg_.chunk_tiles > 0) {
     // many short-lived CTAs: a group takes a run of `chunk_tiles` consecutive tiles and leaves
     const int t = cfg_.chunk_tiles;
@@ -601,7 +601,7 @@ void GpuReplica::launch(bool do_rx, bool do_tx, int sweeps) {
   int grid, chunk, per_group;
   grid_for_launch(params_.tile_count, &grid, &chunk, &per_group);
   params_.chunk = chunk;
-  check(launch_round(params_, cfg_.shape, grid, comm_), "round kernel");
+  check(launch_round(params_, grid, comm_), "round kernel");
   last_parity_ = params_.parity;
   next_window_ = (w + 1) % nw;
   if (next_window_ == 0) cycle_no_++;

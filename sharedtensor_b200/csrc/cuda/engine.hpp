@@ -43,7 +43,7 @@ struct GpuConfig {
   int bits = 8;              // bits per element of a frame: 1 (sign frames), 2, 4 or 8 (integer frames)
   int sweeps = 0;            // passes over the tensor per launch of the engine thread (0 = one)
   int poll_deadline_us = 1000;  // upper bound of every wait inside the round kernel
-  int shape = 1;             // make-up of the round kernel's CTAs, see launch_round
+  int shape = 1;             // 0 or 1: without effect (was the number of groups of a CTA)
   bool yield_to_updates = true;  // a running round kernel gives up its SMs when addFromTensor has an update ready
   bool comm_high_priority = false;  // comm stream at the highest stream priority (switches yield_to_updates off)
   int chunk_tiles = 0;       // > 0: short-lived CTAs, a group takes this many consecutive tiles (0: one CTA per SM per launch)

@@ -1134,13 +1134,13 @@ __device__ __forceinline__ void service_warp(const RoundParams& p, GroupShared& 
 
 }  // namespace
 
-template <int Q, int kGroups, int kKind>
-__global__ void __launch_bounds__(kGroups * kGroupThreads, 1) round_kernel(const __grid_constant__ RoundParams p) {
-  __shared__ GroupShared shared[kGroups];
+template <int Q, int kKind>
+__global__ void __launch_bounds__(kRoundGroups * kGroupThreads, 1) round_kernel(const __grid_constant__ RoundParams p) {
+  __shared__ GroupShared shared[kRoundGroups];
   extern __shared__ __align__(128) uint8_t dynamic[];  // [group][two stages of frames], and for an inner node [group][link][element of the tile]
   constexpr int kIn = kStaged<kKind>, kStageBytes = 2 * kIn * kFrameRoom<Q>;
   const int g = int(threadIdx.x) / kGroupThreads, warp = (int(threadIdx.x) % kGroupThreads) >> 5, lane = threadIdx.x & 31;
-  if (threadIdx.x < kGroups) {
+  if (threadIdx.x < kRoundGroups) {
     GroupShared& sh = shared[threadIdx.x];
     sh.armed = 0;
     sh.claim = 0;
@@ -1156,8 +1156,8 @@ __global__ void __launch_bounds__(kGroups * kGroupThreads, 1) round_kernel(const
   if (!p.follows_window) asm volatile("griddepcontrol.wait;" ::: "memory");
   __syncthreads();  // the only CTA-wide barrier: from here on the groups, and the two kinds of warp, run on their own
   uint8_t* const stages = dynamic + g * kStageBytes;
-  float* const stash = reinterpret_cast<float*>(dynamic + kGroups * kStageBytes) + (kKind == kInner ? g * kMaxLinks * kTile : 0);
-  if (warp == kComputeWarps) service_warp(p, shared[g], stages, kIn, kFrameRoom<Q>, g, kGroups, lane);
+  float* const stash = reinterpret_cast<float*>(dynamic + kRoundGroups * kStageBytes) + (kKind == kInner ? g * kMaxLinks * kTile : 0);
+  if (warp == kComputeWarps) service_warp(p, shared[g], stages, kIn, kFrameRoom<Q>, g, kRoundGroups, lane);
   else compute_warp<Q, kKind>(p, shared[g], stash, stages, warp, lane);
 }
 
@@ -1229,28 +1229,28 @@ int launch_count_unacknowledged(const RoundParams& p, uint32_t* count, void* str
 // ----------------------------------------------------------------------------------------------
 // launcher
 // ----------------------------------------------------------------------------------------------
-template <int Q, int kGroups, int kKind>
-constexpr int kDynamicBytes = kGroups * (2 * kStaged<kKind> * kFrameRoom<Q> + (kKind == kInner ? kMaxLinks * kTile * 4 : 0));
+template <int Q, int kKind>
+constexpr int kDynamicBytes = kRoundGroups * (2 * kStaged<kKind> * kFrameRoom<Q> + (kKind == kInner ? kMaxLinks * kTile * 4 : 0));
 
 // Loads the kernel and, once per device, gives it its shared memory.
-template <int Q, int kGroups, int kKind>
+template <int Q, int kKind>
 static int load_round_l() {
   static std::atomic<uint64_t> loaded{0};
   int dev = 0;
   cudaGetDevice(&dev);
   if ((loaded.load(std::memory_order_relaxed) >> (dev & 63)) & 1u) return 0;
-  const cudaError_t e = cudaFuncSetAttribute(round_kernel<Q, kGroups, kKind>, cudaFuncAttributeMaxDynamicSharedMemorySize, kDynamicBytes<Q, kGroups, kKind>);
+  const cudaError_t e = cudaFuncSetAttribute(round_kernel<Q, kKind>, cudaFuncAttributeMaxDynamicSharedMemorySize, kDynamicBytes<Q, kKind>);
   if (e == cudaSuccess) loaded.fetch_or(1ull << (dev & 63), std::memory_order_relaxed);
   return int(e);
 }
 
-template <int Q, int kGroups, int kKind>
+template <int Q, int kKind>
 static int launch_round_l(const RoundParams& p, int ctas, cudaStream_t stream) {
-  if (const int e = load_round_l<Q, kGroups, kKind>()) return e;
+  if (const int e = load_round_l<Q, kKind>()) return e;
   cudaLaunchConfig_t cfg{};
   cfg.gridDim = dim3(ctas);
-  cfg.blockDim = dim3(kGroups * kGroupThreads);
-  cfg.dynamicSmemBytes = kDynamicBytes<Q, kGroups, kKind>;
+  cfg.blockDim = dim3(kRoundGroups * kGroupThreads);
+  cfg.dynamicSmemBytes = kDynamicBytes<Q, kKind>;
   cfg.stream = stream;
   // The launch may move in while the kernel before it in the stream is running out (and is cheaper to issue so: 2.4 instead
   // of 2.9 us).  A window that follows another of its cycle starts at once: the two have no tile in common.  Any other launch
@@ -1260,38 +1260,33 @@ static int launch_round_l(const RoundParams& p, int ctas, cudaStream_t stream) {
   early.val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = &early;
   cfg.numAttrs = 1;
-  return int(cudaLaunchKernelEx(&cfg, round_kernel<Q, kGroups, kKind>, p));
+  return int(cudaLaunchKernelEx(&cfg, round_kernel<Q, kKind>, p));
 }
 
 // `ctas` == 0: only loads the kernel
 template <int Q>
-static int launch_round_q(const RoundParams& p, int shape, int ctas, cudaStream_t stream) {
-  if (shape != 0 && shape != 1) return int(cudaErrorInvalidValue);
-  if (p.n_links > 1) return ctas ? launch_round_l<Q, 2, kInner>(p, ctas, stream) : load_round_l<Q, 2, kInner>();
-  if (p.n_in > 1) return ctas ? launch_round_l<Q, 2, kMember>(p, ctas, stream) : load_round_l<Q, 2, kMember>();
-  if (round_groups(shape, p.n_links, p.n_in) == 3) return ctas ? launch_round_l<Q, 3, kLeaf>(p, ctas, stream) : load_round_l<Q, 3, kLeaf>();
-  return ctas ? launch_round_l<Q, 2, kLeaf>(p, ctas, stream) : load_round_l<Q, 2, kLeaf>();
+static int launch_round_q(const RoundParams& p, int ctas, cudaStream_t stream) {
+  if (p.n_links > 1) return ctas ? launch_round_l<Q, kInner>(p, ctas, stream) : load_round_l<Q, kInner>();
+  if (p.n_in > 1) return ctas ? launch_round_l<Q, kMember>(p, ctas, stream) : load_round_l<Q, kMember>();
+  return ctas ? launch_round_l<Q, kLeaf>(p, ctas, stream) : load_round_l<Q, kLeaf>();
 }
 
-static int launch_round_any(const RoundParams& p, int shape, int ctas, cudaStream_t stream) {
+static int launch_round_any(const RoundParams& p, int ctas, cudaStream_t stream) {
   switch (p.bits) {
-    case 1: return launch_round_q<1>(p, shape, ctas, stream);
-    case 2: return launch_round_q<2>(p, shape, ctas, stream);
-    case 4: return launch_round_q<4>(p, shape, ctas, stream);
-    case 8: return launch_round_q<8>(p, shape, ctas, stream);
+    case 1: return launch_round_q<1>(p, ctas, stream);
+    case 2: return launch_round_q<2>(p, ctas, stream);
+    case 4: return launch_round_q<4>(p, ctas, stream);
+    case 8: return launch_round_q<8>(p, ctas, stream);
     default: return int(cudaErrorInvalidValue);
   }
 }
 
-// Groups of a CTA: two with 96 registers a thread; for a leaf shape 0 asks for three with 72.
-int round_groups(int shape, int n_links, int n_in) { return shape == 0 && n_links == 1 && n_in <= 1 ? 3 : 2; }
+int load_round(const RoundParams& p) { return launch_round_any(p, 0, nullptr); }
 
-int load_round(const RoundParams& p, int shape) { return launch_round_any(p, shape, 0, nullptr); }
-
-int launch_round(const RoundParams& p, int shape, int ctas, void* stream_v) {
+int launch_round(const RoundParams& p, int ctas, void* stream_v) {
   if (p.n_links < 1 || p.n_links > kMaxLinks || p.sweeps < 1 || ctas < 1) return int(cudaErrorInvalidValue);
   if (p.ring_slots < 2 || p.ring_slots > 64 || (p.ring_slots & (p.ring_slots - 1))) return int(cudaErrorInvalidValue);
-  return launch_round_any(p, shape, ctas, static_cast<cudaStream_t>(stream_v));
+  return launch_round_any(p, ctas, static_cast<cudaStream_t>(stream_v));
 }
 
 }  // namespace st

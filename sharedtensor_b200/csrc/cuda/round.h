@@ -126,13 +126,13 @@ enum StatusWord : int {
 };
 
 // Launchers.  `stream` is a cudaStream_t passed as void*.  Return a cudaError_t as int.
-// `shape` picks the CTA's make-up: 1 = two groups, 0 = three groups where there is one link with one ring (one CTA per SM
-// either way).  A group is eight compute warps and one service warp.
-int launch_round(const RoundParams& p, int shape, int ctas, void* stream);
+// One CTA per SM of two groups, with 96 registers a thread (three groups with 72, for a leaf, measured the same).  A group is
+// eight compute warps and one service warp.
+constexpr int kRoundGroups = 2;
+int launch_round(const RoundParams& p, int ctas, void* stream);
 // Loads the kernel that launch_round would run (code is otherwise loaded on a kernel's first launch, which takes up to some
 // tens of milliseconds).
-int load_round(const RoundParams& p, int shape);
-int round_groups(int shape, int n_links, int n_in);
+int load_round(const RoundParams& p);
 // Takes back the frames of one out-ring that the receiver never acknowledged: their steps are subtracted from the
 // link's mirror and the ring's send counters fall back to the credits.  *taken_back (device) counts the tile-frames.
 int launch_unsend(float* mirror, const uint8_t* payload_remote, uint32_t* tx_seq, const uint32_t* credit, int n_tiles, int ring_slots,
