@@ -123,7 +123,9 @@ class SharedTensor:
             self._b.step(rounds)
 
     def flush(self, timeout: float = 30.0) -> bool:
-        """Waits until this replica has nothing left to send and nothing arriving."""
+        """Waits until this replica has nothing left to send and nothing arriving; False if that takes longer than `timeout`
+        seconds.  It speaks for this replica and its neighbours: they have taken in what they were sent.  What they pass on
+        to replicas further down the tree is theirs to flush."""
         with _Range(self.cfg.nvtx, "sharedtensor.flush"):
             return self._b.flush(timeout)
 

@@ -824,10 +824,9 @@ uint32_t GpuReplica::unacknowledged() {
 }
 
 // Three passes of the engine thread in a row, begun after the caller's updates have run, that get to look at all tiles and
-// find nothing to do; for as
-// long as a neighbour may need to take in what it was sent and pass it on (two busy passes at HBM rate) no pass that did;
-// and every frame acknowledged (a neighbour may be gone, or have no engine running: after a tenth of a second of quiet the
-// frames count as delivered, they are in its memory).
+// find nothing to do; for as long as a neighbour may need to take in what it was sent and answer it (two busy passes at HBM
+// rate) no pass that did; and every frame acknowledged (a neighbour may be gone, or have no engine running: after a tenth of
+// a second of quiet the frames count as delivered, they are in its memory).
 bool GpuReplica::flush(void* user_stream, int64_t timeout_ms) {
   DeviceGuard g(device_);
   // The limit covers the wait for another thread's flush and for the caller's stream too.
@@ -877,9 +876,9 @@ void GpuReplica::engine_loop() {
   ::prctl(PR_SET_TIMERSLACK, 1000UL, 0, 0, 0);  // 1 us instead of the default 50 us: the idle pauses start at 10 us
   const size_t depth = ev_round_.size();
   // A few pinned words per launch in flight: tiles handled, groups that left early, and waits that ran out so far, read once
-  // that launch has finished.  The read runs on
-  // a stream of its own behind an event, so that the comm stream goes from one launch straight to the next; a later
-  // launch may already have added to the count by then, which only moves work from one difference to the next.
+  // that launch has finished.  The read runs on a stream of its own behind an event, so that the comm stream goes from one
+  // launch straight to the next; a later launch may already have added to the counts by then, which only moves work from
+  // one difference to the one before it.
   uint64_t* work_host = status_host_ + kDsTotalWords;  // behind the part status() uses
   uint64_t work_seen = 0, cut_seen = 0;
   uint64_t r = 0;

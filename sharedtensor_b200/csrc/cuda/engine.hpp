@@ -127,8 +127,8 @@ class GpuReplica {
   void start_engine();
   void stop_engine();
   bool engine_running() const { return engine_on_.load(); }
-  // With the engine running: waits until the work queued on `user_stream` is done and the rounds have gone quiet; false
-  // when they have not within the time given.
+  // With the engine running: waits until the work queued on `user_stream` is done, the rounds have gone quiet and the
+  // neighbours have acknowledged what they were sent; false when that has not come about within the time given.
   bool flush(void* user_stream, int64_t timeout_ms);
   int ring_peers() const { return ring_peers_.load(); }
   // Ends the engine thread's idle pause at once.  `from_neighbour` marks a doorbell that came over a socket; the

@@ -18,9 +18,10 @@
 //                 reference src/sharedtensor.c:176-177, two socket writes).
 //
 // What bounds it.  Large tensors: HBM; a visit moves 12 to 18 bytes of values, mirror and frames per element.  Two groups
-// keep 64 KB of loads in flight per SM and the next tile is on its way into the L2 meanwhile.  100 M elements on one link:
-// 0.237 ms to send, 0.328 ms to receive and send, 0.332 ms to receive (0.324, 0.439 and 0.426 ms with tiles staged in
-// shared memory by bulk copies for two groups of four warps, four windows instead of three and no overlap between them).
+// keep 64 KB of loads in flight per SM and the next tile is on its way into the L2 meanwhile.  100 M elements on one link,
+// each pass by itself with a wait for the GPU on both sides: 0.231 ms to send, 0.327 ms to receive and send, 0.305 ms to
+// receive (0.324, 0.439 and 0.426 ms with tiles staged in shared memory by bulk copies for two groups of four warps, four
+// windows instead of three and no overlap between them).
 // Small tensors: latency.  A launch over one tile takes 10 us in the kernel, of which the look at the tile takes 2, the
 // tile 3 and the fence 2; some hundred tiles take 23 us, of which the fence takes 5 to 8 (see the publication below).
 //

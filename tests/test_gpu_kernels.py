@@ -523,8 +523,9 @@ def test_join_while_the_default_stream_is_busy(cu):
 
 
 def test_bounded_wait_runs_out_and_the_replica_recovers(cu):
-    """The copy barrier of one tile is told to expect more bytes than are copied: the group that owns the tile gives
-    up after the configured limit, stores nothing of that tile, reports it, and the next ordinary round converges."""
+    """One tile is never handed to the compute warps: the group that owns it gives up after the configured limit, has
+    stored nothing of that tile, reports it, and the next ordinary round converges.  (Waits that run out while the warps
+    are at a tile: test_gpu_round_kinds.py.)"""
     n = 2 * 4096
     torch.manual_seed(3)
     A, B = _replica(cu, n, deadline_us=200), _replica(cu, n, deadline_us=200)
