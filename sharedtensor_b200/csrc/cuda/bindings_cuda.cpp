@@ -47,6 +47,7 @@ PYBIND11_MODULE(_cuda, m) {
                                     "wait_timeouts"};
   });
   m.def("vmm_available", &vmm_available);
+  m.def("unix_same_process", &unix_same_process);
   m.def("memcpy_d2d", [](uintptr_t dst, uintptr_t src, size_t bytes) {
     ck(int(cudaMemcpy(ptr<void>(dst), ptr<void>(src), bytes, cudaMemcpyDeviceToDevice)), "cudaMemcpy");
   });
@@ -159,11 +160,15 @@ PYBIND11_MODULE(_cuda, m) {
       .def("free_edge_block", &GpuReplica::free_edge_block)
       .def("edge_block_ptr", [](GpuReplica& r, int id) { return reinterpret_cast<uintptr_t>(r.edge_block(id).ptr); })
       .def("edge_block_is_vmm", [](GpuReplica& r, int id) { return !r.edge_block(id).plain; })
-      .def("attach_peer", [](GpuReplica& r, int link, int block, uintptr_t remote) { return r.attach_peer(link, block, ptr<void>(remote)); })
+      .def("attach_peer",
+           [](GpuReplica& r, int link, int block, uintptr_t remote, bool same_gpu) { return r.attach_peer(link, block, ptr<void>(remote), same_gpu); },
+           py::arg("link"), py::arg("block"), py::arg("remote"), py::arg("same_gpu") = false)
       .def("detach_peer", &GpuReplica::detach_peer)
       .def("unsend_unacknowledged", &GpuReplica::unsend_unacknowledged)
       .def("n_links", &GpuReplica::n_links)
       .def("n_peers", &GpuReplica::n_peers)
+      .def("one_gpu", &GpuReplica::one_gpu)
+      .def("device", &GpuReplica::device)
       .def("load_values", [](GpuReplica& r, uintptr_t src, uintptr_t s) { r.load_values(ptr<float>(src), strm(s)); })
       .def("add", [](GpuReplica& r, uintptr_t d, uintptr_t s) { r.add(ptr<float>(d), strm(s)); })
       .def("sub_add", [](GpuReplica& r, uintptr_t a, uintptr_t b, uintptr_t s) { r.sub_add(ptr<float>(a), ptr<float>(b), strm(s)); })

@@ -239,7 +239,7 @@ void GpuReplica::free_edge_block(int id) {
   blocks_[id].used = false;
 }
 
-int GpuReplica::attach_peer(int link, int local_block, void* remote_base) {
+int GpuReplica::attach_peer(int link, int local_block, void* remote_base, bool same_gpu) {
   DeviceGuard g(device_);
   std::lock_guard<std::mutex> lk(mu_);
   if (link < 0 || link >= kMaxLinks || !links_[link].used) throw std::invalid_argument("attach_peer: no such link");
@@ -255,6 +255,7 @@ int GpuReplica::attach_peer(int link, int local_block, void* remote_base) {
       check(cudaMemsetAsync(p.tx_seq, 0, size_t(n_tiles_) * 4, S(comm_)), "memset");
       p.link = link;
       p.local_block = local_block;
+      p.same_gpu = same_gpu;
       p.remote = static_cast<uint8_t*>(remote_base);
       p.used = true;
       // whatever the link still had to say must be looked at again
@@ -316,6 +317,11 @@ int GpuReplica::n_peers() const {
   return c;
 }
 
+bool GpuReplica::one_gpu() const {
+  std::lock_guard<std::mutex> lk(mu_);
+  return params_.one_gpu != 0;
+}
+
 void GpuReplica::publish_pending() {
   // Ring numbering is about to change.  Every round ends with its publish kernel, so once the
   // stream has drained nothing refers to the old numbering any more.
@@ -341,8 +347,10 @@ void GpuReplica::rebuild_params() {
   }
   params_.n_links = dense;
   int r = 0;
+  params_.one_gpu = 1;
   for (auto& p : peers_) {
     if (!p.used) continue;
+    if (!p.same_gpu) params_.one_gpu = 0;
     uint8_t* local = static_cast<uint8_t*>(blocks_[p.local_block].mem.ptr);
     InRing& in = params_.in[r];
     in.payload = local + layout_.off_payload;

@@ -79,14 +79,16 @@ class GpuReplica {
   void free_edge_block(int id);
   const VmmBlock& edge_block(int id) const { return blocks_[id].mem; }
   // Frames from the neighbour arrive in local block `local_block`; frames to it go to its block, mapped
-  // at `remote_base` in this process (same layout).  Returns a peer id.
-  int attach_peer(int link, int local_block, void* remote_base);
+  // at `remote_base` in this process (same layout).  `same_gpu`: the neighbour is a replica of this process on this replica's
+  // GPU (while all are, rounds publish at device scope).  Returns a peer id.
+  int attach_peer(int link, int local_block, void* remote_base, bool same_gpu = false);
   void detach_peer(int peer);
   // The neighbour behind `peer` is gone: the frames it never acknowledged (they are still in its ring, which stays
   // mapped) are taken off the link's mirror again.  Returns how many tile-frames that were.  Call before detach_peer.
   uint64_t unsend_unacknowledged(int peer);
   int n_links() const;
   int n_peers() const;
+  bool one_gpu() const;                // every ring stays on this GPU
 
   // ---- data path ----
   void load_values(const float* src, void* user_stream);
@@ -159,6 +161,7 @@ class GpuReplica {
     bool used = false;
     int link = -1;
     int local_block = -1;
+    bool same_gpu = false;
     uint8_t* remote = nullptr;
     uint32_t* rx_seq = nullptr;
     uint32_t* tx_seq = nullptr;

@@ -568,7 +568,7 @@ class GpuNode {
         rep_->add_gate_held(carry);
         rep_->sync();
       }
-      int pid = rep_->attach_peer(link, block, remote.ptr);
+      int pid = rep_->attach_peer(link, block, remote.ptr, reply.device == device_ && unix_same_process(us));
       {
         std::lock_guard<std::mutex> g(mu_);
         Edge& e = edges_[kSlotUp];
@@ -708,7 +708,7 @@ class GpuNode {
       if (!sent) break;
       // state transfer: one pass over the replica, in stream order with the rounds
       rep_->push_snapshot(link, reinterpret_cast<float*>(static_cast<uint8_t*>(child_values.ptr) + kGuardBytes));
-      int pid = rep_->attach_peer(link, block, remote.ptr);
+      int pid = rep_->attach_peer(link, block, remote.ptr, h.device == device_ && unix_same_process(us));
       {
         std::lock_guard<std::mutex> g(mu_);
         Edge& e = edges_[slot];

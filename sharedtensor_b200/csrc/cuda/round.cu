@@ -7,7 +7,8 @@
 //                 in-rings, credits of the out-rings (all loads in flight together).  For every tile with something to
 //                 do it writes a descriptor (tile, which frames arrived, which rings have room, what each link may
 //                 hear) into a bank and arms the bank.  Tiles that all eight compute warps have finished are published
-//                 together behind a system-scope fence: sequence flags to the receivers, credits to the senders.
+//                 together behind a fence (system scope, or device scope if all rings stay on this GPU): sequence flags
+//                 to the receivers, credits to the senders.
 //   compute warps walk through the bank, each on its own 512 elements of every tile.  A lane owns four 16-byte pieces
 //                 128 elements apart, so that every access to values, mirrors and frames is a full, coalesced line:
 //                 values and mirror are loaded straight into registers, the frames that arrived are decoded
@@ -22,8 +23,9 @@
 // each pass by itself with a wait for the GPU on both sides: 0.231 ms to send, 0.327 ms to receive and send, 0.305 ms to
 // receive (0.324, 0.439 and 0.426 ms with tiles staged in shared memory by bulk copies for two groups of four warps, four
 // windows instead of three and no overlap between them).
-// Small tensors: latency.  A launch over one tile takes 10 us in the kernel, of which the look at the tile takes 2, the
-// tile 3 and the fence 2; some hundred tiles take 23 us, of which the fence takes 5 to 8 (see the publication below).
+// Small tensors: latency.  A launch over one tile takes 6 us in the kernel, of which the look at the tile takes 2.3 and the
+// tile 2; 811 tiles that are received and sent (sign frames) take 25 us when they are published at system scope and 17.5 at
+// device scope (see the publication below).
 //
 // Nothing in here waits for another GPU.  The waits are on this group's own warps and copies, and every one is bounded.
 // When one runs out, no visit is left half done: the warps go by the same answer, frames that are not in their stage are
@@ -1027,9 +1029,14 @@ __device__ __forceinline__ void service_warp(const RoundParams& p, GroupShared& 
       // ---- publish: when nothing is in hand, and earlier when half a bank has piled up, so that a neighbour does not
       // wait for the end of a long launch.  Not more often: a system-scope fence takes 1.5 us on a quiet GPU and 3.9 us as
       // soon as 37 or more SMs have one under way (measured: 2815 and 7400 cycles), and a fence that finds others under
-      // way waits for those first.  A fence behind every tile made the last one of a launch take 8 us.
+      // way waits for those first: at the end of a launch of 296 groups it takes 1.5 to 10 us, 4.4 in the middle.  A fence
+      // behind every tile made the last one of a launch take 8 us.
+      // Where the far end of every ring is memory of this GPU, whoever reads the flags is within device scope, and a fence of
+      // that scope takes 0.2 to 1.0 us there, 0.5 in the middle.
       if (finished != published && (finished == armed || finished - published >= uint32_t(kBank / 2))) {
-        asm volatile("fence.acq_rel.sys;" ::: "memory");  // the payloads are performed before the flags that announce them
+        // the payloads are performed before the flags that announce them
+        if (p.one_gpu) asm volatile("fence.acq_rel.gpu;" ::: "memory");
+        else asm volatile("fence.acq_rel.sys;" ::: "memory");
         for (; published != finished; published += min(finished - published, uint32_t(at_once))) {
           if (int32_t(finished - published) <= t) continue;
           const uint32_t entry = (published + uint32_t(t)) % kBank;

@@ -76,6 +76,7 @@ struct RoundParams {
   int32_t zero_other;            // first launch of a cycle: clear the other half for the cycle after this one
   int32_t follows_window;        // the launch before this one in the stream is the window before this one, of the same cycle
   int32_t do_rx, do_tx;          // receiver-only / sender-only launches
+  int32_t one_gpu;               // every ring's far end is memory of this GPU, of a replica in this process
   int32_t sweeps;                // passes over the tensor in this launch (>= 1)
   uint32_t wait_ns;              // upper bound of every wait on the kernel's own warps and copies
   int32_t stall_tile;            // test hook: a wait for this tile runs out (-1: none)

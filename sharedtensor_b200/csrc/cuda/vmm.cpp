@@ -350,6 +350,12 @@ bool unix_send_fd(int sock, int fd_to_send, const void* msg, size_t msg_len) {
   return r == ssize_t(iov.iov_len);
 }
 
+bool unix_same_process(int sock) {
+  struct ucred c;
+  socklen_t len = sizeof(c);
+  return ::getsockopt(sock, SOL_SOCKET, SO_PEERCRED, &c, &len) == 0 && len == sizeof(c) && c.pid == ::getpid();
+}
+
 bool unix_recv_fd(int sock, int* fd_out, void* msg, size_t msg_len, int timeout_ms) {
   if (fd_out) *fd_out = -1;
   struct pollfd pfd = {sock, POLLIN, 0};

@@ -41,5 +41,6 @@ int unix_listen_abstract(const std::string& name, std::string* err);  // returns
 int unix_connect_abstract(const std::string& name, int timeout_ms);   // returns fd or -1
 bool unix_send_fd(int sock, int fd_to_send, const void* msg, size_t msg_len);
 bool unix_recv_fd(int sock, int* fd_out, void* msg, size_t msg_len, int timeout_ms);
+bool unix_same_process(int sock);  // the other end of the connection is in this process
 
 }  // namespace st

@@ -14,8 +14,9 @@ def connect_local(a, b):
     if la < 0 or lb < 0:
         raise RuntimeError("no free link")
     ba, bb = a.alloc_edge_block(), b.alloc_edge_block()
-    a.attach_peer(la, ba, b.edge_block_ptr(bb))
-    b.attach_peer(lb, bb, a.edge_block_ptr(ba))
+    same_gpu = a.device() == b.device()
+    a.attach_peer(la, ba, b.edge_block_ptr(bb), same_gpu)
+    b.attach_peer(lb, bb, a.edge_block_ptr(ba), same_gpu)
     return la, lb
 
 
@@ -31,5 +32,5 @@ def connect_mesh(replicas):
     for i, ri in enumerate(replicas):
         for j, rj in enumerate(replicas):
             if i != j:
-                ri.attach_peer(links[i], blocks[(i, j)], rj.edge_block_ptr(blocks[(j, i)]))
+                ri.attach_peer(links[i], blocks[(i, j)], rj.edge_block_ptr(blocks[(j, i)]), ri.device() == rj.device())
     return links
