@@ -133,13 +133,19 @@ __device__ __forceinline__ float4 load4(const float* p) {
   return v;
 }
 
+// Tiles are taken from the last to the first, the other way round than an update takes them.  A training loop pulls after it
+// has pushed: the pull then begins with the values that are still in the L2, and the next push with those that the pull has
+// read last.  For 50 M elements pushUpdate + copyToTensor take 174 us instead of 182, for 100 M 371 instead of 379; below some
+// 20 M, where everything stays in the L2 anyway, it makes no difference.  (Hints that the other tensors are the first to leave
+// the L2 add nothing to that, hints that the values are the last to leave take it away again.)
 // VEC: the source is aligned.  The destination is (launch_snapshot moves both on to its first whole vector).
 template <class T, bool VEC>
 __global__ void __launch_bounds__(kEwThreads, 8) snapshot_kernel(const float* src, T* dst, int64_t n, int head, UpdateMarks m) {
   constexpr bool kBf16 = sizeof(T) == 2;
   const int64_t n_tiles = (n + kTile - 1) / kTile;
   wait_for_stream();
-  for (int64_t tile = blockIdx.x; tile < n_tiles; tile += gridDim.x) {
+  for (int64_t turn = blockIdx.x; turn < n_tiles; turn += gridDim.x) {
+    const int64_t tile = n_tiles - 1 - turn;
     if ((tile + 1) * kTile <= n) {
       const float* s4 = src + tile * kTile + threadIdx.x * 4;
       float4 v[kVecs];

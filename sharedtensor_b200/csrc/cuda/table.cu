@@ -43,12 +43,14 @@ void ck(cudaError_t e, const char* what) {
 }
 
 // ADD: arena += tensors (reductions at the L2), then the change marks of the arena tiles it touched, as an update does.
-// Otherwise tensors = arena.  Chunks are walked in arena order, every CTA takes every gridDim-th.
+// Otherwise tensors = arena.  Every CTA takes every gridDim-th chunk, in arena order when it adds and from the end when it
+// copies: a pull begins with what the push before it has left in the L2 (see snapshot_kernel; GPT-2 small, push and pull:
+// 406 us instead of 415).
 template <bool ADD>
 __global__ void __launch_bounds__(kThreads, 8) table_kernel(float* __restrict__ arena, const Chunk* __restrict__ chunks, uint32_t n_chunks,
                                                             uint32_t first_tensor, const __grid_constant__ Pointers ptrs, UpdateMarks m) {
-  for (uint32_t c = blockIdx.x; c < n_chunks; c += gridDim.x) {
-    const Chunk ch = chunks[c];
+  for (uint32_t turn = blockIdx.x; turn < n_chunks; turn += gridDim.x) {
+    const Chunk ch = chunks[ADD ? turn : n_chunks - 1 - turn];
     float* const t = ptrs.p[ch.tensor - first_tensor] + ch.arena;
     float* const a = arena + ch.arena;
     // Whole vectors on the side that is added to or written (the arena's chunks are aligned, a tensor may start anywhere);
@@ -260,14 +262,16 @@ static void launch_table(float* arena, const std::vector<uintptr_t>& ptrs, const
   const int n = int(ptrs.size());
   UpdateMarks inner = m;
   inner.yield_word = nullptr;
-  for (int k0 = 0; k0 < n; k0 += kPtrs) {
-    const int k1 = std::min(n, k0 + kPtrs);
+  const int launches = (n + kPtrs - 1) / kPtrs;
+  for (int i = 0; i < launches; i++) {
+    const int k0 = (ADD ? i : launches - 1 - i) * kPtrs, k1 = std::min(n, k0 + kPtrs);
+    const bool last = i == launches - 1;
     Pointers p;
     for (int k = k0; k < k1; k++) p.p[k - k0] = reinterpret_cast<float*>(ptrs[k] - uintptr_t(offsets[k]) * 4);
     const uint32_t c0 = first_chunk[k0], count = first_chunk[k1] - c0;
-    if (count == 0 && (k1 < n || m.yield_word == nullptr)) continue;
+    if (count == 0 && (!last || m.yield_word == nullptr)) continue;
     table_kernel<ADD><<<count ? blocks_for(count) : 1, kThreads, 0, static_cast<cudaStream_t>(stream)>>>(arena, chunks + c0, count, uint32_t(k0), p,
-                                                                                                         k1 == n ? m : inner);
+                                                                                                         last ? m : inner);
     ck(cudaGetLastError(), "kernel launch");
   }
 }
