@@ -609,6 +609,8 @@ void GpuReplica::launch(bool do_rx, bool do_tx, int sweeps) {
   int grid, chunk, per_group;
   grid_for_launch(params_.tile_count, &grid, &chunk, &per_group);
   params_.chunk = chunk;
+  params_.tiles_each = params_.tile_count / (grid * kRoundGroups);
+  params_.groups_more = params_.tile_count % (grid * kRoundGroups);
   check(launch_round(params_, grid, comm_), "round kernel");
   last_parity_ = params_.parity;
   next_window_ = (w + 1) % nw;

@@ -644,18 +644,19 @@ __device__ __forceinline__ void compute_warp(const RoundParams& p, GroupShared& 
       d = sh.desc[entry];
       c++;
     }
-    if (live && warp == 0 && lane == 0) {
-      // The next tile on its way into the L2.  One tile ahead is best: a window of 25 M elements that receives and sends
-      // takes 92 us so, 115 us with two tiles ahead and 153 us with four.
+    // The next tile on its way into the L2, once this one's loads are under way (ahead of them, a mesh of eight takes 643 us
+    // instead of 620, three sign rounds of 3.3 M elements 51 instead of 49).  One tile ahead is best: a window of 25 M elements
+    // that receives and sends takes 92 us so, 115 us with two tiles ahead and 153 us with four; without, three rounds of 100 M
+    // elements on one link take 1278 us instead of 1157.
+    auto prefetch_next = [&]() {
       const uint32_t ahead = c;  // (c is the next tile's number by now)
-      if (int32_t(ld_shared_acquire(&sh.armed) - ahead) > 0) {
-        const TileDesc& e = sh.desc[ahead % kBank];
-        if (!(e.flags & kDescNoValues)) bulk_prefetch_l2(p.values + size_t(e.tile) * kTile, kTile * 4);
-        for (int l = 0; l < L; l++) bulk_prefetch_l2(p.mirror[l] + size_t(e.tile) * kTile, kTile * 4);
-        if (kIn == 0 || e.n_frames == 1)
-          for (int j = 0; j < e.n_frames; j++) bulk_prefetch_l2(frame_at(sh.frames[ahead % kBank][j]), uint32_t(p.payload_bytes));
-      }
-    }
+      if (!live || warp != 0 || lane != 0 || int32_t(ld_shared_acquire(&sh.armed) - ahead) <= 0) return;
+      const TileDesc& e = sh.desc[ahead % kBank];
+      if (!(e.flags & kDescNoValues)) bulk_prefetch_l2(p.values + size_t(e.tile) * kTile, kTile * 4);
+      for (int l = 0; l < L; l++) bulk_prefetch_l2(p.mirror[l] + size_t(e.tile) * kTile, kTile * 4);
+      if (kIn == 0 || e.n_frames == 1)
+        for (int j = 0; j < e.n_frames; j++) bulk_prefetch_l2(frame_at(sh.frames[ahead % kBank][j]), uint32_t(p.payload_bytes));
+    };
     const int in_tile = warp * kWarpElems + lane * 4;
     const size_t off = size_t(d.tile) * kTile + in_tile;
     const int left = int(min(int64_t(kTile), p.n - int64_t(d.tile) * kTile)) - in_tile;  // (used by sign frames only)
@@ -670,6 +671,7 @@ __device__ __forceinline__ void compute_warp(const RoundParams& p, GroupShared& 
       for (int i = 0; i < kPieces; i++) v[i] = load_v ? load_piece(vp + i * 128) : Piece{0ull, 0ull};
 #pragma unroll
       for (int i = 0; i < kPieces; i++) k[i] = live ? load_piece(p.mirror[0] + off + i * 128) : Piece{0ull, 0ull};
+      prefetch_next();
       if (d.n_frames == 1) {
         const uint64_t e = frames[0];
         const bool for0 = kOneLink || !live || (e & 15u) == 0;
@@ -694,6 +696,7 @@ __device__ __forceinline__ void compute_warp(const RoundParams& p, GroupShared& 
         }
       };
       if (kOneLink) fetch();
+      prefetch_next();
       const uint32_t st = d.stage & 1u;
       if (kIn > 0 && live) {
         // A warp whose stage is not filled in time reads the frames from the ring, where they stay until the tile is
@@ -819,27 +822,32 @@ __device__ __forceinline__ void compute_warp(const RoundParams& p, GroupShared& 
 // a power of two above one, 32 / R tiles are looked at together, and every look costs two round trips to the L2 whatever R is.
 // All 32 lanes run the same control flow; decisions taken from words that change under the warp's feet are taken by one
 // lane, or on a ballot.
+// What it does before the first tile is armed and after the last one is finished is the fixed part of every launch, a chain of
+// one warp's instructions.  It is compiled for each kind of replica, so that a leaf has no loops over links and rings and no
+// ballots among its lanes, and divides nothing and reads no clock on that way: the first tile of a launch is armed after 2.1 us
+// instead of 3.1 (a member's after 2.9 instead of 3.8), and three rounds over 811 tiles of sign frames take 49 us instead of 54.
+template <int kKind>
 __device__ __forceinline__ void service_warp(const RoundParams& p, GroupShared& sh, uint8_t* stages, int staged_frames, int frame_room, int g, int n_groups, int lane) {
   // The group's tiles: a run of `chunk` consecutive tiles, or (chunk == 0) every gstride-th tile of the launch's window.
   // The groups of a CTA are a grid apart, so that the odd tiles of the last turn fall on all SMs alike.
   const int gidx = p.chunk > 0 ? int(blockIdx.x) * n_groups + g : g * int(gridDim.x) + int(blockIdx.x);
   const int gid0 = p.chunk > 0 ? gidx * p.chunk : gidx;
   const int gstride = p.chunk > 0 ? 1 : int(gridDim.x) * n_groups;
-  const int my_count = p.chunk > 0 ? max(0, min(p.chunk, p.tile_count - gid0))
-                                   : (p.tile_count > gid0 ? (p.tile_count - gid0 + gstride - 1) / gstride : 0);
+  const int my_count = p.chunk > 0 ? max(0, min(p.chunk, p.tile_count - gid0)) : p.tiles_each + (gid0 < p.groups_more ? 1 : 0);
   const int gid = p.tile_begin + gid0;
   const uint32_t smask = uint32_t(p.ring_slots) - 1u;
   const uint64_t limit_ns = p.wait_ns;
   uint64_t* const launch_words = p.status + (p.parity ? kDsLaunch1 : kDsLaunch0);
-  const unsigned long long sent_before = blockIdx.x == 0 && g == 0 && lane == 0 ? p.status[kDsFramesSent] : 0ull;  // for the trace
+  unsigned long long sent_before = 0;             // for the trace
 
   // ---- this lane's ring pair and its place among the tiles looked at together
-  int log2_rings = 1;                             // (16 tiles at most, so that the next look fits into the bank in time)
-  while ((1 << log2_rings) < max(p.n_in, p.n_out)) log2_rings++;
+  constexpr bool kLeafOnly = kKind == kLeaf, kOneLink = kKind != kInner;
+  const int n_links = kOneLink ? 1 : p.n_links, rings = kLeafOnly ? 1 : max(p.n_in, p.n_out);
+  const int log2_rings = rings > 4 ? 3 : (rings > 2 ? 2 : 1);  // (16 tiles at most, so that the next look fits into the bank in time)
   const int at_once = 32 >> log2_rings;           // tiles of one look
   const int r = lane >> (5 - log2_rings), t = lane & (at_once - 1);
-  uint32_t same_tile = 0;                         // the lanes of this lane's tile, one per ring, in ring order
-  for (int i = 0; i < (1 << log2_rings); i++) same_tile |= 1u << (i * at_once + t);
+  // the lanes of this lane's tile, one per ring, in ring order
+  const uint32_t same_tile = kLeafOnly ? 1u << lane : (log2_rings == 3 ? 0x11111111u : (log2_rings == 2 ? 0x01010101u : 0x00010001u)) << t;
   const uint32_t below = (1u << lane) - 1u;
   const bool is_in = r < p.n_in && p.do_rx, is_out = r < p.n_out && p.do_tx;
   InRing in{};
@@ -855,10 +863,14 @@ __device__ __forceinline__ void service_warp(const RoundParams& p, GroupShared& 
   bool aborted = false, yielded = false;
   bool ran_out = false;                             // a wait of a compute warp did
 
-  if (p.zero_other && blockIdx.x == 0 && g == 0 && lane == 0) {
+  // Bookkeeping of the launch, done behind the first look's loads.
+  auto begin_launch = [&]() {
+    if (blockIdx.x != 0 || g != 0) return;
     uint64_t* other = p.status + (p.parity ? kDsLaunch0 : kDsLaunch1);  // the next cycle's half
-    for (int i = 0; i < 8; i++) other[i] = 0;
-  }
+    if (p.zero_other && lane < 8) other[lane] = 0;
+    if (lane == 0) sent_before = p.status[kDsFramesSent];
+  };
+  if (my_count == 0) begin_launch();
   auto update_waiting = [&]() -> bool {
     const uint32_t y = p.yield_flag != nullptr && lane == 0 ? ld_cg_u32(p.yield_flag) : 0u;
     return __any_sync(0xffffffffu, y != 0);
@@ -868,7 +880,7 @@ __device__ __forceinline__ void service_warp(const RoundParams& p, GroupShared& 
     const uint32_t armed_before = armed;
     int looked = 0;           // tiles of the group looked at in this sweep
     uint32_t idle = 0;
-    uint64_t t_last = globaltimer_ns();
+    uint64_t t_last = 0;      // (read when there has been nothing to do for some looks: reading the clock takes its time)
     while (true) {
       // ---- the frames of the next tiles that have several on their way into shared memory, as stages become free
       while (staged_frames > 0 && staged != handed && !ran_out) {
@@ -895,7 +907,7 @@ __device__ __forceinline__ void service_warp(const RoundParams& p, GroupShared& 
         ST_CRUMB(g, 2);
         const uint32_t y = p.yield_flag != nullptr && lane == 0 ? ld_cg_u32(p.yield_flag) : 0u;
         const int j = looked + t;
-        const bool valid = j < my_count;
+        const bool valid = j < my_count && (!kLeafOnly || r == 0);
         const int tile = gid + j * gstride;
         looked += at_once;
         uint32_t dirty = 0, rx = 0, tx = 0, credit = 0, avail = 0;
@@ -938,9 +950,16 @@ __device__ __forceinline__ void service_warp(const RoundParams& p, GroupShared& 
             if (avail) (void)ld_acquire_sys(fl + size_t((rx + avail - 1u) & smask) * p.n_tiles);
           }
         }
-        dirty = __shfl_sync(0xffffffffu, dirty, t);
+        if (looked == at_once && sweep == 0) begin_launch();
         const bool room = is_out && (tx - credit) < uint32_t(p.ring_slots);
-        const uint32_t in1 = __ballot_sync(0xffffffffu, avail >= 1), in2 = __ballot_sync(0xffffffffu, avail >= 2), in3 = __ballot_sync(0xffffffffu, avail >= 3);
+        // (a leaf's lane has its tile to itself)
+        uint32_t in1 = avail >= 1 ? same_tile : 0u, in2 = avail >= 2 ? same_tile : 0u, in3 = avail >= 3 ? same_tile : 0u;
+        if (!kLeafOnly) {
+          dirty = __shfl_sync(0xffffffffu, dirty, t);
+          in1 = __ballot_sync(0xffffffffu, avail >= 1);
+          in2 = __ballot_sync(0xffffffffu, avail >= 2);
+          in3 = __ballot_sync(0xffffffffu, avail >= 3);
+        }
         const bool any_in = (in1 & same_tile) != 0, work = valid && (dirty != 0 || any_in);
         if (__any_sync(0xffffffffu, y != 0)) {  // an update is waiting for SMs: hand out nothing more
           if (dirty && r == 0) st_cg_u32(p.tile_state + tile, 1u);
@@ -954,35 +973,38 @@ __device__ __forceinline__ void service_warp(const RoundParams& p, GroupShared& 
         // gets a frame when the tile changed here (its mark) or when another link brought something to pass on.
         uint32_t flags = 0;
         bool goes_out = false;
-        for (int l = 0; l < p.n_links; l++) {
-          const uint32_t here = __ballot_sync(0xffffffffu, avail != 0 && in.link == l) & same_tile;
-          const uint32_t outs = __ballot_sync(0xffffffffu, is_out && out.link == l) & same_tile;
-          const uint32_t full = __ballot_sync(0xffffffffu, is_out && out.link == l && !room) & same_tile;
+        for (int l = 0; l < n_links; l++) {
+          uint32_t here, outs, full;
+          if (kLeafOnly) {
+            here = in1;
+            outs = is_out ? same_tile : 0u;
+            full = is_out && !room ? same_tile : 0u;
+          } else if (kOneLink) {
+            here = in1 & same_tile;
+            outs = __ballot_sync(0xffffffffu, is_out) & same_tile;
+            full = __ballot_sync(0xffffffffu, is_out && !room) & same_tile;
+          } else {
+            here = __ballot_sync(0xffffffffu, avail != 0 && in.link == l) & same_tile;
+            outs = __ballot_sync(0xffffffffu, is_out && out.link == l) & same_tile;
+            full = __ballot_sync(0xffffffffu, is_out && out.link == l && !room) & same_tile;
+          }
           const bool want = dirty != 0 || (in1 & same_tile & ~here) != 0;
           const bool ok = want && outs != 0 && full == 0;
           flags |= (ok ? kDescTxOk << l : 0u) | (here ? kDescRxLink << l : 0u) | (want ? kDescTxWant << l : 0u);
-          goes_out |= ok && is_out && out.link == l;
+          goes_out |= ok && is_out && (kOneLink || out.link == l);
         }
         // A tile of a one-link replica that carries no mark is here only to receive: nothing is said on the link, so
         // the values themselves are not needed.
-        if (p.n_links == 1 && dirty == 0) flags |= kDescNoValues;
-        const uint32_t sends = __ballot_sync(0xffffffffu, goes_out) & same_tile;
+        if (n_links == 1 && dirty == 0) flags |= kDescNoValues;
+        const uint32_t sends = kLeafOnly ? (goes_out ? same_tile : 0u) : __ballot_sync(0xffffffffu, goes_out) & same_tile;
         const int n_frames = __popc(in1 & same_tile) + __popc(in2 & same_tile) + __popc(in3 & same_tile);
-        const uint32_t several = __ballot_sync(0xffffffffu, work && r == 0 && n_frames > 1);
+        const uint32_t several = staged_frames > 0 ? __ballot_sync(0xffffffffu, work && r == 0 && n_frames > 1) : 0u;
         const uint32_t pos = armed + __popc(work_tiles & ((1u << t) - 1u)), entry = pos % kBank;
         if (work) {
           if (r == 0) {
             sh.desc[entry] = TileDesc{tile, flags, uint16_t(n_frames), uint16_t(__popc(sends)), stage_no + __popc(several & ((1u << t) - 1u))};
             sh.done[entry] = 0;
             sh.dirty[entry] = dirty;
-          }
-          if (pos == finished) {  // (the compute warps see to the later ones)
-            if (r == 0) {
-              if (!(flags & kDescNoValues)) bulk_prefetch_l2(p.values + size_t(tile) * kTile, kTile * 4);
-              for (int l = 0; l < p.n_links; l++) bulk_prefetch_l2(p.mirror[l] + size_t(tile) * kTile, kTile * 4);
-            }
-            for (uint32_t f = 0; f < avail && (staged_frames == 0 || n_frames == 1); f++)
-              bulk_prefetch_l2(in.payload + (size_t((rx + f) & smask) * p.n_tiles + tile) * p.payload_bytes, uint32_t(p.payload_bytes));
           }
           const uint32_t before = same_tile & below;
           uint64_t* list = &sh.frames[entry][__popc(in1 & before) + __popc(in2 & before) + __popc(in3 & before)];
@@ -1000,7 +1022,17 @@ __device__ __forceinline__ void service_warp(const RoundParams& p, GroupShared& 
         handed = stalled ? armed + __popc(work_tiles & ((1u << (__ffs(stalled) - 1)) - 1u)) : armed + __popc(work_tiles);
         __syncwarp();
         if (lane == 0) st_shared_release(&sh.armed, handed);
-        if (armed == finished) t_last = globaltimer_ns();
+        // The lines of a tile that is begun at once (the compute warps see to the later ones): all of them, while the warps are on
+        // their way to asking for the first.  A hub and its leaves over 16 M elements take 517 us so, 522 without; a mesh of
+        // eight, whose members begin with bulk copies of their frames, 603 without and 617 so.
+        if (kKind != kMember && work && pos == finished) {
+          if (r == 0) {
+            if (!(flags & kDescNoValues)) bulk_prefetch_l2(p.values + size_t(tile) * kTile, kTile * 4);
+            for (int l = 0; l < n_links; l++) bulk_prefetch_l2(p.mirror[l] + size_t(tile) * kTile, kTile * 4);
+          }
+          for (uint32_t f = 0; f < avail; f++)
+            bulk_prefetch_l2(in.payload + (size_t((rx + f) & smask) * p.n_tiles + tile) * p.payload_bytes, uint32_t(p.payload_bytes));
+        }
         armed += __popc(work_tiles);
         stage_no += __popc(several);
         if (stalled) looked = my_count;
@@ -1022,7 +1054,6 @@ __device__ __forceinline__ void service_warp(const RoundParams& p, GroupShared& 
       if (more) {
         __syncwarp();  // (nor does a ballot) what each lane has acquired of its tile comes before the fence and the flags of any lane
         finished += more;
-        t_last = globaltimer_ns();
         idle = 0;
       }
       const bool last = finished == armed && (looked >= my_count || yielded || aborted || ran_out);
@@ -1038,11 +1069,11 @@ __device__ __forceinline__ void service_warp(const RoundParams& p, GroupShared& 
         if (p.one_gpu) asm volatile("fence.acq_rel.gpu;" ::: "memory");
         else asm volatile("fence.acq_rel.sys;" ::: "memory");
         for (; published != finished; published += min(finished - published, uint32_t(at_once))) {
-          if (int32_t(finished - published) <= t) continue;
+          if (int32_t(finished - published) <= t || (kLeafOnly && r != 0)) continue;
           const uint32_t entry = (published + uint32_t(t)) % kBank;
           const TileDesc d = sh.desc[entry];
           const uint32_t done = sh.done[entry], moved = sh.moved[entry][r];
-          if ((moved & 4u) && ((done >> (kDoneNonsilentShift + 4 * out.link)) & 0xfu)) {
+          if ((moved & 4u) && ((done >> (kDoneNonsilentShift + (kOneLink ? 0 : 4 * out.link))) & 0xfu)) {
             const uint32_t seq = sh.tx[entry][r];
             st_relaxed_sys(out.flags_remote + size_t((seq - 1u) & smask) * p.n_tiles + d.tile, seq);
             st_cg_u32(out.tx_seq + d.tile, seq);
@@ -1056,7 +1087,7 @@ __device__ __forceinline__ void service_warp(const RoundParams& p, GroupShared& 
           }
           if (r == 0) {
             bool left = done >= kDoneFailed;
-            for (int l = 0; l < p.n_links; l++) {
+            for (int l = 0; l < n_links; l++) {
               if (((done >> (kDoneNonsilentShift + 4 * l)) & 0xfu) == 0) continue;
               left = true;  // more may be left to say (or nothing could be said at all)
               if (!(d.flags & (kDescTxOk << l)) && p.do_tx) n_blocked++;
@@ -1073,7 +1104,7 @@ __device__ __forceinline__ void service_warp(const RoundParams& p, GroupShared& 
       }
       if (last) break;
       if (more) continue;
-      idle++;
+      if (++idle == 1024u) t_last = globaltimer_ns();
       // (The time by the clock and in looks, like the waits of the compute warps.  The second time it is longer than all the
       // waits of a compute warp in one tile: one on a stage, one per link on an exchange.)
       const bool late = __any_sync(0xffffffffu, idle > 2048u && globaltimer_ns() - t_last > (aborted ? 8 : 2) * limit_ns);
@@ -1161,14 +1192,16 @@ __global__ void __launch_bounds__(kRoundGroups * kGroupThreads, 1) round_kernel(
       mbar_init(&sh.full[u], 1);
       mbar_init(&sh.empty[u], kComputeWarps);
     }
-    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+    if (kIn > 0) {  // (bulk copies will complete on them)
+      asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+      asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+    }
   }
   if (!p.follows_window) asm volatile("griddepcontrol.wait;" ::: "memory");
   __syncthreads();  // the only CTA-wide barrier: from here on the groups, and the two kinds of warp, run on their own
   uint8_t* const stages = dynamic + g * kStageBytes;
   float* const stash = reinterpret_cast<float*>(dynamic + kRoundGroups * kStageBytes) + (kKind == kInner ? g * kMaxLinks * kTile : 0);
-  if (warp == kComputeWarps) service_warp(p, shared[g], stages, kIn, kFrameRoom<Q>, g, kRoundGroups, lane);
+  if (warp == kComputeWarps) service_warp<kKind>(p, shared[g], stages, kIn, kFrameRoom<Q>, g, kRoundGroups, lane);
   else compute_warp<Q, kKind>(p, shared[g], stash, stages, warp, lane);
 }
 

@@ -82,6 +82,7 @@ struct RoundParams {
   int32_t stall_tile;            // test hook: a wait for this tile runs out (-1: none)
   int32_t stall_warp;            // -1: it is never handed to the compute warps; w: compute warp w does not come to its waits; 8 + w: it comes late
   int32_t chunk;                 // > 0: a group owns this many consecutive tiles; 0: every (groups in the grid)-th tile
+  int32_t tiles_each, groups_more; // chunk == 0: tiles of a group, and how many groups have one more than that
   const uint32_t* yield_flag;    // non-zero while an update is waiting for SMs: groups hand out no more tiles and leave
   uint32_t* dbg;                 // debug builds: progress marks in mapped host memory, 8 words per CTA (else null)
 };
