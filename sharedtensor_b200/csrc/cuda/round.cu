@@ -480,12 +480,13 @@ __device__ __forceinline__ bool claim_tile(GroupShared& sh, uint32_t c) {
 // The frames of a tile, as the service warp listed them: address | link, in ring order and sequence order.
 __device__ __forceinline__ const uint8_t* frame_at(uint64_t e) { return reinterpret_cast<const uint8_t*>(e & ~15ull); }
 
-__device__ __forceinline__ void get_stash(const float* stash, int link, Piece (&x)[kPieces]) {
-#pragma unroll
-  for (int i = 0; i < kPieces; i++) {
-    const ulonglong2 y = *reinterpret_cast<const ulonglong2*>(stash + link * kTile + i * 128);
-    x[i] = {y.x, y.y};
-  }
+// Piece i of this lane's part of a link's plane of the group's stash: what arrived on the link.
+__device__ __forceinline__ Piece get_part(const float* stash, int link, int i) {
+  const ulonglong2 y = *reinterpret_cast<const ulonglong2*>(stash + link * kTile + i * 128);
+  return {y.x, y.y};
+}
+__device__ __forceinline__ void put_part(float* stash, int link, int i, const Piece& x) {
+  *reinterpret_cast<ulonglong2*>(stash + link * kTile + i * 128) = make_ulonglong2(x.a, x.b);
 }
 
 // What kind of replica a kernel is for: a leaf of the tree (one link, one ring in), a member of a mesh group (one link,
@@ -507,15 +508,9 @@ constexpr int kStaged = kKind == kMember ? 8 : 0;
 template <int Q, bool kStash, int kIn>
 __device__ __forceinline__ void decode_frames(const uint64_t* list, const uint8_t* staged, bool in_stage, int count, uint32_t live, uint64_t* empty, int log2_block,
                                               int warp, int lane, int left, float* stash, Piece (&total)[kPieces]) {
-  Piece mine[kPieces];
-  int cur = -1;
   uint32_t seen = 0;
 #pragma unroll
   for (int i = 0; i < kPieces; i++) total[i] = {0ull, 0ull};
-  auto put = [&](int link) {
-#pragma unroll
-    for (int i = 0; i < kPieces; i++) *reinterpret_cast<ulonglong2*>(stash + link * kTile + i * 128) = make_ulonglong2(mine[i].a, mine[i].b);
-  };
 #pragma unroll 1
   for (int j = 0; j < count; j++) {
     FrameRegs f{};
@@ -523,25 +518,19 @@ __device__ __forceinline__ void decode_frames(const uint64_t* list, const uint8_
       if (in_stage && j < kIn) load_staged<Q>(staged + j * kFrameRoom<Q>, warp, lane, log2_block, f);
       else load_frame<Q>(frame_at(list[j]), warp, lane, log2_block, f);
     }
-    if (kStash) {
-      const int link = live ? int(list[j] & 15u) : 0;
-      if (link != cur) {
-        if (cur >= 0) put(cur);
-#pragma unroll
-        for (int i = 0; i < kPieces; i++) mine[i] = {0ull, 0ull};
-        if ((seen >> link) & 1u) get_stash(stash, link, mine);
-        cur = link;
-        seen |= 1u << link;
-      }
-    }
+    const int link = kStash && live ? int(list[j] & 15u) : 0;
+    const bool again = (seen >> link) & 1u;
+    seen |= 1u << link;
 #pragma unroll
     for (int i = 0; i < kPieces; i++) {
-      const Piece st = frame_steps<Q>(f.w[i], f.code(i), Q == 1 ? valid4(left, i) : 0xfu);
+      Piece st = frame_steps<Q>(f.w[i], f.code(i), Q == 1 ? valid4(left, i) : 0xfu);
       add4(total[i], st);
-      if (kStash) add4(mine[i], st);
+      if (kStash) {
+        if (again) add4(st, get_part(stash, link, i));
+        put_part(stash, link, i, st);
+      }
     }
   }
-  if (kStash && cur >= 0) put(cur);
   if (kIn == 0) return;
   __syncwarp();
   if (live && in_stage && lane == 0) mbar_arrive(empty);  // the stage may be filled again when all warps have read it
@@ -664,8 +653,23 @@ __device__ __forceinline__ void compute_warp(const RoundParams& p, GroupShared& 
     Piece v[kPieces], k[kPieces];
     const uint64_t* frames = sh.frames[entry];
     const bool load_v = live && (d.flags & kDescNoValues) == 0;
-    int applied = -1;  // the link whose mirror has been given what arrived on it
-    if (d.n_frames <= 1) {
+    float* const stash = group_stash + in_tile;
+    if (!kOneLink) {
+      // What arrived, then the values into it.  Nothing is held in registers beyond that and the mirror of the link in hand, and
+      // the values' maxima are taken once for all links: the kernel spills nothing, and a hub with two leaves takes 638 us for
+      // its rounds over 30 M elements instead of 657.  (More would not help: with 72 registers and three groups, or the next
+      // link's mirror loaded ahead into registers, the warps wait for memory longer instead, 545 and 505 us against 502 for a hub
+      // and three leaves over 16 M.  The L2 serves some 10 TB/s at that point.)
+      prefetch_next();
+      decode_frames<Q, true, 0>(frames, nullptr, false, d.n_frames, live, nullptr, lb, warp, lane, left, stash, v);
+#pragma unroll
+      for (int i = 0; i < kPieces; i++) k[i] = live ? load_piece(vp + i * 128) : Piece{0ull, 0ull};
+#pragma unroll
+      for (int i = 0; i < kPieces; i++) {
+        if (live && (v[i].a | v[i].b)) red_add_piece(vp + i * 128, v[i]);
+        add4(v[i], k[i]);
+      }
+    } else if (d.n_frames <= 1) {
       // the common case: everything is fetched at once, and the one frame's steps never have to be kept
 #pragma unroll
       for (int i = 0; i < kPieces; i++) v[i] = load_v ? load_piece(vp + i * 128) : Piece{0ull, 0ull};
@@ -673,29 +677,23 @@ __device__ __forceinline__ void compute_warp(const RoundParams& p, GroupShared& 
       for (int i = 0; i < kPieces; i++) k[i] = live ? load_piece(p.mirror[0] + off + i * 128) : Piece{0ull, 0ull};
       prefetch_next();
       if (d.n_frames == 1) {
-        const uint64_t e = frames[0];
-        const bool for0 = kOneLink || !live || (e & 15u) == 0;
         FrameRegs f{};
-        if (live) load_frame<Q>(frame_at(e), warp, lane, lb, f);
+        if (live) load_frame<Q>(frame_at(frames[0]), warp, lane, lb, f);
 #pragma unroll
         for (int i = 0; i < kPieces; i++) {
           const Piece s = frame_steps<Q>(f.w[i], f.code(i), Q == 1 ? valid4(left, i) : 0xfu);
           if (f.code(i)) red_add_piece(vp + i * 128, s);
           add4(v[i], s);
-          if (for0) add4(k[i], s);
+          add4(k[i], s);
         }
-        if (for0) applied = 0;
       }
     } else {
-      // (one link: values and mirror on their way while the frames are decoded)
-      auto fetch = [&]() {
+      // (values and mirror on their way while the frames are decoded)
 #pragma unroll
-        for (int i = 0; i < kPieces; i++) {
-          v[i] = load_v ? load_piece(vp + i * 128) : Piece{0ull, 0ull};
-          k[i] = live ? load_piece(p.mirror[0] + off + i * 128) : Piece{0ull, 0ull};
-        }
-      };
-      if (kOneLink) fetch();
+      for (int i = 0; i < kPieces; i++) {
+        v[i] = load_v ? load_piece(vp + i * 128) : Piece{0ull, 0ull};
+        k[i] = live ? load_piece(p.mirror[0] + off + i * 128) : Piece{0ull, 0ull};
+      }
       prefetch_next();
       const uint32_t st = d.stage & 1u;
       if (kIn > 0 && live) {
@@ -705,39 +703,49 @@ __device__ __forceinline__ void compute_warp(const RoundParams& p, GroupShared& 
         if (!unstaged) unstaged = !__all_sync(0xffffffffu, !held(p, d.tile, warp) && mbar_wait_bounded(&sh.full[st], (d.stage >> 1) & 1u, 2ull * p.wait_ns));
       }
       Piece acc[kPieces];
-      decode_frames<Q, !kOneLink, kIn>(frames, stages + st * (kIn * kFrameRoom<Q>), !unstaged, d.n_frames, live, &sh.empty[st], lb, warp, lane, left,
-                                       group_stash + in_tile, acc);
-      if (!kOneLink) fetch();
+      decode_frames<Q, false, kIn>(frames, stages + st * (kIn * kFrameRoom<Q>), !unstaged, d.n_frames, live, &sh.empty[st], lb, warp, lane, left, nullptr, acc);
 #pragma unroll
       for (int i = 0; i < kPieces; i++) {
         if (live) red_add_piece(vp + i * 128, acc[i]);
         add4(v[i], acc[i]);
-        if (kOneLink) add4(k[i], acc[i]);
+        add4(k[i], acc[i]);
       }
-      if (kOneLink) applied = 0;
     }
+    auto larger = [](float a, float b) { return fmaxf(a, b); };
+    // over the chunks of a piece row and the piece rows: blocks of up to 512 elements
+    auto over_block = [&](float m) {
+      if (lb >= 6) {
+        m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, 8));
+        if (lb >= 7) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, 16));
+        if (lb >= 8) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, 1));
+        if (lb >= 9) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, 2));
+      }
+      return m;
+    };
+    float vmax = 0.f;  // an inner node: the largest |value| of each block, the same for all links
+    if (!kOneLink) {
+      float vs[kPieces];
+#pragma unroll
+      for (int i = 0; i < kPieces; i++) {
+        vs[i] = maxabs(v[i]);
+      }
+      vmax = over_block(reduce_pieces(vs, lane, larger));
+    }
+    const int n_links = live ? L : 1;  // (once through the code of a link is enough to fetch it)
     uint32_t finished = kDoneWarp;
     bool failed = false;
-    for (int l = 0; l < L; l++) {
+#pragma unroll 1
+    for (int l = 0; l < n_links; l++) {
       float* const kp = p.mirror[l] + off;
-      if (!kOneLink && l > 0) {
+      if (!kOneLink) {
 #pragma unroll
         for (int i = 0; i < kPieces; i++) k[i] = live ? load_piece(kp + i * 128) : Piece{0ull, 0ull};
       }
       bool changed = false;
       if (d.flags & (kDescRxLink << l)) {
-        if (!kOneLink && applied != l) {
-          if (d.n_frames == 1) {
-            FrameRegs f{};
-            if (live) load_frame<Q>(frame_at(frames[0]), warp, lane, lb, f);
+        if (!kOneLink) {
 #pragma unroll
-            for (int i = 0; i < kPieces; i++) add4(k[i], frame_steps<Q>(f.w[i], f.code(i), Q == 1 ? valid4(left, i) : 0xfu));
-          } else {
-            Piece acc[kPieces];
-            get_stash(group_stash + in_tile, l, acc);
-#pragma unroll
-            for (int i = 0; i < kPieces; i++) add4(k[i], acc[i]);
-          }
+          for (int i = 0; i < kPieces; i++) add4(k[i], get_part(stash, l, i));
         }
         changed = true;
       }
@@ -746,17 +754,14 @@ __device__ __forceinline__ void compute_warp(const RoundParams& p, GroupShared& 
 #pragma unroll
         for (int i = 0; i < kPieces; i++) {
           xs[i] = maxabs({sub2(v[i].a, k[i].a), sub2(v[i].b, k[i].b)});
-          vs[i] = maxabs(v[i]);
+          if (kOneLink) vs[i] = maxabs(v[i]);
         }
-        auto larger = [](float a, float b) { return fmaxf(a, b); };
-        float xm = reduce_pieces(xs, lane, larger), vm = reduce_pieces(vs, lane, larger);
+        float xm = reduce_pieces(xs, lane, larger), vm = kOneLink ? reduce_pieces(vs, lane, larger) : vmax;
         if (kOneLink || l == 0) res_max0 = fmaxf(res_max0, xm); else if (l == 1) res_max1 = fmaxf(res_max1, xm); else res_max2 = fmaxf(res_max2, xm);
         // blocks of more than 32 elements: over the chunks of a piece row, the piece rows, the warps
         if (lb >= 6) {
-          xm = fmaxf(xm, __shfl_xor_sync(0xffffffffu, xm, 8)); vm = fmaxf(vm, __shfl_xor_sync(0xffffffffu, vm, 8));
-          if (lb >= 7) { xm = fmaxf(xm, __shfl_xor_sync(0xffffffffu, xm, 16)); vm = fmaxf(vm, __shfl_xor_sync(0xffffffffu, vm, 16)); }
-          if (lb >= 8) { xm = fmaxf(xm, __shfl_xor_sync(0xffffffffu, xm, 1)); vm = fmaxf(vm, __shfl_xor_sync(0xffffffffu, vm, 1)); }
-          if (lb >= 9) { xm = fmaxf(xm, __shfl_xor_sync(0xffffffffu, xm, 2)); vm = fmaxf(vm, __shfl_xor_sync(0xffffffffu, vm, 2)); }
+          xm = over_block(xm);
+          if (kOneLink) vm = over_block(vm);
           if (lb >= 10 && live) {
             float2 m = make_float2(-1.f, -1.f);
             if (!failed) m = kOneLink ? exchange_apart(p, sh, exchanges, d.tile, warp, lane, xm, vm) : exchange(p, sh, exchanges, d.tile, warp, lane, xm, vm);
