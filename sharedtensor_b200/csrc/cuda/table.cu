@@ -31,7 +31,9 @@ namespace {
 constexpr int kThreads = 256;
 constexpr uint32_t kChunk = 4096;     // a CTA's step: four 16-byte accesses per thread
 constexpr int64_t kSumRange = 2048;   // the sums: elements of the arena that a CTA takes at least
-constexpr int kSumCtas = 148 * 8;
+constexpr int kSumLoads = 8;          // 16-byte loads of a thread in flight
+constexpr int kSumCtasPerSm = 4;
+constexpr int kSumCtas = 148 * kSumCtasPerSm;
 constexpr int kPtrs = 256;            // tensors of one launch: their addresses travel as kernel parameters
 
 struct Pointers {
@@ -109,11 +111,12 @@ __global__ void __launch_bounds__(kThreads, 8) table_kernel(float* __restrict__ 
 // segment ends: nobody waits for a last wave, and a CTA reduces over its threads once per chunk.  Whoever finishes a
 // segment's last chunk adds the segment's partial sums up in their fixed order, so that the result does not depend on who
 // that is, and writes it to the host.  One launch instead of three.
-__global__ void __launch_bounds__(kThreads, 8) table_sums_kernel(const float* __restrict__ arena, const SumChunk* __restrict__ chunks,
+// Bound by HBM, which likes fewer CTAs with more loads each: 124 M elements are read in 78 us so, in 82 by eight CTAs per SM with
+// four loads each.  Warp 0 sees to a finished chunk while the others have the next one's loads under way.
+__global__ void __launch_bounds__(kThreads, kSumCtasPerSm) table_sums_kernel(const float* __restrict__ arena, const SumChunk* __restrict__ chunks,
                                                                  const uint32_t* __restrict__ first_chunk, const SumSegment* __restrict__ segments, double* __restrict__ partials,
                                                                  uint32_t* __restrict__ counters, double* __restrict__ out, int n_seg) {
-  __shared__ double red[kThreads / 32];
-  __shared__ bool s_last;
+  __shared__ double red[2][kThreads / 32];  // two chunks: the other warps may be one ahead of warp 0
   const bool aligned = (reinterpret_cast<uintptr_t>(arena) & 15) == 0;
   const uint32_t c1 = first_chunk[blockIdx.x + 1];
   for (uint32_t c = first_chunk[blockIdx.x]; c < c1; c++) {
@@ -123,39 +126,35 @@ __global__ void __launch_bounds__(kThreads, 8) table_sums_kernel(const float* __
     if (aligned) {
       const float4* x = reinterpret_cast<const float4*>(arena + ch.begin);  // (segments start on multiples of four)
       const uint32_t n4 = ch.count / 4;
-      uint32_t i = threadIdx.x;
-      for (; i + 3 * kThreads < n4; i += 4 * kThreads) {
-        float4 v[4];
+      for (uint32_t i = threadIdx.x; i < n4; i += kSumLoads * kThreads) {
+        float4 v[kSumLoads];
 #pragma unroll
-        for (int u = 0; u < 4; u++) v[u] = __ldcs(x + i + u * kThreads);
+        for (int u = 0; u < kSumLoads; u++) v[u] = i + u * kThreads < n4 ? __ldcs(x + i + u * kThreads) : make_float4(0.f, 0.f, 0.f, 0.f);
 #pragma unroll
-        for (int u = 0; u < 4; u++) {
+        for (int u = 0; u < kSumLoads; u++) {
           s0 += double(v[u].x) * double(v[u].x) + double(v[u].y) * double(v[u].y);
           s1 += double(v[u].z) * double(v[u].z) + double(v[u].w) * double(v[u].w);
         }
-      }
-      for (; i < n4; i += kThreads) {
-        const float4 v = __ldcs(x + i);
-        s0 += double(v.x) * double(v.x) + double(v.y) * double(v.y);
-        s1 += double(v.z) * double(v.z) + double(v.w) * double(v.w);
       }
       at = n4 * 4;
     }
     for (uint32_t i = at + threadIdx.x; i < ch.count; i += kThreads) s0 += double(arena[ch.begin + i]) * double(arena[ch.begin + i]);
     double acc = s0 + s1;
     for (int o = 16; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
-    if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = acc;
+    double* const mine = red[c & 1u];
+    if ((threadIdx.x & 31) == 0) mine[threadIdx.x >> 5] = acc;
     __syncthreads();
+    if (threadIdx.x >= 32) continue;
     const SumSegment sg = segments[ch.segment];
+    uint32_t last = 0;
     if (threadIdx.x == 0) {
       double t = 0.0;
-      for (int w = 0; w < kThreads / 32; w++) t += red[w];
+      for (int w = 0; w < kThreads / 32; w++) t += mine[w];
       __stcg(partials + c, t);
       __threadfence();
-      s_last = atomicAdd(counters + ch.segment, 1u) == sg.chunks - 1;
+      last = atomicAdd(counters + ch.segment, 1u) == sg.chunks - 1 ? 1u : 0u;
     }
-    __syncthreads();
-    if (s_last && threadIdx.x < 32) {
+    if (__shfl_sync(0xffffffffu, last, 0)) {
       __threadfence();
       double t = 0.0;
       for (uint32_t i = threadIdx.x; i < sg.chunks; i += 32) t += __ldcg(partials + sg.first + i);
@@ -172,7 +171,6 @@ __global__ void __launch_bounds__(kThreads, 8) table_sums_kernel(const float* __
         out[n_seg + ch.segment] = double(e);
       }
     }
-    __syncthreads();  // red and s_last are reused by the next chunk
   }
 }
 
