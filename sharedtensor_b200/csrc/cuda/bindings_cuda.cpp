@@ -27,6 +27,43 @@ static std::vector<uintptr_t> unpack(const py::bytes& b) {  // packed addresses
   std::memcpy(out.data(), v.data(), out.size() * sizeof(uintptr_t));
   return out;
 }
+// The magnitudes of a table as {name: {"sumsq": float, "rms_exp": int}}.  The dicts are made while the kernel runs, and only their
+// values are filled in when it is done: 123 us for the 148 tensors of GPT-2 small, 127 with lists that Python makes them of.
+static py::dict table_magnitudes(TablePlan& t, const py::list& names, uintptr_t arena, uintptr_t s) {
+  const size_t n = names.size();
+  if (int(n) != t.tensors()) throw std::invalid_argument("one name per tensor of the table");
+  const py::str keys[2] = {py::str("sumsq"), py::str("rms_exp")};
+  auto set = [](PyObject* d, PyObject* key, PyObject* value) {
+    if (value == nullptr || PyDict_SetItem(d, key, value) != 0) throw py::error_already_set();
+  };
+  std::unique_lock<std::mutex> lock;
+  {
+    py::gil_scoped_release release;  // (whoever holds the lock may be waiting for the interpreter)
+    lock = t.lock_scales();
+    t.start_scales(ptr<float>(arena), strm(s));
+  }
+  auto finish = [&] {
+    py::gil_scoped_release release;
+    return t.finish_scales(strm(s));
+  };
+  py::dict out;
+  std::vector<py::dict> of(n);
+  try {
+    for (size_t k = 0; k < n; k++) {
+      for (const py::str& key : keys) set(of[k].ptr(), key.ptr(), Py_None);
+      set(out.ptr(), PyList_GET_ITEM(names.ptr(), Py_ssize_t(k)), of[k].ptr());
+    }
+  } catch (...) {
+    finish();  // (the kernel writes what the next one to hold the lock is to use)
+    throw;
+  }
+  const double* const host = finish();
+  for (size_t k = 0; k < n; k++) {
+    set(of[k].ptr(), keys[0].ptr(), py::float_(host[k]).ptr());
+    set(of[k].ptr(), keys[1].ptr(), py::int_(int(host[n + k])).ptr());
+  }
+  return out;
+}
 static void ck(int e, const char* what) {
   if (e != 0) throw std::runtime_error(std::string(what) + ": " + cudaGetErrorString(cudaError_t(e)));
 }
@@ -134,7 +171,7 @@ PYBIND11_MODULE(_cuda, m) {
       .def("bind", [](TablePlan& t, const py::object& device, const py::object& pinned, uintptr_t s) {  // two tensors, kept alive with the plan
         t.bind(ptr<void>(device.attr("data_ptr")().cast<uintptr_t>()), ptr<void>(pinned.attr("data_ptr")().cast<uintptr_t>()), strm(s));
       }, py::keep_alive<1, 2>(), py::keep_alive<1, 3>())
-      .def("scales", [](TablePlan& t, uintptr_t arena, uintptr_t s) { py::gil_scoped_release rel; return t.scales(ptr<float>(arena), strm(s)); });
+      .def("scales", &table_magnitudes);
 
   py::class_<GpuReplica>(m, "GpuReplica")
       .def(py::init<int, int64_t, const GpuConfig&>())

@@ -282,9 +282,8 @@ void TablePlan::copy(const float* arena, const std::vector<uintptr_t>& ptrs, con
   launch_table<false>(const_cast<float*>(arena), ptrs, offsets_, chunks_, first_chunk_, m, stream);
 }
 
-std::pair<std::vector<double>, std::vector<int>> TablePlan::scales(const float* arena, void* stream) {
+void TablePlan::start_scales(const float* arena, void* stream) {
   OnDevice on(device_);
-  std::lock_guard<std::mutex> lk(mu_);
   for (int k = 0; k < n_; k++) {  // (segments without elements)
     host_[k] = 0.0;
     host_[n_ + k] = -128.0;
@@ -293,11 +292,13 @@ std::pair<std::vector<double>, std::vector<int>> TablePlan::scales(const float* 
     table_sums_kernel<<<n_sum_ctas_, kThreads, 0, static_cast<cudaStream_t>(stream)>>>(arena, sum_chunks_, sum_first_, sum_segments_, partials_, counters_,
                                                                                       host_, n_);
     ck(cudaGetLastError(), "kernel launch");
-    ck(cudaStreamSynchronize(static_cast<cudaStream_t>(stream)), "cudaStreamSynchronize");
   }
-  std::vector<int> exps(n_);
-  for (int k = 0; k < n_; k++) exps[k] = int(host_[n_ + k]);
-  return {std::vector<double>(host_, host_ + n_), std::move(exps)};
+}
+
+const double* TablePlan::finish_scales(void* stream) {
+  OnDevice on(device_);
+  if (n_sum_ctas_) ck(cudaStreamSynchronize(static_cast<cudaStream_t>(stream)), "cudaStreamSynchronize");
+  return host_;
 }
 
 }  // namespace st

@@ -4,7 +4,6 @@
 #pragma once
 #include <cstdint>
 #include <mutex>
-#include <utility>
 #include <vector>
 
 #include "round.h"
@@ -28,8 +27,12 @@ class TablePlan {
   // tensors() addresses.
   void add(float* arena, const std::vector<uintptr_t>& ptrs, const UpdateMarks& m, void* stream) const;
   void copy(const float* arena, const std::vector<uintptr_t>& ptrs, const UpdateMarks& m, void* stream) const;
-  // Per segment the sum of squares and floor(log2(rms)) (-128: all zero) of `arena`; waits for the stream.
-  std::pair<std::vector<double>, std::vector<int>> scales(const float* arena, void* stream);
+  // Per segment the sum of squares and floor(log2(rms)) (-128: all zero) of `arena`: starts the kernel that reads them / waits
+  // for the stream and returns the sums, then the exponents.  The lock is held from before the one until what the other
+  // returned has been read.
+  std::unique_lock<std::mutex> lock_scales() { return std::unique_lock<std::mutex>(mu_); }
+  void start_scales(const float* arena, void* stream);
+  const double* finish_scales(void* stream);
 
  private:
   int device_, n_;
@@ -45,7 +48,7 @@ class TablePlan {
   double* partials_ = nullptr;
   uint32_t* counters_ = nullptr;        // chunks of a segment that are done (zero between launches)
   double* host_ = nullptr;              // pinned: sums, then exponents
-  std::mutex mu_;                       // scales() uses partials_, counters_ and host_
+  std::mutex mu_;                       // the magnitudes use partials_, counters_ and host_
 };
 
 }  // namespace st

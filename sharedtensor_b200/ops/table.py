@@ -134,8 +134,7 @@ class SharedTable:
         native = self._native_plan()
         if native is not None and (flat is None or flat.get_device() == self.shared.device.index):
             arena = native[0].values_ptr() if flat is None else flat.data_ptr()
-            sums_l, exps_l = native[1].scales(arena, _stream(self.shared.device))
-            return {k: {"sumsq": s, "rms_exp": e} for k, s, e in zip(self.layout.names, sums_l, exps_l)}
+            return native[1].scales(self.layout.names, arena, _stream(self.shared.device))
         src = flat
         if src is None:
             src = self._flat()
