@@ -40,6 +40,26 @@ struct Pointers {
   float* p[kPtrs];                    // less the tensor's offset, so that an arena element's number finds its tensor element
 };
 
+// Each of these kernels may be launched while the one before it in the stream runs out (which also is cheaper to issue, 2.4
+// instead of 2.9 us), and waits for it before it touches anything that another one writes.
+__device__ __forceinline__ void wait_for_stream() {
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+}
+template <class... P, class... A>
+cudaError_t launch_early(void (*kernel)(P...), int blocks, void* stream, A&&... args) {
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = dim3(blocks);
+  cfg.blockDim = dim3(kThreads);
+  cfg.stream = static_cast<cudaStream_t>(stream);
+  cudaLaunchAttribute early{};
+  early.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  early.val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = &early;
+  cfg.numAttrs = 1;
+  return cudaLaunchKernelEx(&cfg, kernel, P(args)...);
+}
+
 void ck(cudaError_t e, const char* what) {
   if (e != cudaSuccess) throw std::runtime_error(std::string("table of tensors: ") + what + ": " + cudaGetErrorString(e));
 }
@@ -51,6 +71,7 @@ void ck(cudaError_t e, const char* what) {
 template <bool ADD>
 __global__ void __launch_bounds__(kThreads, 8) table_kernel(float* __restrict__ arena, const Chunk* __restrict__ chunks, uint32_t n_chunks,
                                                             uint32_t first_tensor, const __grid_constant__ Pointers ptrs, UpdateMarks m) {
+  wait_for_stream();
   for (uint32_t turn = blockIdx.x; turn < n_chunks; turn += gridDim.x) {
     const Chunk ch = chunks[ADD ? turn : n_chunks - 1 - turn];
     float* const t = ptrs.p[ch.tensor - first_tensor] + ch.arena;
@@ -118,8 +139,9 @@ __global__ void __launch_bounds__(kThreads, kSumCtasPerSm) table_sums_kernel(con
                                                                  uint32_t* __restrict__ counters, double* __restrict__ out, int n_seg) {
   __shared__ double red[2][kThreads / 32];  // two chunks: the other warps may be one ahead of warp 0
   const bool aligned = (reinterpret_cast<uintptr_t>(arena) & 15) == 0;
-  const uint32_t c1 = first_chunk[blockIdx.x + 1];
-  for (uint32_t c = first_chunk[blockIdx.x]; c < c1; c++) {
+  const uint32_t c0 = first_chunk[blockIdx.x], c1 = first_chunk[blockIdx.x + 1];
+  wait_for_stream();
+  for (uint32_t c = c0; c < c1; c++) {
     const SumChunk ch = chunks[c];
     double s0 = 0.0, s1 = 0.0;
     uint32_t at = 0;
@@ -268,9 +290,7 @@ static void launch_table(float* arena, const std::vector<uintptr_t>& ptrs, const
     for (int k = k0; k < k1; k++) p.p[k - k0] = reinterpret_cast<float*>(ptrs[k] - uintptr_t(offsets[k]) * 4);
     const uint32_t c0 = first_chunk[k0], count = first_chunk[k1] - c0;
     if (count == 0 && (!last || m.yield_word == nullptr)) continue;
-    table_kernel<ADD><<<count ? blocks_for(count) : 1, kThreads, 0, static_cast<cudaStream_t>(stream)>>>(arena, chunks + c0, count, uint32_t(k0), p,
-                                                                                                         last ? m : inner);
-    ck(cudaGetLastError(), "kernel launch");
+    ck(launch_early(table_kernel<ADD>, count ? blocks_for(count) : 1, stream, arena, chunks + c0, count, uint32_t(k0), p, last ? m : inner), "kernel launch");
   }
 }
 
@@ -289,9 +309,7 @@ void TablePlan::start_scales(const float* arena, void* stream) {
     host_[n_ + k] = -128.0;
   }
   if (n_sum_ctas_) {
-    table_sums_kernel<<<n_sum_ctas_, kThreads, 0, static_cast<cudaStream_t>(stream)>>>(arena, sum_chunks_, sum_first_, sum_segments_, partials_, counters_,
-                                                                                      host_, n_);
-    ck(cudaGetLastError(), "kernel launch");
+    ck(launch_early(table_sums_kernel, n_sum_ctas_, stream, arena, sum_chunks_, sum_first_, sum_segments_, partials_, counters_, host_, n_), "kernel launch");
   }
 }
 
