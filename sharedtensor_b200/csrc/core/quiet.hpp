@@ -1,5 +1,5 @@
-// What the engine thread tells a flush: how many launches it has looked back on, and the last of them that found work or
-// did not get to look.
+// What the engine thread tells a flush: how many launches it has looked back on, the last of them that found work or did not
+// get to look, and the last that found frames no neighbour had acknowledged.
 #pragma once
 #include <algorithm>
 #include <atomic>
@@ -14,8 +14,9 @@ class QuietWatch {
   void launched() { launched_.fetch_add(1); }
   // `cut_short`: a group left before it had looked at its tiles (an update wanted the SMs, a wait ran out).  That says nothing
   // about them, so the launch does not count as one that found nothing.
-  void looked(bool found_work, bool cut_short, uint64_t now_ns) {
+  void looked(bool found_work, bool cut_short, uint64_t now_ns, bool unacknowledged = false) {
     const uint64_t n = looked_.load() + 1;
+    if (unacknowledged) open_launch_.store(n);
     if (found_work || cut_short) {
       busy_ns_.store(now_ns);
       busy_launch_.store(n);
@@ -31,6 +32,11 @@ class QuietWatch {
     const uint64_t n = looked_.load(), busy = busy_launch_.load();
     return n >= std::max(before, busy) + count;
   }
+  // The last `count` launches found every frame acknowledged.
+  bool acknowledged(uint64_t count) const {
+    const uint64_t n = looked_.load(), open = open_launch_.load();
+    return n >= open + count;
+  }
   // How long no launch has found work, counted from `start_ns` at the earliest.  The engine thread may have found some since
   // the caller took the time.
   uint64_t quiet_for(uint64_t start_ns, uint64_t now_ns) const {
@@ -39,7 +45,7 @@ class QuietWatch {
   }
 
  private:
-  std::atomic<uint64_t> launched_{0}, looked_{0}, busy_launch_{0}, busy_ns_{0};
+  std::atomic<uint64_t> launched_{0}, looked_{0}, busy_launch_{0}, busy_ns_{0}, open_launch_{0};
 };
 
 }  // namespace st

@@ -158,9 +158,10 @@ PYBIND11_MODULE(_cuda, m) {
       .def(py::init<>())
       .def("begin", &QuietWatch::begin)
       .def("launched", &QuietWatch::launched)
-      .def("looked", &QuietWatch::looked)
+      .def("looked", &QuietWatch::looked, py::arg("found_work"), py::arg("cut_short"), py::arg("now_ns"), py::arg("unacknowledged") = false)
       .def("launches", &QuietWatch::launches)
       .def("quiet_launches", &QuietWatch::quiet_launches)
+      .def("acknowledged", &QuietWatch::acknowledged)
       .def("quiet_for", &QuietWatch::quiet_for);
 
   py::class_<TablePlan>(m, "TablePlan")

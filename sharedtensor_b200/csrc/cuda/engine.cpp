@@ -18,10 +18,9 @@ cudaEvent_t E(void* p) { return static_cast<cudaEvent_t>(p); }
 size_t align_up(size_t v, size_t a) { return (v + a - 1) / a * a; }
 
 // Pinned words behind the copy of the status block: what the engine thread reads back per launch in flight (at most four),
-// and the results of two kernels.
+// and the result of a kernel.
 constexpr int64_t kLongestWaitMs = 1000ll * 3600 * 24 * 365;  // (a year, in nanoseconds, is far from the end of 64 bits)
-constexpr int kHostRead = kDsYields - kDsTilesProcessed + 1, kHostUnsend = 4 * kHostRead, kHostUnacknowledged = kHostUnsend + 1,
-              kHostExtraWords = kHostUnacknowledged + 1;
+constexpr int kHostRead = kDsUnacknowledged - kDsTilesProcessed + 1, kHostUnsend = 4 * kHostRead, kHostExtraWords = kHostUnsend + 1;
 
 struct DeviceGuard {
   int prev = -1;
@@ -169,7 +168,6 @@ GpuReplica::~GpuReplica() {
   for (void* e : ev_round_) cudaEventDestroy(E(e));
   for (void* e : ev_kernel_) cudaEventDestroy(E(e));
   if (stat_) cudaStreamDestroy(S(stat_));
-  if (flush_) cudaStreamDestroy(S(flush_));
   if (ev_user_) cudaEventDestroy(E(ev_user_));
   if (ev_comm_) cudaEventDestroy(E(ev_comm_));
   if (comm_) cudaStreamDestroy(S(comm_));
@@ -326,7 +324,6 @@ void GpuReplica::publish_pending() {
   // Ring numbering is about to change.  Every round ends with its publish kernel, so once the
   // stream has drained nothing refers to the old numbering any more.
   cudaStreamSynchronize(S(comm_));
-  if (flush_) cudaStreamSynchronize(S(flush_));  // (a flush counts frames over the old edges)
 }
 
 void GpuReplica::rebuild_params() {
@@ -810,33 +807,11 @@ void GpuReplica::idle_pause(uint64_t us) {
   wake_pending_ = false;
 }
 
-// Frames (per tile and ring) that no neighbour has acknowledged yet.
-uint32_t GpuReplica::unacknowledged() {
-  uint32_t* const count = reinterpret_cast<uint32_t*>(status_host_ + kDsTotalWords + kHostUnacknowledged);
-  {
-    // The engine thread needs the mutex for the pass that takes the acknowledgements in: it is held for the launch only.
-    // (An edge is not taken down while the kernel looks at it, see publish_pending.)
-    std::lock_guard<std::mutex> lk(mu_);
-    if (!flush_) {
-      cudaStream_t st;
-      check(cudaStreamCreateWithFlags(&st, cudaStreamNonBlocking), "cudaStreamCreate");
-      flush_ = st;
-    }
-    *count = 0;
-    check(launch_count_unacknowledged(params_, count, flush_), "count_unacknowledged kernel");
-  }
-  const cudaError_t e = cudaStreamSynchronize(S(flush_));
-  if (e != cudaSuccess) {
-    std::lock_guard<std::mutex> lk(mu_);
-    check(e, "cudaStreamSynchronize");
-  }
-  return *reinterpret_cast<volatile uint32_t*>(count);
-}
-
 // Three passes of the engine thread in a row, begun after the caller's updates have run, that get to look at all tiles and
 // find nothing to do; for as long as a neighbour may need to take in what it was sent and answer it (two busy passes at HBM
-// rate) no pass that did; and every frame acknowledged (a neighbour may be gone, or have no engine running: after a tenth of
-// a second of quiet the frames count as delivered, they are in its memory).
+// rate) no pass that did; and every frame acknowledged, as the passes themselves find when they look at the tiles (a kernel of
+// its own that counted, and the wait for it, kept a pair of 1 Mi elements 10 us longer a flush).  A neighbour may be gone, or
+// have no engine running: after a tenth of a second of quiet the frames count as delivered, they are in its memory.
 bool GpuReplica::flush(void* user_stream, int64_t timeout_ms) {
   DeviceGuard g(device_);
   // The limit covers the wait for another thread's flush and for the caller's stream too.
@@ -853,20 +828,13 @@ bool GpuReplica::flush(void* user_stream, int64_t timeout_ms) {
   }
   const uint64_t start = steady_ns();
   const uint64_t quiet_ns = 100000ull + uint64_t(n_padded_) * 2 * 18 / 6000;   // 18 bytes an element and pass, 6000 bytes a ns
-  const uint64_t before = watch_.launches(), passes = 3ull * uint64_t(n_windows());
-  uint64_t woken = 0, asked_at = 0, pause_ns = 20000;
+  const uint64_t before = watch_.launches(), windows = uint64_t(n_windows()), passes = 3 * windows;
+  // the launches of one pass, and as many more as may be in flight with its first: what that one counts may be read with theirs
+  const uint64_t pass = windows + ev_round_.size() - 1;
+  uint64_t woken = 0;
   while (engine_on_.load()) {
     const uint64_t now = steady_ns(), quiet = watch_.quiet_for(start, now);
-    if (quiet >= quiet_ns && watch_.quiet_launches(before, passes)) {
-      bool arrived = quiet >= quiet_ns + 100000000ull;
-      if (!arrived && now - asked_at >= pause_ns) {
-        // (asked less and less often: a neighbour that takes its time is not to be slowed down by the question)
-        arrived = unacknowledged() == 0;
-        asked_at = steady_ns();
-        pause_ns = pause_ns < 640000 ? pause_ns * 2 : pause_ns;
-      }
-      if (arrived && watch_.quiet_launches(before, passes)) return true;  // (still so)
-    }
+    if (quiet >= quiet_ns && watch_.quiet_launches(before, passes) && (quiet >= quiet_ns + 100000000ull || watch_.acknowledged(pass))) return true;
     if (ring_peers_.load() == 0) return true;  // the last neighbour has gone
     if (now - entered > limit) break;
     if (woken == 0 || now - woken > 2000000ull) {
@@ -885,12 +853,12 @@ void GpuReplica::engine_loop() {
   cudaSetDevice(device_);
   ::prctl(PR_SET_TIMERSLACK, 1000UL, 0, 0, 0);  // 1 us instead of the default 50 us: the idle pauses start at 10 us
   const size_t depth = ev_round_.size();
-  // A few pinned words per launch in flight: tiles handled, groups that left early, and waits that ran out so far, read once
-  // that launch has finished.  The read runs on a stream of its own behind an event, so that the comm stream goes from one
+  // A few pinned words per launch in flight: tiles handled, groups that left early, waits that ran out and frames found without
+  // an acknowledgement so far, read once that launch has finished.  The read runs on a stream of its own behind an event, so that the comm stream goes from one
   // launch straight to the next; a later launch may already have added to the counts by then, which only moves work from
   // one difference to the one before it.
   uint64_t* work_host = status_host_ + kDsTotalWords;  // behind the part status() uses
-  uint64_t work_seen = 0, cut_seen = 0;
+  uint64_t work_seen = 0, cut_seen = 0, open_seen = 0;
   uint64_t r = 0;
   watch_.begin();
   uint64_t idle_rounds = 0;
@@ -927,8 +895,10 @@ void GpuReplica::engine_loop() {
       const uint64_t now = words[0], cut = words[kDsYields - kDsTilesProcessed] + words[kDsWaitTimeouts - kDsTilesProcessed];
       work = now > work_seen ? now - work_seen : 0;
       work_seen = now > work_seen ? now : work_seen;
-      watch_.looked(work != 0, cut != cut_seen, steady_ns());  // what flush() watches
+      const uint64_t open = words[kDsUnacknowledged - kDsTilesProcessed];
+      watch_.looked(work != 0, cut != cut_seen, steady_ns(), open != open_seen);  // what flush() watches
       cut_seen = cut;
+      open_seen = open;
     }
     if (work != 0) epoch_++;
     quiet_launches = work == 0 ? quiet_launches + 1 : 0;

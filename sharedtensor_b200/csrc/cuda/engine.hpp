@@ -176,7 +176,6 @@ class GpuReplica {
   void fill_guards(const VmmBlock& b, size_t used_bytes);
   UpdateMarks ask_for_sms(void* user_stream, bool marks);
   void updated();
-  uint32_t unacknowledged();
   void check(int cuda_err, const char* what);
   void engine_loop();
   void order_after_user(void* user_stream);
@@ -218,7 +217,6 @@ class GpuReplica {
   std::vector<void*> ev_round_;       // per launch in flight: its work count has been read back
   std::vector<void*> ev_kernel_;      // per launch in flight: the kernel has finished (comm stream)
   void* stat_ = nullptr;               // cudaStream_t: reads work counts back beside the comm stream, so that launches follow each other without a copy in between
-  void* flush_ = nullptr;              // cudaStream_t: flush() counts unacknowledged frames beside the rounds (made on first use)
   std::timed_mutex flush_mu_;          // one flush at a time; taken before mu_
   mutable std::mutex mu_;
   std::mutex gate_mu_;                 // taken before mu_ by every update from outside the rounds

@@ -862,6 +862,7 @@ __device__ __forceinline__ void service_warp(const RoundParams& p, GroupShared& 
 
   bool handed_on = false;   // the next window's launch has been let in
   uint32_t n_done = 0, n_tx = 0, n_rx = 0, n_blocked = 0, n_pending = 0, n_sweeps = 0;  // per lane, added up at the end
+  bool open = false;        // this lane has found frames that have not been acknowledged
   uint32_t armed = 0, finished = 0, published = 0;  // tiles armed, finished by the compute warps, published so far
   uint32_t handed = 0, staged = 0;                  // tiles the compute warps may start, and those of them whose frames have been seen to
   uint32_t stage_no = 0, stage_issued = 0;          // tiles with two frames or more found so far, and those staged
@@ -956,6 +957,7 @@ __device__ __forceinline__ void service_warp(const RoundParams& p, GroupShared& 
           }
         }
         if (looked == at_once && sweep == 0) begin_launch();
+        open |= tx != credit;  // (the flush() of a replica asks the passes whether its frames have been taken in)
         const bool room = is_out && (tx - credit) < uint32_t(p.ring_slots);
         // (a leaf's lane has its tile to itself)
         uint32_t in1 = avail >= 1 ? same_tile : 0u, in2 = avail >= 2 ? same_tile : 0u, in3 = avail >= 3 ? same_tile : 0u;
@@ -1156,6 +1158,7 @@ __device__ __forceinline__ void service_warp(const RoundParams& p, GroupShared& 
   n_rx = __reduce_add_sync(0xffffffffu, n_rx);
   n_blocked = __reduce_add_sync(0xffffffffu, n_blocked);
   n_pending = __reduce_add_sync(0xffffffffu, n_pending);
+  open = __any_sync(0xffffffffu, open);
   if (lane == 0) {
     ST_CRUMB(g, 10);
     auto count = [&](uint64_t* w, unsigned long long by) {
@@ -1166,6 +1169,7 @@ __device__ __forceinline__ void service_warp(const RoundParams& p, GroupShared& 
     count(p.status + kDsFramesSent, n_tx);
     count(p.status + kDsFramesRecv, n_rx);
     count(p.status + kDsBlockedNoCredit, n_blocked);
+    count(p.status + kDsUnacknowledged, open ? 1 : 0);
     count(launch_words + kDlWork, n_done);
     count(launch_words + kDlPending, n_pending);
     if (blockIdx.x == 0 && g == 0) {
@@ -1259,19 +1263,6 @@ int launch_unsend(float* mirror, const uint8_t* payload_remote, uint32_t* tx_seq
     case 8: unsend_kernel<8><<<n_tiles, kComputeWarps * 32, 0, s>>>(mirror, payload_remote, tx_seq, credit, n_tiles, ring_slots, payload_bytes, log2_block, n, tb); break;
     default: return int(cudaErrorInvalidValue);
   }
-  return int(cudaGetLastError());
-}
-
-__global__ void __launch_bounds__(256) unacknowledged_kernel(const __grid_constant__ RoundParams p, uint32_t* __restrict__ count) {
-  uint32_t n = 0;
-  for (int tile = blockIdx.x * 256 + threadIdx.x; tile < p.n_tiles; tile += gridDim.x * 256)
-    for (int r = 0; r < p.n_out; r++) n += ld_cg_u32(p.out[r].tx_seq + tile) - ld_relaxed_sys(p.out[r].credit + tile);
-  n = __reduce_add_sync(0xffffffffu, n);
-  if ((threadIdx.x & 31) == 0 && n) atomicAdd_system(count, n);
-}
-int launch_count_unacknowledged(const RoundParams& p, uint32_t* count, void* stream) {
-  const int blocks = (p.n_tiles + 255) / 256;
-  unacknowledged_kernel<<<blocks < 32 ? blocks : 32, 256, 0, static_cast<cudaStream_t>(stream)>>>(p, count);
   return int(cudaGetLastError());
 }
 

@@ -99,9 +99,10 @@ enum DevStatus : int {
   kDsErrors,           // bit mask, see kErr*
   kDsWaitTimeouts,
   kDsYields,           // groups that left early because an update was waiting
-  kDsLaunch0 = 8,      // per-launch words of parity 0: work, pending tiles, residual maxima of links 0..2 (fp32 bits)
-  kDsLaunch1 = 16,     // ... of parity 1
-  kDsTrace = 24,       // ring of kTraceEntries records {globaltimer ns, round, tiles handled by group 0, frames sent so far}
+  kDsUnacknowledged,   // groups that found frames their receivers had not acknowledged
+  kDsLaunch0,          // per-launch words of parity 0: work, pending tiles, residual maxima of links 0..2 (fp32 bits)
+  kDsLaunch1 = kDsLaunch0 + 8,  // ... of parity 1
+  kDsTrace = kDsLaunch1 + 8,    // ring of kTraceEntries records {globaltimer ns, round, tiles handled by group 0, frames sent so far}
   kTraceEntries = 64,
   kTraceWords = 4,
   kDsTotalWords = kDsTrace + kTraceEntries * kTraceWords
@@ -139,8 +140,6 @@ int load_round(const RoundParams& p);
 // link's mirror and the ring's send counters fall back to the credits.  *taken_back (device) counts the tile-frames.
 int launch_unsend(float* mirror, const uint8_t* payload_remote, uint32_t* tx_seq, const uint32_t* credit, int n_tiles, int ring_slots,
                   int payload_bytes, int log2_block, int bits, int64_t n, uint64_t* taken_back, void* stream);
-// Adds to *count (pinned host memory) the frames that have been sent and not yet acknowledged, over all rings and tiles.
-int launch_count_unacknowledged(const RoundParams& p, uint32_t* count, void* stream);
 
 // Element-wise kernels (copyToTensor / addFromTensor / pushUpdate; src/sharedtensor.c:435-446, 334-344).
 // What an update or a snapshot does besides its data; null pointers: nothing.
