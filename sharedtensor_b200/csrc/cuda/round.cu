@@ -1,6 +1,6 @@
 // The sync-round kernel for sm_100a (see round.h for the protocol and ../core/codec.hpp for the arithmetic).
 //
-// A CTA holds up to three independent groups; a group is eight compute warps and one service warp and owns every n-th
+// A CTA holds two independent groups; a group is eight compute warps and one service warp and owns every n-th
 // tile of the tensor.  The two kinds of warp talk through a few words of shared memory:
 //
 //   service warp  looks at several of the group's tiles at once, a lane per tile and ring: change mark, sequence flags of the
@@ -657,9 +657,9 @@ __device__ __forceinline__ void compute_warp(const RoundParams& p, GroupShared& 
     if (!kOneLink) {
       // What arrived, then the values into it.  Nothing is held in registers beyond that and the mirror of the link in hand, and
       // the values' maxima are taken once for all links: the kernel spills nothing, and a hub with two leaves takes 638 us for
-      // its rounds over 30 M elements instead of 657.  (More would not help: with 72 registers and three groups, or the next
-      // link's mirror loaded ahead into registers, the warps wait for memory longer instead, 545 and 505 us against 502 for a hub
-      // and three leaves over 16 M.  The L2 serves some 10 TB/s at that point.)
+      // its rounds over 30 M elements instead of 657.  (More would not help: with 72 registers and three groups the warps
+      // wait for memory longer instead, 524 us against 511 for a hub and three leaves over 16 M, and the next link's mirror loaded
+      // ahead into registers gives 505 against 502.  The L2 serves some 10 TB/s at that point.)
       prefetch_next();
       decode_frames<Q, true, 0>(frames, nullptr, false, d.n_frames, live, nullptr, lb, warp, lane, left, stash, v);
 #pragma unroll
