@@ -20,7 +20,7 @@
 //
 // What bounds it.  Large tensors: HBM; a visit moves 12 to 18 bytes of values, mirror and frames per element.  Two groups
 // keep 64 KB of loads in flight per SM and the next tile is on its way into the L2 meanwhile.  100 M elements on one link,
-// each pass by itself with a wait for the GPU on both sides: 0.231 ms to send, 0.327 ms to receive and send, 0.305 ms to
+// each pass by itself with a wait for the GPU on both sides: 0.223 ms to send, 0.319 ms to receive and send, 0.299 ms to
 // receive (0.324, 0.439 and 0.426 ms with tiles staged in shared memory by bulk copies for two groups of four warps, four
 // windows instead of three and no overlap between them).
 // Small tensors: latency.  A launch over one tile takes 6 us in the kernel, of which the look at the tile takes 2.3 and the
@@ -634,7 +634,8 @@ __device__ __forceinline__ void compute_warp(const RoundParams& p, GroupShared& 
       c++;
     }
     // The next tile on its way into the L2, once this one's loads are under way (ahead of them, a mesh of eight takes 643 us
-    // instead of 620, three sign rounds of 3.3 M elements 51 instead of 49).  One tile ahead is best: a window of 25 M elements
+    // instead of 620, three sign rounds of 3.3 M elements 51 instead of 49), but ahead of them in a visit that only sends and
+    // has little else to wait for: 100 M elements are sent in 223 us so, in 241 the other way round.  One tile ahead is best: a window of 25 M elements
     // that receives and sends takes 92 us so, 115 us with two tiles ahead and 153 us with four; without, three rounds of 100 M
     // elements on one link take 1278 us instead of 1157.
     auto prefetch_next = [&]() {
@@ -671,12 +672,13 @@ __device__ __forceinline__ void compute_warp(const RoundParams& p, GroupShared& 
       }
     } else if (d.n_frames <= 1) {
       // the common case: everything is fetched at once, and the one frame's steps never have to be kept
+      if (d.n_frames == 0) prefetch_next();
 #pragma unroll
       for (int i = 0; i < kPieces; i++) v[i] = load_v ? load_piece(vp + i * 128) : Piece{0ull, 0ull};
 #pragma unroll
       for (int i = 0; i < kPieces; i++) k[i] = live ? load_piece(p.mirror[0] + off + i * 128) : Piece{0ull, 0ull};
-      prefetch_next();
       if (d.n_frames == 1) {
+        prefetch_next();
         FrameRegs f{};
         if (live) load_frame<Q>(frame_at(frames[0]), warp, lane, lb, f);
 #pragma unroll
