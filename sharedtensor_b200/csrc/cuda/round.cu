@@ -20,7 +20,7 @@
 //
 // What bounds it.  Large tensors: HBM; a visit moves 12 to 18 bytes of values, mirror and frames per element.  Two groups
 // keep 64 KB of loads in flight per SM and the next tile is on its way into the L2 meanwhile.  100 M elements on one link,
-// each pass by itself with a wait for the GPU on both sides: 0.223 ms to send, 0.319 ms to receive and send, 0.299 ms to
+// each pass by itself with a wait for the GPU on both sides: 0.216 ms to send, 0.315 ms to receive and send, 0.295 ms to
 // receive (0.324, 0.439 and 0.426 ms with tiles staged in shared memory by bulk copies for two groups of four warps, four
 // windows instead of three and no overlap between them).
 // Small tensors: latency.  A launch over one tile takes 6 us in the kernel, of which the look at the tile takes 2.3 and the
@@ -500,6 +500,12 @@ template <int Q>
 constexpr int kFrameRoom = Q * 512 + 128;
 template <int kKind>
 constexpr int kStaged = kKind == kMember ? 8 : 0;
+// Who asks the L2 for the lines of the next tile: the service warp, a lane per array, or a compute warp, whose own part of the
+// tile in hand waits meanwhile.  With the service warp three rounds of 100 M elements on one link take 1144 us instead of 1159, a
+// hub and two leaves over 30 M 632 instead of 644 (the pass of a hub with three links over 32 Mi alone 248 instead of 305).  A mesh member's service warp has copies to see to (mesh of eight: 603
+// instead of 601), and in the shorter visits of sign frames it comes late (3.3 M elements: 50.9 instead of 49.9).
+template <int Q, int kKind>
+constexpr bool kServiceAhead = kKind != kMember && Q > 1;
 
 // total = the sum of the steps of the tile's frames, in list order; kStash: what came on each link is summed up besides, and
 // left in this lane's part of the link's stash (shared memory; a frame is decoded once, however many links hear of it: a hub
@@ -633,14 +639,14 @@ __device__ __forceinline__ void compute_warp(const RoundParams& p, GroupShared& 
       d = sh.desc[entry];
       c++;
     }
-    // The next tile on its way into the L2, once this one's loads are under way (ahead of them, a mesh of eight takes 643 us
-    // instead of 620, three sign rounds of 3.3 M elements 51 instead of 49), but ahead of them in a visit that only sends and
-    // has little else to wait for: 100 M elements are sent in 223 us so, in 241 the other way round.  One tile ahead is best: a window of 25 M elements
-    // that receives and sends takes 92 us so, 115 us with two tiles ahead and 153 us with four; without, three rounds of 100 M
-    // elements on one link take 1278 us instead of 1157.
+    // Where the service warp does not do it: the next tile on its way into the L2, once this one's loads are under way (ahead of
+    // them, a mesh of eight takes 643 us instead of 620, three sign rounds of 3.3 M elements 51 instead of 49), but ahead of them
+    // in a visit that only sends and has little else to wait for.  One tile ahead is best: a window of 25 M elements that receives
+    // and sends takes 92 us so, 115 us with two tiles ahead and 153 us with four; without, three rounds of 100 M elements on one
+    // link take 1278 us instead of 1157.
     auto prefetch_next = [&]() {
       const uint32_t ahead = c;  // (c is the next tile's number by now)
-      if (!live || warp != 0 || lane != 0 || int32_t(ld_shared_acquire(&sh.armed) - ahead) <= 0) return;
+      if (kServiceAhead<Q, kKind> || !live || warp != 0 || lane != 0 || int32_t(ld_shared_acquire(&sh.armed) - ahead) <= 0) return;
       const TileDesc& e = sh.desc[ahead % kBank];
       if (!(e.flags & kDescNoValues)) bulk_prefetch_l2(p.values + size_t(e.tile) * kTile, kTile * 4);
       for (int l = 0; l < L; l++) bulk_prefetch_l2(p.mirror[l] + size_t(e.tile) * kTile, kTile * 4);
@@ -833,7 +839,7 @@ __device__ __forceinline__ void compute_warp(const RoundParams& p, GroupShared& 
 // one warp's instructions.  It is compiled for each kind of replica, so that a leaf has no loops over links and rings and no
 // ballots among its lanes, and divides nothing and reads no clock on that way: the first tile of a launch is armed after 2.1 us
 // instead of 3.1 (a member's after 2.9 instead of 3.8), and three rounds over 811 tiles of sign frames take 49 us instead of 54.
-template <int kKind>
+template <int Q, int kKind>
 __device__ __forceinline__ void service_warp(const RoundParams& p, GroupShared& sh, uint8_t* stages, int staged_frames, int frame_room, int g, int n_groups, int lane) {
   // The group's tiles: a run of `chunk` consecutive tiles, or (chunk == 0) every gstride-th tile of the launch's window.
   // The groups of a CTA are a grid apart, so that the odd tiles of the last turn fall on all SMs alike.
@@ -868,6 +874,7 @@ __device__ __forceinline__ void service_warp(const RoundParams& p, GroupShared& 
   uint32_t armed = 0, finished = 0, published = 0;  // tiles armed, finished by the compute warps, published so far
   uint32_t handed = 0, staged = 0;                  // tiles the compute warps may start, and those of them whose frames have been seen to
   uint32_t stage_no = 0, stage_issued = 0;          // tiles with two frames or more found so far, and those staged
+  uint32_t ahead = 0;                               // the last tile whose lines have been asked for ahead of time
   bool aborted = false, yielded = false;
   bool ran_out = false;                             // a wait of a compute warp did
 
@@ -1048,6 +1055,16 @@ __device__ __forceinline__ void service_warp(const RoundParams& p, GroupShared& 
         idle = 0;
         continue;
       }
+      // ---- the next tile on its way into the L2, once the compute warps have started on the one before it
+      if (kServiceAhead<Q, kKind> && int32_t(handed - finished) > 1 && ahead != finished + 1u &&
+          (*reinterpret_cast<volatile uint32_t*>(&sh.claim) & ~kStop) > finished) {
+        ahead = finished + 1u;
+        const TileDesc e = sh.desc[ahead % kBank];
+        if (lane == 0 && !(e.flags & kDescNoValues)) bulk_prefetch_l2(p.values + size_t(e.tile) * kTile, kTile * 4);
+        if (lane >= 1 && lane <= n_links) bulk_prefetch_l2(p.mirror[lane - 1] + size_t(e.tile) * kTile, kTile * 4);
+        if (lane >= 8 && lane - 8 < int(e.n_frames)) bulk_prefetch_l2(frame_at(sh.frames[ahead % kBank][lane - 8]), uint32_t(p.payload_bytes));
+        __syncwarp();
+      }
       // ---- the next window's launch may move in on SMs that run dry: its tiles are others than this launch's
       if (!handed_on && looked >= my_count && armed - finished <= 2u) {
         asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
@@ -1212,7 +1229,7 @@ __global__ void __launch_bounds__(kRoundGroups * kGroupThreads, 1) round_kernel(
   __syncthreads();  // the only CTA-wide barrier: from here on the groups, and the two kinds of warp, run on their own
   uint8_t* const stages = dynamic + g * kStageBytes;
   float* const stash = reinterpret_cast<float*>(dynamic + kRoundGroups * kStageBytes) + (kKind == kInner ? g * kMaxLinks * kTile : 0);
-  if (warp == kComputeWarps) service_warp<kKind>(p, shared[g], stages, kIn, kFrameRoom<Q>, g, kRoundGroups, lane);
+  if (warp == kComputeWarps) service_warp<Q, kKind>(p, shared[g], stages, kIn, kFrameRoom<Q>, g, kRoundGroups, lane);
   else compute_warp<Q, kKind>(p, shared[g], stash, stages, warp, lane);
 }
 
