@@ -1056,14 +1056,15 @@ __device__ __forceinline__ void service_warp(const RoundParams& p, GroupShared& 
         continue;
       }
       // ---- the next tile on its way into the L2, once the compute warps have started on the one before it
-      if (kServiceAhead<Q, kKind> && int32_t(handed - finished) > 1 && ahead != finished + 1u &&
-          (*reinterpret_cast<volatile uint32_t*>(&sh.claim) & ~kStop) > finished) {
-        ahead = finished + 1u;
-        const TileDesc e = sh.desc[ahead % kBank];
-        if (lane == 0 && !(e.flags & kDescNoValues)) bulk_prefetch_l2(p.values + size_t(e.tile) * kTile, kTile * 4);
-        if (lane >= 1 && lane <= n_links) bulk_prefetch_l2(p.mirror[lane - 1] + size_t(e.tile) * kTile, kTile * 4);
-        if (lane >= 8 && lane - 8 < int(e.n_frames)) bulk_prefetch_l2(frame_at(sh.frames[ahead % kBank][lane - 8]), uint32_t(p.payload_bytes));
-        __syncwarp();
+      if (kServiceAhead<Q, kKind> && int32_t(handed - finished) > 1 && ahead != finished + 1u) {
+        const uint32_t begun = lane == 0 ? *reinterpret_cast<volatile uint32_t*>(&sh.claim) & ~kStop : 0u;
+        if (__shfl_sync(0xffffffffu, begun, 0) > finished) {
+          ahead = finished + 1u;
+          const TileDesc e = sh.desc[ahead % kBank];
+          if (lane == 0 && !(e.flags & kDescNoValues)) bulk_prefetch_l2(p.values + size_t(e.tile) * kTile, kTile * 4);
+          if (lane >= 1 && lane <= n_links) bulk_prefetch_l2(p.mirror[lane - 1] + size_t(e.tile) * kTile, kTile * 4);
+          if (lane >= 8 && lane - 8 < int(e.n_frames)) bulk_prefetch_l2(frame_at(sh.frames[ahead % kBank][lane - 8]), uint32_t(p.payload_bytes));
+        }
       }
       // ---- the next window's launch may move in on SMs that run dry: its tiles are others than this launch's
       if (!handed_on && looked >= my_count && armed - finished <= 2u) {
