@@ -175,9 +175,10 @@ __global__ void __launch_bounds__(kThreads, kSumCtasPerSm) table_sums_kernel(con
       __stcg(partials + c, t);
       __threadfence();
       last = atomicAdd(counters + ch.segment, 1u) == sg.chunks - 1 ? 1u : 0u;
+      if (last) __threadfence();  // the other chunks' partial sums come with the count that says they are there ...
     }
     if (__shfl_sync(0xffffffffu, last, 0)) {
-      __threadfence();
+      __syncwarp();               // ... for the whole warp: a shuffle orders no memory
       double t = 0.0;
       for (uint32_t i = threadIdx.x; i < sg.chunks; i += 32) t += __ldcg(partials + sg.first + i);
       for (int o = 16; o > 0; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);

@@ -40,3 +40,12 @@ def test_the_service_warp_takes_no_branch_on_what_each_lane_has_read_for_itself(
     assert len(found) > 20
     for c in found:
         assert not reads.search(c) or "lane == 0" in c, c
+
+
+def test_what_one_lane_knows_to_be_there_is_ordered_for_the_warp_that_reads_it():
+    """Table magnitudes: lane 0 counts a chunk and learns that it was the last one, then all lanes read what other CTAs have
+    written.  A shuffle orders no memory: lane 0's fence behind the count and a warp barrier behind the shuffle do."""
+    body = _body(_code("table.cu"), "table_sums_kernel")
+    count, told, read = body.index("atomicAdd(counters"), body.index("__shfl_sync(0xffffffffu, last, 0)"), body.index("__ldcg(partials")
+    assert count < told < read
+    assert "__threadfence()" in body[count:told] and "__syncwarp()" in body[told:read]
