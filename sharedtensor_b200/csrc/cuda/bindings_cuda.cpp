@@ -5,6 +5,7 @@
 
 #include <cuda_runtime_api.h>
 
+#include <algorithm>
 #include <cstring>
 #include <string_view>
 
@@ -29,9 +30,9 @@ static std::vector<uintptr_t> unpack(const py::bytes& b) {  // packed addresses
 }
 // The magnitudes of a table as {name: {"sumsq": float, "rms_exp": int}}.  The dicts are made while the kernel runs, and only their
 // values are filled in when it is done: 123 us for the 148 tensors of GPT-2 small, 127 with lists that Python makes them of.
-static py::dict table_magnitudes(TablePlan& t, const py::list& names, uintptr_t arena, uintptr_t s) {
-  const size_t n = names.size();
-  if (int(n) != t.tensors()) throw std::invalid_argument("one name per tensor of the table");
+static py::dict table_magnitudes(TablePlan& t, const py::object& sequence, uintptr_t arena, uintptr_t s) {
+  const py::tuple names(sequence);  // as they are now: the interpreter is let go below, and the sequence is the caller's to change
+  const size_t tensors = size_t(t.tensors()), n = std::min(names.size(), tensors);
   const py::str keys[2] = {py::str("sumsq"), py::str("rms_exp")};
   auto set = [](PyObject* d, PyObject* key, PyObject* value) {
     if (value == nullptr || PyDict_SetItem(d, key, value) != 0) throw py::error_already_set();
@@ -51,7 +52,7 @@ static py::dict table_magnitudes(TablePlan& t, const py::list& names, uintptr_t 
   try {
     for (size_t k = 0; k < n; k++) {
       for (const py::str& key : keys) set(of[k].ptr(), key.ptr(), Py_None);
-      set(out.ptr(), PyList_GET_ITEM(names.ptr(), Py_ssize_t(k)), of[k].ptr());
+      set(out.ptr(), PyTuple_GET_ITEM(names.ptr(), Py_ssize_t(k)), of[k].ptr());
     }
   } catch (...) {
     finish();  // (the kernel writes what the next one to hold the lock is to use)
@@ -60,7 +61,7 @@ static py::dict table_magnitudes(TablePlan& t, const py::list& names, uintptr_t 
   const double* const host = finish();
   for (size_t k = 0; k < n; k++) {
     set(of[k].ptr(), keys[0].ptr(), py::float_(host[k]).ptr());
-    set(of[k].ptr(), keys[1].ptr(), py::int_(int(host[n + k])).ptr());
+    set(of[k].ptr(), keys[1].ptr(), py::int_(int(host[tensors + k])).ptr());
   }
   return out;
 }

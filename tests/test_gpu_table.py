@@ -1,10 +1,13 @@
 """The kernels over a table of tensors against PyTorch."""
 import math
+import threading
+import time
 
 import pytest
 import torch
 
 import sharedtensor
+from sharedtensor_b200 import _native
 
 pytestmark = pytest.mark.gpu
 
@@ -151,3 +154,33 @@ def test_every_push_reaches_the_other_replica(free_port):
     finally:
         b.close()
         a.close()
+
+
+def test_magnitudes_go_by_the_names_of_the_call(free_port):
+    """Another thread may change the names while the call waits for its turn, and any sequence of names will do."""
+    init = _table([100, 5000, 3])
+    tab = sharedtensor.createOrFetchTable("127.0.0.1", free_port, init)
+    try:
+        want, got = tab.scales(), []
+        busy = torch.cuda.Stream()
+
+        def read_behind(ns):
+            with torch.cuda.stream(busy):
+                if ns:
+                    _native.cuda().delay(ns, busy.cuda_stream)
+                got.append(tab.scales())
+
+        threads = [threading.Thread(target=read_behind, args=(ns,)) for ns in (1_000_000_000, 0)]
+        for t in threads:
+            t.start()
+            time.sleep(0.2)
+        tab.layout.names[0] = "another"
+        for t in threads:
+            t.join()
+        assert got == [want, want]
+        tab.layout.names = tuple(init)
+        assert tab.scales() == want
+        tab.layout.names = list(init)[:2]
+        assert tab.scales() == {k: want[k] for k in list(init)[:2]}
+    finally:
+        tab.close()
