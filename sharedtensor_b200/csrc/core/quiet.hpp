@@ -37,6 +37,13 @@ class QuietWatch {
     const uint64_t n = looked_.load(), open = open_launch_.load();
     return n >= open + count;
   }
+  // Three passes (of `windows` launches each), all begun after launch number `before`, count nothing to do, and the last one no
+  // frame without an acknowledgement (unless nobody is waited for: `alone`).  What a launch counts may be read along with the
+  // counts of up to `ahead` launches before it, as many as may be in flight behind a launch whose counts are read: so that the
+  // last pass has surely looked at all tiles and found nothing, nothing may have been counted in those either.
+  bool settled(uint64_t before, uint64_t windows, uint64_t ahead, bool alone) const {
+    return quiet_launches(before, std::max(3 * windows, windows + ahead)) && (alone || acknowledged(windows + ahead));
+  }
   // How long no launch has found work, counted from `start_ns` at the earliest.  The engine thread may have found some since
   // the caller took the time.
   uint64_t quiet_for(uint64_t start_ns, uint64_t now_ns) const {

@@ -163,6 +163,7 @@ PYBIND11_MODULE(_cuda, m) {
       .def("launches", &QuietWatch::launches)
       .def("quiet_launches", &QuietWatch::quiet_launches)
       .def("acknowledged", &QuietWatch::acknowledged)
+      .def("settled", &QuietWatch::settled)
       .def("quiet_for", &QuietWatch::quiet_for);
 
   py::class_<TablePlan>(m, "TablePlan")

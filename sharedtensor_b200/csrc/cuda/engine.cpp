@@ -828,13 +828,11 @@ bool GpuReplica::flush(void* user_stream, int64_t timeout_ms) {
   }
   const uint64_t start = steady_ns();
   const uint64_t quiet_ns = 100000ull + uint64_t(n_padded_) * 2 * 18 / 6000;   // 18 bytes an element and pass, 6000 bytes a ns
-  const uint64_t before = watch_.launches(), windows = uint64_t(n_windows()), passes = 3 * windows;
-  // the launches of one pass, and as many more as may be in flight with its first: what that one counts may be read with theirs
-  const uint64_t pass = windows + ev_round_.size() - 1;
+  const uint64_t before = watch_.launches(), windows = uint64_t(n_windows()), ahead = ev_round_.size() - 1;
   uint64_t woken = 0;
   while (engine_on_.load()) {
     const uint64_t now = steady_ns(), quiet = watch_.quiet_for(start, now);
-    if (quiet >= quiet_ns && watch_.quiet_launches(before, passes) && (quiet >= quiet_ns + 100000000ull || watch_.acknowledged(pass))) return true;
+    if (quiet >= quiet_ns && watch_.settled(before, windows, ahead, quiet >= quiet_ns + 100000000ull)) return true;
     if (ring_peers_.load() == 0) return true;  // the last neighbour has gone
     if (now - entered > limit) break;
     if (woken == 0 || now - woken > 2000000ull) {
