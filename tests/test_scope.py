@@ -18,6 +18,38 @@ def connect_undeclared(a, b):
     return a.attach_peer(la, ba, b.edge_block_ptr(bb)), b.attach_peer(lb, bb, a.edge_block_ptr(ba))
 
 
+@pytest.fixture
+def system_scope(monkeypatch):
+    """Edges of which nothing is said about where their far end lives."""
+    attach = _native.cuda().GpuReplica.attach_peer
+    monkeypatch.setattr(_native.cuda().GpuReplica, "attach_peer", lambda r, link, block, remote, same_gpu=False: attach(r, link, block, remote))
+    a, b = [_native.cuda().GpuReplica(0, 5000, _native.cuda().GpuConfig()) for _ in range(2)]
+    connect_local(a, b)
+    assert not a.one_gpu() and not b.one_gpu()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("bits,block", [(1, 256), (1, 4096), (2, 1024), (4, 32), (8, 32), (8, 4096)])
+@pytest.mark.parametrize("topology,members", [("mesh", 3), ("mesh", 8), ("star", 4)])
+def test_group_bit_exact_at_system_scope(system_scope, topology, members, bits, block):
+    """Members, an inner node and its leaves, in every format, as they are between processes and GPUs."""
+    kinds.test_round_bit_exact_in_a_group(topology, members, bits, block)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("topology,members", [("mesh", 2), ("mesh", 4), ("star", 4)])
+def test_many_tiles_per_group_at_system_scope(system_scope, topology, members):
+    """Half a bank of descriptors is published before the pass has ended."""
+    kinds.test_round_bit_exact_with_many_tiles_per_group(topology, members)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("bits,block", [(1, 1024), (8, 32), (8, 4096)])
+@pytest.mark.parametrize("topology,members", [("mesh", 2), ("mesh", 4), ("star", 4)])
+def test_a_wait_that_runs_out_at_system_scope(system_scope, topology, members, bits, block):
+    kinds.test_a_wait_that_runs_out_leaves_no_visit_half_done(topology, members, bits, block, 3)
+
+
 @pytest.mark.gpu
 @pytest.mark.parametrize("members", [2, 4])
 def test_round_bit_exact_at_system_scope(monkeypatch, members):
