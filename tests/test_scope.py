@@ -99,11 +99,17 @@ def test_whether_the_other_end_of_a_socket_is_in_this_process():
                 assert cu.unix_same_process(here.fileno()) and cu.unix_same_process(conn.fileno())
         child = mp.get_context("spawn").Process(target=_connect_and_wait, args=(name,))
         child.start()
-        conn, _ = server.accept()
-        with conn:
-            assert not cu.unix_same_process(conn.fileno())
-            conn.send(b"x")
-        child.join(60)
+        try:
+            server.settimeout(60)  # (a child that fails never comes)
+            conn, _ = server.accept()
+            with conn:
+                assert not cu.unix_same_process(conn.fileno())
+                conn.send(b"x")
+            child.join(60)
+            assert child.exitcode == 0
+        finally:
+            child.kill()  # (does nothing to one that has ended)
+            child.join()
     assert not cu.unix_same_process(-1)
 
 
