@@ -321,8 +321,8 @@ bool GpuReplica::one_gpu() const {
 }
 
 void GpuReplica::publish_pending() {
-  // Ring numbering is about to change.  Every round ends with its publish kernel, so once the
-  // stream has drained nothing refers to the old numbering any more.
+  // Ring numbering is about to change.  A launch publishes what it has handled before it ends, so once the stream has drained
+  // nothing refers to the old numbering any more.
   cudaStreamSynchronize(S(comm_));
 }
 
@@ -852,9 +852,9 @@ void GpuReplica::engine_loop() {
   ::prctl(PR_SET_TIMERSLACK, 1000UL, 0, 0, 0);  // 1 us instead of the default 50 us: the idle pauses start at 10 us
   const size_t depth = ev_round_.size();
   // A few pinned words per launch in flight: tiles handled, groups that left early, waits that ran out and frames found without
-  // an acknowledgement so far, read once that launch has finished.  The read runs on a stream of its own behind an event, so that the comm stream goes from one
-  // launch straight to the next; a later launch may already have added to the counts by then, which only moves work from
-  // one difference to the one before it.
+  // an acknowledgement so far, read once that launch has finished.  The read runs on a stream of its own behind an event, so
+  // that the comm stream goes from one launch straight to the next.  Later launches, depth - 1 of them at most, may already have
+  // added to the counts by then: what they found is then told with an earlier launch (see QuietWatch::settled).
   uint64_t* work_host = status_host_ + kDsTotalWords;  // behind the part status() uses
   uint64_t work_seen = 0, cut_seen = 0, open_seen = 0;
   uint64_t r = 0;

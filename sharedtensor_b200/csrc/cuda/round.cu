@@ -501,9 +501,12 @@ constexpr int kFrameRoom = Q * 512 + 128;
 template <int kKind>
 constexpr int kStaged = kKind == kMember ? 8 : 0;
 // Who asks the L2 for the lines of the next tile: the service warp, a lane per array, or a compute warp, whose own part of the
-// tile in hand waits meanwhile.  With the service warp three rounds of 100 M elements on one link take 1144 us instead of 1159, a
-// hub and two leaves over 30 M 632 instead of 644 (the pass of a hub with three links over 32 Mi alone 248 instead of 305).  A mesh member's service warp has copies to see to (mesh of eight: 603
-// instead of 601), and in the shorter visits of sign frames it comes late (3.3 M elements: 50.9 instead of 49.9).
+// tile in hand waits meanwhile.  With the service warp three rounds of 100 M elements on one link take 1144 us instead of 1159,
+// a hub and two leaves over 30 M 632 instead of 644 (the pass of a hub with three links over 32 Mi alone 248 instead of 305).
+// For a mesh member, whose service warp has copies to see to, it makes no difference (mesh of eight: 603 and 601).  In a leaf's
+// short visits of sign frames the service warp comes late (3.3 M elements: 50.9 instead of 49.9).  That is no reason for an
+// inner node with sign frames, which the rule takes along: with the service warp a hub and three leaves over 16 M elements
+// would take 524 us instead of 531, a hub and two over 30 M 658 instead of 668 (3.3 M: 107 and 107).
 template <int Q, int kKind>
 constexpr bool kServiceAhead = kKind != kMember && Q > 1;
 
@@ -639,11 +642,12 @@ __device__ __forceinline__ void compute_warp(const RoundParams& p, GroupShared& 
       d = sh.desc[entry];
       c++;
     }
-    // Where the service warp does not do it: the next tile on its way into the L2, once this one's loads are under way (ahead of
-    // them, a mesh of eight takes 643 us instead of 620, three sign rounds of 3.3 M elements 51 instead of 49), but ahead of them
-    // in a visit that only sends and has little else to wait for.  One tile ahead is best: a window of 25 M elements that receives
-    // and sends takes 92 us so, 115 us with two tiles ahead and 153 us with four; without, three rounds of 100 M elements on one
-    // link take 1278 us instead of 1157.
+    // Where the service warp does not do it: the next tile on its way into the L2.  A leaf and a mesh member ask once this
+    // tile's loads are under way (ahead of them, a mesh of eight takes 643 us instead of 620, three sign rounds of 3.3 M elements
+    // on one link 51 instead of 49), but ahead of them in a visit that only sends and has little else to wait for; an inner node
+    // with sign frames, whose loads are spread over its visit, asks at the start.  One tile ahead is best: a window of 25 M
+    // elements that receives and sends takes 92 us so, 115 us with two tiles ahead and 153 us with four; without, three rounds of
+    // 100 M elements on one link take 1278 us instead of 1157.
     auto prefetch_next = [&]() {
       const uint32_t ahead = c;  // (c is the next tile's number by now)
       if (kServiceAhead<Q, kKind> || !live || warp != 0 || lane != 0 || int32_t(ld_shared_acquire(&sh.armed) - ahead) <= 0) return;
@@ -664,9 +668,9 @@ __device__ __forceinline__ void compute_warp(const RoundParams& p, GroupShared& 
     if (!kOneLink) {
       // What arrived, then the values into it.  Nothing is held in registers beyond that and the mirror of the link in hand, and
       // the values' maxima are taken once for all links: the kernel spills nothing, and a hub with two leaves takes 638 us for
-      // its rounds over 30 M elements instead of 657.  (More would not help: with 72 registers and three groups the warps
-      // wait for memory longer instead, 524 us against 511 for a hub and three leaves over 16 M, and the next link's mirror loaded
-      // ahead into registers gives 505 against 502.  The L2 serves some 10 TB/s at that point.)
+      // its rounds over 30 M elements instead of 657.  (While a compute warp asked for the next tile's lines, and held up the
+      // group with it, more did not help: 72 registers and three groups gave 524 us against 511 for a hub and three leaves over
+      // 16 M, the next link's mirror loaded ahead into registers 505 against 502.  Neither has been measured since.)
       prefetch_next();
       decode_frames<Q, true, 0>(frames, nullptr, false, d.n_frames, live, nullptr, lb, warp, lane, left, stash, v);
 #pragma unroll
@@ -1038,7 +1042,7 @@ __device__ __forceinline__ void service_warp(const RoundParams& p, GroupShared& 
         handed = stalled ? armed + __popc(work_tiles & ((1u << (__ffs(stalled) - 1)) - 1u)) : armed + __popc(work_tiles);
         __syncwarp();
         if (lane == 0) st_shared_release(&sh.armed, handed);
-        // The lines of a tile that is begun at once (the compute warps see to the later ones): all of them, while the warps are on
+        // The lines of a tile that is begun at once (for the later ones see kServiceAhead): all of them, while the warps are on
         // their way to asking for the first.  A hub and its leaves over 16 M elements take 517 us so, 522 without; a mesh of
         // eight, whose members begin with bulk copies of their frames, 603 without and 617 so.
         if (kKind != kMember && work && pos == finished) {
