@@ -598,7 +598,7 @@ void GpuReplica::launch(bool do_rx, bool do_tx, int sweeps) {
   params_.tile_count = (w == nw - 1) ? n_tiles_ - w * wt : wt;
   params_.round = round_no_++;
   params_.parity = cycle_no_ & 1;
-  params_.zero_other = w == 0 ? 1 : 0;
+  params_.zero_other = w == nw - 1 ? 1 : 0;  // (until then status() reads it)
   params_.follows_window = w != 0 ? 1 : 0;
   params_.do_rx = do_rx ? 1 : 0;
   params_.do_tx = do_tx ? 1 : 0;

@@ -1318,7 +1318,8 @@ static int launch_round_l(const RoundParams& p, int ctas, cudaStream_t stream) {
   cfg.stream = stream;
   // The launch may move in while the kernel before it in the stream is running out (and is cheaper to issue so: 2.4 instead
   // of 2.9 us).  A window that follows another of its cycle starts at once: the two have no tile in common.  Any other launch
-  // waits for the stream first.  (A cycle's first window clears counters that the launch before it may still add to.)
+  // waits for the stream first.  (A cycle's last window clears the counters of the cycle before, which was
+  // complete when this cycle's first window began.)
   cudaLaunchAttribute early{};
   early.id = cudaLaunchAttributeProgrammaticStreamSerialization;
   early.val.programmaticStreamSerializationAllowed = 1;

@@ -73,7 +73,7 @@ struct RoundParams {
   int32_t round;                 // number of this launch's first sweep (bookkeeping only)
   int32_t tile_begin, tile_count; // the window of the tensor this launch covers
   int32_t parity;                // which half of the per-cycle counters this launch uses (a cycle = one pass over all windows)
-  int32_t zero_other;            // first launch of a cycle: clear the other half for the cycle after this one
+  int32_t zero_other;            // last launch of a cycle: clear the other half for the cycle after this one
   int32_t follows_window;        // the launch before this one in the stream is the window before this one, of the same cycle
   int32_t do_rx, do_tx;          // receiver-only / sender-only launches
   int32_t one_gpu;               // every ring's far end is memory of this GPU, of a replica in this process

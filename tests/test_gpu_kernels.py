@@ -435,6 +435,25 @@ def test_updates_commute_with_rounds(cu):
     assert A.check_guards() == 0 and B.check_guards() == 0
 
 
+def test_status_in_the_middle_of_a_pass_tells_of_the_pass_before(cu):
+    """Three windows and a neighbour that takes nothing in: once its rings are full (two frames do not say everything), every
+    pass finds all tiles and leaves them."""
+    n = 40 * 4096 + 11
+    A, B = _replica(cu, n, window=16, slots=2), _replica(cu, n, window=16, slots=2)
+    connect_local(A, B)
+    values = torch.randn(n, device="cuda")
+    A.load_values(values.data_ptr(), _stream())
+    for _ in range(10):
+        A.round()
+    work, pending = [cu.status_names().index(k) for k in ("last_work_count", "pending_tiles")]
+    A.start_engine()
+    try:
+        told = [A.status() for _ in range(300)]
+    finally:
+        A.stop_engine()
+    assert {s[work] for s in told} == {A.tiles()} and {s[pending] for s in told} == {A.tiles()}
+
+
 def test_windowed_launches_cover_the_tensor(cu):
     """A tensor that is covered in several launches per pass (windows of 16 tiles here): manual rounds make whole
     passes, the engine thread goes from window to window, and both see every tile."""
